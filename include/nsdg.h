@@ -429,6 +429,12 @@ int nsdg_kernel_warm_stats(nsdg_kernel* k, nsdg_warm_stats* out);
  * Mixed-precision handles use the parallelogram stress kernel when it is at
  * most 1e-9. */
 int nsdg_mesh_parallelogram_mismatch(size_t nx, size_t ny, const double* coords, int dg_comp, double* mismatch);
+/* Host only (no GPU): the largest relative FP64 difference between the exact
+ * mEVP stress operators of a mesh (coords as for nsdg_kernel_initialise,
+ * lon/lat radians when is_spherical) and those rebuilt from the element map's
+ * derivatives at the Gauss points, as the sum-factorised stress kernels take
+ * them. */
+int nsdg_mesh_metric_mismatch(size_t nx, size_t ny, const double* coords, int is_spherical, double* mismatch);
 /* Host only (no GPU): every check that admits the parallelogram kernels, as
  * out[4]: 0 the mEVP stress operators' mismatch (as above), 1 the transport
  * cell operators rebuilt from the coefficients, 2 the largest off-diagonal of

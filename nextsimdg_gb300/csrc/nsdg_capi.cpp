@@ -109,6 +109,8 @@ struct nsdg_kernel {
     double *u0 = nullptr, *v0 = nullptr, *cgH = nullptr, *cgA = nullptr, *uGrad = nullptr, *vGrad = nullptr;
     double *c1 = nullptr, *c1b = nullptr, *fau = nullptr, *fav = nullptr, *rhfc = nullptr, *gu = nullptr, *gv = nullptr;
     double *Pg = nullptr, *contrib = nullptr;
+    StressGeometry geo {};   // the element maps of the sum-factorised stress kernels
+    double* Pw = nullptr;    // their weighted pressure
     double *velx = nullptr, *vely = nullptr, *nvX = nullptr, *nvY = nullptr;
     double *phiA = nullptr, *k1 = nullptr; // 3 fields x dg x N
     double *velx8 = nullptr, *vely8 = nullptr, *nvX8 = nullptr, *nvY8 = nullptr;
@@ -387,6 +389,8 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     bucketComps.clear();
     stepNumber = 0;
     readCache = 0;
+    geo = StressGeometry {};
+    Pw = nullptr;
 
     // --- host mesh (DynamicsKernel.hpp:44-75) ---
     mesh = HostMesh();
@@ -462,6 +466,12 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         add(8 * N); add(8 * N); add(3 * nXe); add(3 * nYe); add(24 * N); add(24 * N);
     }
     add(3 * Ncg1); add(8 * N); add(8 * N); add(8 * N); add(Ncg);
+    StressMetric metric;
+    if (P.precision == NSDG_PRECISION_FP64 && !bbm) {
+        buildStressMetric(mesh, metric);
+        add(metric.k.size()); add(metric.n.size()); add(metric.m.size()); add(metric.w.size());
+        add(9 * N);
+    }
     if (P.precision == NSDG_PRECISION_FP64 && !bbm && !mesh.spherical)
         add(324 * pairsLd(N), 8);                 // float-pair stress operators
     if (P.precision == NSDG_PRECISION_MIXED && !bbm) {
@@ -570,6 +580,13 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         dops.wdam = upd(ops.wdam);
         dops.hsize = upd(ops.hsize);
     }
+    if (!metric.k.empty()) {
+        geo.rect = metric.rect;
+        geo.k = upd(metric.k);
+        geo.n = metric.n.empty() ? nullptr : upd(metric.n);
+        geo.m = metric.m.empty() ? nullptr : upd(metric.m);
+        geo.w = upd(metric.w);
+    }
     if (e != cudaSuccess)
         return fail(NSDG_ERR_CUDA, std::string("initialise: upload failed: ") + cudaGetErrorString(e));
     auto z = [&](size_t n) {
@@ -593,6 +610,8 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     rhfc = z(Ncg); gu = z(Ncg); gv = z(Ncg);
     Pg = z(9 * N);
     contrib = z(18 * N);
+    if (geo.k)
+        Pw = z(9 * N);
     velx = z(size_t(dg) * N);
     vely = z(size_t(dg) * N);
     nvX = z(ED * nXe);
@@ -963,16 +982,18 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
         const MevpParams mp = mevpParams(dt);
         MevpNodeState st { u, v, u0, v0, cgH, cgA, uo, vo, ua, va, uGrad, vGrad, c1, c1b, fau, fav, rhfc, gu, gv };
         if (prep) {
-            // the mixed path forms its FP32 node constants in one kernel
-            if (!mixed())
-                LCH(launchMevpPrepNodes(s, dm, st, mp));
             // a full mixed-precision update also records the sub-cycle's
             // start (the warm-start features of the next update) inside
             // the two preparation kernels
             const bool save = loop && mixed();
-            LCH(launchMevpPrepElements(s, dm, dg, hice, cice, Pg, mp, mixed() ? hP32 : nullptr,
-                save ? tdiv32 : nullptr, save ? tdivLast : nullptr));
-            if (mixed())
+            const bool weighted = !mixed() && fp64Stress == 0;
+            LCH(launchMevpPrepElements(s, dm, dg, hice, cice, weighted ? Pw : Pg, mp, mixed() ? hP32 : nullptr,
+                save ? tdiv32 : nullptr, save ? tdivLast : nullptr, weighted ? geo.w : nullptr));
+            // after the elements' preparation: the first stress kernel reads
+            // its pressure before it waits for the launch just before it
+            if (!mixed())
+                LCH(launchMevpPrepNodes(s, dm, st, mp));
+            else
                 LCH(launchMevpPrepNodes32(s, dm, st, st32, dops.invm2, mp, save ? uLast : nullptr,
                     save ? vLast : nullptr));
         }
@@ -990,7 +1011,7 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
                     else if (opsPairs && fp64Stress == 1)
                         LCH(launchMevpStressPairs(s, dm, opsPairs, pairsLdN, u, v, Pg, contrib, mp));
                     else
-                        LCH(launchMevpStress(s, dm, dops, u, v, Pg, contrib, mp));
+                        LCH(launchMevpStress(s, dm, geo, u, v, Pw, contrib, mp));
                     LCH(launchMevpMomentum(s, dm, dops, st, contrib, mp, derr));
                 } else {
                     LCH(launchStress32(s, mp, derr));
@@ -2106,9 +2127,9 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
             if (k->opsPairs && k->fp64Stress == 1)
                 return launchMevpStressPairs(k->stream, k->dm, k->opsPairs, k->pairsLdN, k->u, k->v, k->Pg,
                     k->contrib, mp);
-            return launchMevpStress(k->stream, k->dm, k->dops, k->u, k->v, k->Pg, k->contrib, mp);
+            return launchMevpStress(k->stream, k->dm, k->geo, k->u, k->v, k->Pw, k->contrib, mp);
         case 9:
-            return launchMevpStress(k->stream, k->dm, k->dops, k->u, k->v, k->Pg, k->contrib, mp);
+            return launchMevpStress(k->stream, k->dm, k->geo, k->u, k->v, k->Pw, k->contrib, mp);
         case 10:
             return launchMevpStressPairs(k->stream, k->dm, k->opsPairs, k->pairsLdN, k->u, k->v, k->Pg, k->contrib,
                 mp);
@@ -2950,6 +2971,34 @@ int nsdg_mesh_parallelogram_mismatch(size_t nx, size_t ny, const double* coords,
     AffineStressOps aff;
     buildAffineStressOps(m, ops, m.nelements(), 0.0, aff);
     *mismatch = aff.worst;
+    return NSDG_OK;
+}
+
+int nsdg_mesh_metric_mismatch(size_t nx, size_t ny, const double* coords, int is_spherical, double* mismatch)
+{
+    if (!coords || !mismatch || nx < 1 || ny < 1)
+        return NSDG_ERR_BAD_ARG;
+    HostMesh m;
+    m.spherical = is_spherical != 0;
+    m.nx = nx;
+    m.ny = ny;
+    const size_t nn = (nx + 1) * (ny + 1);
+    m.vx.resize(nn);
+    m.vy.resize(nn);
+    for (size_t i = 0; i < nn; ++i) {
+        m.vx[i] = coords[2 * i];
+        m.vy[i] = coords[2 * i + 1];
+        if (!std::isfinite(m.vx[i]) || !std::isfinite(m.vy[i]))
+            return NSDG_ERR_BAD_ARG;
+    }
+    if (m.spherical)
+        m.rotatePoleToGreenland();
+    m.ice.assign(nx * ny, 1);
+    ElementOps ops;
+    buildElementOps(m, 1, false, ops);
+    StressMetric metric;
+    buildStressMetric(m, metric);
+    *mismatch = stressMetricMismatch(m, ops, metric);
     return NSDG_OK;
 }
 

@@ -435,6 +435,112 @@ void transportOps(const HostMesh& m, int dg, ElementOps& ops, unsigned threads)
 
 } // namespace
 
+void buildStressMetric(const HostMesh& m, StressMetric& out, unsigned threads)
+{
+    const Basis& b = basis();
+    const size_t N = m.nelements(), nx = m.nx, ny = m.ny, sv = nx + 1;
+    out = StressMetric();
+    out.rect = !m.spherical;
+    for (size_t j = 0; j <= ny && out.rect; ++j)
+        for (size_t i = 0; i <= nx && out.rect; ++i)
+            out.rect = m.vx[j * sv + i] == m.vx[i] && m.vy[j * sv + i] == m.vy[j * sv];
+    out.k.assign((out.rect ? 2 : 36) * N, 0.0);
+    out.w.assign(9 * N, 0.0);
+    if (!out.rect)
+        out.n.assign(9 * N, 0.0);
+    if (m.spherical)
+        out.m.assign(9 * N, 0.0);
+    parallelFor(N, threads, [&](size_t lo, size_t hi) {
+        Geom g;
+        for (size_t e = lo; e < hi; ++e) {
+            geometry(m, e, 3, g);
+            double iw[9], sum = 0;
+            for (int q = 0; q < 9; ++q) {
+                const double w = b.weight(3, q);
+                const double nu = (q % 3 == 1 ? -2.0 : 1.0) * (q / 3 == 1 ? -2.0 : 1.0);
+                out.w[q * N + e] = 2.0 * (w * g.J[q]);
+                iw[q] = nu / (w * g.J[q] * (m.spherical ? g.cl[q] : 1.0));
+                sum += nu * iw[q];
+            }
+            if (out.rect) {
+                const double kx = 0.5 * g.deta[1][4] / g.J[4];
+                out.k[e] = g.dxi[0][4] / g.deta[1][4];
+                out.k[N + e] = 1.0 / (kx * kx);
+                for (int q = 0; q < 9; ++q)
+                    out.w[q * N + e] *= kx;
+                continue;
+            }
+            for (int q = 0; q < 9; ++q) {
+                const double hx = 0.5 / (g.J[q] * (m.spherical ? kEarthRadius * g.cl[q] : 1.0));
+                const double hy = 0.5 / (g.J[q] * (m.spherical ? kEarthRadius : 1.0));
+                out.k[q * N + e] = g.deta[1][q] * hx;
+                out.k[(9 + q) * N + e] = -g.dxi[1][q] * hx;
+                out.k[(18 + q) * N + e] = -g.deta[0][q] * hy;
+                out.k[(27 + q) * N + e] = g.dxi[0][q] * hy;
+                out.n[q * N + e] = iw[q] / sum;
+                if (m.spherical)
+                    out.m[q * N + e] = 0.5 * g.sl[q] / (g.cl[q] * kEarthRadius);
+            }
+        }
+    });
+}
+
+double stressMetricMismatch(const HostMesh& m, const ElementOps& ops, const StressMetric& s, unsigned threads)
+{
+    const Basis& b = basis();
+    const size_t N = m.nelements();
+    const bool sph = m.spherical;
+    double worst = 0;
+    std::mutex mu;
+    parallelFor(N, threads, [&](size_t lo, size_t hi) {
+        double mine = 0;
+        for (size_t e = lo; e < hi; ++e) {
+            // K_x, K_y and the metric term at the points [q][j], P [q][r]
+            double K[3][9][9], P[9][9];
+            for (int q = 0; q < 9; ++q) {
+                double k[4];
+                const double kx = s.rect ? 1.0 / std::sqrt(s.k[N + e]) : 1.0;
+                for (int c = 0; c < 4; ++c)
+                    k[c] = s.rect ? (c == 0 ? kx : c == 3 ? kx * s.k[e] : 0.0) : s.k[(9 * c + q) * N + e];
+                for (int j = 0; j < 9; ++j) {
+                    const double px = b.phix(2, j, 3, q), py = b.phiy(2, j, 3, q);
+                    K[0][q][j] = 2.0 * (k[0] * px + k[1] * py);
+                    K[1][q][j] = 2.0 * (k[2] * px + k[3] * py);
+                    K[2][q][j] = sph ? 2.0 * s.m[q * N + e] * b.phi(2, j, 3, q) : 0.0;
+                }
+                for (int r = 0; r < 9; ++r) {
+                    const double nu = (r % 3 == 1 ? -2.0 : 1.0) * (r / 3 == 1 ? -2.0 : 1.0);
+                    P[q][r] = (q == r ? 1.0 : 0.0) - (s.rect ? 0.0 : s.n[q * N + e] * nu);
+                }
+            }
+            const std::vector<double>* G[3] = { &ops.gx, &ops.gy, &ops.gm };
+            const std::vector<double>* A[3] = { &ops.a1, &ops.a2, &ops.a3 };
+            for (int c = 0; c < (sph ? 3 : 2); ++c) {
+                double gm = 0, gd = 0, am = 0, ad = 0;
+                for (int q = 0; q < 9; ++q)
+                    for (int j = 0; j < 9; ++j) {
+                        double g = 0; // (P K)[q][j]; the divergence K^T P^T w J is its transpose
+                        for (int r = 0; r < 9; ++r)
+                            g += P[q][r] * K[c][r][j];
+                        const double at = 0.5 * s.w[q * N + e] * g * (s.rect ? std::sqrt(s.k[N + e]) : 1.0);
+                        const double xg = (*G[c])[(q * 9 + j) * N + e], xa = (*A[c])[(j * 9 + q) * N + e];
+                        gm = std::max(gm, std::fabs(xg));
+                        gd = std::max(gd, std::fabs(xg - g));
+                        am = std::max(am, std::fabs(xa));
+                        ad = std::max(ad, std::fabs(xa - at));
+                    }
+                if (gm > 0)
+                    mine = std::max(mine, gd / gm);
+                if (am > 0)
+                    mine = std::max(mine, ad / am);
+            }
+        }
+        std::lock_guard<std::mutex> lk(mu);
+        worst = std::max(worst, mine);
+    });
+    return worst;
+}
+
 bool buildAffineStressOps(const HostMesh& m, const ElementOps& ops, size_t ld, double tol,
     AffineStressOps& out, unsigned threads)
 {

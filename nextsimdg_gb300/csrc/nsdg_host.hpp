@@ -118,6 +118,29 @@ struct ElementOps {
 void buildElementOps(const HostMesh& m, int dg, bool stressTransport, ElementOps& ops,
     unsigned threads = 0);
 
+// The element map at the 3 x 3 Gauss points, as the sum-factorised stress
+// kernels take it (nsdg_sumfact.cuh has the formulas): with (x_xi, y_xi,
+// x_eta, y_eta) the map's derivatives, J its determinant and, on a sphere,
+// the lon derivatives over R cos(lat) and the lat derivatives over R,
+//   k = (y_eta, -y_xi, -x_eta, x_xi) / (2 J)        (half strains)
+//   n = W^{-1} nu / (nu W^{-1} nu),  W = w J [cos lat],  nu = (1,-2,1) x (1,-2,1)
+//   m = tan(lat) / (2 R)                              (spherical meshes)
+//   w = 2 w_q J
+// A mesh whose vertices form a tensor grid (rect) has k_x = 1 / (2 dx) and
+// k_y = 1 / (2 dy) at every point and needs no n: it keeps k = (k_y / k_x,
+// 1 / k_x^2) per element, and w = 2 w_q J k_x.
+struct StressMetric {
+    bool rect = false;
+    std::vector<double> k; // [2][N] (rect) or [4][9][N]
+    std::vector<double> n; // [9][N], empty on rectangles
+    std::vector<double> m; // [9][N], spherical only
+    std::vector<double> w; // [9][N]
+};
+void buildStressMetric(const HostMesh& m, StressMetric& out, unsigned threads = 0);
+// The largest relative difference between an element's operators (gx, gy,
+// a1, a2 and on a sphere gm, a3 of `ops`) and those rebuilt from `s`.
+double stressMetricMismatch(const HostMesh& m, const ElementOps& ops, const StressMetric& s, unsigned threads = 0);
+
 // Parallelogram (affine) elements.  When every element is a parallelogram,
 // its Jacobian is constant and the mEVP stress operators are fixed linear
 // combinations of the unit-square ones: with (x_xi, y_xi, x_eta, y_eta) the

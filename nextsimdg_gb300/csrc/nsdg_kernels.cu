@@ -1403,7 +1403,7 @@ __global__ void __launch_bounds__(kBlock) kMevpPrepNodes(size_t n, MevpNodeState
 template <int DG>
 __global__ void __launch_bounds__(kBlock) kMevpPrepElements(size_t N, const double* __restrict__ h,
     const double* __restrict__ a, double* __restrict__ Pg, double Pstar, double invAlpha, float* __restrict__ hP32,
-    const float* __restrict__ tdiv32, float* __restrict__ tdivLast)
+    const float* __restrict__ tdiv32, float* __restrict__ tdivLast, const double* __restrict__ weight)
 {
     const size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
     if (e >= N)
@@ -1430,7 +1430,7 @@ __global__ void __launch_bounds__(kBlock) kMevpPrepElements(size_t N, const doub
             Pg[q * N + e] = 0.125 * pa;
             hP32[q * N + e] = static_cast<float>(0.5 * pa);
         } else {
-            Pg[q * N + e] = pa;
+            Pg[q * N + e] = weight ? 0.25 * pa * weight[q * N + e] : pa;
         }
     }
 }
@@ -1444,109 +1444,15 @@ __global__ void __launch_bounds__(kBlock) kMevpPrepElements(size_t N, const doub
 // is observed only through that divergence, and the update is linear in s:
 //   s' = (1 - 1/alpha) s + iMJwPSI f    =>   divS s' = (1 - 1/alpha) divS s + (divS iMJwPSI) f
 // so each element keeps its 18 divergence coefficients tdiv instead of the 24
-// stress coefficients and applies the 9 x 9 operators A = divS iMJwPSI,
-// precomputed in FP64 on the host.  This drops the separate projection and
-// divergence products (216 + 288 FMA) for 324 FMA on an FP64-issue-bound
-// kernel.  The strain at the Gauss points comes straight from the 9 velocity
-// nodes through G = psi^T iMgrad (9 x 9), so the strain coefficients are not
-// formed either.  Land cells keep tdiv = 0 (the reference's divergence skips
-// them).  Pg holds P/alpha at the 9 Gauss points.
-//
-// Thread layout: three threads per element (kStressParts), 64 elements per
-// block.  Phase 1: thread `part` computes the strain, Delta and the stress
-// increments at Gauss points 3*part .. 3*part+2 and leaves them in shared
-// memory.  Phase 2: the same thread updates the divergence coefficients of
-// nodes 3*part .. 3*part+2.  Same FP64 work as one thread per element, three
-// times the warps to hide the operator loads.
+// stress coefficients and applies A = divS iMJwPSI.  The FP64 element kernel
+// is in nsdg_stress_sumfact.cu; the operator kernels below split an element
+// over three threads (kStressParts), 64 elements per block: in phase 1 thread
+// `part` computes the strain, Delta and the stress increments at Gauss points
+// 3*part .. 3*part+2 and leaves them in shared memory, in phase 2 it updates
+// the divergence coefficients of nodes 3*part .. 3*part+2.  Land cells keep
+// tdiv = 0 (the reference's divergence skips them).
 constexpr int kStressElems = 64;
 constexpr int kStressParts = 3;
-
-// SPH: spherical metric terms (CGDynamicsKernel.cpp:331-334, 348-351): the
-// strain gains e11 -= iMM v, e12 += iMM u / 2 (through the composite G_m),
-// the divergence gains +divM s12 (x) and -divM s11 (y) (through A_3).
-template <bool SPH>
-__global__ void __launch_bounds__(kStressElems * kStressParts) kMevpStress(DevMesh m, DevOps o,
-    const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ Pg,
-    double* __restrict__ tdiv, MevpParams p)
-{
-    __shared__ double fs[3][9][kStressElems];
-    const int le = threadIdx.x % kStressElems;
-    const int part = threadIdx.x / kStressElems; // warp-uniform
-    const size_t N = m.N;
-    const size_t e = blockIdx.x * size_t(kStressElems) + le;
-    const bool active = e < N && m.ice[e];
-    if (active) {
-        const size_t s2 = 2 * size_t(m.nx) + 1;
-        const size_t ix = static_cast<unsigned>(e) % static_cast<unsigned>(m.nx), iy = static_cast<unsigned>(e) / static_cast<unsigned>(m.nx);
-        const size_t base = 2 * s2 * iy + 2 * ix;
-        double ul[9], vl[9];
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-            const size_t nd = base + (j % 3) + (j / 3) * s2;
-            ul[j] = u[nd];
-            vl[j] = v[nd];
-        }
-        const double dmin2 = p.DeltaMin * p.DeltaMin;
-#pragma unroll
-        for (int qq = 0; qq < 3; ++qq) {
-            const int q = 3 * part + qq;
-            double ex = 0.0, ey = 0.0, exv = 0.0, eyu = 0.0;
-#pragma unroll
-            for (int j = 0; j < 9; ++j) {
-                const double gxq = o.gx[(q * 9 + j) * N + e];
-                const double gyq = o.gy[(q * 9 + j) * N + e];
-                ex = fma(gxq, ul[j], ex);
-                ey = fma(gyq, vl[j], ey);
-                exv = fma(gxq, vl[j], exv);
-                eyu = fma(gyq, ul[j], eyu);
-            }
-            if constexpr (SPH) {
-                double mu = 0.0, mv = 0.0;
-#pragma unroll
-                for (int j = 0; j < 9; ++j) {
-                    const double gmq = o.gm[(q * 9 + j) * N + e];
-                    mu = fma(gmq, ul[j], mu);
-                    mv = fma(gmq, vl[j], mv);
-                }
-                ex -= mv;
-                eyu += mu;
-            }
-            // e11 = ex, e22 = ey, e12 = (exv + eyu) / 2
-            const double sxy = exv + eyu;
-            const double d2 = dmin2 + 1.25 * (ex * ex + ey * ey) + 1.50 * ex * ey + 0.25 * sxy * sxy;
-            const double Pa = Pg[q * N + e];
-            const double z8 = 0.125 * Pa * rsqrt(d2); // P / (8 alpha Delta)
-            const double hP = 0.5 * Pa;
-            fs[0][q][le] = fma(z8, fma(5.0, ex, 3.0 * ey), -hP);
-            fs[1][q][le] = z8 * sxy; // P / (4 alpha Delta) e12
-            fs[2][q][le] = fma(z8, fma(5.0, ey, 3.0 * ex), -hP);
-        }
-    }
-    __syncthreads();
-    if (!active)
-        return;
-    const double keep = p.keepd;
-#pragma unroll
-    for (int jj = 0; jj < 3; ++jj) {
-        const int j = 3 * part + jj;
-        double ax = 0.0, ay = 0.0;
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const double a1 = o.a1[(j * 9 + q) * N + e];
-            const double a2 = o.a2[(j * 9 + q) * N + e];
-            const double f11 = fs[0][q][le], f12 = fs[1][q][le], f22 = fs[2][q][le];
-            ax = fma(a1, f11, fma(a2, f12, ax));
-            ay = fma(a1, f12, fma(a2, f22, ay));
-            if constexpr (SPH) {
-                const double a3 = o.a3[(j * 9 + q) * N + e];
-                ax = fma(a3, f12, ax);
-                ay = fma(-a3, f11, ay);
-            }
-        }
-        tdiv[j * N + e] = fma(tdiv[j * N + e], keep, ax);
-        tdiv[(9 + j) * N + e] = fma(tdiv[(9 + j) * N + e], keep, ay);
-    }
-}
 
 // Gathers the divergence contributions of the (up to four) ice cells around
 // a CG2 node in the reference's scatter order (even cell rows first, then
@@ -3117,27 +3023,17 @@ cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNode
 }
 
 cudaError_t launchMevpPrepElements(cudaStream_t s, const DevMesh& m, int dg, const double* h,
-    const double* a, double* Pg, const MevpParams& p, float* hP32, const float* tdiv32, float* tdivLast)
+    const double* a, double* Pg, const MevpParams& p, float* hP32, const float* tdiv32, float* tdivLast,
+    const double* weight)
 {
     const unsigned g = blocksFor(m.N);
     const double ia = 1.0 / p.alpha;
     switch (dg) {
-    case 1: kMevpPrepElements<1><<<g, kBlock, 0, s>>>(m.N, h, a, Pg, p.Pstar, ia, hP32, tdiv32, tdivLast); break;
-    case 3: kMevpPrepElements<3><<<g, kBlock, 0, s>>>(m.N, h, a, Pg, p.Pstar, ia, hP32, tdiv32, tdivLast); break;
-    case 6: kMevpPrepElements<6><<<g, kBlock, 0, s>>>(m.N, h, a, Pg, p.Pstar, ia, hP32, tdiv32, tdivLast); break;
+    case 1: kMevpPrepElements<1><<<g, kBlock, 0, s>>>(m.N, h, a, Pg, p.Pstar, ia, hP32, tdiv32, tdivLast, weight); break;
+    case 3: kMevpPrepElements<3><<<g, kBlock, 0, s>>>(m.N, h, a, Pg, p.Pstar, ia, hP32, tdiv32, tdivLast, weight); break;
+    case 6: kMevpPrepElements<6><<<g, kBlock, 0, s>>>(m.N, h, a, Pg, p.Pstar, ia, hP32, tdiv32, tdivLast, weight); break;
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
-}
-
-cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const DevOps& o, const double* u,
-    const double* v, const double* Pg, double* tdiv, const MevpParams& pIn)
-{
-    const MevpParams p = withDerived(pIn);
-    if (o.gm)
-        kMevpStress<true><<<blocksFor(m.N, kStressElems), kStressElems * kStressParts, 0, s>>>(m, o, u, v, Pg, tdiv, p);
-    else
-        kMevpStress<false><<<blocksFor(m.N, kStressElems), kStressElems * kStressParts, 0, s>>>(m, o, u, v, Pg, tdiv, p);
     return cudaGetLastError();
 }
 

@@ -181,20 +181,30 @@ inline MevpParams withDerived(MevpParams p)
 cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st,
     const MevpParams& p);
 // P at the 3x3 Gauss points from h and A (MEVPStressUpdateStep.hpp:54-57,75-77):
-// Pg = P/alpha, or, for the mixed-precision kernels (hP32 given),
+// Pg = P/alpha, or Pg = weight P/(4 alpha) with a weight per point ([9][N],
+// StressGeometry::w), or, for the mixed-precision kernels (hP32 given),
 // Pg = P/(8 alpha) (FP64, the viscosity numerator) and hP32 = P/(2 alpha).
 // tdivLast (mixed precision, optional): also copies tdiv32 there (the
 // sub-cycle's starting divergence, a warm-start feature).
 cudaError_t launchMevpPrepElements(cudaStream_t s, const DevMesh& m, int dg, const double* h,
     const double* a, double* Pg, const MevpParams& p, float* hP32 = nullptr, const float* tdiv32 = nullptr,
-    float* tdivLast = nullptr);
+    float* tdivLast = nullptr, const double* weight = nullptr);
 // One mEVP iteration, element part, carried in divergence space: the strain at
 // the Gauss points, Delta, and the relaxed update of the element's stress
 // divergence contributions tdiv[18][N] = (divS1 s11 + divS2 s12, divS1 s12 +
 // divS2 s22) at its 9 CG2 nodes (CGDynamicsKernel.cpp:300-398,
-// MEVPStressUpdateStep.hpp:30-118).  Pg holds P/alpha at the Gauss points.
-cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const DevOps& o, const double* u,
-    const double* v, const double* Pg, double* tdiv, const MevpParams& p);
+// MEVPStressUpdateStep.hpp:30-118), by sum factorisation (nsdg_sumfact.cuh).
+// Device copy of StressMetric (nsdg_host.hpp).
+struct StressGeometry {
+    const double* k = nullptr; // [2][N] on rectangles, else [4][9][N]
+    const double* n = nullptr; // [9][N] (null on rectangles)
+    const double* m = nullptr; // [9][N] (spherical meshes)
+    const double* w = nullptr; // [9][N]
+    bool rect = false;
+};
+// Pw holds w P/(4 alpha) at the Gauss points.
+cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const StressGeometry& geo, const double* u,
+    const double* v, const double* Pw, double* tdiv, const MevpParams& p);
 // The benchmark forcing on the cell centres (nsdg_forcing.cu):
 // BenchmarkAtmosphere.cpp:29-77 and BenchmarkOcean.cpp:15-39.
 struct BenchmarkWindArgs {

@@ -86,6 +86,21 @@ def parallelogram_checks(coords, nx: int, ny: int, dg_comp: int = 6) -> dict:
             "bbm": float(out[3])}
 
 
+def metric_mismatch(coords, nx: int, ny: int, is_spherical: bool = False) -> float:
+    """Host only: the largest relative FP64 difference between a mesh's exact
+    mEVP stress operators and those rebuilt from the element map's derivatives
+    at the Gauss points (nsdg_mesh_metric_mismatch)."""
+    lib = _lib.load()
+    c = _f64(coords)
+    if c.size != 2 * (nx + 1) * (ny + 1):
+        raise ValueError("coords must hold (nx+1)(ny+1) vertices x 2")
+    out = c_double()
+    st = lib.nsdg_mesh_metric_mismatch(nx, ny, _ptr(c), int(bool(is_spherical)), byref(out))
+    if st != _lib.NSDG_OK:
+        raise NsdgError(st, "metric_mismatch failed")
+    return out.value
+
+
 def mesh_dirichlet(mask, nx: int, ny: int) -> list:
     """Host only: the closed (Dirichlet) element sides a handle derives from
     its mask at initialise, as four ascending arrays of element ids (bottom,
