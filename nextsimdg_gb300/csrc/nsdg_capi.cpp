@@ -107,7 +107,7 @@ struct nsdg_kernel {
     double *avgU = nullptr, *avgV = nullptr;
     // per-step work
     double *u0 = nullptr, *v0 = nullptr, *cgH = nullptr, *cgA = nullptr, *uGrad = nullptr, *vGrad = nullptr;
-    double *c1 = nullptr, *c1b = nullptr, *fau = nullptr, *fav = nullptr, *rhfc = nullptr, *gu = nullptr, *gv = nullptr;
+    double *nodeA = nullptr, *nodeKu = nullptr, *nodeKv = nullptr, *nodeIm = nullptr; // FP64 mEVP node constants
     double *Pg = nullptr, *contrib = nullptr;
     StressGeometry geo {};   // the element maps of the sum-factorised stress kernels
     double* Pw = nullptr;    // their weighted pressure
@@ -458,7 +458,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     // state and work
     add(size_t(dg) * N); add(size_t(dg) * N); add(N); add(size_t(dg) * N);
     add(8 * N); add(8 * N); add(8 * N);
-    for (int i = 0; i < 25; ++i) add(Ncg);
+    for (int i = 0; i < 22; ++i) add(Ncg);
     add(9 * N); add(18 * N);
     add(size_t(dg) * N); add(size_t(dg) * N); add(ED * nXe); add(ED * nYe);
     add(3 * size_t(dg) * N); add(3 * size_t(dg) * N);
@@ -606,8 +606,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     s22 = z(8 * N);
     u = z(Ncg); v = z(Ncg); uo = z(Ncg); vo = z(Ncg); ua = z(Ncg); va = z(Ncg);
     avgU = z(Ncg); avgV = z(Ncg); u0 = z(Ncg); v0 = z(Ncg); cgH = z(Ncg); cgA = z(Ncg);
-    uGrad = z(Ncg); vGrad = z(Ncg); c1 = z(Ncg); c1b = z(Ncg); fau = z(Ncg); fav = z(Ncg);
-    rhfc = z(Ncg); gu = z(Ncg); gv = z(Ncg);
+    uGrad = z(Ncg); vGrad = z(Ncg); nodeA = z(Ncg); nodeKu = z(Ncg); nodeKv = z(Ncg); nodeIm = z(Ncg);
     Pg = z(9 * N);
     contrib = z(18 * N);
     if (geo.k)
@@ -980,7 +979,8 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
     const int nS = P.n_steps;
     if (!bbm) {
         const MevpParams mp = mevpParams(dt);
-        MevpNodeState st { u, v, u0, v0, cgH, cgA, uo, vo, ua, va, uGrad, vGrad, c1, c1b, fau, fav, rhfc, gu, gv };
+        MevpNodeState st { u, v, u0, v0, cgH, cgA, uo, vo, ua, va, uGrad, vGrad, nodeA, nodeKu, nodeKv,
+            nodeIm };
         if (prep) {
             // a full mixed-precision update also records the sub-cycle's
             // start (the warm-start features of the next update) inside
@@ -992,7 +992,7 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
             // after the elements' preparation: the first stress kernel reads
             // its pressure before it waits for the launch just before it
             if (!mixed())
-                LCH(launchMevpPrepNodes(s, dm, st, mp));
+                LCH(launchMevpPrepNodes(s, dm, st, dops.invm2, mp));
             else
                 LCH(launchMevpPrepNodes32(s, dm, st, st32, dops.invm2, mp, save ? uLast : nullptr,
                     save ? vLast : nullptr));
@@ -1012,7 +1012,7 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
                         LCH(launchMevpStressPairs(s, dm, opsPairs, pairsLdN, u, v, Pg, contrib, mp));
                     else
                         LCH(launchMevpStress(s, dm, geo, u, v, Pw, contrib, mp));
-                    LCH(launchMevpMomentum(s, dm, dops, st, contrib, mp, derr));
+                    LCH(launchMevpMomentum(s, dm, st, contrib, mp, derr));
                 } else {
                     LCH(launchStress32(s, mp, derr));
                     LCH(launchMevpMomentum32(s, dm, st32, tdiv32, mp, derr));
@@ -2094,7 +2094,7 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
     MevpParams mp { k->P.rho_ice, k->P.F_atm, k->P.F_ocean, k->P.fc, k->P.gravity, k->P.Pstar, k->P.DeltaMin,
         k->P.alpha, k->P.beta, dt };
     MevpNodeState st { k->u, k->v, k->u0, k->v0, k->cgH, k->cgA, k->uo, k->vo, k->ua, k->va, k->uGrad,
-        k->vGrad, k->c1, k->c1b, k->fau, k->fav, k->rhfc, k->gu, k->gv };
+        k->vGrad, k->nodeA, k->nodeKu, k->nodeKv, k->nodeIm };
     const double rad = 0x1.1df46a2529d39p-6;
     BbmParams bp { k->P.rho_ice, k->P.F_atm, k->P.F_ocean, k->P.fc, k->P.gravity, dt / k->P.n_steps,
         double(k->P.n_steps), std::cos(rad * k->P.ocean_turning_angle), std::sin(rad * k->P.ocean_turning_angle),
@@ -2141,7 +2141,7 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
                 return launchMevpMomentum32(k->stream, k->dm, k->st32, k->tdiv32, mp, k->derr);
             return bbm ? launchBbmMomentum(k->stream, k->dm, k->dops, bs, k->contrib, bp, k->derr,
                              k->mixed() ? k->invmHL : nullptr, (k->mixed() && k->bbmK0) ? &k->bbmConst : nullptr)
-                       : launchMevpMomentum(k->stream, k->dm, k->dops, st, k->contrib, mp, k->derr);
+                       : launchMevpMomentum(k->stream, k->dm, st, k->contrib, mp, k->derr);
         case 3:
         case 4:
             return k->launchStress32(k->stream, mp, k->derr, kernel_id == 4 ? 1 : 0);

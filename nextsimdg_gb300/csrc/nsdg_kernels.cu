@@ -18,6 +18,7 @@ __constant__ ConstTables32 cT32;
 #include "nsdg_kernels.hpp"
 #include "nsdg_visc_ff.hpp"
 #include "nsdg_tma.cuh"
+#include "nsdg_seed64.cuh"
 
 namespace nsdg {
 
@@ -1375,7 +1376,8 @@ __global__ void __launch_bounds__(kBlock) kSSHToCG2(DevMesh m, const double* __r
 // ===========================================================================
 // mEVP
 // ===========================================================================
-__global__ void __launch_bounds__(kBlock) kMevpPrepNodes(size_t n, MevpNodeState st, MevpParams p)
+__global__ void __launch_bounds__(kBlock) kMevpPrepNodes(size_t n, MevpNodeState st,
+    const double* __restrict__ invm2, MevpParams p)
 {
     const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
     if (i >= n)
@@ -1385,19 +1387,14 @@ __global__ void __launch_bounds__(kBlock) kMevpPrepNodes(size_t n, MevpNodeState
     const double H = fmax(st.cgH[i], 1.e-4);
     st.cgA[i] = A;
     st.cgH[i] = H;
-    st.u0[i] = st.u[i];
-    st.v0[i] = st.v[i];
     const double rhoH = p.rho_ice * H;
-    const double c1 = rhoH / p.dt;
-    st.c1[i] = c1;
-    st.c1b[i] = c1 * (1.0 + p.beta);
+    const double rc1 = p.dt / rhoH;
     const double ua = st.ua[i], va = st.va[i];
-    const double absatm = sqrt(ua * ua + va * va);
-    st.fau[i] = p.F_atm * absatm * ua;
-    st.fav[i] = p.F_atm * absatm * va;
-    st.rhfc[i] = rhoH * p.fc;
-    st.gu[i] = rhoH * p.gravity * st.uGrad[i];
-    st.gv[i] = rhoH * p.gravity * st.vGrad[i];
+    const double fatm = p.F_atm * sqrt(ua * ua + va * va);
+    st.a[i] = A * p.F_ocean * rc1;
+    st.ku[i] = st.u[i] + (A * (fatm * ua) - rhoH * p.gravity * st.uGrad[i]) * rc1;
+    st.kv[i] = st.v[i] + (A * (fatm * va) - rhoH * p.gravity * st.vGrad[i]) * rc1;
+    st.im[i] = invm2[i] * rc1;
 }
 
 template <int DG>
@@ -1490,7 +1487,14 @@ __device__ __forceinline__ void gatherDivergence(const DevMesh& m, int i2, int j
     dy = ay;
 }
 
-__global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, DevOps o, MevpNodeState st,
+// The FP64 node update, divided through by c1 = rho H / dt (kMevpPrepNodes):
+//   u_new = (beta u + ku + a |u_o - u| u_o - fc dt u + im dSx) / (1 + beta + a |u_o - u|)
+// and likewise v with + fc dt v (VPCGDynamicsKernel.hpp:132-172).  Bound by
+// FP64 issue: about 28 FP64 instructions per node, with the square root and
+// the reciprocal from FP32 seeds (CUDA's were more than half of the 60
+// before); 513 x 513 nodes 17.7 us instead of 26.8 us, 129 x 129
+// 2.9 us instead of 6.2 us (latency of the dependent chain).
+__global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, MevpNodeState st,
     const double* __restrict__ contrib, MevpParams p, int* __restrict__ err)
 {
     const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
@@ -1498,23 +1502,21 @@ __global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, DevOps o, Mev
         return;
     const int s2 = 2 * m.nx + 1;
     const int i2 = static_cast<int>(static_cast<unsigned>(i) % static_cast<unsigned>(s2)), j2 = static_cast<int>(static_cast<unsigned>(i) / static_cast<unsigned>(s2));
+    // before the wait for the stress kernel: what the step prepared, and the
+    // velocity, which the node kernel before that one wrote
     const bool dir = m.cg2Dir[i] != 0;
+    const double a = st.a[i], ku = st.ku[i], kv = st.kv[i], im = st.im[i];
+    const double u = st.u[i], v = st.v[i];
+    const double uo = st.uo[i], vo = st.vo[i];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     double dSx = 0.0, dSy = 0.0;
     if (!dir)
         gatherDivergence(m, i2, j2, contrib, dSx, dSy);
-    const double u = st.u[i], v = st.v[i];
-    const double uo = st.uo[i], vo = st.vo[i];
-    const double uOcnRel = uo - u, vOcnRel = v - vo;
-    const double absocn = sqrt(uOcnRel * uOcnRel + vOcnRel * vOcnRel);
-    const double A = st.cgA[i];
-    const double c1 = st.c1[i];
-    const double invm = o.invm2[i];
-    const double rden = 1.0 / (st.c1b[i] + A * p.F_ocean * absocn);
-    const double focn = p.F_ocean * absocn;
-    double un = rden * (c1 * (p.beta * u + st.u0[i]) + A * (st.fau[i] + focn * uo) - st.rhfc[i] * u
-        - st.gu[i] + dSx * invm);
-    double vn = rden * (c1 * (p.beta * v + st.v0[i]) + A * (st.fav[i] + focn * vo) + st.rhfc[i] * v
-        - st.gv[i] + dSy * invm);
+    const double ur = uo - u, vr = vo - v;
+    const double f = a * sf::sqrt64(fma(ur, ur, vr * vr));
+    const double rden = sf::recip64(p.onePlusBeta + f);
+    double un = rden * fma(p.betaMinus, u, fma(f, uo, fma(dSx, im, ku)));
+    double vn = rden * fma(p.betaPlus, v, fma(f, vo, fma(dSy, im, kv)));
     if (!isfinite(un) || !isfinite(vn))
         atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
     if (dir) {
@@ -3016,9 +3018,10 @@ cudaError_t launchSSHGradient(cudaStream_t s, const DevMesh& m, const DevOps& o,
     return cudaGetLastError();
 }
 
-cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const MevpParams& p)
+cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* invm2,
+    const MevpParams& p)
 {
-    kMevpPrepNodes<<<blocksFor(m.Ncg), kBlock, 0, s>>>(m.Ncg, st, p);
+    kMevpPrepNodes<<<blocksFor(m.Ncg), kBlock, 0, s>>>(m.Ncg, st, invm2, p);
     return cudaGetLastError();
 }
 
@@ -3037,11 +3040,20 @@ cudaError_t launchMevpPrepElements(cudaStream_t s, const DevMesh& m, int dg, con
     return cudaGetLastError();
 }
 
-cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const DevOps& o, const MevpNodeState& st,
-    const double* contrib, const MevpParams& p, int* err)
+cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* contrib,
+    const MevpParams& pIn, int* err)
 {
-    kMevpMomentum<<<blocksFor(m.Ncg), kBlock, 0, s>>>(m, o, st, contrib, p, err);
-    return cudaGetLastError();
+    const MevpParams p = withDerived(pIn);
+    cudaLaunchConfig_t cfg {};
+    cfg.gridDim = dim3(blocksFor(m.Ncg));
+    cfg.blockDim = dim3(kBlock);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kMevpMomentum, m, st, contrib, p, err);
 }
 
 cudaError_t launchMevpPrepNodes32(cudaStream_t s, const DevMesh& m, const MevpNodeState& st64,

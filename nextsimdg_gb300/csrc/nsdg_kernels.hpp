@@ -148,20 +148,19 @@ struct MevpNodeState {
     const double* va;
     const double* uGrad;
     const double* vGrad;
-    double* c1;      // rho H / dt
-    double* c1b;     // rho H / dt * (1 + beta)
-    double* fau;     // F_atm |wind| uwind
-    double* fav;
-    double* rhfc;    // rho H fc
-    double* gu;      // rho H g dxSSH
-    double* gv;
+    // the FP64 path's step constants, over c1 = rho H / dt:
+    double* a;  // A F_ocean / c1
+    double* ku; // u0 + (A F_atm |wind| uwind - rho H g dxSSH) / c1
+    double* kv;
+    double* im; // (1 / lumped mass) / c1
 };
 struct MevpParams {
     double rho_ice, F_atm, F_ocean, fc, gravity, Pstar, DeltaMin, alpha, beta, dt;
-    // derived on the host by withDerived() in every stress launcher, so that
+    // derived on the host by withDerived() in the stress and node launchers, so that
     // no thread spends FP64 instructions (about 1/60 of the FP32 rate on
     // GB300) on a division or a square of the parameters
     double keepd = 0;                          // 1 - 1/alpha
+    double onePlusBeta = 0, betaMinus = 0, betaPlus = 0; // 1 + beta, beta -+ fc dt
     float keep = 0, dmin2f = 0, F_oceanf = 0;  // FP32 copies (dmin2f: DeltaMin^2)
     float dmin2lo = 0;                         // DeltaMin^2 - dmin2f (its float-pair low part)
     float betaf = 0, onePlusBetaf = 0, fcdtf = 0; // beta, 1 + beta, fc dt
@@ -169,6 +168,9 @@ struct MevpParams {
 inline MevpParams withDerived(MevpParams p)
 {
     p.keepd = 1.0 - 1.0 / p.alpha;
+    p.onePlusBeta = 1.0 + p.beta;
+    p.betaMinus = p.beta - p.fc * p.dt;
+    p.betaPlus = p.beta + p.fc * p.dt;
     p.keep = static_cast<float>(p.keepd);
     p.dmin2f = static_cast<float>(p.DeltaMin * p.DeltaMin);
     p.dmin2lo = static_cast<float>(std::fma(p.DeltaMin, p.DeltaMin, -static_cast<double>(p.dmin2f)));
@@ -178,7 +180,7 @@ inline MevpParams withDerived(MevpParams p)
     p.fcdtf = static_cast<float>(p.fc * p.dt);
     return p;
 }
-cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st,
+cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* invm2,
     const MevpParams& p);
 // P at the 3x3 Gauss points from h and A (MEVPStressUpdateStep.hpp:54-57,75-77):
 // Pg = P/alpha, or Pg = weight P/(4 alpha) with a weight per point ([9][N],
@@ -239,8 +241,8 @@ cudaError_t launchMevpStressPairsTma(cudaStream_t s, const DevMesh& m, const Pai
 cudaError_t launchPairsSelfTest(cudaStream_t s, size_t n, const double* a, const double* x, double* out);
 // Node gather of the divergence, Dirichlet zero, implicit velocity update and
 // boundary zero (CGDynamicsKernel.cpp:365-444, VPCGDynamicsKernel.hpp:132-172).
-cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const DevOps& o,
-    const MevpNodeState& st, const double* contrib, const MevpParams& p, int* err);
+cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* contrib,
+    const MevpParams& p, int* err);
 
 // --- mEVP, mixed precision (NSDG_PRECISION_MIXED) ----------------------
 // FP32 operators, velocities, divergence coefficients and momentum

@@ -33,6 +33,7 @@
 #include <cstdint>
 
 #include "nsdg_kernels.hpp"
+#include "nsdg_seed64.cuh"
 
 namespace nsdg {
 namespace sf {
@@ -136,40 +137,6 @@ template <typename T> __device__ __forceinline__ void columnT(const T (&x)[3], c
     o[2] = p + q;
 }
 
-// 2 P / (8 alpha Delta) of the weighted pressure pq = w P / (4 alpha) and
-// t = Delta^2, in FP64 from the FP32 seed y0 = rsqrtf(t): with
-// e = 1 - t y0^2 (|e| <= 2^-20), 1/sqrt(t) = y0 (1 + e/2 + 3/8 e^2 + ...),
-// truncated below 2^-60.  Six FP64 instructions.  t outside the range that a
-// normal float seed covers takes CUDA's rsqrt.
-static __device__ __noinline__ double viscositySlow(double pq, double t) { return pq * rsqrt(t); }
-__device__ __forceinline__ double widenSeed(float f)
-{
-    return __longlong_as_double(
-        static_cast<long long>((static_cast<unsigned long long>(__float_as_uint(f)) << 29) + (896ull << 52)));
-}
-// the float nearest below t (truncated), for 2^-120 <= t <= 2^120
-__device__ __forceinline__ float narrowSeed(double t)
-{
-    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(t));
-    return __uint_as_float(static_cast<unsigned>((b - (896ull << 52)) >> 29));
-}
-// t in [2^-120, 2^120] (false for negative values and NaN)
-__device__ __forceinline__ bool seedRange(double t)
-{
-    const unsigned h = static_cast<unsigned>(__double2hiint(t));
-    return h - ((1023u - 120u) << 20) <= (240u << 20);
-}
-__device__ __forceinline__ double viscosity64(double pq, double t)
-{
-    if (!seedRange(t))
-        return viscositySlow(pq, t);
-    const double y = widenSeed(rsqrtf(narrowSeed(t)));
-    const double h = t * y;
-    const double e = fma(-h, y, 1.0);
-    const double c = e * fma(0.375, e, 0.5);
-    const double z = pq * y;
-    return fma(z, c, z);
-}
 // -x / 2 for x >= 0 (subnormal results flushed to zero), on the integer pipe
 __device__ __forceinline__ double minusHalf(double x)
 {
@@ -186,7 +153,7 @@ __device__ __forceinline__ void pointStress64(double a, double b, double s, doub
 {
     const double pl = a + b, mi = a - b;
     const double t = fma(4.0, fma(pl, pl, dminQ), fma(mi, mi, s * s));
-    const double z = viscosity64(pq, t);
+    const double z = timesRsqrt64(pq, t); // 2 P / (8 alpha Delta), weighted
     const double w = fma(z, pl, minusHalf(pq));
     const double d = z * mi;
     f12 = z * s;
