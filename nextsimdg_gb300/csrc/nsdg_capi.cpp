@@ -109,8 +109,16 @@ struct nsdg_kernel {
     double *u0 = nullptr, *v0 = nullptr, *cgH = nullptr, *cgA = nullptr, *uGrad = nullptr, *vGrad = nullptr;
     double *nodeA = nullptr, *nodeKu = nullptr, *nodeKv = nullptr, *nodeIm = nullptr; // FP64 mEVP node constants
     double *Pg = nullptr, *contrib = nullptr;
-    StressGeometry geo {};   // the element maps of the sum-factorised stress kernels
-    double* Pw = nullptr;    // their weighted pressure
+    // the element maps of the sum-factorised stress kernels, the weights and
+    // the weighted pressure (FP64, or pairs of floats on the mixed path)
+    StressGeometry<double> geo {};
+    StressGeometry<float> quad32 {}, aff32 {};
+    const double* metricW = nullptr;
+    double* Pw = nullptr;
+    float2* Pw32 = nullptr;
+    // which pressures the step prepares on the mixed path: the operator
+    // kernel's, the sum-factorised kernels' (an ensemble may run the other)
+    bool pressureOps = false, pressureSf = true;
     double *velx = nullptr, *vely = nullptr, *nvX = nullptr, *nvY = nullptr;
     double *phiA = nullptr, *k1 = nullptr; // 3 fields x dg x N
     double *velx8 = nullptr, *vely8 = nullptr, *nvX8 = nullptr, *nvY8 = nullptr;
@@ -129,11 +137,11 @@ struct nsdg_kernel {
     BbmNodeConst32 bbmConst { nullptr, nullptr };
     bool bbmK0 = false;
     float *cellX8_32 = nullptr, *cellY8_32 = nullptr; // FP32 DG8 stress-transport operators
-    // which FP32 stress kernel the updates use (chosen by timing at
-    // initialise): 0 operators by global loads, 1 operator tiles by TMA,
-    // 2 parallelogram coefficients (when the mesh allows it)
-    int stressKind = 1;
-    int viscMode = 2;                // FP64 viscosity form of the parallelogram kernel
+    // which FP32 stress kernel the updates use: 0 the element map's
+    // derivatives at the Gauss points from global memory, 1 operator tiles by
+    // TMA, 2 parallelogram coefficients (when the mesh allows it)
+    int stressKind = 0;
+    int viscMode = 3;                // viscosity form of the parallelogram kernel
     // FP64 path: the element stress kernel, 0 = FP64 FMA (kMevpStress, the
     // default), 1 = float-pair products (kMevpStressPairs), 2 = the same with
     // TMA-staged operators (kMevpStressPairsTma); Cartesian mEVP.  The
@@ -169,10 +177,9 @@ struct nsdg_kernel {
     {
         const int kind = variant < 0 ? stressKind : variant;
         if (kind == 2 && affCoef)
-            return launchMevpStress32Affine(s, dm, affCoef, affLd, st32.u, st32.v, Pg, tdiv32, mp,
-                vm < 0 ? viscMode : vm);
+            return launchMevpStress32Affine(s, dm, aff32, st32.u, st32.v, Pw32, tdiv32, mp, vm < 0 ? viscMode : vm);
         return kind == 1 ? launchMevpStress32Tma(s, dm, maps32, st32.u, st32.v, Pg, hP32, tdiv32, mp, errWord)
-                         : launchMevpStress32(s, dm, dops32, st32.u, st32.v, Pg, hP32, tdiv32, mp);
+                         : launchMevpStress32(s, dm, quad32, st32.u, st32.v, Pw32, tdiv32, mp);
     }
     int chooseStress32();
     float* tdiv32 = nullptr;
@@ -389,8 +396,12 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     bucketComps.clear();
     stepNumber = 0;
     readCache = 0;
-    geo = StressGeometry {};
+    geo = {};
+    quad32 = {};
+    aff32 = {};
     Pw = nullptr;
+    Pw32 = nullptr;
+    affCoef = nullptr;
 
     // --- host mesh (DynamicsKernel.hpp:44-75) ---
     mesh = HostMesh();
@@ -467,10 +478,12 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     }
     add(3 * Ncg1); add(8 * N); add(8 * N); add(8 * N); add(Ncg);
     StressMetric metric;
-    if (P.precision == NSDG_PRECISION_FP64 && !bbm) {
-        buildStressMetric(mesh, metric);
-        add(metric.k.size()); add(metric.n.size()); add(metric.m.size()); add(metric.w.size());
-        add(9 * N);
+    if (!bbm) {
+        buildStressMetric(mesh, P.precision == NSDG_PRECISION_FP64, metric);
+        const size_t sz = P.precision == NSDG_PRECISION_FP64 ? 8 : 4;
+        add(metric.k.size(), sz); add(metric.n.size(), sz); add(metric.m.size(), sz);
+        add(4 * N, 4);                            // the same on parallelograms
+        add(9 * N); add(9 * N);                   // weights, weighted pressure
     }
     if (P.precision == NSDG_PRECISION_FP64 && !bbm && !mesh.spherical)
         add(324 * pairsLd(N), 8);                 // float-pair stress operators
@@ -580,12 +593,14 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         dops.wdam = upd(ops.wdam);
         dops.hsize = upd(ops.hsize);
     }
-    if (!metric.k.empty()) {
-        geo.rect = metric.rect;
-        geo.k = upd(metric.k);
-        geo.n = metric.n.empty() ? nullptr : upd(metric.n);
-        geo.m = metric.m.empty() ? nullptr : upd(metric.m);
-        geo.w = upd(metric.w);
+    if (!bbm) {
+        metricW = upd(metric.w);
+        if (!mixed()) {
+            geo.rect = metric.rect;
+            geo.k = upd(metric.k);
+            geo.n = metric.n.empty() ? nullptr : upd(metric.n);
+            geo.m = metric.m.empty() ? nullptr : upd(metric.m);
+        }
     }
     if (e != cudaSuccess)
         return fail(NSDG_ERR_CUDA, std::string("initialise: upload failed: ") + cudaGetErrorString(e));
@@ -609,8 +624,10 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     uGrad = z(Ncg); vGrad = z(Ncg); nodeA = z(Ncg); nodeKu = z(Ncg); nodeKv = z(Ncg); nodeIm = z(Ncg);
     Pg = z(9 * N);
     contrib = z(18 * N);
-    if (geo.k)
+    if (!bbm) {
         Pw = z(9 * N);
+        Pw32 = reinterpret_cast<float2*>(Pw);
+    }
     velx = z(size_t(dg) * N);
     vely = z(size_t(dg) * N);
     nvX = z(ED * nXe);
@@ -747,6 +764,9 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
             if (e == cudaSuccess)
                 e = makeStressMaps(dops32, &maps32);
         }
+        quad32.k = upf(metric.k);
+        quad32.n = upf(metric.n);
+        quad32.m = mesh.spherical ? upf(metric.m) : nullptr;
         if (!mesh.spherical) {
             // parallelogram meshes: 5 coefficients per element replace the
             // operator block (the rebuilt operators must match the exact
@@ -759,9 +779,11 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
                     e = cudaErrorMemoryAllocation;
                 else if (e == cudaSuccess)
                     e = cudaMemcpy(affCoef, aff.coef.data(), aff.coef.size() * sizeof(float), cudaMemcpyHostToDevice);
-                if (e == cudaSuccess)
-                    e = uploadAffineReference(aff.ref);
                 affLd = ld;
+                std::vector<double> centre(4 * N); // the map is the same at every point
+                for (size_t c = 0; c < 4; ++c)
+                    std::copy_n(metric.k.begin() + (9 * c + 4) * N, N, centre.begin() + c * N);
+                aff32.k = upf(centre);
             }
             affWorst = aff.worst;
             // the transport on the same coefficients: the rebuilt cell
@@ -829,66 +851,33 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     return ok();
 }
 
-// Picks the FP32 stress kernel.  A parallelogram mesh takes the coefficient
-// kernel (5 coefficients instead of 324 operator entries per element; its
-// results differ from the others' by FP32 rounding only, and ensembles of
+// Picks the FP32 stress kernel: on a parallelogram mesh the coefficient kernel
+// (its results differ from the others' by FP32 rounding only, and ensembles of
 // such members take it too, so a member's single run and its ensemble run
-// agree bit for bit).  Otherwise the two operator kernels (tiles through TMA
-// into shared memory, or direct global loads), which compute identical
-// values, are timed on this mesh and the faster is kept: which wins depends
-// on the grid size and the number of resident blocks.
+// agree bit for bit), otherwise the kernel on the map's derivatives at the
+// Gauss points, which reads 430 bytes per element and iteration where the
+// operator kernel streams 1,580 (2,228 on a sphere).
 int nsdg_kernel::chooseStress32()
 {
-    // NSDG_STRESS_KERNEL=global|tma|affine fixes the choice (for profilers,
-    // whose serialised launches make the timing below meaningless)
-    // NSDG_VISC_FORM=0..4 fixes the FP64 viscosity form of the
-    // parallelogram kernel (0 rsqrt, 1 Newton, 2 Newton with integer
-    // conversions, 3 float pairs, 4 float pairs checked against form 2 with
-    // form 2 where the check fails: bitwise form 2)
+    // NSDG_STRESS_KERNEL=global|tma|affine fixes the choice
+    // NSDG_VISC_FORM=0..4 fixes the viscosity form of the parallelogram
+    // kernel (0 rsqrt, 1 Newton, 2 Newton with integer conversions, 3 float
+    // pairs, 4 float pairs checked against form 2 with form 2 where the check
+    // fails: bitwise form 2)
     if (const char* env = std::getenv("NSDG_VISC_FORM")) {
         const int f = std::atoi(env);
         if (f >= 0 && f <= 4)
             viscMode = f;
     }
+    stressKind = affCoef ? 2 : 0;
     if (const char* env = std::getenv("NSDG_STRESS_KERNEL")) {
         const char* names[3] = { "global", "tma", "affine" };
         for (int i = 0; i < 3; ++i)
-            if (std::strcmp(env, names[i]) == 0 && (i < 2 || affCoef)) {
+            if (std::strcmp(env, names[i]) == 0 && (i < 2 || affCoef))
                 stressKind = i;
-                return NSDG_OK;
-            }
     }
-    if (affCoef) {
-        stressKind = 2;
-        return NSDG_OK;
-    }
-    const MevpParams mp = mevpParams(120.0);
-    cudaEvent_t a, b;
-    if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess)
-        return fail(NSDG_ERR_CUDA, "initialise: event create failed");
-    float best[2] = { 0, 0 };
-    const int kinds = 2;
-    cudaError_t e = cudaSuccess;
-    for (int variant = 0; variant < kinds && e == cudaSuccess; ++variant) {
-        e = launchStress32(stream, mp, derr, variant);
-        if (e == cudaSuccess) e = cudaEventRecord(a, stream);
-        for (int r = 0; r < 10 && e == cudaSuccess; ++r)
-            e = launchStress32(stream, mp, derr, variant);
-        if (e == cudaSuccess) e = cudaEventRecord(b, stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(b);
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&best[variant], a, b);
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    // the timing launches updated the divergence of the (zero) initial state: reset it
-    if (e == cudaSuccess) e = cudaMemsetAsync(tdiv32, 0, 18 * N * sizeof(float), stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess)
-        return fail(NSDG_ERR_CUDA, std::string("initialise: stress kernel timing: ") + cudaGetErrorString(e));
-    stressKind = 0;
-    for (int variant = 1; variant < kinds; ++variant)
-        if (best[variant] <= best[stressKind])
-            stressKind = variant;
+    pressureOps = stressKind == 1;
+    pressureSf = !pressureOps;
     return NSDG_OK;
 }
 
@@ -986,9 +975,17 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
             // start (the warm-start features of the next update) inside
             // the two preparation kernels
             const bool save = loop && mixed();
-            const bool weighted = !mixed() && fp64Stress == 0;
-            LCH(launchMevpPrepElements(s, dm, dg, hice, cice, weighted ? Pw : Pg, mp, mixed() ? hP32 : nullptr,
-                save ? tdiv32 : nullptr, save ? tdivLast : nullptr, weighted ? geo.w : nullptr));
+            PressureOut po;
+            po.w = metricW;
+            if (!mixed())
+                (fp64Stress == 0 ? po.weighted : po.alpha) = fp64Stress == 0 ? Pw : Pg;
+            else {
+                po.weightedPair = pressureSf ? Pw32 : nullptr;
+                po.visc = pressureOps ? Pg : nullptr;
+                po.half = hP32;
+            }
+            LCH(launchMevpPrepElements(s, dm, dg, hice, cice, po, mp, save ? tdiv32 : nullptr,
+                save ? tdivLast : nullptr));
             // after the elements' preparation: the first stress kernel reads
             // its pressure before it waits for the launch just before it
             if (!mixed())
@@ -2437,10 +2434,10 @@ struct nsdg_ensemble {
     // the sub-cycle as one persistent cooperative launch (parallelogram
     // members only) instead of two launches per iteration
     bool persistent = false;
-    // element phase: 0 tiled global-load kernel, 1 TMA-staged, 2 parallelogram
-    // coefficients (every member a parallelogram mesh)
+    // element phase: 0 the map's derivatives at the Gauss points, 1 TMA-staged
+    // operators, 2 parallelogram coefficients (every member a parallelogram mesh)
     int elementKind = 0;
-    int viscMode = 2;
+    int viscMode = 3;
     cudaError_t launchElements(cudaStream_t s, const EnsembleMember* table, const MevpParams& mp)
     {
         if (elementKind == 2)
@@ -2448,7 +2445,6 @@ struct nsdg_ensemble {
         return elementKind == 1 ? launchMevpStress32TmaBatched(s, table, dTmaMap, tmaBlocks, mp, derr)
                                 : launchMevpStress32Batched(s, table, dStressMap, stressBlocks, mp);
     }
-    std::vector<int> tileW;
     cudaGraphExec_t graph = nullptr;
     double graphDt = -1.0;
     int launches = 0;
@@ -2472,7 +2468,7 @@ struct nsdg_ensemble {
         if (stream)
             cudaStreamDestroy(stream);
     }
-    EnsembleMember describe(nsdg_kernel* k, int tw) const
+    EnsembleMember describe(nsdg_kernel* k) const
     {
         EnsembleMember d {};
         d.nx = k->dm.nx;
@@ -2482,110 +2478,29 @@ struct nsdg_ensemble {
         d.ice = k->dm.ice;
         d.cg2Dir = k->dm.cg2Dir;
         d.invm2 = k->dops.invm2;
-        d.o = k->dops32;
         d.st = k->st32;
         d.Pg = k->Pg;
         d.hP = k->hP32;
+        d.Pw = k->Pw32;
         d.tdiv = k->tdiv32;
         d.maps = k->maps32;
-        d.affCoef = k->affCoef;
-        d.affLd = k->affLd;
-        d.tileW = tw;
-        d.tileH = stressElementsPerBlock() / tw;
-        d.tilesX = (d.nx + tw - 1) / tw;
+        d.quad = k->quad32;
+        d.aff = k->aff32;
         return d;
     }
-    static int stressBlocksOf(const EnsembleMember& d) { return d.tilesX * ((d.ny + d.tileH - 1) / d.tileH); }
+    static int stressBlocksOf(const EnsembleMember& d)
+    {
+        return static_cast<int>((d.N + kQuadElems - 1) / kQuadElems);
+    }
     static int nodeBlocksOf(const EnsembleMember& d)
     {
         return static_cast<int>((d.Ncg + nodesPerBlock() - 1) / nodesPerBlock());
     }
     static int tmaBlocksOf(const EnsembleMember& d) { return static_cast<int>((d.N + kTmaElems - 1) / kTmaElems); }
-    int chooseElementKernel();
-    int autotune();
+    void chooseElementKernel();
     int build();
     int ensureGraph(double dt);
 };
-
-// Project-written autotuner: for every grid size in the ensemble, times the
-// batched element kernel on that member alone for each tile shape
-// (tileW x tileH, tileW * tileH = elements per block) and keeps the fastest.
-// The divergence coefficients of the timing runs go to a scratch buffer, so
-// the members' state is not touched.
-int nsdg_ensemble::autotune()
-{
-    const int E = stressElementsPerBlock();
-    std::vector<int> candidates;
-    for (int w = E; w >= 8; w /= 2)
-        candidates.push_back(w);
-    size_t maxN = 0;
-    for (auto* k : members)
-        maxN = std::max(maxN, k->N);
-    void* scratch = nullptr;
-    EnsembleMember* dOne = nullptr;
-    uint16_t* dMap = nullptr;
-    size_t mapLen = 1;
-    for (auto* k : members)
-        for (int w : candidates)
-            mapLen = std::max(mapLen, static_cast<size_t>(stressBlocksOf(describe(k, w))));
-    if (cudaMalloc(&scratch, 18 * maxN * sizeof(float)) != cudaSuccess
-        || cudaMalloc(&dOne, sizeof(EnsembleMember)) != cudaSuccess
-        || cudaMalloc(&dMap, mapLen * sizeof(uint16_t)) != cudaSuccess) {
-        cudaFree(scratch);
-        cudaFree(dOne);
-        return fail(NSDG_ERR_CUDA, "ensemble autotune: allocation failed");
-    }
-    cudaMemsetAsync(dMap, 0, mapLen * sizeof(uint16_t), stream);
-    cudaMemsetAsync(scratch, 0, 18 * maxN * sizeof(float), stream);
-    std::map<std::pair<int, int>, int> best;
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    const nsdg_params& P = members[0]->P;
-    MevpParams mp { P.rho_ice, P.F_atm, P.F_ocean, P.fc, P.gravity, P.Pstar, P.DeltaMin, P.alpha, P.beta, 120.0 };
-    cudaError_t e = cudaSuccess;
-    for (size_t mi = 0; mi < members.size() && e == cudaSuccess; ++mi) {
-        nsdg_kernel* k = members[mi];
-        const auto key = std::make_pair(k->dm.nx, k->dm.ny);
-        if (best.count(key))
-            continue;
-        float bestMs = 1e30f;
-        int bestW = E;
-        for (int w : candidates) {
-            EnsembleMember d = describe(k, w);
-            d.tdiv = static_cast<float*>(scratch);
-            d.stressBlock0 = 0;
-            const int blocks = stressBlocksOf(d);
-            e = cudaMemcpyAsync(dOne, &d, sizeof(d), cudaMemcpyHostToDevice, stream);
-            for (int r = 0; r < 3 && e == cudaSuccess; ++r) // warm-up
-                e = launchMevpStress32Batched(stream, dOne, dMap, blocks, mp);
-            if (e == cudaSuccess) e = cudaEventRecord(a, stream);
-            for (int r = 0; r < 10 && e == cudaSuccess; ++r)
-                e = launchMevpStress32Batched(stream, dOne, dMap, blocks, mp);
-            if (e == cudaSuccess) e = cudaEventRecord(b, stream);
-            if (e == cudaSuccess) e = cudaEventSynchronize(b);
-            float ms = 0.f;
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, a, b);
-            if (e == cudaSuccess && ms < bestMs) {
-                bestMs = ms;
-                bestW = w;
-            }
-        }
-        best[key] = bestW;
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    cudaStreamSynchronize(stream);
-    cudaFree(scratch);
-    cudaFree(dOne);
-    cudaFree(dMap);
-    if (e != cudaSuccess)
-        return fail(NSDG_ERR_CUDA, std::string("ensemble autotune: ") + cudaGetErrorString(e));
-    tileW.clear();
-    for (auto* k : members)
-        tileW.push_back(best[std::make_pair(k->dm.nx, k->dm.ny)]);
-    return NSDG_OK;
-}
 
 int nsdg_ensemble::build()
 {
@@ -2593,7 +2508,7 @@ int nsdg_ensemble::build()
     std::vector<uint16_t> smap, nmap, tmap, pmap;
     const size_t perP = static_cast<size_t>(persistentNodesPerBlock());
     for (size_t mi = 0; mi < members.size(); ++mi) {
-        EnsembleMember d = describe(members[mi], tileW[mi]);
+        EnsembleMember d = describe(members[mi]);
         d.stressBlock0 = static_cast<int>(smap.size());
         d.nodeBlock0 = static_cast<int>(nmap.size());
         d.tmaBlock0 = static_cast<int>(tmap.size());
@@ -2635,78 +2550,33 @@ int nsdg_ensemble::build()
     if (e == cudaSuccess) e = cudaMemset(derr, 0, sizeof(int));
     if (e != cudaSuccess)
         return fail(NSDG_ERR_CUDA, std::string("ensemble: upload failed: ") + cudaGetErrorString(e));
-    return chooseElementKernel();
+    chooseElementKernel();
+    // the members' steps prepare the pressure this ensemble's kernel reads
+    for (auto* k : members) {
+        bool& need = elementKind == 1 ? k->pressureOps : k->pressureSf;
+        if (!need)
+            k->dropGraphs();
+        need = true;
+    }
+    return NSDG_OK;
 }
 
-// Times the element phase of the whole ensemble with the tiled global-load
-// kernel (autotuned tiles) and with the TMA-staged kernel, the divergence
-// redirected to scratch so that no member's state changes, and keeps the
-// faster.
-int nsdg_ensemble::chooseElementKernel()
+// Parallelogram members take the coefficient kernel (as their single runs do)
+// when every member has coefficients, otherwise all take the kernel on the
+// map's derivatives; NSDG_STRESS_KERNEL fixes the choice.
+void nsdg_ensemble::chooseElementKernel()
 {
-    size_t total = 0;
-    for (auto* k : members)
-        total += 18 * k->N;
-    std::vector<EnsembleMember> table;
-    void* scratch = nullptr;
-    EnsembleMember* dT = nullptr;
-    if (cudaMalloc(&scratch, total * sizeof(float)) != cudaSuccess
-        || cudaMalloc(&dT, members.size() * sizeof(EnsembleMember)) != cudaSuccess) {
-        cudaFree(scratch);
-        return fail(NSDG_ERR_CUDA, "ensemble: timing allocation failed");
-    }
-    std::vector<EnsembleMember> host(members.size());
-    cudaError_t e = cudaMemcpy(host.data(), dMembers, host.size() * sizeof(EnsembleMember), cudaMemcpyDeviceToHost);
-    size_t off = 0;
-    for (size_t mi = 0; mi < host.size(); ++mi) {
-        host[mi].tdiv = static_cast<float*>(scratch) + off;
-        off += 18 * members[mi]->N;
-    }
-    if (e == cudaSuccess) e = cudaMemcpy(dT, host.data(), host.size() * sizeof(EnsembleMember), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(scratch, 0, total * sizeof(float));
-    const nsdg_params& P = members[0]->P;
-    MevpParams mp { P.rho_ice, P.F_atm, P.F_ocean, P.fc, P.gravity, P.Pstar, P.DeltaMin, P.alpha, P.beta, 120.0 };
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    float ms[2] = { 0, 0 };
-    for (int variant = 0; variant < 2 && e == cudaSuccess; ++variant) {
-        auto launch = [&]() {
-            return variant == 0 ? launchMevpStress32Batched(stream, dT, dStressMap, stressBlocks, mp)
-                                : launchMevpStress32TmaBatched(stream, dT, dTmaMap, tmaBlocks, mp, derr);
-        };
-        for (int r = 0; r < 2 && e == cudaSuccess; ++r)
-            e = launch();
-        if (e == cudaSuccess) e = cudaEventRecord(a, stream);
-        for (int r = 0; r < 10 && e == cudaSuccess; ++r)
-            e = launch();
-        if (e == cudaSuccess) e = cudaEventRecord(b, stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(b);
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms[variant], a, b);
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    cudaStreamSynchronize(stream);
-    cudaFree(scratch);
-    cudaFree(dT);
-    if (e != cudaSuccess)
-        return fail(NSDG_ERR_CUDA, std::string("ensemble: element kernel timing: ") + cudaGetErrorString(e));
-    elementKind = ms[1] <= ms[0] ? 1 : 0;
-    // parallelogram members take the coefficient kernel (as their single
-    // runs do), when every member has coefficients
     bool allAffine = true;
     for (auto* k : members)
         allAffine = allAffine && k->affCoef != nullptr;
-    if (allAffine) {
-        elementKind = 2;
+    elementKind = allAffine ? 2 : 0;
+    if (allAffine)
         viscMode = members[0]->viscMode;
-    }
     if (const char* env = std::getenv("NSDG_STRESS_KERNEL")) {
         if (std::strcmp(env, "tma") == 0) elementKind = 1;
         if (std::strcmp(env, "global") == 0) elementKind = 0;
         if (std::strcmp(env, "affine") == 0 && allAffine) elementKind = 2;
     }
-    return NSDG_OK;
 }
 
 int nsdg_ensemble::ensureGraph(double dt)
@@ -2806,7 +2676,7 @@ int nsdg_ensemble_create(nsdg_kernel* const* members, int n_members, nsdg_ensemb
     }
     for (auto* k : ens->members)
         cudaStreamSynchronize(k->stream);
-    if (ens->autotune() != NSDG_OK || ens->build() != NSDG_OK) {
+    if (ens->build() != NSDG_OK) {
         delete ens;
         return NSDG_ERR_CUDA;
     }
@@ -2930,8 +2800,8 @@ int nsdg_ensemble_tile(nsdg_ensemble* ens, int member, int* tile_w, int* tile_h)
         *tile_w = kTmaElems; // consecutive elements (operators staged by TMA, or parallelogram coefficients)
         *tile_h = 1;
     } else {
-        *tile_w = ens->tileW[member];
-        *tile_h = stressElementsPerBlock() / ens->tileW[member];
+        *tile_w = kQuadElems; // consecutive elements
+        *tile_h = 1;
     }
     return NSDG_OK;
 }
@@ -2996,9 +2866,12 @@ int nsdg_mesh_metric_mismatch(size_t nx, size_t ny, const double* coords, int is
     m.ice.assign(nx * ny, 1);
     ElementOps ops;
     buildElementOps(m, 1, false, ops);
-    StressMetric metric;
-    buildStressMetric(m, metric);
-    *mismatch = stressMetricMismatch(m, ops, metric);
+    *mismatch = 0;
+    for (const bool rect : { true, false }) { // a tensor grid has both forms
+        StressMetric metric;
+        buildStressMetric(m, rect, metric);
+        *mismatch = std::max(*mismatch, stressMetricMismatch(m, ops, metric));
+    }
     return NSDG_OK;
 }
 

@@ -435,12 +435,12 @@ void transportOps(const HostMesh& m, int dg, ElementOps& ops, unsigned threads)
 
 } // namespace
 
-void buildStressMetric(const HostMesh& m, StressMetric& out, unsigned threads)
+void buildStressMetric(const HostMesh& m, bool allowRect, StressMetric& out, unsigned threads)
 {
     const Basis& b = basis();
     const size_t N = m.nelements(), nx = m.nx, ny = m.ny, sv = nx + 1;
     out = StressMetric();
-    out.rect = !m.spherical;
+    out.rect = allowRect && !m.spherical;
     for (size_t j = 0; j <= ny && out.rect; ++j)
         for (size_t i = 0; i <= nx && out.rect; ++i)
             out.rect = m.vx[j * sv + i] == m.vx[i] && m.vy[j * sv + i] == m.vy[j * sv];

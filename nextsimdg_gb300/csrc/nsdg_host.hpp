@@ -136,7 +136,8 @@ struct StressMetric {
     std::vector<double> m; // [9][N], spherical only
     std::vector<double> w; // [9][N]
 };
-void buildStressMetric(const HostMesh& m, StressMetric& out, unsigned threads = 0);
+// With allowRect false the general form is built on every mesh.
+void buildStressMetric(const HostMesh& m, bool allowRect, StressMetric& out, unsigned threads = 0);
 // The largest relative difference between an element's operators (gx, gy,
 // a1, a2 and on a sphere gm, a3 of `ops`) and those rebuilt from `s`.
 double stressMetricMismatch(const HostMesh& m, const ElementOps& ops, const StressMetric& s, unsigned threads = 0);

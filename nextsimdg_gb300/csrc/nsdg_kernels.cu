@@ -16,9 +16,8 @@ __constant__ ConstTables32 cT32;
 
 #include "nsdg_common.cuh"
 #include "nsdg_kernels.hpp"
-#include "nsdg_visc_ff.hpp"
 #include "nsdg_tma.cuh"
-#include "nsdg_seed64.cuh"
+#include "nsdg_sumfact.cuh"
 
 namespace nsdg {
 
@@ -1399,8 +1398,8 @@ __global__ void __launch_bounds__(kBlock) kMevpPrepNodes(size_t n, MevpNodeState
 
 template <int DG>
 __global__ void __launch_bounds__(kBlock) kMevpPrepElements(size_t N, const double* __restrict__ h,
-    const double* __restrict__ a, double* __restrict__ Pg, double Pstar, double invAlpha, float* __restrict__ hP32,
-    const float* __restrict__ tdiv32, float* __restrict__ tdivLast, const double* __restrict__ weight)
+    const double* __restrict__ a, PressureOut out, double Pstar, double invAlpha, const float* __restrict__ tdiv32,
+    float* __restrict__ tdivLast)
 {
     const size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
     if (e >= N)
@@ -1423,11 +1422,19 @@ __global__ void __launch_bounds__(kBlock) kMevpPrepElements(size_t N, const doub
         const double hq = fmax(hs, 0.0);
         const double aq = fmin(fmax(as, 0.0), 1.0);
         const double pa = Pstar * hq * exp(-20.0 * (1.0 - aq)) * invAlpha;
-        if (hP32) {
-            Pg[q * N + e] = 0.125 * pa;
-            hP32[q * N + e] = static_cast<float>(0.5 * pa);
-        } else {
-            Pg[q * N + e] = weight ? 0.25 * pa * weight[q * N + e] : pa;
+        const size_t at = q * N + e;
+        if (out.weighted)
+            out.weighted[at] = 0.25 * pa * out.w[at];
+        if (out.weightedPair) {
+            const double x = 0.25 * pa * out.w[at];
+            const float hi = static_cast<float>(x);
+            out.weightedPair[at] = make_float2(hi, static_cast<float>(x - static_cast<double>(hi)));
+        }
+        if (out.alpha)
+            out.alpha[at] = pa;
+        if (out.visc) {
+            out.visc[at] = 0.125 * pa;
+            out.half[at] = static_cast<float>(0.5 * pa);
         }
     }
 }
@@ -1441,14 +1448,13 @@ __global__ void __launch_bounds__(kBlock) kMevpPrepElements(size_t N, const doub
 // is observed only through that divergence, and the update is linear in s:
 //   s' = (1 - 1/alpha) s + iMJwPSI f    =>   divS s' = (1 - 1/alpha) divS s + (divS iMJwPSI) f
 // so each element keeps its 18 divergence coefficients tdiv instead of the 24
-// stress coefficients and applies A = divS iMJwPSI.  The FP64 element kernel
-// is in nsdg_stress_sumfact.cu; the operator kernels below split an element
-// over three threads (kStressParts), 64 elements per block: in phase 1 thread
-// `part` computes the strain, Delta and the stress increments at Gauss points
+// stress coefficients and applies A = divS iMJwPSI.  The element kernels are
+// in nsdg_stress_sumfact.cu; the TMA-staged operator kernel below splits an
+// element over three threads (kStressParts): in phase 1 thread `part` computes
+// the strain, Delta and the stress increments at Gauss points
 // 3*part .. 3*part+2 and leaves them in shared memory, in phase 2 it updates
 // the divergence coefficients of nodes 3*part .. 3*part+2.  Land cells keep
 // tdiv = 0 (the reference's divergence skips them).
-constexpr int kStressElems = 64;
 constexpr int kStressParts = 3;
 
 // Gathers the divergence contributions of the (up to four) ice cells around
@@ -1570,113 +1576,13 @@ __global__ void __launch_bounds__(kBlock) kMevpPrepNodes32(size_t n, MevpNodeSta
         dir[i] ? 1.f : 0.f);
 }
 
-// The FP64 kernel kMevpStress with FP32 operators and state.  The strain
-// invariant 1.25(e11^2+e22^2) + 1.5 e11 e22 + e12^2 is formed in FP32 from the
-// FP32 strain (it is a positive-definite quadratic form: no cancellation);
-// Delta = sqrt(invariant + DeltaMin^2) and the viscosity P/(8 alpha Delta) are
-// evaluated in FP64 (Pg holds P/(8 alpha), hP = P/(2 alpha) in FP32); the
-// stress increments and the divergence update are FP32.
-// Body of the mixed-precision element kernel for element e handled by thread
-// (le, part) of a block of kStressElems x kStressParts threads; shared by the
-// single-grid and the batched (ensemble) kernels.
-__device__ __forceinline__ void mevpStress32Element(int nx, size_t N, bool active, size_t e, int le, int part,
-    const DevOps32& o, const float* __restrict__ u, const float* __restrict__ v, const double* __restrict__ Pg,
-    const float* __restrict__ hPg, float* __restrict__ tdiv, const MevpParams& p, float (*fs)[9][kStressElems])
-{
-    if (active) {
-        const size_t s2 = 2 * size_t(nx) + 1;
-        const size_t ix = static_cast<unsigned>(e) % static_cast<unsigned>(nx);
-        const size_t iy = static_cast<unsigned>(e) / static_cast<unsigned>(nx);
-        const size_t base = 2 * s2 * iy + 2 * ix;
-        float ul[9], vl[9];
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-            const size_t nd = base + (j % 3) + (j / 3) * s2;
-            ul[j] = u[nd];
-            vl[j] = v[nd];
-        }
-        const double dmin = p.DeltaMin; // Delta^2 = inv + DeltaMin^2 with one rounding (FMA)
-#pragma unroll
-        for (int qq = 0; qq < 3; ++qq) {
-            const int q = 3 * part + qq;
-            float ex = 0.f, ey = 0.f, exv = 0.f, eyu = 0.f;
-#pragma unroll
-            for (int j = 0; j < 9; ++j) {
-                const float gxq = o.gx[(q * 9 + j) * o.ld + e];
-                const float gyq = o.gy[(q * 9 + j) * o.ld + e];
-                ex = fmaf(gxq, ul[j], ex);
-                ey = fmaf(gyq, vl[j], ey);
-                exv = fmaf(gxq, vl[j], exv);
-                eyu = fmaf(gyq, ul[j], eyu);
-            }
-            if (o.gm) { // spherical metric term
-                float mu = 0.f, mv = 0.f;
-#pragma unroll
-                for (int j = 0; j < 9; ++j) {
-                    const float gmq = o.gm[(q * 9 + j) * o.ld + e];
-                    mu = fmaf(gmq, ul[j], mu);
-                    mv = fmaf(gmq, vl[j], mv);
-                }
-                ex -= mv;
-                eyu += mu;
-            }
-            const float sxy = exv + eyu;
-            const float inv = 1.25f * (ex * ex + ey * ey) + 1.50f * ex * ey + 0.25f * sxy * sxy;
-            const float z8 = static_cast<float>(Pg[q * N + e] * rsqrt(fma(dmin, dmin, static_cast<double>(inv))));
-            const float hP = hPg[q * N + e];
-            fs[0][q][le] = fmaf(z8, fmaf(5.f, ex, 3.f * ey), -hP);
-            fs[1][q][le] = z8 * sxy;
-            fs[2][q][le] = fmaf(z8, fmaf(5.f, ey, 3.f * ex), -hP);
-        }
-    }
-    __syncthreads();
-    if (!active)
-        return;
-    const float keep = p.keep;
-#pragma unroll
-    for (int jj = 0; jj < 3; ++jj) {
-        const int j = 3 * part + jj;
-        float ax = 0.f, ay = 0.f;
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const float a1 = o.a1[(j * 9 + q) * o.ld + e];
-            const float a2 = o.a2[(j * 9 + q) * o.ld + e];
-            const float f11 = fs[0][q][le], f12 = fs[1][q][le], f22 = fs[2][q][le];
-            ax = fmaf(a1, f11, fmaf(a2, f12, ax));
-            ay = fmaf(a1, f12, fmaf(a2, f22, ay));
-            if (o.a3) {
-                const float a3 = o.a3[(j * 9 + q) * o.ld + e];
-                ax = fmaf(a3, f12, ax);
-                ay = fmaf(-a3, f11, ay);
-            }
-        }
-        tdiv[j * N + e] = fmaf(tdiv[j * N + e], keep, ax);
-        tdiv[(9 + j) * N + e] = fmaf(tdiv[(9 + j) * N + e], keep, ay);
-    }
-}
-
-// The FP64 kernel kMevpStress with FP32 operators and state.  The strain
-// invariant 1.25(e11^2+e22^2) + 1.5 e11 e22 + e12^2 is formed in FP32 from the
-// FP32 strain (it is a positive-definite quadratic form: no cancellation);
-// Delta = sqrt(invariant + DeltaMin^2) and the viscosity P/(8 alpha Delta) are
-// evaluated in FP64; the stress increments and the divergence update are FP32.
-__global__ void __launch_bounds__(kStressElems * kStressParts) kMevpStress32(DevMesh m, DevOps32 o,
-    const float* __restrict__ u, const float* __restrict__ v, const double* __restrict__ Pg,
-    const float* __restrict__ hP, float* __restrict__ tdiv, MevpParams p)
-{
-    __shared__ float fs[3][9][kStressElems];
-    const int le = threadIdx.x % kStressElems;
-    const int part = threadIdx.x / kStressElems;
-    const size_t e = blockIdx.x * size_t(kStressElems) + le;
-    const bool active = e < m.N && m.ice[e];
-    mevpStress32Element(m.nx, m.N, active, e, le, part, o, u, v, Pg, hP, tdiv, p, fs);
-}
-
 // ---------------------------------------------------------------------------
 // TMA-staged FP32 stress kernel
 // ---------------------------------------------------------------------------
-// The arithmetic of mevpStress32Element, with the operator entries of a
-// block's 32 elements brought into shared memory by 2-D TMA copies that
+// The element update with the 9 x 9 operators in FP32 (the strain invariant
+// 1.25(e11^2+e22^2) + 1.5 e11 e22 + e12^2 is positive definite: no
+// cancellation; Delta = sqrt(invariant + DeltaMin^2) and the viscosity in
+// FP64), with the operator entries of a block's 32 elements brought into shared memory by 2-D TMA copies that
 // complete on mbarriers: first the strain rows (G_x, G_y: box {32 elements,
 // 162 rows}, 20.7 KB), then, into the same buffer once the strain phase has
 // read it, the divergence rows (A_1, A_2).  One 24 KB buffer per block keeps
@@ -1837,244 +1743,6 @@ __global__ void __launch_bounds__(kTmaElems * kStressParts) kMevpStress32Tma(con
     stress32TmaBlock<SPH>(&mapG, &mapA, m.nx, m.N, m.ice, u, v, Pg, hPg, tdiv, p, err, blockIdx.x * kTmaElems, smem);
 }
 
-// ---------------------------------------------------------------------------
-// FP32 stress kernel for parallelogram meshes
-// ---------------------------------------------------------------------------
-// On a mesh of parallelograms every element's operators are combinations of
-// the unit-square ones with 5 coefficients per element (c0..c3 the Jacobian
-// entries, c4 = 1/J; the host derives them and checks the rebuilt operators
-// against the exact ones).  The unit-square operators sit in constant memory
-// and each warp handles a fixed third of the Gauss points and nodes, so their
-// entries are compile-time constant-bank operands; per element-iteration the
-// kernel streams 5 coefficients, P/(8 alpha), P/(2 alpha), the divergence and
-// the velocities instead of 324 operator entries.
-namespace {
-constexpr int kAffElems = 32;
-__constant__ float cAff[4][81]; // G_xi [q][j], G_eta [q][j], A_xi [j][q], A_eta [j][q]
-
-// float <-> double by exponent rebiasing on the integer pipe (GB300 executes
-// FP64 at about 1/60 of its FP32 rate): exact for positive normal
-// floats; a value below the smallest normal float maps to zero.
-__device__ __forceinline__ double widenPos(float f)
-{
-    const unsigned long long b = (static_cast<unsigned long long>(__float_as_uint(f)) << 29) + (896ull << 52);
-    return __longlong_as_double(static_cast<long long>(b));
-}
-// f / 2 for a positive normal float f (exact)
-__device__ __forceinline__ double widenHalfPos(float f)
-{
-    const unsigned long long b = (static_cast<unsigned long long>(__float_as_uint(f)) << 29) + (895ull << 52);
-    return __longlong_as_double(static_cast<long long>(b));
-}
-__device__ __forceinline__ double widenNonneg(float f)
-{
-    return __float_as_uint(f) >= 0x00800000u ? widenPos(f) : 0.0;
-}
-// d >= 0 and below 2^128: nearest float (ties away from zero); 0 below the
-// smallest normal float
-__device__ __forceinline__ float narrowPos(double d)
-{
-    const long long b = __double_as_longlong(d);
-    const long long r = (b - (896ll << 52) + (1ll << 28)) >> 29;
-    return b >= (897ll << 52) ? __uint_as_float(static_cast<unsigned>(r)) : 0.f;
-}
-} // namespace
-
-// P/(8 alpha Delta) with Delta = sqrt(t), t = inv + DeltaMin^2 formed in FP64
-// with one rounding (FMA), evaluated in FP64.  VM 0: CUDA's rsqrt(double).
-// VM 1 and 2: one Newton-Raphson step for the reciprocal square root,
-// y1 = y0 + y0 (1 - t y0^2) / 2, in FP64 from the FP32 seed
-// y0 = rsqrtf(inv + DeltaMin^2) (relative error of y1: 1.5 e0^2 + FP64
-// rounding, e0 <= 2^-21 for the seed and its FP32 argument, i.e. below
-// 1e-12); VM 2 converts between float and double on the integer pipe (y0/2
-// by the exponent bias).  Five FP64 instructions per Gauss point in VM 2.
-// VM 3: the same Newton step from the same seed with float pairs on the FP32
-// pipe (nsdg_visc_ff.hpp: one FP64 subtraction per Gauss point; dmin2lo is
-// the low part of DeltaMin^2).  VM 4: VM 3's float pairs with the check of
-// nsdg_ff::viscFloatFloatChecked, and VM 2's FP64 operations from the same
-// seed wherever the check cannot prove the pair's rounding equal to theirs
-// (near a float rounding boundary: about 1e-4 of the Gauss points): bitwise
-// VM 2's result with one FP64 subtraction per Gauss point instead of five
-// FP64 instructions (measured slower than VM 2 on GB300: the float-pair
-// arithmetic and the check cost more issue than the FP64 pipe they free).
-__device__ __forceinline__ float viscNewton64(float inv, double Pa, double dmin, float y0)
-{
-    const double t = fma(dmin, dmin, widenNonneg(inv));
-    const double yd = widenPos(y0);
-    const double h = t * yd;
-    const double e2 = fma(-h, widenHalfPos(y0), 0.5); // (1 - t y0^2) / 2
-    const double z = Pa * yd;
-    return narrowPos(fma(z, e2, z));
-}
-
-template <int VM>
-__device__ __forceinline__ float viscosity8(float inv, double Pa, double dmin, float dmin2f, float dmin2lo)
-{
-    if constexpr (VM == 3) {
-        return nsdg_ff::viscFloatFloat(inv, Pa, dmin2f, dmin2lo, rsqrtf(inv + dmin2f));
-    } else if constexpr (VM == 4) {
-        const float y0 = rsqrtf(inv + dmin2f);
-        bool exact;
-        const float z = nsdg_ff::viscFloatFloatChecked(inv, Pa, dmin2f, dmin2lo, y0, exact);
-        return exact ? z : viscNewton64(inv, Pa, dmin, y0);
-    } else {
-        const double td = VM == 2 ? widenNonneg(inv) : static_cast<double>(inv);
-        const double t = fma(dmin, dmin, td);
-        if constexpr (VM == 0) {
-            return static_cast<float>(Pa * rsqrt(t));
-        } else {
-            const float y0 = rsqrtf(inv + dmin2f);
-            const double yd = VM == 1 ? static_cast<double>(y0) : widenPos(y0);
-            const double yh = VM == 1 ? 0.5 * yd : widenHalfPos(y0);
-            const double h = t * yd;
-            const double e2 = fma(-h, yh, 0.5); // (1 - t y0^2) / 2
-            const double z = Pa * yd;
-            const double z8 = fma(z, e2, z);
-            return VM == 1 ? static_cast<float>(z8) : narrowPos(z8);
-        }
-    }
-}
-
-template <int PART, int VM>
-__device__ __forceinline__ void affineStrain(const float (&ul)[9], const float (&vl)[9], const float (&c)[5],
-    const double (&Pa)[3], const float (&hP)[3], double dmin, float dmin2f, float dmin2lo,
-    float (*fs)[9][kAffElems], int le)
-{
-#pragma unroll
-    for (int qq = 0; qq < 3; ++qq) {
-        constexpr int q0 = 3 * PART;
-        const int q = q0 + qq;
-        float ux = 0.f, ue = 0.f, vx = 0.f, ve = 0.f;
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-            const float gx = cAff[0][q * 9 + j], ge = cAff[1][q * 9 + j];
-            ux = fmaf(gx, ul[j], ux);
-            ue = fmaf(ge, ul[j], ue);
-            vx = fmaf(gx, vl[j], vx);
-            ve = fmaf(ge, vl[j], ve);
-        }
-        const float ex = c[4] * fmaf(c[0], ux, c[1] * ue);  // G_x u
-        const float ey = c[4] * fmaf(c[2], vx, c[3] * ve);  // G_y v
-        const float exv = c[4] * fmaf(c[0], vx, c[1] * ve); // G_x v
-        const float eyu = c[4] * fmaf(c[2], ux, c[3] * ue); // G_y u
-        const float sxy = exv + eyu;
-        const float inv = 1.25f * (ex * ex + ey * ey) + 1.50f * ex * ey + 0.25f * sxy * sxy;
-        const float z8 = viscosity8<VM>(inv, Pa[qq], dmin, dmin2f, dmin2lo);
-        const float f11 = fmaf(z8, fmaf(5.f, ex, 3.f * ey), -hP[qq]);
-        const float f12 = z8 * sxy;
-        const float f22 = fmaf(z8, fmaf(5.f, ey, 3.f * ex), -hP[qq]);
-        // the Gauss-point weights of A_xi and A_eta in A_1 f11 + A_2 f12 and
-        // A_1 f12 + A_2 f22
-        fs[0][q][le] = fmaf(c[0], f11, c[2] * f12);
-        fs[1][q][le] = fmaf(c[1], f11, c[3] * f12);
-        fs[2][q][le] = fmaf(c[0], f12, c[2] * f22);
-        fs[3][q][le] = fmaf(c[1], f12, c[3] * f22);
-    }
-}
-
-template <int PART>
-__device__ __forceinline__ void affineDivergence(float (*fs)[9][kAffElems], int le, size_t e, size_t N,
-    float* __restrict__ tdiv, float keep, const float (&told)[6])
-{
-    float w[4][9];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int q = 0; q < 9; ++q)
-            w[k][q] = fs[k][q][le];
-#pragma unroll
-    for (int jj = 0; jj < 3; ++jj) {
-        const int j = 3 * PART + jj;
-        float ax = 0.f, ay = 0.f;
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const float axi = cAff[2][j * 9 + q], aet = cAff[3][j * 9 + q];
-            ax = fmaf(axi, w[0][q], fmaf(aet, w[1][q], ax));
-            ay = fmaf(axi, w[2][q], fmaf(aet, w[3][q], ay));
-        }
-        tdiv[j * N + e] = fmaf(told[jj], keep, ax);
-        tdiv[(9 + j) * N + e] = fmaf(told[3 + jj], keep, ay);
-    }
-}
-
-// One block of the parallelogram stress kernel: elements x0 .. x0+31 of a
-// grid (shared by the single-grid and the batched ensemble kernels).
-template <int VM>
-__device__ __forceinline__ void affineBlock(int nx, size_t N, const uint8_t* __restrict__ ice,
-    const float* __restrict__ coef, size_t ld, const float* __restrict__ u, const float* __restrict__ v,
-    const double* __restrict__ Pg, float* __restrict__ tdiv, const MevpParams& p, size_t x0,
-    float (*fs)[9][kAffElems])
-{
-    const int le = threadIdx.x % kAffElems;
-    const int part = threadIdx.x / kAffElems; // one warp per third of the Gauss points / nodes
-    const size_t e = x0 + le;
-    const bool active = e < N && ice[e];
-    // step constants first: a programmatic dependent launch overlaps them
-    // with the previous kernel's tail.  So does this element's divergence
-    // from the previous iteration: no launch triggers its dependents early,
-    // so this kernel starts only after the node kernel before it has exited,
-    // and that kernel read the divergence only after the stress kernel that
-    // wrote it had completed; the node kernel only reads it.
-    float c[5], ul[9], vl[9], hP[3], told[6];
-    double Pa[3];
-    if (active) {
-#pragma unroll
-        for (int jj = 0; jj < 3; ++jj) {
-            told[jj] = tdiv[(3 * part + jj) * N + e];
-            told[3 + jj] = tdiv[(9 + 3 * part + jj) * N + e];
-        }
-#pragma unroll
-        for (int k = 0; k < 5; ++k)
-            c[k] = coef[k * ld + e];
-#pragma unroll
-        for (int qq = 0; qq < 3; ++qq) {
-            Pa[qq] = Pg[(3 * part + qq) * N + e];
-            // P/(2 alpha) = 4 P/(8 alpha): an exact power-of-two scaling,
-            // rounded to float on the integer pipe (the value the prep kernel
-            // stores for the other element kernels)
-            hP[qq] = narrowPos(__longlong_as_double(__double_as_longlong(Pa[qq]) + (2ll << 52)));
-        }
-    }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (active) {
-        const size_t s2 = 2 * size_t(nx) + 1;
-        const size_t ix = static_cast<unsigned>(e) % static_cast<unsigned>(nx);
-        const size_t iy = static_cast<unsigned>(e) / static_cast<unsigned>(nx);
-        const size_t base = 2 * s2 * iy + 2 * ix;
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-            const size_t nd = base + (j % 3) + (j / 3) * s2;
-            ul[j] = u[nd];
-            vl[j] = v[nd];
-        }
-        const double dmin = p.DeltaMin;
-        const float dmin2f = p.dmin2f, dmin2lo = p.dmin2lo;
-        switch (part) {
-        case 0: affineStrain<0, VM>(ul, vl, c, Pa, hP, dmin, dmin2f, dmin2lo, fs, le); break;
-        case 1: affineStrain<1, VM>(ul, vl, c, Pa, hP, dmin, dmin2f, dmin2lo, fs, le); break;
-        default: affineStrain<2, VM>(ul, vl, c, Pa, hP, dmin, dmin2f, dmin2lo, fs, le); break;
-        }
-    }
-    __syncthreads();
-    if (!active)
-        return;
-    const float keep = p.keep;
-    switch (part) {
-    case 0: affineDivergence<0>(fs, le, e, N, tdiv, keep, told); break;
-    case 1: affineDivergence<1>(fs, le, e, N, tdiv, keep, told); break;
-    default: affineDivergence<2>(fs, le, e, N, tdiv, keep, told); break;
-    }
-}
-
-template <int VM>
-__global__ void __launch_bounds__(kAffElems * kStressParts, 12) kMevpStress32Affine(DevMesh m,
-    const float* __restrict__ coef, size_t ld, const float* __restrict__ u, const float* __restrict__ v,
-    const double* __restrict__ Pg, float* __restrict__ tdiv, MevpParams p)
-{
-    __shared__ float fs[4][9][kAffElems];
-    affineBlock<VM>(m.nx, m.N, m.ice, coef, ld, u, v, Pg, tdiv, p, blockIdx.x * size_t(kAffElems), fs);
-}
-
 // Self-test of the FP64 viscosity forms: out[3 n] = P/(8 alpha Delta) for
 // every VM (0, 1, 2) at each (inv, Pa).
 __global__ void kViscositySelfTest(size_t n, const float* __restrict__ inv, const double* __restrict__ Pa,
@@ -2185,27 +1853,9 @@ __global__ void __launch_bounds__(kBlock) kMevpMomentum32(DevMesh m, MevpNodeSta
 
 // ---------------------------------------------------------------------------
 // Batched ensemble: one launch covers the elements (nodes) of every member.
-// Block b belongs to member blockMember[b]; within the member, stress blocks
-// map to 2D tiles of tileW x tileH elements (tileW * tileH = kStressElems,
-// chosen per grid size by the ensemble's autotuner) and node blocks to
-// consecutive runs of kBlock CG2 nodes.
+// Block b belongs to member blockMember[b]; within the member, blocks map to
+// consecutive runs of elements or of kBlock CG2 nodes.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kStressElems * kStressParts) kMevpStress32Batched(
-    const EnsembleMember* __restrict__ members, const uint16_t* __restrict__ blockMember, MevpParams p)
-{
-    __shared__ float fs[3][9][kStressElems];
-    const EnsembleMember& M = members[blockMember[blockIdx.x]];
-    const int b = static_cast<int>(blockIdx.x) - M.stressBlock0;
-    const int le = threadIdx.x % kStressElems;
-    const int part = threadIdx.x / kStressElems;
-    const int tx = b % M.tilesX, ty = b / M.tilesX;
-    const int ix = tx * M.tileW + le % M.tileW, iy = ty * M.tileH + le / M.tileW;
-    const bool inside = ix < M.nx && iy < M.ny;
-    const size_t e = inside ? size_t(iy) * M.nx + ix : 0;
-    const bool active = inside && M.ice[e];
-    mevpStress32Element(M.nx, M.N, active, e, le, part, M.o, M.st.u, M.st.v, M.Pg, M.hP, M.tdiv, p, fs);
-}
-
 // Self-test of the bounded wait: one thread waits on an mbarrier that nothing
 // will complete (expected arrivals 1, none made), records whether the wait
 // ran out, and the barrier is left behind with the block.
@@ -2230,22 +1880,12 @@ __global__ void __launch_bounds__(kTmaElems * kStressParts) kMevpStress32TmaBatc
         smem);
 }
 
-template <int VM>
-__global__ void __launch_bounds__(kAffElems * kStressParts, 12) kMevpStress32AffineBatched(
-    const EnsembleMember* __restrict__ members, const uint16_t* __restrict__ blockMember, MevpParams p)
-{
-    __shared__ float fs[4][9][kAffElems];
-    const EnsembleMember& M = members[blockMember[blockIdx.x]];
-    const size_t x0 = size_t(static_cast<int>(blockIdx.x) - M.tmaBlock0) * kAffElems;
-    affineBlock<VM>(M.nx, M.N, M.ice, M.affCoef, M.affLd, M.st.u, M.st.v, M.Pg, M.tdiv, p, x0, fs);
-}
-
 // ---------------------------------------------------------------------------
 // Persistent sub-cycle of a parallelogram ensemble: one cooperative launch
 // runs all mEVP iterations of every member, the element phase and the node
 // phase as grid-stride loops over the same block maps as the per-phase
 // launches, separated by grid barriers.  Each element and node is computed
-// by the same arithmetic in the same order as in kMevpStress32AffineBatched
+// by the same arithmetic in the same order as in kMevpStress32Batched
 // and kMevpMomentum32Batched, so the results are bitwise the same.
 //
 // The grid barrier is the project's own, with a bounded wait: bar[0] counts
@@ -2292,15 +1932,17 @@ __global__ void __launch_bounds__(kAffElems * kStressParts) kEnsembleSubcyclePer
     const uint16_t* __restrict__ nodeMap, int nodeBlocks, MevpParams p, int iterations, unsigned* __restrict__ bar,
     int* __restrict__ err)
 {
-    __shared__ float fs[4][9][kAffElems];
+    __shared__ sf::Exchange<float, kAffElems> ex;
+    const sf::Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
     __shared__ int okShared;
     constexpr int kThreads = kAffElems * kStressParts;
     for (int it = 0; it < iterations; ++it) {
         for (int b = blockIdx.x; b < elemBlocks; b += gridDim.x) {
             const EnsembleMember& M = members[elemMap[b]];
             const size_t x0 = size_t(b - M.tmaBlock0) * kAffElems;
-            affineBlock<VM>(M.nx, M.N, M.ice, M.affCoef, M.affLd, M.st.u, M.st.v, M.Pg, M.tdiv, p, x0, fs);
-            __syncthreads(); // the next work block reuses fs
+            sf::stressBlock<float, sf::AFFINE, VM, kAffElems>(M.nx, M.N, M.ice, M.aff, M.st.u, M.st.v, M.Pw, M.tdiv,
+                rh, p.keep, x0, ex, nullptr);
+            __syncthreads(); // the next work block reuses ex
         }
         if (!gridBarrierBounded(bar, err, &okShared))
             break;
@@ -2438,6 +2080,7 @@ template <typename T> struct BbmOps {
     size_t ld = 0;
 };
 
+__constant__ float cAff[4][81]; // G_xi [q][j], G_eta [q][j], A_xi [j][q], A_eta [j][q]
 // The unit square's BBM operators for the parallelogram-mesh kernel (with
 // cAff's strain operators): iMJwPSI [k][q], the damage projection [k][q],
 // D_xi and D_eta [j][k] (divS1 = c0 D_xi + c1 D_eta, divS2 = c2 D_xi +
@@ -3026,15 +2669,14 @@ cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNode
 }
 
 cudaError_t launchMevpPrepElements(cudaStream_t s, const DevMesh& m, int dg, const double* h,
-    const double* a, double* Pg, const MevpParams& p, float* hP32, const float* tdiv32, float* tdivLast,
-    const double* weight)
+    const double* a, const PressureOut& out, const MevpParams& p, const float* tdiv32, float* tdivLast)
 {
     const unsigned g = blocksFor(m.N);
     const double ia = 1.0 / p.alpha;
     switch (dg) {
-    case 1: kMevpPrepElements<1><<<g, kBlock, 0, s>>>(m.N, h, a, Pg, p.Pstar, ia, hP32, tdiv32, tdivLast, weight); break;
-    case 3: kMevpPrepElements<3><<<g, kBlock, 0, s>>>(m.N, h, a, Pg, p.Pstar, ia, hP32, tdiv32, tdivLast, weight); break;
-    case 6: kMevpPrepElements<6><<<g, kBlock, 0, s>>>(m.N, h, a, Pg, p.Pstar, ia, hP32, tdiv32, tdivLast, weight); break;
+    case 1: kMevpPrepElements<1><<<g, kBlock, 0, s>>>(m.N, h, a, out, p.Pstar, ia, tdiv32, tdivLast); break;
+    case 3: kMevpPrepElements<3><<<g, kBlock, 0, s>>>(m.N, h, a, out, p.Pstar, ia, tdiv32, tdivLast); break;
+    case 6: kMevpPrepElements<6><<<g, kBlock, 0, s>>>(m.N, h, a, out, p.Pstar, ia, tdiv32, tdivLast); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -3211,28 +2853,6 @@ cudaError_t uploadAffineReference(const double ref[4][81])
     return cudaMemcpyToSymbol(cAff, h, sizeof(h));
 }
 
-cudaError_t launchMevpStress32Affine(cudaStream_t s, const DevMesh& m, const float* coef, size_t ld, const float* u,
-    const float* v, const double* Pg, float* tdiv, const MevpParams& pIn, int viscosityMode)
-{
-    const MevpParams p = withDerived(pIn);
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(blocksFor(m.N, kAffElems));
-    cfg.blockDim = dim3(kAffElems * kStressParts);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    switch (viscosityMode) {
-    case 0: return cudaLaunchKernelEx(&cfg, kMevpStress32Affine<0>, m, coef, ld, u, v, Pg, tdiv, p);
-    case 1: return cudaLaunchKernelEx(&cfg, kMevpStress32Affine<1>, m, coef, ld, u, v, Pg, tdiv, p);
-    case 3: return cudaLaunchKernelEx(&cfg, kMevpStress32Affine<3>, m, coef, ld, u, v, Pg, tdiv, p);
-    case 4: return cudaLaunchKernelEx(&cfg, kMevpStress32Affine<4>, m, coef, ld, u, v, Pg, tdiv, p);
-    default: return cudaLaunchKernelEx(&cfg, kMevpStress32Affine<2>, m, coef, ld, u, v, Pg, tdiv, p);
-    }
-}
-
 cudaError_t launchViscositySelfTest(cudaStream_t s, size_t n, const float* inv, const double* Pa, double dmin,
     float* out)
 {
@@ -3254,13 +2874,6 @@ cudaError_t launchViscositySelfTestChecked(cudaStream_t s, size_t n, const float
     return cudaGetLastError();
 }
 
-cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const DevOps32& o, const float* u,
-    const float* v, const double* Pg, const float* hP, float* tdiv, const MevpParams& pIn)
-{
-    const MevpParams p = withDerived(pIn);
-    kMevpStress32<<<blocksFor(m.N, kStressElems), kStressElems * kStressParts, 0, s>>>(m, o, u, v, Pg, hP, tdiv, p);
-    return cudaGetLastError();
-}
 cudaError_t launchMevpMomentum32(cudaStream_t s, const DevMesh& m, const MevpNodeState32& st,
     const float* tdiv, const MevpParams& pIn, int* err)
 {
@@ -3275,13 +2888,6 @@ cudaError_t launchMevpMomentum32(cudaStream_t s, const DevMesh& m, const MevpNod
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kMevpMomentum32, m, st, tdiv, p, err);
-}
-cudaError_t launchMevpStress32Batched(cudaStream_t s, const EnsembleMember* members, const uint16_t* blockMember,
-    int blocks, const MevpParams& pIn)
-{
-    const MevpParams p = withDerived(pIn);
-    kMevpStress32Batched<<<blocks, kStressElems * kStressParts, 0, s>>>(members, blockMember, p);
-    return cudaGetLastError();
 }
 cudaError_t launchMevpMomentum32Batched(cudaStream_t s, const EnsembleMember* members, const uint16_t* blockMember,
     int blocks, const MevpParams& pIn, int* err)
@@ -3314,27 +2920,6 @@ cudaError_t launchMevpStress32TmaBatched(cudaStream_t s, const EnsembleMember* m
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kMevpStress32TmaBatched, members, blockMember, p, err);
 }
-cudaError_t launchMevpStress32AffineBatched(cudaStream_t s, const EnsembleMember* members,
-    const uint16_t* blockMember, int blocks, const MevpParams& pIn, int viscosityMode)
-{
-    const MevpParams p = withDerived(pIn);
-    static_assert(kAffElems == kTmaElems, "the parallelogram and TMA kernels share the block map");
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(kAffElems * kStressParts);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    switch (viscosityMode) {
-    case 0: return cudaLaunchKernelEx(&cfg, kMevpStress32AffineBatched<0>, members, blockMember, p);
-    case 1: return cudaLaunchKernelEx(&cfg, kMevpStress32AffineBatched<1>, members, blockMember, p);
-    case 4: return cudaLaunchKernelEx(&cfg, kMevpStress32AffineBatched<4>, members, blockMember, p);
-    default: return cudaLaunchKernelEx(&cfg, kMevpStress32AffineBatched<2>, members, blockMember, p);
-    }
-}
 int persistentNodesPerBlock() { return kAffElems * kStressParts; }
 
 cudaError_t launchEnsembleSubcyclePersistent(cudaStream_t s, const EnsembleMember* members, const uint16_t* elemMap,
@@ -3347,7 +2932,8 @@ cudaError_t launchEnsembleSubcyclePersistent(cudaStream_t s, const EnsembleMembe
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     auto kern = viscosityMode == 0 ? kEnsembleSubcyclePersistent<0>
         : viscosityMode == 1 ? kEnsembleSubcyclePersistent<1>
-        : viscosityMode == 4 ? kEnsembleSubcyclePersistent<4> : kEnsembleSubcyclePersistent<2>;
+        : viscosityMode == 2 ? kEnsembleSubcyclePersistent<2>
+        : viscosityMode == 4 ? kEnsembleSubcyclePersistent<4> : kEnsembleSubcyclePersistent<3>;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, kAffElems * kStressParts, 0);
     if (e != cudaSuccess)
         return e;
@@ -3371,7 +2957,6 @@ cudaError_t launchEnsembleSubcyclePersistent(cudaStream_t s, const EnsembleMembe
     return cudaLaunchKernelEx(&cfg, kern, members, elemMap, elemBlocks, nodeMap, nodeBlocks, p, iterations, bar, err);
 }
 
-int stressElementsPerBlock() { return kStressElems; }
 int nodesPerBlock() { return kBlock; }
 
 cudaError_t launchWidenVelocity(cudaStream_t s, size_t n, const float* u32, const float* v32, double* u, double* v)

@@ -182,30 +182,35 @@ inline MevpParams withDerived(MevpParams p)
 }
 cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* invm2,
     const MevpParams& p);
-// P at the 3x3 Gauss points from h and A (MEVPStressUpdateStep.hpp:54-57,75-77):
-// Pg = P/alpha, or Pg = weight P/(4 alpha) with a weight per point ([9][N],
-// StressGeometry::w), or, for the mixed-precision kernels (hP32 given),
-// Pg = P/(8 alpha) (FP64, the viscosity numerator) and hP32 = P/(2 alpha).
+// P at the 3x3 Gauss points from h and A (MEVPStressUpdateStep.hpp:54-57,75-77),
+// in every form whose target is given ([9][N] each).
+struct PressureOut {
+    double* alpha = nullptr;        // P/alpha (the float-pair FP64 kernels)
+    double* visc = nullptr;         // P/(8 alpha), with half (the mixed TMA kernel)
+    float* half = nullptr;          // P/(2 alpha)
+    double* weighted = nullptr;     // w P/(4 alpha) (the sum-factorised FP64 kernels)
+    float2* weightedPair = nullptr; // the same as a pair of floats (mixed)
+    const double* w = nullptr;      // StressMetric::w
+};
 // tdivLast (mixed precision, optional): also copies tdiv32 there (the
 // sub-cycle's starting divergence, a warm-start feature).
 cudaError_t launchMevpPrepElements(cudaStream_t s, const DevMesh& m, int dg, const double* h,
-    const double* a, double* Pg, const MevpParams& p, float* hP32 = nullptr, const float* tdiv32 = nullptr,
-    float* tdivLast = nullptr, const double* weight = nullptr);
+    const double* a, const PressureOut& out, const MevpParams& p, const float* tdiv32 = nullptr,
+    float* tdivLast = nullptr);
 // One mEVP iteration, element part, carried in divergence space: the strain at
 // the Gauss points, Delta, and the relaxed update of the element's stress
 // divergence contributions tdiv[18][N] = (divS1 s11 + divS2 s12, divS1 s12 +
 // divS2 s22) at its 9 CG2 nodes (CGDynamicsKernel.cpp:300-398,
 // MEVPStressUpdateStep.hpp:30-118), by sum factorisation (nsdg_sumfact.cuh).
 // Device copy of StressMetric (nsdg_host.hpp).
-struct StressGeometry {
-    const double* k = nullptr; // [2][N] on rectangles, else [4][9][N]
-    const double* n = nullptr; // [9][N] (null on rectangles)
-    const double* m = nullptr; // [9][N] (spherical meshes)
-    const double* w = nullptr; // [9][N]
+template <typename T> struct StressGeometry {
+    const T* k = nullptr; // [2][N] on rectangles (FP64), [4][N] on parallelograms (FP32), else [4][9][N]
+    const T* n = nullptr; // [9][N] (null on rectangles and parallelograms)
+    const T* m = nullptr; // [9][N] (spherical meshes)
     bool rect = false;
 };
 // Pw holds w P/(4 alpha) at the Gauss points.
-cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const StressGeometry& geo, const double* u,
+cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const StressGeometry<double>& geo, const double* u,
     const double* v, const double* Pw, double* tdiv, const MevpParams& p);
 // The benchmark forcing on the cell centres (nsdg_forcing.cu):
 // BenchmarkAtmosphere.cpp:29-77 and BenchmarkOcean.cpp:15-39.
@@ -312,17 +317,24 @@ cudaError_t launchMevpPrepNodes32(cudaStream_t s, const DevMesh& m, const MevpNo
     const MevpNodeState32& st32, const double* invm2, const MevpParams& p,
     float* uLast = nullptr, float* vLast = nullptr);
 // (the Dirichlet flags of the nodes come from m.cg2Dir)
-// kMevpStress32 for parallelogram meshes: the unit-square operators
-// (G_xi, G_eta [q][j], A_xi, A_eta [j][q]) in constant memory, uploaded once
-// per device (they depend only on the basis), and 5 coefficients per element
-// ([5][ld]).  viscosityMode selects the FP64 evaluation of P/(8 alpha Delta):
-// 0 CUDA's rsqrt(double), 1 a Newton step from an FP32 seed, 2 the same with
-// float/double conversions on the integer pipe; 3 the same Newton step with
-// float pairs on the FP32 pipe (nsdg_visc_ff.hpp); 4 form 3 checked against
-// form 2's rounding, with form 2 where the check fails (bitwise form 2).
+// The unit square's strain operators (G_xi, G_eta [q][j]) for the
+// parallelogram BBM kernel, in constant memory (they depend only on the basis).
 cudaError_t uploadAffineReference(const double ref[4][81]);
-cudaError_t launchMevpStress32Affine(cudaStream_t s, const DevMesh& m, const float* coef, size_t ld, const float* u,
-    const float* v, const double* Pg, float* tdiv, const MevpParams& p, int viscosityMode);
+// The sum-factorised element kernels with FP32 state (nsdg_sumfact.cuh), Pw
+// the weighted pressure as pairs of floats: on parallelograms (4 coefficients
+// per element) and on general quadrilaterals or a sphere.  viscosityMode
+// selects the evaluation of P/(8 alpha Delta) on parallelograms: 3, the
+// default, the Newton step with float pairs on the FP32 pipe
+// (nsdg_visc_ff.hpp); 0 CUDA's rsqrt(double), 1 the Newton step from an FP32
+// seed in FP64, 2 the same with float/double conversions on the integer pipe;
+// 4 form 3 checked against form 2's rounding, with form 2 where the check
+// fails (bitwise form 2).
+constexpr int kAffElems = 32;  // elements per block
+constexpr int kQuadElems = 64;
+cudaError_t launchMevpStress32Affine(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo,
+    const float* u, const float* v, const float2* Pw, float* tdiv, const MevpParams& p, int viscosityMode);
+cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo, const float* u,
+    const float* v, const float2* Pw, float* tdiv, const MevpParams& p);
 // out[k n + i] = P/(8 alpha Delta) of (inv[i], Pa[i]) by viscosity mode k = 0, 1, 2.
 cudaError_t launchViscositySelfTest(cudaStream_t s, size_t n, const float* inv, const double* Pa, double dmin,
     float* out);
@@ -332,8 +344,6 @@ cudaError_t launchViscositySelfTestFF(cudaStream_t s, size_t n, const float* inv
 // out[i] = P/(8 alpha Delta) of (inv[i], Pa[i]) by viscosity mode 4.
 cudaError_t launchViscositySelfTestChecked(cudaStream_t s, size_t n, const float* inv, const double* Pa,
     double dmin, float* out);
-cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const DevOps32& o, const float* u,
-    const float* v, const double* Pg, const float* hP, float* tdiv, const MevpParams& p);
 cudaError_t launchMevpMomentum32(cudaStream_t s, const DevMesh& m,
     const MevpNodeState32& st, const float* tdiv, const MevpParams& p, int* err);
 // One member of a batched ensemble (device-resident table entry).
@@ -343,18 +353,16 @@ struct EnsembleMember {
     const uint8_t* ice;
     const uint8_t* cg2Dir;
     const double* invm2;
-    DevOps32 o;
     MevpNodeState32 st;
     const double* Pg;
     const float* hP;
+    const float2* Pw;
     float* tdiv;
-    int tileW, tileH, tilesX;
     int stressBlock0, nodeBlock0;
     int tmaBlock0;   // first block of this member in the TMA-staged / parallelogram batched launch
     int nodeBlockP;  // first block of this member in the persistent sub-cycle's node phase
     StressMaps maps; // the member's tensor maps (64-byte aligned inside the device table)
-    const float* affCoef; // [5][affLd] parallelogram coefficients (null: not a parallelogram mesh)
-    size_t affLd;
+    StressGeometry<float> quad, aff; // aff.k null: not a parallelogram mesh
 };
 // The whole mEVP sub-cycle of a parallelogram ensemble (every member has
 // coefficients) as one cooperative, persistent launch: `iterations` times the
@@ -379,7 +387,6 @@ cudaError_t launchMevpStress32TmaBatched(cudaStream_t s, const EnsembleMember* m
 // member must have coefficients); blocks as for the TMA-staged launch.
 cudaError_t launchMevpStress32AffineBatched(cudaStream_t s, const EnsembleMember* members,
     const uint16_t* blockMember, int blocks, const MevpParams& p, int viscosityMode);
-int stressElementsPerBlock();
 int nodesPerBlock();
 
 // u, v (FP64) from the FP32 iterate at the end of the sub-cycle

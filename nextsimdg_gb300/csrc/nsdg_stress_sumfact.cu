@@ -1,4 +1,6 @@
-// nsdg_stress_sumfact.cu — the FP64 mEVP element kernel (nsdg_sumfact.cuh).
+// nsdg_stress_sumfact.cu — the sum-factorised mEVP element kernels
+// (nsdg_sumfact.cuh): FP64, mixed precision, and mixed precision batched over
+// an ensemble's members.
 #include "nsdg_sumfact.cuh"
 
 namespace nsdg {
@@ -6,18 +8,7 @@ namespace {
 
 using namespace sf;
 
-// One mEVP iteration in divergence space, FP64: tdiv <- (1 - 1/alpha) tdiv +
-// K^T P^T f(P K u).  Three threads per element, in three warps of a block of
-// kElems elements: warp R takes node column R (the eta maps of its three
-// nodes), then Gauss row R (the xi maps, strain, stress increments, the
-// transposed xi maps), then node column R again (the transposed eta maps); the
-// 24 and 36 values in between go through shared memory, as do the sums of the
-// two projections on general quadrilaterals.
-//
-// On rectangles the strain is carried over k_x (strain' = strain / k_x, the
-// eta derivatives times rho = k_y / k_x, DeltaMin^2 over k_x^2) and k_x is
-// part of the pressure's weight, so only rho is multiplied in.
-//
+// FP64.
 // Bound by FP64 issue: about 480 FP64 instructions per element on rectangles,
 // 720 on quadrilaterals and 800 on a sphere; at the rate cuBLAS DGEMM reaches
 // (0.55 T FMA/s) 57 us for 256 x 256 rectangles.  Timed alone (CUDA events):
@@ -28,258 +19,120 @@ using namespace sf;
 // 64 x 64 one warp per SM waits out every instruction's latency (17.1 us).
 constexpr int kElems = 32;
 
-struct Exchange {
-    union {
-        struct {
-            double v[2][3][3][kElems];  // [u, v][Gauss row][column]: values on the columns
-            double dv[2][3][3][kElems]; // eta derivatives
-        } in;
-        struct {
-            double x[2][3][3][kElems]; // to the transposed interpolation
-            double y[2][3][3][kElems]; // to the transposed derivative
-        } out;
-    };
-};
-
-// The block's three warps meet here from different instances of the row code:
-// a barrier by its number (PTX bar.sync counts warps, whatever their place in
-// the code).
-__device__ __forceinline__ void rowsBarrier() { asm volatile("bar.sync 1, %0;" ::"n"(3 * kElems) : "memory"); }
-
-// sum over the element's three warps of each thread's c[0..2]
-__device__ __forceinline__ void sumRows(double (*part)[3][kElems], int R, int le, double (&c)[3])
-{
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        part[R][k][le] = c[k];
-    rowsBarrier();
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        c[k] = part[0][k][le] + part[1][k][le] + part[2][k][le];
-}
-
-template <int R, Geometry GEO>
-__device__ __forceinline__ void row64(bool active, size_t e, size_t N, const StressGeometry& geo,
-    const double (&pq)[3], double rho, double dminQ, Exchange& ex, double (*sums)[3][3][kElems], int le)
-{
-    double I[3], D[3], uxi[3], uet[3], vxi[3], vet[3], f11[3], f12[3], f22[3], x[3], y[3];
-    [[maybe_unused]] double up[3], vp[3];
-    const Scaled<double> sc(GEO == RECT ? rho : 1.0);
-    auto take = [&](int c) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            I[i] = ex.in.v[c][R][i][le];
-            D[i] = ex.in.dv[c][R][i][le];
-        }
-    };
-    take(0);
-    deriv(I, uxi);
-    if constexpr (GEO == RECT)
-        sc.interp(D, uet);
-    else
-        interp(D, uet);
-    if constexpr (GEO == SPHERE)
-        interp(I, up);
-    take(1);
-    deriv(I, vxi);
-    if constexpr (GEO == RECT)
-        sc.interp(D, vet);
-    else
-        interp(D, vet);
-    if constexpr (GEO == SPHERE)
-        interp(I, vp);
-    if constexpr (GEO == RECT) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            pointStress64(uxi[i], vet[i], uet[i] + vxi[i], pq[i], dminQ, f11[i], f12[i], f22[i]);
-        rowsBarrier(); // every warp has taken its row: the buffer changes hands
-        auto put = [&](int c, const double (&fx)[3], const double (&fy)[3]) {
-            derivT(fx, x);
-            sc.interpT(fy, y);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                ex.out.x[c][R][i][le] = x[i];
-                ex.out.y[c][R][i][le] = y[i];
-            }
-        };
-        put(0, f11, f12);
-        put(1, f12, f22);
-    } else {
-        double k0[3], k1[3], k2[3], k3[3], nq[3], a[3], b[3], s[3];
-        [[maybe_unused]] double mq[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const size_t q = 3 * R + i;
-            k0[i] = active ? geo.k[q * N + e] : 0.0;
-            k1[i] = active ? geo.k[(9 + q) * N + e] : 0.0;
-            k2[i] = active ? geo.k[(18 + q) * N + e] : 0.0;
-            k3[i] = active ? geo.k[(27 + q) * N + e] : 0.0;
-            nq[i] = active ? geo.n[q * N + e] : 0.0;
-            a[i] = fma(k0[i], uxi[i], k1[i] * uet[i]);
-            b[i] = fma(k2[i], vxi[i], k3[i] * vet[i]);
-            s[i] = fma(k2[i], uxi[i], fma(k3[i], uet[i], fma(k0[i], vxi[i], k1[i] * vet[i])));
-            if constexpr (GEO == SPHERE) {
-                mq[i] = active ? geo.m[q * N + e] : 0.0;
-                a[i] = fma(-mq[i], vp[i], a[i]);
-                s[i] = fma(mq[i], up[i], s[i]);
-            }
-        }
-        constexpr double nr = R == 1 ? -2.0 : 1.0; // nu on this row: nr, -2 nr, nr
-        // P: subtract n (nu . g)
-        double c[3] = { nr * fma(-2.0, a[1], a[0] + a[2]), nr * fma(-2.0, b[1], b[0] + b[2]),
-            nr * fma(-2.0, s[1], s[0] + s[2]) };
-        sumRows(sums[0], R, le, c);
-        double d[3] = { 0.0, 0.0, 0.0 };
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            pointStress64(fma(-c[0], nq[i], a[i]), fma(-c[1], nq[i], b[i]), fma(-c[2], nq[i], s[i]), pq[i], dminQ,
-                f11[i], f12[i], f22[i]);
-            d[0] = fma(nq[i], f11[i], d[0]);
-            d[1] = fma(nq[i], f22[i], d[1]);
-            d[2] = fma(nq[i], f12[i], d[2]);
-        }
-        // P^T: subtract nu (n . f)
-        sumRows(sums[1], R, le, d);
-        double t0[3], t1[3], t2[3], t3[3];
-        [[maybe_unused]] double mu[3], mv[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double w = i == 1 ? -2.0 * nr : nr;
-            f11[i] = fma(-w, d[0], f11[i]);
-            f22[i] = fma(-w, d[1], f22[i]);
-            f12[i] = fma(-w, d[2], f12[i]);
-            t0[i] = fma(k0[i], f11[i], k2[i] * f12[i]);
-            t1[i] = fma(k1[i], f11[i], k3[i] * f12[i]);
-            t2[i] = fma(k0[i], f12[i], k2[i] * f22[i]);
-            t3[i] = fma(k1[i], f12[i], k3[i] * f22[i]);
-            if constexpr (GEO == SPHERE) {
-                mu[i] = mq[i] * f12[i];
-                mv[i] = -mq[i] * f11[i];
-            }
-        }
-        auto put = [&](int c, const double (&tx)[3], const double (&ty)[3], [[maybe_unused]] const double (&tm)[3]) {
-            derivT(tx, x);
-            interpT(ty, y);
-            if constexpr (GEO == SPHERE) {
-                double z[3];
-                interpT(tm, z);
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-                    x[i] += z[i];
-            }
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                ex.out.x[c][R][i][le] = x[i];
-                ex.out.y[c][R][i][le] = y[i];
-            }
-        };
-        if constexpr (GEO == SPHERE) {
-            put(0, t0, t1, mu);
-            put(1, t2, t3, mv);
-        } else {
-            put(0, t0, t1, t0);
-            put(1, t2, t3, t2);
-        }
-    }
-}
-
 template <Geometry GEO>
-__global__ void __launch_bounds__(3 * kElems) kMevpStress(DevMesh m, StressGeometry geo, const double* __restrict__ u,
-    const double* __restrict__ v, const double* __restrict__ Pw, double* __restrict__ tdiv, double dminQ, double keep)
+__global__ void __launch_bounds__(3 * kElems) kMevpStress(DevMesh m, StressGeometry<double> geo,
+    const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ Pw,
+    double* __restrict__ tdiv, Rheology<double> rh, double keep)
 {
-    __shared__ Exchange ex;
+    __shared__ Exchange<double, kElems> ex;
     __shared__ double sums[GEO == RECT ? 1 : 2][3][3][kElems];
-    const int le = threadIdx.x % kElems, R = threadIdx.x / kElems;
-    const size_t N = m.N, e = blockIdx.x * size_t(kElems) + le;
-    const bool active = e < N && m.ice[e];
-    // everything the previous two launches do not write comes before the wait
-    // (the divergence was written two launches ago by this kernel and is only
-    // read by the node kernel in between)
-    double pq[3] = { 0.0, 0.0, 0.0 }, told[6], rho = 0.0;
-    if (active) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            pq[i] = Pw[(3 * R + i) * N + e];
-        if constexpr (GEO == RECT) {
-            rho = geo.k[e];
-            dminQ *= geo.k[N + e];
-        }
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            told[r] = tdiv[(3 * r + R) * N + e];
-            told[3 + r] = tdiv[(9 + 3 * r + R) * N + e];
-        }
-    }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    {
-        double n[2][3] = { { 0.0, 0.0, 0.0 }, { 0.0, 0.0, 0.0 } };
-        if (active) {
-            const unsigned s2 = 2u * static_cast<unsigned>(m.nx) + 1u;
-            const unsigned ix = static_cast<unsigned>(e) % static_cast<unsigned>(m.nx);
-            const unsigned iy = static_cast<unsigned>(e) / static_cast<unsigned>(m.nx);
-            const size_t base = 2 * size_t(s2) * iy + 2 * ix + R;
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                n[0][r] = u[base + size_t(r) * s2];
-                n[1][r] = v[base + size_t(r) * s2];
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            double vr[3], dr[3];
-            interpDeriv(n[c], vr, dr);
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                ex.in.v[c][r][R][le] = vr[r];
-                ex.in.dv[c][r][R][le] = dr[r];
-            }
-        }
-    }
-    __syncthreads();
-    switch (R) {
-    case 0: row64<0, GEO>(active, e, N, geo, pq, rho, dminQ, ex, sums, le); break;
-    case 1: row64<1, GEO>(active, e, N, geo, pq, rho, dminQ, ex, sums, le); break;
-    default: row64<2, GEO>(active, e, N, geo, pq, rho, dminQ, ex, sums, le); break;
-    }
-    __syncthreads();
-    if (!active)
-        return;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        double x[3], y[3], o[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            x[r] = ex.out.x[c][r][R][le];
-            y[r] = ex.out.y[c][r][R][le];
-        }
-        columnT(x, y, o);
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-            tdiv[(9 * c + 3 * r + R) * N + e] = fma(told[3 * c + r], keep, o[r]);
-    }
+    stressBlock<double, GEO, 0, kElems>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, rh, keep, blockIdx.x * size_t(kElems),
+        ex, sums);
 }
 
-} // namespace
-
-cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const StressGeometry& geo, const double* u,
-    const double* v, const double* Pw, double* tdiv, const MevpParams& pIn)
+// Mixed precision: FP32 velocities, divergence and arithmetic, Delta^2 and the
+// viscosity in float pairs.  Per element and iteration 260 bytes on
+// parallelograms (divergence 144, weighted pressure 72, coefficients 16, its
+// share of the velocities) and 430 on quadrilaterals (+ 180 of map, 216 on a
+// sphere), where the 9 x 9 operators were 1,580 (2,228).  Bound by L2 / HBM
+// traffic: 14.0 us for 512 x 512 parallelograms = 4.9 TB/s (24.9 us with dense
+// unit-square operators and the viscosity in FP64, which was bound by FP64
+// issue), 9.6 us for 384 x 320 quadrilaterals (42.7 us with TMA-staged
+// operators), 7.3 us for 301 x 257 cells of a sphere (38.6 us).
+template <Geometry GEO, int VM, int E>
+__global__ void __launch_bounds__(3 * E) kMevpStress32(DevMesh m, StressGeometry<float> geo,
+    const float* __restrict__ u, const float* __restrict__ v, const float2* __restrict__ Pw, float* __restrict__ tdiv,
+    Rheology<float> rh, float keep)
 {
-    const MevpParams p = withDerived(pIn);
-    const double dminQ = 0.25 * (p.DeltaMin * p.DeltaMin);
+    __shared__ Exchange<float, E> ex;
+    __shared__ float sums[GEO == AFFINE ? 1 : 2][3][3][E];
+    stressBlock<float, GEO, VM, E>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, rh, keep, blockIdx.x * size_t(E), ex, sums);
+}
+
+// One launch over the elements of every member of an ensemble: block b belongs
+// to member blockMember[b] and covers E consecutive elements of it.
+template <Geometry GEO, int VM, int E>
+__global__ void __launch_bounds__(3 * E) kMevpStress32Batched(const EnsembleMember* __restrict__ members,
+    const uint16_t* __restrict__ blockMember, Rheology<float> rh, float keep)
+{
+    __shared__ Exchange<float, E> ex;
+    __shared__ float sums[GEO == AFFINE ? 1 : 2][3][3][E];
+    const EnsembleMember& M = members[blockMember[blockIdx.x]];
+    const int b = static_cast<int>(blockIdx.x) - (GEO == AFFINE ? M.tmaBlock0 : M.stressBlock0);
+    stressBlock<float, GEO, VM, E>(M.nx, M.N, M.ice, GEO == AFFINE ? M.aff : M.quad, M.st.u, M.st.v, M.Pw, M.tdiv, rh,
+        keep, size_t(b) * E, ex, sums);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch(cudaStream_t s, void (*kernel)(KArgs...), size_t blocks, int threads, Args... args)
+{
     cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(static_cast<unsigned>((m.N + kElems - 1) / kElems));
-    cfg.blockDim = dim3(3 * kElems);
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+    cfg.blockDim = dim3(threads);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (geo.rect)
-        return cudaLaunchKernelEx(&cfg, kMevpStress<RECT>, m, geo, u, v, Pw, tdiv, dminQ, p.keepd);
-    if (geo.m)
-        return cudaLaunchKernelEx(&cfg, kMevpStress<SPHERE>, m, geo, u, v, Pw, tdiv, dminQ, p.keepd);
-    return cudaLaunchKernelEx(&cfg, kMevpStress<QUAD>, m, geo, u, v, Pw, tdiv, dminQ, p.keepd);
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+} // namespace
+
+cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const StressGeometry<double>& geo, const double* u,
+    const double* v, const double* Pw, double* tdiv, const MevpParams& pIn)
+{
+    const MevpParams p = withDerived(pIn);
+    const Rheology<double> rh { 0.25 * (p.DeltaMin * p.DeltaMin) };
+    const size_t blocks = (m.N + kElems - 1) / kElems;
+    auto kernel = geo.rect ? kMevpStress<RECT> : geo.m ? kMevpStress<SPHERE> : kMevpStress<QUAD>;
+    return launch(s, kernel, blocks, 3 * kElems, m, geo, u, v, Pw, tdiv, rh, p.keepd);
+}
+
+cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo, const float* u,
+    const float* v, const float2* Pw, float* tdiv, const MevpParams& pIn)
+{
+    const MevpParams p = withDerived(pIn);
+    const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
+    auto kernel = geo.m ? kMevpStress32<SPHERE, 3, kQuadElems> : kMevpStress32<QUAD, 3, kQuadElems>;
+    return launch(s, kernel, (m.N + kQuadElems - 1) / kQuadElems, 3 * kQuadElems, m, geo, u, v, Pw, tdiv, rh, p.keep);
+}
+
+cudaError_t launchMevpStress32Affine(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo,
+    const float* u, const float* v, const float2* Pw, float* tdiv, const MevpParams& pIn, int viscosityMode)
+{
+    const MevpParams p = withDerived(pIn);
+    const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
+    void (*kernels[5])(DevMesh, StressGeometry<float>, const float*, const float*, const float2*, float*,
+        Rheology<float>, float)
+        = { kMevpStress32<AFFINE, 0, kAffElems>, kMevpStress32<AFFINE, 1, kAffElems>,
+              kMevpStress32<AFFINE, 2, kAffElems>, kMevpStress32<AFFINE, 3, kAffElems>,
+              kMevpStress32<AFFINE, 4, kAffElems> };
+    const int vm = viscosityMode >= 0 && viscosityMode <= 4 ? viscosityMode : 3;
+    return launch(s, kernels[vm], (m.N + kAffElems - 1) / kAffElems, 3 * kAffElems, m, geo, u, v, Pw, tdiv, rh, p.keep);
+}
+
+cudaError_t launchMevpStress32Batched(cudaStream_t s, const EnsembleMember* members, const uint16_t* blockMember,
+    int blocks, const MevpParams& pIn)
+{
+    const MevpParams p = withDerived(pIn);
+    const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
+    return launch(s, kMevpStress32Batched<QUAD, 3, kQuadElems>, blocks, 3 * kQuadElems, members, blockMember, rh,
+        p.keep);
+}
+
+cudaError_t launchMevpStress32AffineBatched(cudaStream_t s, const EnsembleMember* members,
+    const uint16_t* blockMember, int blocks, const MevpParams& pIn, int viscosityMode)
+{
+    const MevpParams p = withDerived(pIn);
+    const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
+    void (*kernels[5])(const EnsembleMember*, const uint16_t*, Rheology<float>, float)
+        = { kMevpStress32Batched<AFFINE, 0, kAffElems>, kMevpStress32Batched<AFFINE, 1, kAffElems>,
+              kMevpStress32Batched<AFFINE, 2, kAffElems>, kMevpStress32Batched<AFFINE, 3, kAffElems>,
+              kMevpStress32Batched<AFFINE, 4, kAffElems> };
+    const int vm = viscosityMode >= 0 && viscosityMode <= 4 ? viscosityMode : 3;
+    return launch(s, kernels[vm], blocks, 3 * kAffElems, members, blockMember, rh, p.keep);
 }
 
 } // namespace nsdg

@@ -34,6 +34,7 @@
 
 #include "nsdg_kernels.hpp"
 #include "nsdg_seed64.cuh"
+#include "nsdg_viscosity.cuh"
 
 namespace nsdg {
 namespace sf {
@@ -144,15 +145,36 @@ __device__ __forceinline__ double minusHalf(double x)
     return hi >= (2 << 20) ? __hiloint2double((hi - (1 << 20)) | static_cast<int>(0x80000000u), __double2loint(x)) : 0.0;
 }
 
+// How an element's map is given: one pair (k_y / k_x, 1 / k_x^2) on
+// rectangles, four derivatives on parallelograms, four per Gauss point else.
+enum Geometry { RECT = 0, AFFINE = 1, QUAD = 2, SPHERE = 3 };
+
+// What the stress increments take besides the strain: the weighted pressure
+// pq = w P / (4 alpha) (FP32 kernels: as a pair of floats, 48 bits) and
+// DeltaMin^2.
+template <typename T> struct Rheology;
+template <> struct Rheology<double> {
+    using Weight = double;
+    double dminQ; // DeltaMin^2 / 4
+    static __device__ __forceinline__ double none() { return 0.0; }
+};
+template <> struct Rheology<float> {
+    using Weight = float2;
+    float d2h, d2l; // DeltaMin^2 as a pair of floats
+    double dmin;
+    static __device__ __forceinline__ float2 none() { return make_float2(0.f, 0.f); }
+};
+
 // The stress increments (times the weight in pq) of one Gauss point:
 // f11, f12, f22 of P/(8 alpha Delta) (5 e11 + 3 e22) - P/(2 alpha) etc. from
 // a = e11/2, b = e22/2, s = e12 and Delta^2 = DeltaMin^2 + 4 (a + b)^2 + (a - b)^2 + s^2
-// (MEVPStressUpdateStep.hpp:63-77, 80-116).  dminQ = DeltaMin^2 / 4.
-__device__ __forceinline__ void pointStress64(double a, double b, double s, double pq, double dminQ, double& f11,
-    double& f12, double& f22)
+// (MEVPStressUpdateStep.hpp:63-77, 80-116).
+template <int VM>
+__device__ __forceinline__ void pointStress(double a, double b, double s, double pq, const Rheology<double>& rh,
+    double& f11, double& f12, double& f22)
 {
     const double pl = a + b, mi = a - b;
-    const double t = fma(4.0, fma(pl, pl, dminQ), fma(mi, mi, s * s));
+    const double t = fma(4.0, fma(pl, pl, rh.dminQ), fma(mi, mi, s * s));
     const double z = timesRsqrt64(pq, t); // 2 P / (8 alpha Delta), weighted
     const double w = fma(z, pl, minusHalf(pq));
     const double d = z * mi;
@@ -160,9 +182,307 @@ __device__ __forceinline__ void pointStress64(double a, double b, double s, doub
     f11 = fma(4.0, w, d);
     f22 = fma(4.0, w, -d);
 }
+// FP32: the invariant is a sum of squares (no cancellation); Delta^2 and the
+// viscosity in float pairs (VM 3, the default) or in FP64 (VM 0, 1, 2; 4 is
+// 3 checked against 2)
+template <int VM>
+__device__ __forceinline__ void pointStress(float a, float b, float s, float2 pq, const Rheology<float>& rh,
+    float& f11, float& f12, float& f22)
+{
+    const float pl = a + b, mi = a - b;
+    const float inv = fmaf(4.f * pl, pl, fmaf(mi, mi, s * s));
+    float z;
+    if constexpr (VM == 3)
+        z = nsdg_ff::viscPair(inv, pq.x, pq.y, rh.d2h, rh.d2l, rsqrtf(inv + rh.d2h));
+    else
+        z = viscosity8<VM>(inv, static_cast<double>(pq.x) + static_cast<double>(pq.y), rh.dmin, rh.d2h, rh.d2l);
+    const float w = fmaf(z, pl, -0.5f * pq.x);
+    const float d = z * mi;
+    f12 = z * s;
+    f11 = fmaf(4.f, w, d);
+    f22 = fmaf(4.f, w, -d);
+}
 
-// How an element's map is given.
-enum Geometry { RECT = 0, QUAD = 1, SPHERE = 2 };
+// One mEVP iteration in divergence space: tdiv <- (1 - 1/alpha) tdiv +
+// K^T P^T f(P K u).  Three threads per element, in three warps of a block of
+// E elements: warp R takes node column R (the eta maps of its three
+// nodes), then Gauss row R (the xi maps, strain, stress increments, the
+// transposed xi maps), then node column R again (the transposed eta maps); the
+// 24 and 36 values in between go through shared memory, as do the sums of the
+// two projections on general quadrilaterals.
+//
+// On rectangles the strain is carried over k_x (strain' = strain / k_x, the
+// eta derivatives times rho = k_y / k_x, DeltaMin^2 over k_x^2) and k_x is
+// part of the pressure's weight, so only rho is multiplied in.
+template <typename T, int E> struct Exchange {
+    union {
+        struct {
+            T v[2][3][3][E];  // [u, v][Gauss row][column]: values on the columns
+            T dv[2][3][3][E]; // eta derivatives
+        } in;
+        struct {
+            T x[2][3][3][E]; // to the transposed interpolation
+            T y[2][3][3][E]; // to the transposed derivative
+        } out;
+    };
+};
+
+// The block's three warps meet here from different instances of the row code:
+// a barrier by its number (PTX bar.sync counts warps, whatever their place in
+// the code).
+template <int E> __device__ __forceinline__ void rowsBarrier()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(3 * E) : "memory");
+}
+
+// sum over the element's three warps of each thread's c[0..2]
+template <typename T, int E>
+__device__ __forceinline__ void sumRows(T (*part)[3][E], int R, int le, T (&c)[3])
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        part[R][k][le] = c[k];
+    rowsBarrier<E>();
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        c[k] = part[0][k][le] + part[1][k][le] + part[2][k][le];
+}
+
+template <int R, typename T, Geometry GEO, int VM, int E>
+__device__ __forceinline__ void gaussRow(bool active, size_t e, size_t N, const StressGeometry<T>& geo,
+    const typename Rheology<T>::Weight (&pq)[3], const T (&ke)[4], const Rheology<T>& rh, Exchange<T, E>& ex,
+    T (*sums)[3][3][E], int le)
+{
+    T I[3], D[3], uxi[3], uet[3], vxi[3], vet[3], f11[3], f12[3], f22[3], x[3], y[3];
+    [[maybe_unused]] T up[3], vp[3];
+    const Scaled<T> sc(GEO == RECT ? ke[0] : T(1));
+    auto take = [&](int c) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            I[i] = ex.in.v[c][R][i][le];
+            D[i] = ex.in.dv[c][R][i][le];
+        }
+    };
+    take(0);
+    deriv(I, uxi);
+    if constexpr (GEO == RECT)
+        sc.interp(D, uet);
+    else
+        interp(D, uet);
+    if constexpr (GEO == SPHERE)
+        interp(I, up);
+    take(1);
+    deriv(I, vxi);
+    if constexpr (GEO == RECT)
+        sc.interp(D, vet);
+    else
+        interp(D, vet);
+    if constexpr (GEO == SPHERE)
+        interp(I, vp);
+    if constexpr (GEO == RECT) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            pointStress<VM>(uxi[i], vet[i], uet[i] + vxi[i], pq[i], rh, f11[i], f12[i], f22[i]);
+        rowsBarrier<E>(); // every warp has taken its row: the buffer changes hands
+        auto put = [&](int c, const T (&fx)[3], const T (&fy)[3]) {
+            derivT(fx, x);
+            sc.interpT(fy, y);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                ex.out.x[c][R][i][le] = x[i];
+                ex.out.y[c][R][i][le] = y[i];
+            }
+        };
+        put(0, f11, f12);
+        put(1, f12, f22);
+    } else if constexpr (GEO == AFFINE) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            pointStress<VM>(fmaT(ke[0], uxi[i], ke[1] * uet[i]), fmaT(ke[2], vxi[i], ke[3] * vet[i]),
+                fmaT(ke[2], uxi[i], fmaT(ke[3], uet[i], fmaT(ke[0], vxi[i], ke[1] * vet[i]))), pq[i], rh, f11[i],
+                f12[i], f22[i]);
+        rowsBarrier<E>();
+        auto put = [&](int c, const T (&f)[3], const T (&h)[3]) {
+            T p[3], q[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                p[i] = fmaT(ke[0], f[i], ke[2] * h[i]);
+                q[i] = fmaT(ke[1], f[i], ke[3] * h[i]);
+            }
+            derivT(p, x);
+            interpT(q, y);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                ex.out.x[c][R][i][le] = x[i];
+                ex.out.y[c][R][i][le] = y[i];
+            }
+        };
+        put(0, f11, f12);
+        put(1, f12, f22);
+    } else {
+        T k0[3], k1[3], k2[3], k3[3], nq[3], a[3], b[3], s[3];
+        [[maybe_unused]] T mq[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const size_t q = 3 * R + i;
+            k0[i] = active ? geo.k[q * N + e] : T(0);
+            k1[i] = active ? geo.k[(9 + q) * N + e] : T(0);
+            k2[i] = active ? geo.k[(18 + q) * N + e] : T(0);
+            k3[i] = active ? geo.k[(27 + q) * N + e] : T(0);
+            nq[i] = active ? geo.n[q * N + e] : T(0);
+            a[i] = fmaT(k0[i], uxi[i], k1[i] * uet[i]);
+            b[i] = fmaT(k2[i], vxi[i], k3[i] * vet[i]);
+            s[i] = fmaT(k2[i], uxi[i], fmaT(k3[i], uet[i], fmaT(k0[i], vxi[i], k1[i] * vet[i])));
+            if constexpr (GEO == SPHERE) {
+                mq[i] = active ? geo.m[q * N + e] : T(0);
+                a[i] = fmaT(-mq[i], vp[i], a[i]);
+                s[i] = fmaT(mq[i], up[i], s[i]);
+            }
+        }
+        constexpr T nr = R == 1 ? T(-2) : T(1); // nu on this row: nr, -2 nr, nr
+        // P: subtract n (nu . g)
+        T c[3] = { nr * fmaT(T(-2), a[1], a[0] + a[2]), nr * fmaT(T(-2), b[1], b[0] + b[2]),
+            nr * fmaT(T(-2), s[1], s[0] + s[2]) };
+        sumRows<T, E>(sums[0], R, le, c);
+        T d[3] = { T(0), T(0), T(0) };
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            pointStress<VM>(fmaT(-c[0], nq[i], a[i]), fmaT(-c[1], nq[i], b[i]), fmaT(-c[2], nq[i], s[i]), pq[i], rh,
+                f11[i], f12[i], f22[i]);
+            d[0] = fmaT(nq[i], f11[i], d[0]);
+            d[1] = fmaT(nq[i], f22[i], d[1]);
+            d[2] = fmaT(nq[i], f12[i], d[2]);
+        }
+        // P^T: subtract nu (n . f)
+        sumRows<T, E>(sums[1], R, le, d);
+        T t0[3], t1[3], t2[3], t3[3];
+        [[maybe_unused]] T mu[3], mv[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const T w = i == 1 ? T(-2) * nr : nr;
+            f11[i] = fmaT(-w, d[0], f11[i]);
+            f22[i] = fmaT(-w, d[1], f22[i]);
+            f12[i] = fmaT(-w, d[2], f12[i]);
+            t0[i] = fmaT(k0[i], f11[i], k2[i] * f12[i]);
+            t1[i] = fmaT(k1[i], f11[i], k3[i] * f12[i]);
+            t2[i] = fmaT(k0[i], f12[i], k2[i] * f22[i]);
+            t3[i] = fmaT(k1[i], f12[i], k3[i] * f22[i]);
+            if constexpr (GEO == SPHERE) {
+                mu[i] = mq[i] * f12[i];
+                mv[i] = -mq[i] * f11[i];
+            }
+        }
+        auto put = [&](int c, const T (&tx)[3], const T (&ty)[3], [[maybe_unused]] const T (&tm)[3]) {
+            derivT(tx, x);
+            interpT(ty, y);
+            if constexpr (GEO == SPHERE) {
+                T z[3];
+                interpT(tm, z);
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    x[i] += z[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                ex.out.x[c][R][i][le] = x[i];
+                ex.out.y[c][R][i][le] = y[i];
+            }
+        };
+        if constexpr (GEO == SPHERE) {
+            put(0, t0, t1, mu);
+            put(1, t2, t3, mv);
+        } else {
+            put(0, t0, t1, t0);
+            put(1, t2, t3, t2);
+        }
+    }
+}
+
+// The block of elements x0 .. x0 + E - 1 of a grid of nx cells per row.
+// Launched as a programmatic dependent of the node kernel: what the previous
+// two launches do not write is loaded before the wait (the divergence was
+// written two launches ago by this kernel, and the node kernel in between,
+// which waited for it, only reads it).
+template <typename T, Geometry GEO, int VM, int E>
+__device__ __forceinline__ void stressBlock(int nx, size_t N, const uint8_t* __restrict__ ice,
+    const StressGeometry<T>& geo, const T* __restrict__ u, const T* __restrict__ v,
+    const typename Rheology<T>::Weight* __restrict__ Pw, T* __restrict__ tdiv, Rheology<T> rh, T keep, size_t x0,
+    Exchange<T, E>& ex, T (*sums)[3][3][E])
+{
+    const int le = threadIdx.x % E, R = threadIdx.x / E; // R is the same in a warp
+    const size_t e = x0 + le;
+    const bool active = e < N && ice[e];
+    typename Rheology<T>::Weight pq[3];
+    T told[6], ke[4] = { T(0), T(0), T(0), T(0) };
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        pq[i] = Rheology<T>::none();
+    if (active) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            pq[i] = Pw[(3 * R + i) * N + e];
+        if constexpr (GEO == RECT) {
+            ke[0] = geo.k[e];
+            rh.dminQ *= geo.k[N + e];
+        }
+        if constexpr (GEO == AFFINE)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                ke[c] = geo.k[c * N + e];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            told[r] = tdiv[(3 * r + R) * N + e];
+            told[3 + r] = tdiv[(9 + 3 * r + R) * N + e];
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    {
+        T n[2][3] = { { T(0), T(0), T(0) }, { T(0), T(0), T(0) } };
+        if (active) {
+            const unsigned s2 = 2u * static_cast<unsigned>(nx) + 1u;
+            const unsigned ix = static_cast<unsigned>(e) % static_cast<unsigned>(nx);
+            const unsigned iy = static_cast<unsigned>(e) / static_cast<unsigned>(nx);
+            const size_t base = 2 * size_t(s2) * iy + 2 * ix + R;
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                n[0][r] = u[base + size_t(r) * s2];
+                n[1][r] = v[base + size_t(r) * s2];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            T vr[3], dr[3];
+            interpDeriv(n[c], vr, dr);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                ex.in.v[c][r][R][le] = vr[r];
+                ex.in.dv[c][r][R][le] = dr[r];
+            }
+        }
+    }
+    __syncthreads();
+    switch (R) {
+    case 0: gaussRow<0, T, GEO, VM, E>(active, e, N, geo, pq, ke, rh, ex, sums, le); break;
+    case 1: gaussRow<1, T, GEO, VM, E>(active, e, N, geo, pq, ke, rh, ex, sums, le); break;
+    default: gaussRow<2, T, GEO, VM, E>(active, e, N, geo, pq, ke, rh, ex, sums, le); break;
+    }
+    __syncthreads();
+    if (!active)
+        return;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        T x[3], y[3], o[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            x[r] = ex.out.x[c][r][R][le];
+            y[r] = ex.out.y[c][r][R][le];
+        }
+        columnT(x, y, o);
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            tdiv[(9 * c + 3 * r + R) * N + e] = fmaT(told[3 * c + r], keep, o[r]);
+    }
+}
 
 } // namespace sf
 } // namespace nsdg

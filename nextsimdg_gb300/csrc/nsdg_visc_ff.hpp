@@ -204,6 +204,26 @@ NSDG_FF_HD float viscFloatFloat(float inv, double Pa, float d2h, float d2l, floa
     return z >= 0x1p-126f ? z : 0.f;
 }
 
+// The float-float form for a numerator given as a pair ph + pl (ph the nearest
+// float, pl the nearest float to the rest), as the sum-factorised stress
+// kernels keep it: no FP64 operation.
+NSDG_FF_HD float viscPair(float inv, float ph, float pl, float d2h, float d2l, float y0)
+{
+    const float th = add(inv, d2h);
+    const float bv = sub(th, inv);
+    const float av = sub(th, bv);
+    const float tl = add(add(sub(inv, av), sub(d2h, bv)), d2l);
+    const float p = mul(y0, y0);
+    const float pe = fma(y0, y0, -p);
+    const float q = mul(th, p);
+    const float qe = fma(th, p, -q);
+    const float r = fma(-tl, p, fma(-th, pe, sub(sub(1.f, q), qe)));
+    const float yl = mul(mul(y0, r), 0.5f);
+    const float m = mul(ph, y0);
+    const float me = fma(ph, y0, -m);
+    return add(m, fma(ph, yl, fma(pl, y0, me)));
+}
+
 // The float-float form with a check that its result is bitwise the FP64
 // form's (viscNewton64 with the same seed).  Error bounds, relative to z, for
 // a seed with |r| = |1 - t y0^2| <= 2^-19 (rsqrtf's seed: about 2^-21):

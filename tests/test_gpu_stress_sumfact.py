@@ -4,7 +4,7 @@ a sphere, with land cells, at sizes around the kernels' blocks of 32 elements.""
 import numpy as np
 import pytest
 
-from nextsimdg_gb300.dynamics import MEVPDynamicsKernel
+from nextsimdg_gb300.dynamics import Ensemble, MEVPDynamicsKernel
 from test_stress_metric import _coords
 
 pytestmark = pytest.mark.gpu
@@ -34,3 +34,37 @@ def test_fp64_matches_oracle(gpu, oracle, kind, nx, ny, dg):
     ref = _step(oracle.OracleKernel(0, dg, n_steps=60), kind, nx, ny)
     for name, r in ref.items():
         assert np.abs(got[name] - r).max() <= 1e-10 * max(np.abs(r).max(), 1e-300), name
+
+
+@pytest.mark.parametrize("kind", ["box", "stretched", "sheared", "quads", "sphere"])
+@pytest.mark.parametrize("nx,ny,dg", [(2, 3, 6), (11, 3, 3), (16, 8, 1), (33, 29, 6)])
+def test_mixed_within_the_mixed_bars(gpu, oracle, kind, nx, ny, dg):
+    """The mixed path's bars: velocity 1e-5 m/s, h and A 1e-6 (RMS)."""
+    k = MEVPDynamicsKernel(dg_comp=dg, n_steps=60, precision=1)
+    got = _step(k, kind, nx, ny)
+    ref = _step(oracle.OracleKernel(0, dg, n_steps=60), kind, nx, ny)
+    assert k.stress_variant()[0] == ("global" if kind in ("quads", "sphere") else "affine")
+    for name, bar in (("u", 1e-5), ("v", 1e-5), ("hice", 1e-6), ("cice", 1e-6)):
+        assert np.sqrt(np.mean((got[name] - ref[name]) ** 2)) <= bar, name
+
+
+@pytest.mark.parametrize("kinds", [("quads", "box"), ("quads", "sheared"), ("stretched", "sheared")])
+def test_ensemble_of_mixed_geometries(gpu, kinds):
+    """An ensemble whose members have different maps: bitwise the members'
+    single runs where one kernel serves all members in both, else within FP32
+    rounding of them (1e-5 m/s after two steps)."""
+    sizes = [(13, 11), (37, 9)]
+    ref = [_step(MEVPDynamicsKernel(dg_comp=3, n_steps=60, precision=1), k, *s) for k, s in zip(kinds, sizes)]
+    members = [MEVPDynamicsKernel(dg_comp=3, n_steps=60, precision=1) for _ in kinds]
+    for m, k, s in zip(members, kinds, sizes):
+        _step(m, k, *s, steps=0)
+    ens = Ensemble(members)
+    for i in range(2):
+        ens.update(120.0 * i, 120.0)
+    ens.synchronize()
+    for m, r in zip(members, ref):
+        for name in ("u", "v"):
+            d = m.getDG0Data(name) - r[name]
+            if "quads" not in kinds:
+                assert np.all(d == 0.0), name
+            assert np.sqrt(np.mean(d * d)) <= 1e-5, name
