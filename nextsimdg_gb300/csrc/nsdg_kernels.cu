@@ -1494,12 +1494,15 @@ __device__ __forceinline__ void gatherDivergence(const DevMesh& m, int i2, int j
 }
 
 // The FP64 node update, divided through by c1 = rho H / dt (kMevpPrepNodes):
-//   u_new = (beta u + ku + a |u_o - u| u_o - fc dt u + im dSx) / (1 + beta + a |u_o - u|)
-// and likewise v with + fc dt v (VPCGDynamicsKernel.hpp:132-172).  Bound by
-// FP64 issue: about 28 FP64 instructions per node, with the square root and
+//   u_new = (beta u + ku + f u_o - fc dt u + im dSx) / (1 + beta + f),  f = a |u_o - u|,
+// and likewise v with + fc dt v (VPCGDynamicsKernel.hpp:132-172), as the
+// increment (ku + f u_o + im dSx - (1 + f + fc dt) u) / (1 + beta + f): a
+// rounding of the factors then acts on the increment, where in the quotient
+// it would act on u in each of the iterations with the same sign.  Bound by
+// FP64 issue: about 30 FP64 instructions per node, with the square root and
 // the reciprocal from FP32 seeds (CUDA's were more than half of the 60
-// before); 513 x 513 nodes 17.7 us instead of 26.8 us, 129 x 129
-// 2.9 us instead of 6.2 us (latency of the dependent chain).
+// before); 513 x 513 nodes 18.6 us instead of 26.8 us, 129 x 129
+// 3.0 us instead of 6.2 us (latency of the dependent chain).
 __global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, MevpNodeState st,
     const double* __restrict__ contrib, MevpParams p, int* __restrict__ err)
 {
@@ -1521,8 +1524,8 @@ __global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, MevpNodeState
     const double ur = uo - u, vr = vo - v;
     const double f = a * sf::sqrt64(fma(ur, ur, vr * vr));
     const double rden = sf::recip64(p.onePlusBeta + f);
-    double un = rden * fma(p.betaMinus, u, fma(f, uo, fma(dSx, im, ku)));
-    double vn = rden * fma(p.betaPlus, v, fma(f, vo, fma(dSy, im, kv)));
+    double un = fma(rden, fma(-(p.onePlusFc + f), u, fma(f, uo, fma(dSx, im, ku))), u);
+    double vn = fma(rden, fma(-(p.oneMinusFc + f), v, fma(f, vo, fma(dSy, im, kv))), v);
     if (!isfinite(un) || !isfinite(vn))
         atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
     if (dir) {
@@ -1829,9 +1832,10 @@ __device__ __forceinline__ void mevpMomentum32Node(int nx, int ny, size_t N, siz
     const float uOcnRel = uo - u, vOcnRel = v - vo;
     const float afocn = a * (p.F_oceanf * sqrtf(uOcnRel * uOcnRel + vOcnRel * vOcnRel));
     const float rden = 1.0f / (p.onePlusBetaf + afocn);
-    // (beta u + ku + a focn uo - fc dt u + mx) / (1 + beta + a focn), VPCGDynamicsKernel.hpp:132-172 over c1
-    float un = rden * (p.betaf * u + ku + afocn * uo - p.fcdtf * u + mx);
-    float vn = rden * (p.betaf * v + kv + afocn * vo + p.fcdtf * v + my);
+    // (beta u + ku + a focn uo - fc dt u + mx) / (1 + beta + a focn), VPCGDynamicsKernel.hpp:132-172 over c1,
+    // as the increment of u (kMevpMomentum)
+    float un = fmaf(rden, fmaf(-(p.onePlusFcf + afocn), u, fmaf(afocn, uo, ku + mx)), u);
+    float vn = fmaf(rden, fmaf(-(p.oneMinusFcf + afocn), v, fmaf(afocn, vo, kv + my)), v);
     if (!isfinite(un) || !isfinite(vn))
         atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
     if (dir) {

@@ -160,24 +160,24 @@ struct MevpParams {
     // no thread spends FP64 instructions (about 1/60 of the FP32 rate on
     // GB300) on a division or a square of the parameters
     double keepd = 0;                          // 1 - 1/alpha
-    double onePlusBeta = 0, betaMinus = 0, betaPlus = 0; // 1 + beta, beta -+ fc dt
+    double onePlusBeta = 0, onePlusFc = 0, oneMinusFc = 0; // 1 + beta, 1 +- fc dt
     float keep = 0, dmin2f = 0, F_oceanf = 0;  // FP32 copies (dmin2f: DeltaMin^2)
     float dmin2lo = 0;                         // DeltaMin^2 - dmin2f (its float-pair low part)
-    float betaf = 0, onePlusBetaf = 0, fcdtf = 0; // beta, 1 + beta, fc dt
+    float onePlusBetaf = 0, onePlusFcf = 0, oneMinusFcf = 0;
 };
 inline MevpParams withDerived(MevpParams p)
 {
     p.keepd = 1.0 - 1.0 / p.alpha;
     p.onePlusBeta = 1.0 + p.beta;
-    p.betaMinus = p.beta - p.fc * p.dt;
-    p.betaPlus = p.beta + p.fc * p.dt;
+    p.onePlusFc = 1.0 + p.fc * p.dt;
+    p.oneMinusFc = 1.0 - p.fc * p.dt;
     p.keep = static_cast<float>(p.keepd);
     p.dmin2f = static_cast<float>(p.DeltaMin * p.DeltaMin);
     p.dmin2lo = static_cast<float>(std::fma(p.DeltaMin, p.DeltaMin, -static_cast<double>(p.dmin2f)));
     p.F_oceanf = static_cast<float>(p.F_ocean);
-    p.betaf = static_cast<float>(p.beta);
     p.onePlusBetaf = static_cast<float>(1.0 + p.beta);
-    p.fcdtf = static_cast<float>(p.fc * p.dt);
+    p.onePlusFcf = static_cast<float>(p.onePlusFc);
+    p.oneMinusFcf = static_cast<float>(p.oneMinusFc);
     return p;
 }
 cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* invm2,
