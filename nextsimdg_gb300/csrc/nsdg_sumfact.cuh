@@ -227,14 +227,6 @@ template <typename T, int E> struct Exchange {
     };
 };
 
-// The block's three warps meet here from different instances of the row code:
-// a barrier by its number (PTX bar.sync counts warps, whatever their place in
-// the code).
-template <int E> __device__ __forceinline__ void rowsBarrier()
-{
-    asm volatile("bar.sync 1, %0;" ::"n"(3 * E) : "memory");
-}
-
 // sum over the element's three warps of each thread's c[0..2]
 template <typename T, int E>
 __device__ __forceinline__ void sumRows(T (*part)[3][E], int R, int le, T (&c)[3])
@@ -242,14 +234,14 @@ __device__ __forceinline__ void sumRows(T (*part)[3][E], int R, int le, T (&c)[3
 #pragma unroll
     for (int k = 0; k < 3; ++k)
         part[R][k][le] = c[k];
-    rowsBarrier<E>();
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < 3; ++k)
         c[k] = part[0][k][le] + part[1][k][le] + part[2][k][le];
 }
 
-template <int R, typename T, Geometry GEO, int VM, int E>
-__device__ __forceinline__ void gaussRow(bool active, size_t e, size_t N, const StressGeometry<T>& geo,
+template <typename T, Geometry GEO, int VM, int E>
+__device__ __forceinline__ void gaussRow(int R, bool active, size_t e, size_t N, const StressGeometry<T>& geo,
     const typename Rheology<T>::Weight (&pq)[3], const T (&ke)[4], const Rheology<T>& rh, Exchange<T, E>& ex,
     T (*sums)[3][3][E], int le)
 {
@@ -283,7 +275,7 @@ __device__ __forceinline__ void gaussRow(bool active, size_t e, size_t N, const 
 #pragma unroll
         for (int i = 0; i < 3; ++i)
             pointStress<VM>(uxi[i], vet[i], uet[i] + vxi[i], pq[i], rh, f11[i], f12[i], f22[i]);
-        rowsBarrier<E>(); // every warp has taken its row: the buffer changes hands
+        __syncthreads(); // every warp has taken its row: the buffer changes hands
         auto put = [&](int c, const T (&fx)[3], const T (&fy)[3]) {
             derivT(fx, x);
             sc.interpT(fy, y);
@@ -301,7 +293,7 @@ __device__ __forceinline__ void gaussRow(bool active, size_t e, size_t N, const 
             pointStress<VM>(fmaT(ke[0], uxi[i], ke[1] * uet[i]), fmaT(ke[2], vxi[i], ke[3] * vet[i]),
                 fmaT(ke[2], uxi[i], fmaT(ke[3], uet[i], fmaT(ke[0], vxi[i], ke[1] * vet[i]))), pq[i], rh, f11[i],
                 f12[i], f22[i]);
-        rowsBarrier<E>();
+        __syncthreads();
         auto put = [&](int c, const T (&f)[3], const T (&h)[3]) {
             T p[3], q[3];
 #pragma unroll
@@ -339,7 +331,7 @@ __device__ __forceinline__ void gaussRow(bool active, size_t e, size_t N, const 
                 s[i] = fmaT(mq[i], up[i], s[i]);
             }
         }
-        constexpr T nr = R == 1 ? T(-2) : T(1); // nu on this row: nr, -2 nr, nr
+        const T nr = R == 1 ? T(-2) : T(1); // nu on this row: nr, -2 nr, nr
         // P: subtract n (nu . g)
         T c[3] = { nr * fmaT(T(-2), a[1], a[0] + a[2]), nr * fmaT(T(-2), b[1], b[0] + b[2]),
             nr * fmaT(T(-2), s[1], s[0] + s[2]) };
@@ -461,11 +453,7 @@ __device__ __forceinline__ void stressBlock(int nx, size_t N, const uint8_t* __r
         }
     }
     __syncthreads();
-    switch (R) {
-    case 0: gaussRow<0, T, GEO, VM, E>(active, e, N, geo, pq, ke, rh, ex, sums, le); break;
-    case 1: gaussRow<1, T, GEO, VM, E>(active, e, N, geo, pq, ke, rh, ex, sums, le); break;
-    default: gaussRow<2, T, GEO, VM, E>(active, e, N, geo, pq, ke, rh, ex, sums, le); break;
-    }
+    gaussRow<T, GEO, VM, E>(R, active, e, N, geo, pq, ke, rh, ex, sums, le);
     __syncthreads();
     if (!active)
         return;
