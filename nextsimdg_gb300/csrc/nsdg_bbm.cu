@@ -1,0 +1,725 @@
+// nsdg_bbm.cu — the brittle (BBM) sub-cycle (BBMStressUpdateStep.hpp:31-195,
+// BrittleCGDynamicsKernel.hpp:206-254).
+//
+// Through the sub-steps of a model step the stress and the damage are kept as
+// their values at the 3 x 3 Gauss points instead of 8 and DG coefficients.
+// The update works on point values, and the projection back onto the modes is
+// all that a sub-step needs of the coefficients:
+//   stress   g <- P f,  P = I - n nu^T   (nsdg_sumfact.cuh: one rank is lost)
+//   damage   d <- Psi (Psi^T W Psi)^{-1} Psi^T W d
+// Point values of a field in the modes' span and its coefficients carry the
+// same information, so kBbmLoad forms the values once per step and kBbmStore
+// the coefficients.  Thickness and concentration do not change through the
+// sub-steps either: the terms formed from them (exponentials, powers, roots)
+// are six constants per point and step.
+#include <cmath>
+#include <type_traits>
+
+#include "nsdg_nodes.cuh"
+#include "nsdg_sumfact.cuh"
+
+namespace nsdg {
+namespace {
+
+using namespace sf;
+
+// x^y for x >= 0: by multiplication when y is a small integer (mode 1), times
+// sqrt(x) when it is a small half-integer (mode 2), else pow().  Differs from
+// pow() by a few ulps.
+template <typename T> __device__ __forceinline__ T powByMode(T x, T y, int mode, int k)
+{
+    if (mode == 0)
+        return pow(x, y);
+    T r = T(1);
+    for (int i = 0; i < k; ++i)
+        r *= x;
+    return mode == 2 ? r * sqrt(x) : r;
+}
+
+// 1-D Gauss weights and points on [-1/2, 1/2], Legendre mode 2 there
+constexpr double kG = 0.38729833462074168852;
+constexpr double kL2Norm = 1. / 180.; // sum w L2^2
+__host__ __device__ constexpr double kW(int i) { return i == 1 ? 8. / 18. : 5. / 18.; }
+__host__ __device__ constexpr double kX(int i) { return i == 0 ? -kG : i == 1 ? 0.0 : kG; }
+__host__ __device__ constexpr double kL2(int i) { return (i == 1 ? 0.0 : 0.15) - 1. / 12.; }
+__host__ __device__ constexpr double kN(int i) { return i == 1 ? -5. / 18. : 2. / 9.; } // (nu / w) / sum(nu^2 / w)
+
+// DG mode j (x-y degrees) at Gauss point (ix, iy) and 1 / (its squared norm)
+__device__ constexpr int modeX(int j) { return j == 1 || j == 5 || j == 7 ? 1 : j == 3 || j == 6 ? 2 : 0; }
+__device__ constexpr int modeY(int j) { return j == 2 || j == 5 || j == 6 ? 1 : j == 4 || j == 7 ? 2 : 0; }
+__device__ __forceinline__ constexpr double leg(int n, int i) { return n == 0 ? 1.0 : n == 1 ? kX(i) : kL2(i); }
+__device__ __forceinline__ constexpr double psiAt(int j, int q) { return leg(modeX(j), q % 3) * leg(modeY(j), q / 3); }
+__device__ __forceinline__ constexpr double invNorm(int n) { return n == 0 ? 1.0 : n == 1 ? 12.0 : 180.0; }
+__device__ __forceinline__ constexpr double invNormOf(int j) { return invNorm(modeX(j)) * invNorm(modeY(j)); }
+
+// Step constants and point values from the advected fields.
+template <typename T, int DG>
+__global__ void __launch_bounds__(128) kBbmLoad(size_t N, const double* __restrict__ h, const double* __restrict__ a,
+    const double* __restrict__ damage, const double* __restrict__ s11, const double* __restrict__ s12,
+    const double* __restrict__ s22, const double* __restrict__ hsize, const double* __restrict__ invKx2,
+    BbmPoints<T> pt, BbmParams p)
+{
+    const size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if (e >= N)
+        return;
+    double hc[DG], ac[DG], dc[DG];
+#pragma unroll
+    for (int j = 0; j < DG; ++j) {
+        hc[j] = h[j * N + e];
+        ac[j] = a[j * N + e];
+        dc[j] = damage[j * N + e];
+    }
+    const double size = hsize[e];
+    const double sizeScale = sqrt(0.1 / size);
+    // relax = (1 - dcrit) dt / td, td = size sqrt(2 (1 + nu0) rho) / sqrt(elasticity)
+    const double relaxScale = p.dt / (size * sqrt(2. * (1. + p.nu0) * p.rho_ice));
+    // the kernels' half strains, over k_x on rectangles
+    const double strain = (invKx2 ? 2. / sqrt(invKx2[e]) : 2.) * p.dt * p.young / (1. - p.nu0 * p.nu0);
+#pragma unroll 1
+    for (int q = 0; q < 9; ++q) {
+        double hs = 0.0, as = 0.0, ds = 0.0;
+#pragma unroll
+        for (int j = 0; j < DG; ++j) {
+            const double ps = psiAt(j, q);
+            hs = fma(hc[j], ps, hs);
+            as = fma(ac[j], ps, as);
+            ds = fma(dc[j], ps, ds);
+        }
+        const double hG = fmax(hs, 0.0), aG = fmin(fmax(as, 0.0), 1.0);
+        const double expC = exp(p.compaction_param * (1.0 - aG));
+        const double el = hG * p.young * expC; // elasticity / damage
+        const size_t at = q * N + e;
+        pt.c[0 * 9 * N + at] = static_cast<T>(hG * expC * strain);
+        pt.c[1 * 9 * N + at] = static_cast<T>(
+            p.P0 * powByMode(hG, p.exponent_compression_factor + 1., p.powCmode, p.powCk) * expC);
+        const double tv = p.lambda * powByMode(expC, p.exponent_relaxation_sigma - 1., p.powRmode, p.powRk);
+        // FP64: the viscous relaxation time over damage^(n-1); FP32: dt over it
+        // (the time itself underflows in open water)
+        pt.c[2 * 9 * N + at] = static_cast<T>(sizeof(T) == 8 ? tv : p.dt / tv);
+        pt.c[3 * 9 * N + at] = static_cast<T>(p.C_lab * sizeScale * hG);
+        pt.c[4 * 9 * N + at] = static_cast<T>(p.compr_strength * sizeScale * hG);
+        pt.c[5 * 9 * N + at] = static_cast<T>(relaxScale * sqrt(el));
+        pt.d[at] = static_cast<T>(ds);
+    }
+    const double* src[3] = { s11, s12, s22 };
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+        double m[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            m[j] = src[c][j * N + e];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            double s = 0.0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                s = fma(m[j], psiAt(j, q), s);
+            pt.s[(c * 9 + q) * N + e] = static_cast<T>(s);
+        }
+    }
+}
+
+// The coefficients of the point values (which lie in the modes' span: the
+// unit square's projection gives them on every mesh).
+template <typename T, int DG>
+__global__ void __launch_bounds__(128) kBbmStore(size_t N, BbmPoints<T> pt, double* __restrict__ damage,
+    double* __restrict__ s11, double* __restrict__ s12, double* __restrict__ s22)
+{
+    const size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if (e >= N)
+        return;
+    auto project = [&](const T* src, auto modes, double* out) {
+        double v[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q)
+            v[q] = static_cast<double>(src[q * N + e]);
+#pragma unroll
+        for (int j = 0; j < decltype(modes)::value; ++j) {
+            double s = 0.0;
+#pragma unroll
+            for (int q = 0; q < 9; ++q)
+                s = fma(v[q], psiAt(j, q) * kW(q % 3) * kW(q / 3) * invNormOf(j), s);
+            out[j * N + e] = s;
+        }
+    };
+    project(pt.d, std::integral_constant<int, DG>(), damage);
+    double* dst[3] = { s11, s12, s22 };
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        project(pt.s + size_t(9) * c * N, std::integral_constant<int, 8>(), dst[c]);
+}
+
+// min(max(d, 1e-12), 1) on the integer pipe (NaN gives 1e-12, as fmax does)
+__device__ __forceinline__ double clampDamage(double d)
+{
+    const long long b = __double_as_longlong(d);
+    constexpr long long lo = 0x3d719799812dea11ll, hi = 0x3ff0000000000000ll; // 1e-12, 1
+    const bool nan = (b & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+    return __longlong_as_double(nan || b < lo ? lo : b > hi ? hi : b);
+}
+__device__ __forceinline__ float clampDamage(float d) { return fminf(fmaxf(d, 1e-12f), 1.f); }
+// comparisons on the bit patterns (an FP64 comparison issues at the FP64 rate)
+__device__ __forceinline__ long long bitsT(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ int bitsT(float x) { return __float_as_int(x); }
+__device__ __forceinline__ unsigned long long magnitudeT(double x) { return static_cast<unsigned long long>(bitsT(x)); }
+__device__ __forceinline__ unsigned magnitudeT(float x) { return static_cast<unsigned>(bitsT(x)); }
+template <typename T> __device__ __forceinline__ bool above0(T x) { return bitsT(x) > 0; }
+// min(x, 1) for x >= 0; NaN of either sign (0 / 0 in open water) gives 1, as fmin does
+template <typename T> __device__ __forceinline__ T min1(T x) { return magnitudeT(x) < magnitudeT(T(1)) ? x : T(1); }
+__device__ __forceinline__ bool finiteT(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+__device__ __forceinline__ bool finiteT(float x) { return (__float_as_int(x) & 0x7f800000) != 0x7f800000; }
+__device__ __forceinline__ double recipT(double x) { return recip64(x); }
+__device__ __forceinline__ float recipT(float x) { return 1.f / x; }
+__device__ __forceinline__ double sqrtT(double x) { return sqrt64(x); }
+__device__ __forceinline__ float sqrtT(float x) { return sqrtf(x); }
+
+template <typename T> struct BbmScalars {
+    T dt, nu0, halfOneMinusNu, tanPhi, relaxExp;
+    int powRmode, powRk;
+};
+
+// One Gauss point: the elastic-viscous stress update and the damage
+// (BBMStressUpdateStep.hpp:89-166) from half strains a, b, s times the
+// element's factor in c[0].
+template <typename T>
+__device__ __forceinline__ void bbmPoint(T a, T b, T s, const T (&c)[6], const BbmScalars<T>& k, T& g11, T& g12,
+    T& g22, T& d)
+{
+    d = clampDamage(d);
+    T press = T(-0.5) * (g11 + g22); // -sigma_n
+    T open = T(1);
+    if (above0(press))
+        open = T(1) - min1(c[1] * recipT(press));
+    T mult;
+    if constexpr (sizeof(T) == 8) {
+        const T tv = c[2] * powByMode(d, k.relaxExp, k.powRmode, k.powRk);
+        mult = tv * recipT(fmaT(open, k.dt, tv));
+    } else {
+        const T r = above0(open) ? open * c[2] * powByMode(T(1) / d, k.relaxExp, k.powRmode, k.powRk) : T(0);
+        mult = T(1) / (T(1) + r);
+    }
+    const T du = c[0] * d;
+    g11 = mult * fmaT(du, fmaT(k.nu0, b, a), g11);
+    g22 = mult * fmaT(du, fmaT(k.nu0, a, b), g22);
+    g12 = mult * fmaT(du, k.halfOneMinusNu * s, g12);
+    press = T(-0.5) * (g11 + g22);
+    const T dd = T(0.5) * (g11 - g22);
+    const T tau = sqrtT(fmaT(dd, dd, g12 * g12));
+    // dcrit: cohesion / (tau + tan_phi sigma_n) above the Mohr-Coulomb line,
+    // -compr / sigma_n beyond the compressive strength
+    const T mc = fmaT(-k.tanPhi, press, tau);
+    const bool crush = bitsT(press) > bitsT(c[4]); // press > the strength (>= 0)
+    const T num = crush ? c[4] : c[3], den = crush ? press : mc;
+    T dcrit = T(1);
+    if (above0(den))
+        dcrit = min1(num * recipT(den));
+    const T keep = fmaT(dcrit - T(1), c[5] * sqrtT(d), T(1));
+    d *= keep;
+    g11 *= keep;
+    g12 *= keep;
+    g22 *= keep;
+}
+
+template <typename T, int E> struct BbmShared {
+    Exchange<T, E> ex;
+    T strain[3][3][E];   // nu . strain per row
+    T sum[3][9][E];      // per row: nu . f (3) and the damage's moments (2, or DG)
+};
+
+// Row R of an element: see kBbmStress.
+template <typename T, Geometry GEO, int DG, int E>
+__device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const StressGeometry<T>& geo,
+    const T* __restrict__ wdam, const T* __restrict__ wj, const BbmPoints<T>& pt, const T (&ke)[4], T weight,
+    const T (&c)[3][6], T (&g)[3][3], T (&d)[3], const BbmScalars<T>& k, BbmShared<T, E>& sh, int le)
+{
+    T I[3], D[3], uxi[3], uet[3], vxi[3], vet[3], a[3], b[3], s[3];
+    const Scaled<T> sc(GEO == RECT ? ke[0] : T(1));
+    auto take = [&](int f) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            I[i] = sh.ex.in.v[f][R][i][le];
+            D[i] = sh.ex.in.dv[f][R][i][le];
+        }
+    };
+    take(0);
+    deriv(I, uxi);
+    if constexpr (GEO == RECT)
+        sc.interp(D, uet);
+    else
+        interp(D, uet);
+    take(1);
+    deriv(I, vxi);
+    if constexpr (GEO == RECT)
+        sc.interp(D, vet);
+    else
+        interp(D, vet);
+    const bool mid = R == 1;
+    const T nr = mid ? T(-2) : T(1);
+    [[maybe_unused]] T k0[3], k1[3], k2[3], k3[3], nq[3];
+    if constexpr (GEO == RECT) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            a[i] = uxi[i];
+            b[i] = vet[i];
+            s[i] = uet[i] + vxi[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const size_t q = 3 * R + i;
+            if constexpr (GEO == AFFINE) {
+                k0[i] = ke[0];
+                k1[i] = ke[1];
+                k2[i] = ke[2];
+                k3[i] = ke[3];
+            } else {
+                k0[i] = in ? geo.k[q * N + e] : T(0);
+                k1[i] = in ? geo.k[(9 + q) * N + e] : T(0);
+                k2[i] = in ? geo.k[(18 + q) * N + e] : T(0);
+                k3[i] = in ? geo.k[(27 + q) * N + e] : T(0);
+                nq[i] = in ? geo.n[q * N + e] : T(0);
+            }
+            a[i] = fmaT(k0[i], uxi[i], k1[i] * uet[i]);
+            b[i] = fmaT(k2[i], vxi[i], k3[i] * vet[i]);
+            s[i] = fmaT(k2[i], uxi[i], fmaT(k3[i], uet[i], fmaT(k0[i], vxi[i], k1[i] * vet[i])));
+        }
+        if constexpr (GEO == QUAD) {
+            T l[3] = { nr * fmaT(T(-2), a[1], a[0] + a[2]), nr * fmaT(T(-2), b[1], b[0] + b[2]),
+                nr * fmaT(T(-2), s[1], s[0] + s[2]) };
+            sumRows<T, E>(sh.strain, R, le, l);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                a[i] = fmaT(-l[0], nq[i], a[i]);
+                b[i] = fmaT(-l[1], nq[i], b[i]);
+                s[i] = fmaT(-l[2], nq[i], s[i]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        bbmPoint(a[i], b[i], s[i], c[i], k, g[0][i], g[1][i], g[2][i], d[i]);
+    // P f and the damage's projection: sums over the three rows
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+        sh.sum[R][f][le] = nr * fmaT(T(-2), g[f][1], g[f][0] + g[f][2]);
+    [[maybe_unused]] T m0 = T(0), m1 = T(0), m2 = T(0);
+    if constexpr (GEO == QUAD) {
+#pragma unroll
+        for (int j = 0; j < DG; ++j) {
+            T t = T(0);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                t = fmaT(in ? wdam[(j * 9 + 3 * R + i) * N + e] : T(0), d[i], t);
+            sh.sum[R][3 + j][le] = t;
+        }
+    } else {
+        // the row's Legendre coefficients along xi
+        // (the mean as d[1] plus differences: constants stay exact)
+        const T t2 = fmaT(T(-2), d[1], d[0] + d[2]);
+        m0 = fmaT(T(kW(0)), t2, d[1]);
+        m1 = T(0.5 / kG) * (d[2] - d[0]);
+        m2 = T(0.5 / (kG * kG)) * t2;
+        sh.sum[R][3][le] = m0;
+        sh.sum[R][4][le] = m1;
+        sh.sum[R][5][le] = m2;
+    }
+    __syncthreads();
+    [[maybe_unused]] const T nRow = mid ? T(kN(1)) : T(kN(0));
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+        const T l = sh.sum[0][f][le] + sh.sum[1][f][le] + sh.sum[2][f][le];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            g[f][i] = fmaT(-l, GEO == QUAD ? nq[i] : nRow * T(kN(i)), g[f][i]);
+    }
+    if constexpr (GEO == QUAD) {
+        T cf[DG];
+#pragma unroll
+        for (int j = 0; j < DG; ++j)
+            cf[j] = sh.sum[0][3 + j][le] + sh.sum[1][3 + j][le] + sh.sum[2][3 + j][le];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            T t = T(0);
+#pragma unroll
+            for (int j = 0; j < DG; ++j)
+                t = fmaT(cf[j], mid ? T(psiAt(j, 3 + i)) : R == 0 ? T(psiAt(j, i)) : T(psiAt(j, 6 + i)), t);
+            d[i] = t;
+        }
+    } else {
+        // modes of total degree <= 2 (DG 6), 1 (DG 3) or 0 (DG 1) stay
+        auto at = [&](int m, int r) { return sh.sum[r][3 + m][le]; };
+        auto second = [&](int m) { return fmaT(T(-2), at(m, 1), at(m, 0) + at(m, 2)); };
+        auto mean = [&](int m) { return fmaT(T(kW(0)), second(m), at(m, 1)); };
+        // the row value of the part of a coefficient that is quadratic in eta
+        const T qRow = (mid ? T(kL2(1)) : T(kL2(0))) * T(kW(0) * kL2(0) / kL2Norm);
+        auto quadratic = [&](int m) { return qRow * second(m); };
+        if constexpr (DG == 6) {
+            const T d1 = quadratic(1), d2 = m2 - mean(2);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                d[i] = fmaT(-d2, T(kL2(i)), fmaT(-d1, T(kX(i)), d[i]));
+        } else if constexpr (DG == 3) {
+            const T c0 = m0 - quadratic(0), c1 = mean(1);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                d[i] = fmaT(c1, T(kX(i)), c0);
+        } else {
+            const T c0 = mean(0);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                d[i] = c0;
+        }
+    }
+    if (in) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const size_t q = 3 * R + i;
+            pt.d[q * N + e] = d[i];
+#pragma unroll
+            for (int f = 0; f < 3; ++f)
+                pt.s[(9 * f + q) * N + e] = g[f][i];
+        }
+    }
+    // the divergence K^T (w J g) of this row: xi maps transposed
+    T x[3], y[3];
+    auto put = [&](int f, const T (&tx)[3], const T (&ty)[3]) {
+        derivT(tx, x);
+        if constexpr (GEO == RECT)
+            sc.interpT(ty, y);
+        else
+            interpT(ty, y);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            sh.ex.out.x[f][R][i][le] = x[i];
+            sh.ex.out.y[f][R][i][le] = y[i];
+        }
+    };
+    T w[3];
+    [[maybe_unused]] const T rowWeight = (mid ? T(kW(1)) : T(kW(0))) * weight;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        w[i] = GEO == QUAD ? (in ? wj[(3 * R + i) * N + e] : T(0)) : T(kW(i)) * rowWeight;
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            g[f][i] *= w[i];
+    if constexpr (GEO == RECT) {
+        put(0, g[0], g[1]);
+        put(1, g[1], g[2]);
+    } else {
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+            T p[3], q[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                p[i] = fmaT(k0[i], g[f][i], k2[i] * g[f + 1][i]);
+                q[i] = fmaT(k1[i], g[f][i], k3[i] * g[f + 1][i]);
+            }
+            put(f, p, q);
+        }
+    }
+}
+
+// One sub-step of the stress, the damage and the divergence.  Three threads
+// per element in three warps, as the mEVP kernel (nsdg_sumfact.cuh): node
+// column R, Gauss row R, node column R.
+//
+// Bound by FP64 issue in FP64 (about 1000 FP64 instructions per element where
+// the coefficient form took 3000, most of them in divisions, roots and
+// exponentials) and by memory on the mixed path (900 bytes per element, FP32).
+// Per launch: 96 x 80 rectangles, FP64, 21.7 us (121.8 us with coefficients and
+// per-element operators, 60 blocks of one thread per element); 256 x 256
+// parallelograms, mixed, 11.5 us (45.2 us: conversions of the FP64 state and
+// 168 registers).
+template <typename T, Geometry GEO, int DG, int E>
+__global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T> geo, const T* __restrict__ wdam,
+    const T* __restrict__ wj, const T* __restrict__ u, const T* __restrict__ v, BbmPoints<T> pt,
+    T* __restrict__ contrib, BbmScalars<T> k, int* __restrict__ err)
+{
+    __shared__ BbmShared<T, E> sh;
+    const int le = threadIdx.x % E, R = threadIdx.x / E;
+    const size_t N = m.N, e = blockIdx.x * size_t(E) + le;
+    const bool in = e < N, ice = in && m.ice[e];
+    T ke[4] = { T(0), T(0), T(0), T(0) }, weight = T(0), c[3][6], g[3][3], d[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const size_t q = 3 * R + i;
+#pragma unroll
+        for (int j = 0; j < 6; ++j)
+            c[i][j] = in ? pt.c[(9 * j + q) * N + e] : T(1);
+#pragma unroll
+        for (int f = 0; f < 3; ++f)
+            g[f][i] = in ? pt.s[(9 * f + q) * N + e] : T(0);
+        d[i] = in ? pt.d[q * N + e] : T(1);
+    }
+    if (in) {
+        if constexpr (GEO == RECT) {
+            ke[0] = geo.k[e];
+            weight = wj[e];
+        }
+        if constexpr (GEO == AFFINE) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                ke[j] = geo.k[j * N + e];
+            weight = wj[e];
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    {
+        T n[2][3] = { { T(0), T(0), T(0) }, { T(0), T(0), T(0) } };
+        if (ice) {
+            const unsigned s2 = 2u * static_cast<unsigned>(m.nx) + 1u;
+            const unsigned ix = static_cast<unsigned>(e) % static_cast<unsigned>(m.nx);
+            const unsigned iy = static_cast<unsigned>(e) / static_cast<unsigned>(m.nx);
+            const size_t base = 2 * size_t(s2) * iy + 2 * ix + R;
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                n[0][r] = u[base + size_t(r) * s2];
+                n[1][r] = v[base + size_t(r) * s2];
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+            T vr[3], dr[3];
+            interpDeriv(n[f], vr, dr);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                sh.ex.in.v[f][r][R][le] = vr[r];
+                sh.ex.in.dv[f][r][R][le] = dr[r];
+            }
+        }
+    }
+    __syncthreads();
+    bbmRow<T, GEO, DG, E>(R, e, N, in, geo, wdam, wj, pt, ke, weight, c, g, d, k, sh, le);
+    bool finite = true; // g holds the weighted stress
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            finite = finite && finiteT(g[f][i]);
+    if (in && !finite)
+        atomicOr(err, DEV_ERR_NONFINITE_STRESS);
+    __syncthreads();
+    if (!ice)
+        return;
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+        T x[3], y[3], o[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            x[r] = sh.ex.out.x[f][r][R][le];
+            y[r] = sh.ex.out.y[f][r][R][le];
+        }
+        columnT(x, y, o);
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            contrib[(9 * f + 3 * r + R) * N + e] = o[r];
+    }
+}
+
+// Step constants of the nodes, over dt / (rho H) (BrittleCGDynamicsKernel.hpp:206-254)
+// with c = dt / (rho H):
+//   a = c A F_ocean, kx = c (A F_atm |wind| uwind - rho H g dxSSH), ky likewise,
+//   im = c / lumped mass, and the ocean velocity turned by the ocean angle.
+template <typename T>
+__global__ void __launch_bounds__(128) kBbmPrepNodes(size_t n, BbmNodeState st, BbmNodeConst<T> c,
+    const double* __restrict__ invm2, BbmParams p)
+{
+    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if (i >= n)
+        return;
+    const double A = fmax(fmin(st.cgA[i], 1.0), 1.e-4);
+    const double H = fmax(st.cgH[i], 1.e-4);
+    st.cgA[i] = A;
+    st.cgH[i] = H;
+    st.avgU[i] = 0.0;
+    st.avgV[i] = 0.0;
+    const double rhoH = p.rho_ice * H, cm = p.dt / rhoH;
+    const double ua = st.ua[i], va = st.va[i], uo = st.uo[i], vo = st.vo[i];
+    const double drag = A * p.F_atm * sqrt(ua * ua + va * va);
+    const double im = invm2[i] * cm;
+    c.a[i] = static_cast<T>(cm * A * p.F_ocean);
+    c.kx[i] = static_cast<T>(cm * (drag * ua - rhoH * p.gravity * st.uGrad[i]));
+    c.ky[i] = static_cast<T>(cm * (drag * va - rhoH * p.gravity * st.vGrad[i]));
+    c.im[i] = static_cast<T>(im);
+    if (c.imLo)
+        c.imLo[i] = static_cast<T>(im - static_cast<double>(c.im[i]));
+    c.uo[i] = static_cast<T>(uo);
+    c.vo[i] = static_cast<T>(vo);
+    c.uor[i] = static_cast<T>(uo * p.cosA - vo * p.sinA);
+    c.vor[i] = static_cast<T>(vo * p.cosA + uo * p.sinA);
+    if (c.u != reinterpret_cast<T*>(st.u)) {
+        c.u[i] = static_cast<T>(st.u[i]);
+        c.v[i] = static_cast<T>(st.v[i]);
+    }
+}
+
+template <typename T> struct BbmNodeScalars {
+    T cosA, sinA, fcdt;
+    double invNSteps;
+};
+
+// The node update of one sub-step: with G = c F,
+//   u_new = (al (u + Gx) + be (v + Gy)) / (al^2 + be^2),
+//   v_new = (al (v + Gy) + be (Gx - u)) / (al^2 + be^2)
+// as increments, so that roundings of the factors act on the increment.  Per
+// launch: 193 x 161 nodes, FP64, 5.0 us (12.4 us with hypot, a division and the
+// step's terms formed again in every sub-step); 513 x 513 nodes, mixed, 4.7 us
+// (11.4 us on FP64 arrays).
+template <typename T>
+__global__ void __launch_bounds__(128) kBbmMomentum(DevMesh m, BbmNodeConst<T> c, double* __restrict__ avgU,
+    double* __restrict__ avgV, const T* __restrict__ contrib, BbmNodeScalars<T> k, int* __restrict__ err)
+{
+    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if (i >= m.Ncg)
+        return;
+    const unsigned s2 = 2u * static_cast<unsigned>(m.nx) + 1u;
+    const int i2 = static_cast<int>(static_cast<unsigned>(i) % s2), j2 = static_cast<int>(static_cast<unsigned>(i) / s2);
+    const bool dir = m.cg2Dir[i] != 0;
+    // before the wait for the stress kernel: the step's constants, and what
+    // the node kernel before that one wrote
+    const T a = c.a[i], kx = c.kx[i], ky = c.ky[i], im = c.im[i];
+    const T uo = c.uo[i], vo = c.vo[i], uor = c.uor[i], vor = c.vor[i];
+    const T u = c.u[i], v = c.v[i];
+    const T imLo = sizeof(T) == 4 ? c.imLo[i] : T(0);
+    const double au = avgU[i], av = avgV[i];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    T dSx = T(0), dSy = T(0);
+    if (!dir)
+        gatherDivergence(m, i2, j2, contrib, dSx, dSy);
+    const T ur = uo - u, vr = vo - v;
+    const T cp = a * sqrtT(fmaT(ur, ur, vr * vr));
+    const T cpc = cp * k.cosA, al = T(1) + cpc, be = fmaT(cp, k.sinA, k.fcdt);
+    const T rd = recipT(fmaT(al, al, be * be));
+    T gx = fmaT(dSx, im, kx), gy = fmaT(dSy, im, ky);
+    if constexpr (sizeof(T) == 4) {
+        gx = fmaT(dSx, imLo, gx);
+        gy = fmaT(dSy, imLo, gy);
+    }
+    gx = fmaT(cp, uor, gx);
+    gy = fmaT(cp, vor, gy);
+    T un = fmaT(rd, fmaT(al, fmaT(-cpc, u, gx), be * fmaT(-be, u, v + gy)), u);
+    T vn = fmaT(rd, fmaT(al, fmaT(-cpc, v, gy), be * fmaT(-be, v, gx - u)), v);
+    if (!finiteT(un) || !finiteT(vn))
+        atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
+    if constexpr (sizeof(T) == 8) {
+        avgU[i] = fma(un, k.invNSteps, au);
+        avgV[i] = fma(vn, k.invNSteps, av);
+    } else {
+        avgU[i] = fma(static_cast<double>(un), k.invNSteps, au);
+        avgV[i] = fma(static_cast<double>(vn), k.invNSteps, av);
+    }
+    if (dir)
+        un = vn = T(0);
+    c.u[i] = un;
+    c.v[i] = vn;
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch(cudaStream_t s, void (*kernel)(KArgs...), size_t blocks, int threads, Args... args)
+{
+    cudaLaunchConfig_t cfg {};
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <typename T, int DG>
+cudaError_t stressFor(cudaStream_t s, const DevMesh& m, const BbmElements<T>& el, const T* u, const T* v,
+    T* contrib, const BbmScalars<T>& k, int* err)
+{
+    constexpr int E = kBbmElems;
+    const size_t blocks = (m.N + E - 1) / E;
+    if (el.geo.n)
+        return launch(s, kBbmStress<T, QUAD, DG, E>, blocks, 3 * E, m, el.geo, el.wdam, el.w, u, v, el.pt, contrib, k, err);
+    constexpr Geometry simple = sizeof(T) == 8 ? RECT : AFFINE;
+    return launch(s, kBbmStress<T, simple, DG, E>, blocks, 3 * E, m, el.geo, el.wdam, el.w, u, v, el.pt, contrib, k, err);
+}
+
+} // namespace
+
+template <typename T>
+cudaError_t launchBbmLoad(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, const double* h,
+    const double* a, const double* damage, const double* s11, const double* s12, const double* s22,
+    const double* hsize, const BbmParams& p)
+{
+    const unsigned g = static_cast<unsigned>((m.N + 127) / 128);
+    const double* invKx2 = nullptr;
+    if constexpr (sizeof(T) == 8)
+        invKx2 = el.geo.rect ? el.geo.k + m.N : nullptr;
+    switch (dg) {
+    case 1: kBbmLoad<T, 1><<<g, 128, 0, s>>>(m.N, h, a, damage, s11, s12, s22, hsize, invKx2, el.pt, p); break;
+    case 3: kBbmLoad<T, 3><<<g, 128, 0, s>>>(m.N, h, a, damage, s11, s12, s22, hsize, invKx2, el.pt, p); break;
+    case 6: kBbmLoad<T, 6><<<g, 128, 0, s>>>(m.N, h, a, damage, s11, s12, s22, hsize, invKx2, el.pt, p); break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launchBbmStore(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, double* damage,
+    double* s11, double* s12, double* s22)
+{
+    const unsigned g = static_cast<unsigned>((m.N + 127) / 128);
+    switch (dg) {
+    case 1: kBbmStore<T, 1><<<g, 128, 0, s>>>(m.N, el.pt, damage, s11, s12, s22); break;
+    case 3: kBbmStore<T, 3><<<g, 128, 0, s>>>(m.N, el.pt, damage, s11, s12, s22); break;
+    case 6: kBbmStore<T, 6><<<g, 128, 0, s>>>(m.N, el.pt, damage, s11, s12, s22); break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const BbmNodeState& st, const BbmNodeConst<T>& c,
+    const double* invm2, const BbmParams& p)
+{
+    kBbmPrepNodes<T><<<static_cast<unsigned>((m.Ncg + 127) / 128), 128, 0, s>>>(m.Ncg, st, c, invm2, p);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launchBbmStress(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, const T* u,
+    const T* v, T* contrib, const BbmParams& p, int* err)
+{
+    const BbmScalars<T> k { static_cast<T>(p.dt), static_cast<T>(p.nu0), static_cast<T>(0.5 * (1. - p.nu0)),
+        static_cast<T>(p.tan_phi), static_cast<T>(p.exponent_relaxation_sigma - 1.), p.powRmode, p.powRk };
+    switch (dg) {
+    case 1: return stressFor<T, 1>(s, m, el, u, v, contrib, k, err);
+    case 3: return stressFor<T, 3>(s, m, el, u, v, contrib, k, err);
+    case 6: return stressFor<T, 6>(s, m, el, u, v, contrib, k, err);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template <typename T>
+cudaError_t launchBbmMomentum(cudaStream_t s, const DevMesh& m, const BbmNodeState& st, const BbmNodeConst<T>& c,
+    const T* contrib, const BbmParams& p, int* err)
+{
+    const BbmNodeScalars<T> k { static_cast<T>(p.cosA), static_cast<T>(p.sinA), static_cast<T>(p.dt * p.fc),
+        p.invNSteps };
+    return launch(s, kBbmMomentum<T>, (m.Ncg + 127) / 128, 128, m, c, st.avgU, st.avgV, contrib, k, err);
+}
+
+#define NSDG_BBM_INSTANCES(T)                                                                                       \
+    template cudaError_t launchBbmLoad<T>(cudaStream_t, const DevMesh&, int, const BbmElements<T>&, const double*,  \
+        const double*, const double*, const double*, const double*, const double*, const double*, const BbmParams&); \
+    template cudaError_t launchBbmStore<T>(cudaStream_t, const DevMesh&, int, const BbmElements<T>&, double*,       \
+        double*, double*, double*);                                                                                 \
+    template cudaError_t launchBbmPrepNodes<T>(cudaStream_t, const DevMesh&, const BbmNodeState&,                   \
+        const BbmNodeConst<T>&, const double*, const BbmParams&);                                                   \
+    template cudaError_t launchBbmStress<T>(cudaStream_t, const DevMesh&, int, const BbmElements<T>&, const T*,     \
+        const T*, T*, const BbmParams&, int*);                                                                      \
+    template cudaError_t launchBbmMomentum<T>(cudaStream_t, const DevMesh&, const BbmNodeState&,                    \
+        const BbmNodeConst<T>&, const T*, const BbmParams&, int*);
+NSDG_BBM_INSTANCES(double)
+NSDG_BBM_INSTANCES(float)
+
+} // namespace nsdg

@@ -130,12 +130,14 @@ struct nsdg_kernel {
     float* hP32 = nullptr; // P/(2 alpha) at the Gauss points (mixed precision)
     float *cellX32 = nullptr, *cellY32 = nullptr; // FP32 transport cell operators (mixed precision)
     float* jwA32 = nullptr; // FP32 J w at the advection Gauss points (mixed-precision CG2DG)
-    float2* invmHL = nullptr; // inverse lumped CG2 mass as {hi, lo} floats (mixed precision)
-    BbmOps32 bbm32 {};        // FP32 BBM operators (mixed precision BBM)
-    // mixed BBM: the node terms fixed through the elastic sub-steps (FP32,
-    // formed by the step's node preparation)
-    BbmNodeConst32 bbmConst { nullptr, nullptr };
-    bool bbmK0 = false;
+    // the BBM sub-cycle's elements, node constants and divergence (FP64, or
+    // FP32 on the mixed path)
+    BbmElements<double> bbm64 {};
+    BbmElements<float> bbm32 {};
+    BbmNodeConst<double> bbmNode64 {};
+    BbmNodeConst<float> bbmNode32 {};
+    float* contrib32 = nullptr;
+    bool bbmAffine = false; // the mixed path's parallelogram form
     float *cellX8_32 = nullptr, *cellY8_32 = nullptr; // FP32 DG8 stress-transport operators
     // which FP32 stress kernel the updates use: 0 the element map's
     // derivatives at the Gauss points from global memory, 1 operator tiles by
@@ -454,17 +456,16 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     add(N + 1, 4); add(std::max<size_t>(flags.perEntry.size(), 1), 4);
     // ops
     add(ops.cellX.size()); add(ops.cellY.size()); add(ops.minv.size()); add(ops.jwA.size()); add(ops.jw3.size());
-    add(ops.gx.size()); add(ops.gy.size()); add(ops.a1.size()); add(ops.a2.size());
-    if (bbm) {
-        add(ops.w.size()); add(ops.d1.size()); add(ops.d2.size());
+    const bool pairs = P.precision == NSDG_PRECISION_FP64 && !bbm && !mesh.spherical;
+    if (pairs) {
+        add(ops.gx.size()); add(ops.gy.size()); add(ops.a1.size()); add(ops.a2.size());
     }
     add(ops.dxssh.size()); add(ops.dyssh.size()); add(Ncg); add(Ncg1);
     if (mesh.spherical) {
-        add(ops.gm.size()); add(ops.a3.size() + 1); add(ops.dm.size() + 1);
         add(ops.minvP.size()); add(ops.minv8P.size() + 1);
     }
     if (bbm) {
-        add(ops.cellX8.size()); add(ops.cellY8.size()); add(ops.minv8.size()); add(ops.wdam.size()); add(ops.hsize.size());
+        add(ops.cellX8.size()); add(ops.cellY8.size()); add(ops.minv8.size()); add(ops.hsize.size());
     }
     // state and work
     add(size_t(dg) * N); add(size_t(dg) * N); add(N); add(size_t(dg) * N);
@@ -478,14 +479,20 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     }
     add(3 * Ncg1); add(8 * N); add(8 * N); add(8 * N); add(Ncg);
     StressMetric metric;
-    if (!bbm) {
-        buildStressMetric(mesh, P.precision == NSDG_PRECISION_FP64, metric);
+    buildStressMetric(mesh, P.precision == NSDG_PRECISION_FP64, metric);
+    {
         const size_t sz = P.precision == NSDG_PRECISION_FP64 ? 8 : 4;
         add(metric.k.size(), sz); add(metric.n.size(), sz); add(metric.m.size(), sz);
         add(4 * N, 4);                            // the same on parallelograms
         add(9 * N); add(9 * N);                   // weights, weighted pressure
+        if (bbm) {
+            add(ops.wdam.size(), sz);
+            add(54 * N, sz); add(27 * N, sz); add(9 * N, sz); // step constants and point values
+            for (int i = 0; i < 11; ++i) add(Ncg, sz);        // node constants
+            add(18 * N, 4);
+        }
     }
-    if (P.precision == NSDG_PRECISION_FP64 && !bbm && !mesh.spherical)
+    if (pairs)
         add(324 * pairsLd(N), 8);                 // float-pair stress operators
     if (P.precision == NSDG_PRECISION_MIXED && !bbm) {
         add((mesh.spherical ? 486 : 324) * ops32Ld(N), 4);
@@ -500,16 +507,9 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     if (P.precision == NSDG_PRECISION_MIXED) {
         add(ops.cellX.size(), 4); add(ops.cellY.size(), 4); // FP32 transport operators
         add(ops.jwA.size(), 4);                             // FP32 J w of the CG2DG quadrature
-        add(Ncg, 8);                                        // inverse lumped mass {hi, lo}
     }
     if (P.precision == NSDG_PRECISION_MIXED && bbm) {
-        add(5 * ops32Ld(N), 4);                   // parallelogram coefficients
-        add(4 * Ncg, 4); add(4 * Ncg, 4);         // the node constants of the sub-steps
-        add(ops.gx.size(), 4); add(ops.gy.size(), 4); add(ops.w.size(), 4); add(ops.wdam.size(), 4);
-        add(ops.d1.size(), 4); add(ops.d2.size(), 4); add(ops.cellX8.size(), 4); add(ops.cellY8.size(), 4);
-        if (mesh.spherical) {
-            add(ops.gm.size(), 4); add(ops.dm.size(), 4);
-        }
+        add(ops.cellX8.size(), 4); add(ops.cellY8.size(), 4);
     }
     add((N + 255) / 256 + 1); add(1); add(1, 4);
     bytes += 4096;
@@ -560,24 +560,16 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     dops.minv = upd(ops.minv);
     dops.jwA = upd(ops.jwA);
     dops.jw3 = upd(ops.jw3);
-    dops.gx = upd(ops.gx);
-    dops.gy = upd(ops.gy);
-    dops.a1 = upd(ops.a1);
-    dops.a2 = upd(ops.a2);
-    if (bbm) {
-        dops.w = upd(ops.w);
-        dops.d1 = upd(ops.d1);
-        dops.d2 = upd(ops.d2);
+    if (pairs) {
+        dops.gx = upd(ops.gx);
+        dops.gy = upd(ops.gy);
+        dops.a1 = upd(ops.a1);
+        dops.a2 = upd(ops.a2);
     }
     if (mesh.spherical) {
         dops.minvP = upd(ops.minvP);
         if (bbm)
             dops.minv8P = upd(ops.minv8P);
-        dops.gm = upd(ops.gm);
-        if (bbm)
-            dops.dm = upd(ops.dm);
-        else
-            dops.a3 = upd(ops.a3);
     }
     dops.dxssh = upd(ops.dxssh);
     dops.dyssh = upd(ops.dyssh);
@@ -590,17 +582,14 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         dops.cellX8 = upd(ops.cellX8);
         dops.cellY8 = upd(ops.cellY8);
         dops.minv8 = upd(ops.minv8);
-        dops.wdam = upd(ops.wdam);
         dops.hsize = upd(ops.hsize);
     }
-    if (!bbm) {
-        metricW = upd(metric.w);
-        if (!mixed()) {
-            geo.rect = metric.rect;
-            geo.k = upd(metric.k);
-            geo.n = metric.n.empty() ? nullptr : upd(metric.n);
-            geo.m = metric.m.empty() ? nullptr : upd(metric.m);
-        }
+    metricW = upd(metric.w);
+    if (!mixed()) {
+        geo.rect = metric.rect;
+        geo.k = upd(metric.k);
+        geo.n = metric.n.empty() ? nullptr : upd(metric.n);
+        geo.m = metric.m.empty() ? nullptr : upd(metric.m);
     }
     if (e != cudaSuccess)
         return fail(NSDG_ERR_CUDA, std::string("initialise: upload failed: ") + cudaGetErrorString(e));
@@ -649,7 +638,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     cgTmp = z(Ncg);
     partials = z((N + 255) / 256 + 1);
     dsum = z(1);
-    if (P.precision == NSDG_PRECISION_FP64 && !bbm && !mesh.spherical) {
+    if (pairs) {
         // NSDG_FP64_STRESS=pairs or pairs_tma selects a float-pair stress kernel
         const char* env = std::getenv("NSDG_FP64_STRESS");
         fp64Stress = !env ? 0 : std::strcmp(env, "pairs") == 0 ? 1 : std::strcmp(env, "pairs_tma") == 0 ? 2 : 0;
@@ -676,58 +665,69 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         cellX32 = upf(ops.cellX);
         cellY32 = upf(ops.cellY);
         jwA32 = upf(ops.jwA);
-        std::vector<float2> hl(Ncg);
-        for (size_t i = 0; i < Ncg; ++i) {
-            const float hi = static_cast<float>(invm[i]);
-            hl[i] = make_float2(hi, static_cast<float>(invm[i] - static_cast<double>(hi)));
-        }
-        invmHL = arena.take<float2>(Ncg);
-        if (!invmHL)
-            e = cudaErrorMemoryAllocation;
-        else if (e == cudaSuccess)
-            e = cudaMemcpy(invmHL, hl.data(), Ncg * sizeof(float2), cudaMemcpyHostToDevice);
     }
-    if (mixed() && bbm) {
-        bbm32.gx = upf(ops.gx);
-        bbm32.gy = upf(ops.gy);
-        bbm32.w = upf(ops.w);
-        bbm32.wdam = upf(ops.wdam);
-        bbm32.d1 = upf(ops.d1);
-        bbm32.d2 = upf(ops.d2);
-        bbm32.gm = mesh.spherical ? upf(ops.gm) : nullptr;
-        bbm32.dm = mesh.spherical ? upf(ops.dm) : nullptr;
-        cellX8_32 = upf(ops.cellX8);
-        cellY8_32 = upf(ops.cellY8);
-        bbmConst.k0 = arena.take<float4>(Ncg);
-        bbmConst.k1 = arena.take<float4>(Ncg);
-        if (!bbmConst.k0 || !bbmConst.k1)
-            e = cudaErrorMemoryAllocation;
-        bbmK0 = bbmConst.k0 && bbmConst.k1;
-        // parallelogram meshes: 5 coefficients per element and the unit
-        // square's operators replace the per-element ones in the stress
-        // kernel (NSDG_BBM_STRESS_KERNEL=general keeps those)
-        const char* bk = std::getenv("NSDG_BBM_STRESS_KERNEL");
-        if (!mesh.spherical && !(bk && std::strcmp(bk, "general") == 0)) {
-            AffineStressOps aff;
-            AffineBbmOps abb;
-            const size_t ld = ops32Ld(N);
-            const bool okS = buildAffineStressOps(mesh, ops, ld, 1e-9, aff);
-            const bool okB = okS && buildAffineBbmOps(mesh, ops, 1e-9, abb);
-            affWorst = std::max(aff.worst, abb.worst);
-            if (okS && okB) {
-                float* coef = arena.take<float>(aff.coef.size());
-                if (!coef)
-                    e = cudaErrorMemoryAllocation;
-                else if (e == cudaSuccess)
-                    e = cudaMemcpy(coef, aff.coef.data(), aff.coef.size() * sizeof(float), cudaMemcpyHostToDevice);
-                if (e == cudaSuccess)
-                    e = uploadAffineReference(aff.ref);
-                if (e == cudaSuccess)
-                    e = uploadAffineBbmReference(abb.w, abb.wdam, dg, abb.dxi, abb.deta);
-                if (e == cudaSuccess) {
-                    bbm32.coef = coef;
-                    bbm32.ld = ld;
-                }
+    if (bbm) {
+        // 2 J (times k_x on rectangles) from the weight of the centre point
+        auto perElement = [&]() {
+            std::vector<double> c(metric.w.begin() + 4 * N, metric.w.begin() + 5 * N);
+            for (double& x : c)
+                x *= 81.0 / 16.0;
+            return c;
+        };
+        auto takeAll = [&](auto& el, auto& node, auto zero) {
+            using T = decltype(zero);
+            el.pt.c = arena.take<T>(54 * N);
+            el.pt.s = arena.take<T>(27 * N);
+            el.pt.d = arena.take<T>(9 * N);
+            T** const arrays[] = { &node.a, &node.kx, &node.ky, &node.im, &node.uo, &node.vo, &node.uor, &node.vor,
+                &node.imLo, &node.u, &node.v };
+            for (T** a : arrays)
+                *a = arena.take<T>(Ncg);
+            if (!el.pt.c || !el.pt.s || !el.pt.d || !node.v)
+                e = cudaErrorMemoryAllocation;
+            else if (e == cudaSuccess) // the timing entry may run before the first step
+                e = cudaMemsetAsync(el.pt.c, 0, (reinterpret_cast<char*>(node.v + Ncg)
+                    - reinterpret_cast<char*>(el.pt.c)), stream);
+        };
+        if (!mixed()) {
+            takeAll(bbm64, bbmNode64, 0.0);
+            bbmNode64.imLo = nullptr;
+            bbmNode64.u = u;
+            bbmNode64.v = v;
+            bbm64.geo = geo;
+            bbm64.w = geo.rect ? upd(perElement()) : metricW;
+            bbm64.wdam = geo.rect ? nullptr : upd(ops.wdam);
+        } else {
+            takeAll(bbm32, bbmNode32, 0.f);
+            contrib32 = arena.take<float>(18 * N);
+            if (!contrib32)
+                e = cudaErrorMemoryAllocation;
+            else if (e == cudaSuccess)
+                e = cudaMemsetAsync(contrib32, 0, 18 * N * sizeof(float), stream);
+            cellX8_32 = upf(ops.cellX8);
+            cellY8_32 = upf(ops.cellY8);
+            // parallelogram meshes: 4 coefficients per element
+            // (NSDG_BBM_STRESS_KERNEL=general keeps the map at every point)
+            const char* bk = std::getenv("NSDG_BBM_STRESS_KERNEL");
+            bbmAffine = false;
+            if (!(bk && std::strcmp(bk, "general") == 0)) {
+                AffineStressOps aff;
+                AffineBbmOps abb;
+                bbmAffine = buildAffineStressOps(mesh, ops, ops32Ld(N), 1e-9, aff)
+                    && buildAffineBbmOps(mesh, ops, 1e-9, abb);
+                affWorst = std::max(aff.worst, abb.worst);
+            }
+            if (bbmAffine) {
+                std::vector<double> centre(4 * N);
+                for (size_t c = 0; c < 4; ++c)
+                    std::copy_n(metric.k.begin() + (9 * c + 4) * N, N, centre.begin() + c * N);
+                bbm32.geo.k = upf(centre);
+                bbm32.w = upf(perElement());
+            } else {
+                bbm32.geo.k = upf(metric.k);
+                bbm32.geo.n = upf(metric.n);
+                bbm32.w = upf(metric.w);
+                bbm32.wdam = upf(ops.wdam);
             }
         }
     }
@@ -1026,13 +1026,23 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
             P.exponent_relaxation_sigma, P.exponent_compression_factor, P.tan_phi, P.compr_strength, P.C_lab };
         bbmPowModes(bp);
         BbmNodeState st { u, v, avgU, avgV, cgH, cgA, uo, vo, ua, va, uGrad, vGrad };
-        const BbmNodeConst32* bc = (mixed() && bbmK0) ? &bbmConst : nullptr;
-        LCH(launchBbmPrepNodes(s, dm, st, &bp, bc));
-        for (int it = 0; it < nS; ++it) {
-            LCH(launchBbmStress(s, dm, dops, dg, u, v, hice, cice, damage, s11, s12, s22, contrib, bp, derr,
-                mixed() ? &bbm32 : nullptr));
-            LCH(launchBbmMomentum(s, dm, dops, st, contrib, bp, derr, mixed() ? invmHL : nullptr, bc));
-        }
+        auto subcycle = [&](auto& el, auto& node, auto* div) -> int {
+            // the nodes' preparation last: the first stress kernel reads the
+            // point values before it waits for the launch just before it
+            LCH(launchBbmLoad(s, dm, dg, el, hice, cice, damage, s11, s12, s22, dops.hsize, bp));
+            LCH(launchBbmPrepNodes(s, dm, st, node, dops.invm2, bp));
+            for (int it = 0; it < nS; ++it) {
+                LCH(launchBbmStress(s, dm, dg, el, node.u, node.v, div, bp, derr));
+                LCH(launchBbmMomentum(s, dm, st, node, div, bp, derr));
+            }
+            LCH(launchBbmStore(s, dm, dg, el, damage, s11, s12, s22));
+            return NSDG_OK;
+        };
+        const int sub = mixed() ? subcycle(bbm32, bbmNode32, contrib32) : subcycle(bbm64, bbmNode64, contrib);
+        if (sub != NSDG_OK)
+            return sub;
+        if (mixed())
+            LCH(launchWidenVelocity(s, Ncg, bbmNode32.u, bbmNode32.v, u, v));
     }
 #undef LCH
     return NSDG_OK;
@@ -2116,8 +2126,10 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
             if (!bbm && k->mixed())
                 return k->launchStress32(k->stream, mp, k->derr);
             if (bbm)
-                return launchBbmStress(k->stream, k->dm, k->dops, k->dg, k->u, k->v, k->hice, k->cice, k->damage,
-                    k->s11, k->s12, k->s22, k->contrib, bp, k->derr, k->mixed() ? &k->bbm32 : nullptr);
+                return k->mixed() ? launchBbmStress(k->stream, k->dm, k->dg, k->bbm32, k->bbmNode32.u, k->bbmNode32.v,
+                                       k->contrib32, bp, k->derr)
+                                   : launchBbmStress(k->stream, k->dm, k->dg, k->bbm64, k->u, k->v, k->contrib, bp,
+                                       k->derr);
             if (k->opsPairs && k->fp64Stress == 2)
                 return launchMevpStressPairsTma(k->stream, k->dm, k->pairsMaps, k->u, k->v, k->Pg, k->contrib, mp,
                     k->derr);
@@ -2136,8 +2148,9 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
         case 1:
             if (!bbm && k->mixed())
                 return launchMevpMomentum32(k->stream, k->dm, k->st32, k->tdiv32, mp, k->derr);
-            return bbm ? launchBbmMomentum(k->stream, k->dm, k->dops, bs, k->contrib, bp, k->derr,
-                             k->mixed() ? k->invmHL : nullptr, (k->mixed() && k->bbmK0) ? &k->bbmConst : nullptr)
+            if (bbm && k->mixed())
+                return launchBbmMomentum(k->stream, k->dm, bs, k->bbmNode32, k->contrib32, bp, k->derr);
+            return bbm ? launchBbmMomentum(k->stream, k->dm, bs, k->bbmNode64, k->contrib, bp, k->derr)
                        : launchMevpMomentum(k->stream, k->dm, st, k->contrib, mp, k->derr);
         case 3:
         case 4:
@@ -2205,7 +2218,7 @@ int nsdg_kernel_stress_variant(nsdg_kernel* k, int* kind, double* mismatch)
     if (k->mixed() && k->rheology == NSDG_RHEOLOGY_MEVP)
         *kind = k->stressKind;
     else if (k->mixed())
-        *kind = k->bbm32.coef ? 2 : 0; // BBM: the parallelogram kernel or the per-element operators
+        *kind = k->bbmAffine ? 2 : 0; // BBM: parallelogram coefficients or the map at every point
     else
         *kind = -1;
     *mismatch = k->affWorst;

@@ -18,6 +18,7 @@ __constant__ ConstTables32 cT32;
 #include "nsdg_kernels.hpp"
 #include "nsdg_tma.cuh"
 #include "nsdg_sumfact.cuh"
+#include "nsdg_nodes.cuh"
 
 namespace nsdg {
 
@@ -1154,34 +1155,6 @@ __global__ void __launch_bounds__(kTrX * kTrY, 4) kTransportStageAffine(Transpor
 // reference's reversed-parity stripes), cells in ascending x; then the
 // boundary rows and columns are doubled.
 // ===========================================================================
-// The cells along one direction touching CG2 index i2 (0..2n) and the node's
-// local index in each (0, 1, 2), ascending; kept in registers (no local
-// arrays): n of them
-struct NodeCand {
-    int n, c0, l0, c1, l1;
-};
-__device__ __forceinline__ NodeCand nodeCand(int i2, int n)
-{
-    NodeCand r { 1, 0, 0, 0, 0 };
-    if (i2 & 1) {
-        r.c0 = (i2 - 1) / 2;
-        r.l0 = 1;
-    } else if (i2 >= 2 && i2 / 2 < n) {
-        r.n = 2;
-        r.c0 = i2 / 2 - 1;
-        r.l0 = 2;
-        r.c1 = i2 / 2;
-        r.l1 = 0;
-    } else if (i2 >= 2) {
-        r.c0 = i2 / 2 - 1;
-        r.l0 = 2;
-    } else {
-        r.c0 = i2 / 2;
-        r.l0 = 0;
-    }
-    return r;
-}
-
 template <int DG, int NF>
 __global__ void __launch_bounds__(kBlock) kDG2CG(DevMesh m, const double* __restrict__ in0,
     const double* __restrict__ in1, double* __restrict__ out0, double* __restrict__ out1)
@@ -1456,42 +1429,6 @@ __global__ void __launch_bounds__(kBlock) kMevpPrepElements(size_t N, const doub
 // the divergence coefficients of nodes 3*part .. 3*part+2.  Land cells keep
 // tdiv = 0 (the reference's divergence skips them).
 constexpr int kStressParts = 3;
-
-// Gathers the divergence contributions of the (up to four) ice cells around
-// a CG2 node in the reference's scatter order (even cell rows first, then
-// odd; ascending x) and returns -sum.
-__device__ __forceinline__ void gatherDivergence(const DevMesh& m, int i2, int j2,
-    const double* __restrict__ contrib, double& dx, double& dy)
-{
-    const NodeCand X = nodeCand(i2, m.nx);
-    NodeCand Y = nodeCand(j2, m.ny);
-    if (Y.n == 2 && (Y.c0 & 1)) { // even cell rows first
-        const int c = Y.c0, l = Y.l0;
-        Y.c0 = Y.c1;
-        Y.l0 = Y.l1;
-        Y.c1 = c;
-        Y.l1 = l;
-    }
-    const size_t N = m.N;
-    double ax = 0.0, ay = 0.0;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        if (r < Y.n) {
-            const int cy = r ? Y.c1 : Y.c0, ly = r ? Y.l1 : Y.l0;
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (k < X.n) {
-                    const size_t c = size_t(cy) * m.nx + (k ? X.c1 : X.c0);
-                    const int j = (k ? X.l1 : X.l0) + 3 * ly;
-                    ax -= contrib[j * N + c];
-                    ay -= contrib[(9 + j) * N + c];
-                }
-            }
-        }
-    }
-    dx = ax;
-    dy = ay;
-}
 
 // The FP64 node update, divided through by c1 = rho H / dt (kMevpPrepNodes):
 //   u_new = (beta u + ku + f u_o - fc dt u + im dSx) / (1 + beta + f),  f = a |u_o - u|,
@@ -1982,427 +1919,6 @@ __global__ void kWidenVelocity(size_t n, const float* __restrict__ u32, const fl
 }
 
 // ===========================================================================
-// BBM (BBMStressUpdateStep.hpp:31-195, BrittleCGDynamicsKernel.hpp:206-254)
-// ===========================================================================
-__global__ void __launch_bounds__(kBlock) kBbmPrepNodes(size_t n, BbmNodeState st, BbmParams p,
-    BbmNodeConst32 c)
-{
-    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i >= n)
-        return;
-    const double Ad = fmax(fmin(st.cgA[i], 1.0), 1.e-4);
-    const double Hd = fmax(st.cgH[i], 1.e-4);
-    st.cgA[i] = Ad;
-    st.cgH[i] = Hd;
-    st.avgU[i] = 0.0;
-    st.avgV[i] = 0.0;
-    if (c.k0) {
-        // the FP32 node kernel's sub-step-invariant terms, formed as it forms them
-        const float H = static_cast<float>(Hd), A = static_cast<float>(Ad);
-        const float dt = static_cast<float>(p.dt), rho = static_cast<float>(p.rho_ice);
-        const float ua = static_cast<float>(st.ua[i]), va = static_cast<float>(st.va[i]);
-        const float dragAtm = A * static_cast<float>(p.F_atm) * hypotf(ua, va);
-        const float rhoHg = rho * H * static_cast<float>(p.gravity);
-        c.k0[i] = make_float4(dt / (rho * H), A * static_cast<float>(p.F_ocean), static_cast<float>(st.uo[i]),
-            static_cast<float>(st.vo[i]));
-        c.k1[i] = make_float4(dragAtm * ua, dragAtm * va, rhoHg * static_cast<float>(st.uGrad[i]),
-            rhoHg * static_cast<float>(st.vGrad[i]));
-    }
-}
-
-// The mixed-precision BBM node update from the step's FP32 node constants
-// (kBbmPrepNodes): per sub-step only the velocity, the gathered divergence
-// and the running averages are read.
-__global__ void __launch_bounds__(kBlock) kBbmMomentum32(DevMesh m, BbmNodeState st, BbmNodeConst32 c,
-    const double* __restrict__ contrib, BbmParams p, int* __restrict__ err, const float2* __restrict__ invmHL)
-{
-    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i >= m.Ncg)
-        return;
-    const int s2 = 2 * m.nx + 1;
-    const int i2 = static_cast<int>(static_cast<unsigned>(i) % static_cast<unsigned>(s2)), j2 = static_cast<int>(static_cast<unsigned>(i) / static_cast<unsigned>(s2));
-    const bool dir = m.cg2Dir[i] != 0;
-    const float4 k0 = c.k0[i], k1 = c.k1[i];
-    const float2 im = invmHL[i];
-    double dSx = 0.0, dSy = 0.0;
-    if (!dir)
-        gatherDivergence(m, i2, j2, contrib, dSx, dSy);
-    const float dt = narrowAny(p.dt);
-    const float cosA = narrowAny(p.cosA), sinA = narrowAny(p.sinA);
-    const float dteOverMass = k0.x, AFo = k0.y, uo = k0.z, vo = k0.w;
-    const float uIce = narrowAny(st.u[i]), vIce = narrowAny(st.v[i]);
-    const float cPrime = AFo * hypotf(uo - uIce, vo - vIce);
-    const float alpha = 1.f + dteOverMass * (cPrime * cosA);
-    const float beta = dt * narrowAny(p.fc) + dteOverMass * cPrime * sinA;
-    const float rDenom = 1.f / (alpha * alpha + beta * beta);
-    const float tauX = k1.x + cPrime * (uo * cosA - vo * sinA);
-    const float tauY = k1.y + cPrime * (vo * cosA + uo * sinA);
-    const float fx = narrowAny(dSx), fy = narrowAny(dSy);
-    const float gradX = fmaf(fx, im.y, fx * im.x) - k1.z;
-    const float gradY = fmaf(fy, im.y, fy * im.x) - k1.w;
-    float un = alpha * uIce + beta * vIce + dteOverMass * (alpha * (gradX + tauX) + beta * (gradY + tauY));
-    un *= rDenom;
-    float vn = alpha * vIce - beta * uIce + dteOverMass * (alpha * (gradY + tauY) + beta * (gradX + tauX));
-    vn *= rDenom;
-    if (!isfinite(un) || !isfinite(vn))
-        atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
-    st.avgU[i] += widenAny(un) * p.invNSteps;
-    st.avgV[i] += widenAny(vn) * p.invNSteps;
-    if (dir) {
-        un = 0.f;
-        vn = 0.f;
-    }
-    st.u[i] = widenAny(un);
-    st.v[i] = widenAny(vn);
-}
-
-// x^y for x >= 0: by multiplication when y is a small integer (mode 1), times
-// sqrt(x) when it is a small half-integer (mode 2), else pow().  Differs from
-// pow() by a few ulps.
-template <typename T> __device__ __forceinline__ T powByMode(T x, T y, int mode, int k)
-{
-    if (mode == 0)
-        return pow(x, y);
-    T r = T(1);
-    for (int i = 0; i < k; ++i)
-        r *= x;
-    return mode == 2 ? r * sqrt(x) : r;
-}
-
-// Element operators of the BBM stress kernel in the compute type T.
-template <typename T> struct BbmOps {
-    const T* gx;
-    const T* gy;
-    const T* w;
-    const T* wdam;
-    const T* d1;
-    const T* d2;
-    const double* hsize;
-    const T* gm; // spherical metric terms (null on Cartesian meshes)
-    const T* dm;
-    const float* coef = nullptr; // [5][ld] parallelogram coefficients (AFF kernels)
-    size_t ld = 0;
-};
-
-__constant__ float cAff[4][81]; // G_xi [q][j], G_eta [q][j], A_xi [j][q], A_eta [j][q]
-// The unit square's BBM operators for the parallelogram-mesh kernel (with
-// cAff's strain operators): iMJwPSI [k][q], the damage projection [k][q],
-// D_xi and D_eta [j][k] (divS1 = c0 D_xi + c1 D_eta, divS2 = c2 D_xi +
-// c3 D_eta)
-struct BbmAffTables {
-    float w[72];
-    float wdam[72];
-    float dxi[72];
-    float deta[72];
-};
-__constant__ BbmAffTables cBbmAff;
-
-// BBM stress, damage and divergence for one element.  T = double is the
-// reference's arithmetic; T = float is the mixed-precision kernel (FP32
-// operators and arithmetic, including exp/pow/sqrt; the stress, damage and
-// divergence are stored FP64 for the FP64 transport of the stress fields;
-// the conversions stay on the conversion unit: on the integer pipe, as in the
-// other mixed kernels, this kernel measured 9 % slower).
-// AFF (T = float on a parallelogram mesh): the strain from the unit
-// square's operators and the element's coefficients c (as the mEVP
-// parallelogram kernel), iMJwPSI and the damage projection from constant
-// memory, the divergence as D_xi (c0 s_a + c2 s_b) + D_eta (c1 s_a + c3 s_b):
-// 5 coefficients per element instead of 2 x 81 + 72 + 9 DG + 2 x 72
-// operator entries.
-template <int DG, typename T, bool AFF = false>
-__global__ void __launch_bounds__(kBlock) kBbmStress(DevMesh m, BbmOps<T> o, const double* __restrict__ u,
-    const double* __restrict__ v, const double* __restrict__ h, const double* __restrict__ a,
-    double* __restrict__ damage, double* __restrict__ s11, double* __restrict__ s12,
-    double* __restrict__ s22, double* __restrict__ contrib, BbmParams p, int* __restrict__ err)
-{
-    const size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    const size_t N = m.N;
-    if (e >= N)
-        return;
-    const bool ice = m.ice[e] != 0;
-    const size_t s2 = 2 * size_t(m.nx) + 1;
-    const size_t ix = static_cast<unsigned>(e) % static_cast<unsigned>(m.nx), iy = static_cast<unsigned>(e) / static_cast<unsigned>(m.nx);
-    const size_t base = 2 * s2 * iy + 2 * ix;
-    T ul[9], vl[9];
-#pragma unroll
-    for (int j = 0; j < 9; ++j) {
-        const size_t nd = base + (j % 3) + (j / 3) * s2;
-        ul[j] = ice ? static_cast<T>(u[nd]) : T(0);
-        vl[j] = ice ? static_cast<T>(v[nd]) : T(0);
-    }
-    T hc[DG], ac[DG], dc[DG], c11[8], c12[8], c22[8];
-#pragma unroll
-    for (int j = 0; j < DG; ++j) {
-        hc[j] = static_cast<T>(h[j * N + e]);
-        ac[j] = static_cast<T>(a[j * N + e]);
-        dc[j] = static_cast<T>(damage[j * N + e]);
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        c11[k] = static_cast<T>(s11[k * N + e]);
-        c12[k] = static_cast<T>(s12[k * N + e]);
-        c22[k] = static_cast<T>(s22[k * N + e]);
-    }
-    float cf[5] = { 0.f, 0.f, 0.f, 0.f, 0.f };
-    if constexpr (AFF) {
-#pragma unroll
-        for (int k = 0; k < 5; ++k)
-            cf[k] = o.coef[k * o.ld + e];
-    }
-    const T dt = static_cast<T>(p.dt);
-    const T nu0 = static_cast<T>(p.nu0);
-    const T hi = static_cast<T>(o.hsize[e]);
-    const T scale_coef = sqrt(T(0.1) / hi);
-    const T tdScale = hi * sqrt(T(2.) * (T(1.) + nu0) * static_cast<T>(p.rho_ice));
-    T n11[8], n12[8], n22[8], nd[DG];
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-        n11[k] = n12[k] = n22[k] = T(0);
-#pragma unroll
-    for (int k = 0; k < DG; ++k)
-        nd[k] = T(0);
-#pragma unroll 1
-    for (int q = 0; q < 9; ++q) {
-        T hs = T(0), as = T(0), ds = T(0);
-#pragma unroll
-        for (int j = 0; j < DG; ++j) {
-            hs += hc[j] * tab<T>::psi(3, j, q);
-            as += ac[j] * tab<T>::psi(3, j, q);
-            ds += dc[j] * tab<T>::psi(3, j, q);
-        }
-        const T hG = fmax(hs, T(0));
-        const T aG = fmin(fmax(as, T(0)), T(1));
-        T dG = fmin(fmax(ds, T(1e-12)), T(1));
-        T ex = T(0), ey = T(0), exv = T(0), eyu = T(0);
-        if constexpr (AFF) {
-            float ux = 0.f, ue = 0.f, vx = 0.f, ve = 0.f;
-#pragma unroll
-            for (int j = 0; j < 9; ++j) {
-                const float gx = cAff[0][q * 9 + j], ge = cAff[1][q * 9 + j];
-                ux = fmaf(gx, ul[j], ux);
-                ue = fmaf(ge, ul[j], ue);
-                vx = fmaf(gx, vl[j], vx);
-                ve = fmaf(ge, vl[j], ve);
-            }
-            ex = cf[4] * fmaf(cf[0], ux, cf[1] * ue);
-            ey = cf[4] * fmaf(cf[2], vx, cf[3] * ve);
-            exv = cf[4] * fmaf(cf[0], vx, cf[1] * ve);
-            eyu = cf[4] * fmaf(cf[2], ux, cf[3] * ue);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 9; ++j) {
-                const T gxq = o.gx[(q * 9 + j) * N + e];
-                const T gyq = o.gy[(q * 9 + j) * N + e];
-                ex = fma(gxq, ul[j], ex);
-                ey = fma(gyq, vl[j], ey);
-                exv = fma(gxq, vl[j], exv);
-                eyu = fma(gyq, ul[j], eyu);
-            }
-        }
-        if (!AFF && o.gm) { // spherical: e11 -= iMM v, e12 += iMM u / 2 (CGDynamicsKernel.cpp:331-334)
-            T mu = T(0), mv = T(0);
-#pragma unroll
-            for (int j = 0; j < 9; ++j) {
-                const T gmq = o.gm[(q * 9 + j) * N + e];
-                mu = fma(gmq, ul[j], mu);
-                mv = fma(gmq, vl[j], mv);
-            }
-            ex -= mv;
-            eyu += mu;
-        }
-        const T e11 = ex, e22 = ey, e12 = T(0.5) * (exv + eyu);
-        T g11 = T(0), g12 = T(0), g22 = T(0);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            g11 += c11[k] * tab<T>::psi(3, k, q);
-            g12 += c12[k] * tab<T>::psi(3, k, q);
-            g22 += c22[k] * tab<T>::psi(3, k, q);
-        }
-        T sigma_n = T(0.5) * (g11 + g22);
-        const T expC = exp(static_cast<T>(p.compaction_param) * (T(1.0) - aG));
-        const T Pmax = static_cast<T>(p.P0)
-            * powByMode(hG, static_cast<T>(p.exponent_compression_factor) + T(1.), p.powCmode, p.powCk) * expC;
-        const T tildeP = (sigma_n < T(0)) ? fmin(-Pmax / sigma_n, T(1.0)) : T(0);
-        T multiplicator;
-        if constexpr (sizeof(T) == 8) {
-            const T powalphaexpC
-                = powByMode(dG * expC, static_cast<T>(p.exponent_relaxation_sigma) - T(1), p.powRmode, p.powRk);
-            const T time_viscous = static_cast<T>(p.lambda) * powalphaexpC;
-            multiplicator = time_viscous / (time_viscous + (T(1.) - tildeP) * dt);
-        } else {
-            // lambda (d e^{C(1-A)})^(n-1) underflows FP32 in open water and
-            // 0 / (0 + 0) would follow where tildeP = 1: the same quantity as
-            // 1 / (1 + (1 - tildeP) dt / time_viscous) with the relaxation
-            // time taken in log space
-            const T logTv = log(static_cast<T>(p.lambda))
-                + (static_cast<T>(p.exponent_relaxation_sigma) - T(1))
-                    * (log(dG) + static_cast<T>(p.compaction_param) * (T(1.0) - aG));
-            const T open = T(1.) - tildeP;
-            const T ratio = open > T(0) ? open * dt * exp(-logTv) : T(0);
-            multiplicator = T(1) / (T(1) + ratio);
-        }
-        const T elasticity = hG * static_cast<T>(p.young) * dG * expC;
-        const T Dunit_factor = dt * elasticity / (T(1.) - (nu0 * nu0));
-        g11 += Dunit_factor * (e11 + nu0 * e22);
-        g22 += Dunit_factor * (nu0 * e11 + e22);
-        g12 += Dunit_factor * e12 * (T(1.) - nu0);
-        g11 *= multiplicator;
-        g22 *= multiplicator;
-        g12 *= multiplicator;
-        sigma_n = T(0.5) * (g11 + g22);
-        const T dd = g11 - g22;
-        const T tau = sqrt(T(0.25) * (dd * dd) + g12 * g12);
-        const T tan_phi = static_cast<T>(p.tan_phi);
-        const T cohesion = static_cast<T>(p.C_lab) * scale_coef * hG;
-        const T compr = static_cast<T>(p.compr_strength) * scale_coef * hG;
-        T dcrit = (tau + tan_phi * sigma_n > T(0)) ? cohesion / (tau + tan_phi * sigma_n) : T(1.);
-        dcrit = (sigma_n < -compr) ? -compr / sigma_n : dcrit;
-        dcrit = fmin(dcrit, T(1.0));
-        const T td = tdScale / sqrt(elasticity);
-        const T relax = (T(1.) - dcrit) * dt / td;
-        dG -= dG * relax;
-        g11 -= g11 * relax;
-        g12 -= g12 * relax;
-        g22 -= g22 * relax;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const T wk = AFF ? T(cBbmAff.w[k * 9 + q]) : o.w[(k * 9 + q) * N + e];
-            n11[k] = fma(wk, g11, n11[k]);
-            n12[k] = fma(wk, g12, n12[k]);
-            n22[k] = fma(wk, g22, n22[k]);
-        }
-#pragma unroll
-        for (int k = 0; k < DG; ++k)
-            nd[k] = fma(AFF ? T(cBbmAff.wdam[k * 9 + q]) : o.wdam[(k * 9 + q) * N + e], dG, nd[k]);
-    }
-    bool finite = true;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        s11[k * N + e] = n11[k];
-        s12[k * N + e] = n12[k];
-        s22[k * N + e] = n22[k];
-        finite = finite && isfinite(n11[k]) && isfinite(n12[k]) && isfinite(n22[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < DG; ++k)
-        damage[k * N + e] = nd[k];
-    if (!finite)
-        atomicOr(err, DEV_ERR_NONFINITE_STRESS);
-    if constexpr (AFF) {
-        // divS1 n11 + divS2 n12 = D_xi (c0 n11 + c2 n12) + D_eta (c1 n11 + c3 n12),
-        // divS1 n12 + divS2 n22 likewise
-        T ax[8], bx[8], ay[8], by[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            ax[k] = fmaf(cf[0], n11[k], cf[2] * n12[k]);
-            bx[k] = fmaf(cf[1], n11[k], cf[3] * n12[k]);
-            ay[k] = fmaf(cf[0], n12[k], cf[2] * n22[k]);
-            by[k] = fmaf(cf[1], n12[k], cf[3] * n22[k]);
-        }
-#pragma unroll 1
-        for (int j = 0; j < 9; ++j) {
-            T tx = T(0), ty = T(0);
-            if (ice) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const float dxi = cBbmAff.dxi[j * 8 + k], deta = cBbmAff.deta[j * 8 + k];
-                    tx = fmaf(dxi, ax[k], fmaf(deta, bx[k], tx));
-                    ty = fmaf(dxi, ay[k], fmaf(deta, by[k], ty));
-                }
-            }
-            contrib[j * N + e] = tx;
-            contrib[(9 + j) * N + e] = ty;
-        }
-        return;
-    }
-#pragma unroll 1
-    for (int j = 0; j < 9; ++j) {
-        T tx = T(0), ty = T(0);
-        if (ice) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const T d1 = o.d1[(j * 8 + k) * N + e];
-                const T d2v = o.d2[(j * 8 + k) * N + e];
-                tx = fma(d1, n11[k], fma(d2v, n12[k], tx));
-                ty = fma(d1, n12[k], fma(d2v, n22[k], ty));
-                if (o.dm) { // spherical: +divM s12, -divM s11 (CGDynamicsKernel.cpp:348-351)
-                    const T dmv = o.dm[(j * 8 + k) * N + e];
-                    tx = fma(dmv, n12[k], tx);
-                    ty = fma(-dmv, n11[k], ty);
-                }
-            }
-        }
-        contrib[j * N + e] = tx;
-        contrib[(9 + j) * N + e] = ty;
-    }
-}
-
-// BBM momentum per CG2 node.  T = double is the reference's arithmetic; T =
-// float is the mixed-precision kernel: FP32 arithmetic on the FP64 state, the
-// inverse lumped mass as a hi/lo float pair, the sub-step averages of the
-// velocity accumulated in FP64.
-template <typename T>
-__global__ void __launch_bounds__(kBlock) kBbmMomentum(DevMesh m, DevOps o, BbmNodeState st,
-    const double* __restrict__ contrib, BbmParams p, int* __restrict__ err, const float2* __restrict__ invmHL)
-{
-    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i >= m.Ncg)
-        return;
-    const int s2 = 2 * m.nx + 1;
-    const int i2 = static_cast<int>(static_cast<unsigned>(i) % static_cast<unsigned>(s2)), j2 = static_cast<int>(static_cast<unsigned>(i) / static_cast<unsigned>(s2));
-    const bool dir = m.cg2Dir[i] != 0;
-    double dSx = 0.0, dSy = 0.0;
-    if (!dir)
-        gatherDivergence(m, i2, j2, contrib, dSx, dSy);
-    const T H = static_cast<T>(st.cgH[i]), A = static_cast<T>(st.cgA[i]);
-    const T dt = static_cast<T>(p.dt), rho = static_cast<T>(p.rho_ice);
-    const T cosA = static_cast<T>(p.cosA), sinA = static_cast<T>(p.sinA);
-    const T dteOverMass = dt / (rho * H);
-    const T uIce = static_cast<T>(st.u[i]), vIce = static_cast<T>(st.v[i]);
-    const T uo = static_cast<T>(st.uo[i]), vo = static_cast<T>(st.vo[i]);
-    const T ua = static_cast<T>(st.ua[i]), va = static_cast<T>(st.va[i]);
-    const T cPrime = A * static_cast<T>(p.F_ocean) * hypot(uo - uIce, vo - vIce);
-    const T alpha = 1 + dteOverMass * (cPrime * cosA);
-    const T beta = dt * static_cast<T>(p.fc) + dteOverMass * cPrime * sinA;
-    const T rDenom = 1 / (alpha * alpha + beta * beta);
-    const T dragAtm = A * static_cast<T>(p.F_atm) * hypot(ua, va);
-    const T tauX = dragAtm * ua + cPrime * (uo * cosA - vo * sinA);
-    const T tauY = dragAtm * va + cPrime * (vo * cosA + uo * sinA);
-    T gradX, gradY;
-    if constexpr (sizeof(T) == 8) {
-        const double invm = o.invm2[i];
-        gradX = dSx * invm - p.rho_ice * H * p.gravity * st.uGrad[i];
-        gradY = dSy * invm - p.rho_ice * H * p.gravity * st.vGrad[i];
-    } else {
-        const float2 im = invmHL[i];
-        const float fx = static_cast<float>(dSx), fy = static_cast<float>(dSy);
-        const float rhoHg = rho * H * static_cast<float>(p.gravity);
-        gradX = fmaf(fx, im.y, fx * im.x) - rhoHg * static_cast<float>(st.uGrad[i]);
-        gradY = fmaf(fy, im.y, fy * im.x) - rhoHg * static_cast<float>(st.vGrad[i]);
-    }
-    T un = alpha * uIce + beta * vIce + dteOverMass * (alpha * (gradX + tauX) + beta * (gradY + tauY));
-    un *= rDenom;
-    T vn = alpha * vIce - beta * uIce + dteOverMass * (alpha * (gradY + tauY) + beta * (gradX + tauX));
-    vn *= rDenom;
-    if (!isfinite(un) || !isfinite(vn))
-        atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
-    if constexpr (sizeof(T) == 8) {
-        st.avgU[i] += un / p.nSteps;
-        st.avgV[i] += vn / p.nSteps;
-    } else {
-        const double invSteps = 1.0 / p.nSteps;
-        st.avgU[i] += static_cast<double>(un) * invSteps;
-        st.avgV[i] += static_cast<double>(vn) * invSteps;
-    }
-    if (dir) {
-        un = T(0);
-        vn = T(0);
-    }
-    st.u[i] = un;
-    st.v[i] = vn;
-}
-
-// ===========================================================================
 // Misc
 // ===========================================================================
 __global__ void kIceOceanStress(size_t n, int brittle, const double* __restrict__ u,
@@ -2834,29 +2350,6 @@ cudaError_t launchMevpStress32Tma(cudaStream_t s, const DevMesh& m, const Stress
     return cudaLaunchKernelEx(&cfg, kMevpStress32Tma<false>, maps.g, maps.a, m, u, v, Pg, hP, tdiv, p, err);
 }
 
-cudaError_t uploadAffineBbmReference(const double* w, const double* wdam, int dg, const double* dxi,
-    const double* deta)
-{
-    BbmAffTables t {};
-    for (int r = 0; r < 72; ++r) {
-        t.w[r] = static_cast<float>(w[r]);
-        t.dxi[r] = static_cast<float>(dxi[r]);
-        t.deta[r] = static_cast<float>(deta[r]);
-    }
-    for (int r = 0; r < dg * 9 && r < 72; ++r)
-        t.wdam[r] = static_cast<float>(wdam[r]);
-    return cudaMemcpyToSymbol(cBbmAff, &t, sizeof(t));
-}
-
-cudaError_t uploadAffineReference(const double ref[4][81])
-{
-    float h[4][81];
-    for (int b = 0; b < 4; ++b)
-        for (int r = 0; r < 81; ++r)
-            h[b][r] = static_cast<float>(ref[b][r]);
-    return cudaMemcpyToSymbol(cAff, h, sizeof(h));
-}
-
 cudaError_t launchViscositySelfTest(cudaStream_t s, size_t n, const float* inv, const double* Pa, double dmin,
     float* out)
 {
@@ -2978,63 +2471,6 @@ cudaError_t launchIceOceanStress(cudaStream_t s, size_t n, int brittle, const do
             static_cast<float>(cosA), static_cast<float>(sinA), tx, ty);
     else
         kIceOceanStress<<<blocksFor(n), kBlock, 0, s>>>(n, brittle, u, v, uo, vo, F_ocean, cosA, sinA, tx, ty);
-    return cudaGetLastError();
-}
-
-cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const BbmNodeState& st, const BbmParams* p,
-    const BbmNodeConst32* c)
-{
-    const BbmNodeConst32 none { nullptr, nullptr };
-    kBbmPrepNodes<<<blocksFor(m.Ncg), kBlock, 0, s>>>(m.Ncg, st, p ? *p : BbmParams {}, (c && p) ? *c : none);
-    return cudaGetLastError();
-}
-
-cudaError_t launchBbmStress(cudaStream_t s, const DevMesh& m, const DevOps& o, int dg, const double* u,
-    const double* v, const double* h, const double* a, double* damage, double* s11, double* s12,
-    double* s22, double* contrib, const BbmParams& p, int* err, const BbmOps32* o32)
-{
-    const unsigned g = blocksFor(m.N);
-    if (o32 && o32->coef) {
-        BbmOps<float> of { o32->gx, o32->gy, o32->w, o32->wdam, o32->d1, o32->d2, o.hsize, o32->gm, o32->dm };
-        of.coef = o32->coef;
-        of.ld = o32->ld;
-        switch (dg) {
-        case 1: kBbmStress<1, float, true><<<g, kBlock, 0, s>>>(m, of, u, v, h, a, damage, s11, s12, s22, contrib, p, err); break;
-        case 3: kBbmStress<3, float, true><<<g, kBlock, 0, s>>>(m, of, u, v, h, a, damage, s11, s12, s22, contrib, p, err); break;
-        case 6: kBbmStress<6, float, true><<<g, kBlock, 0, s>>>(m, of, u, v, h, a, damage, s11, s12, s22, contrib, p, err); break;
-        default: return cudaErrorInvalidValue;
-        }
-        return cudaGetLastError();
-    }
-    if (o32) {
-        const BbmOps<float> of { o32->gx, o32->gy, o32->w, o32->wdam, o32->d1, o32->d2, o.hsize, o32->gm, o32->dm };
-        switch (dg) {
-        case 1: kBbmStress<1, float><<<g, kBlock, 0, s>>>(m, of, u, v, h, a, damage, s11, s12, s22, contrib, p, err); break;
-        case 3: kBbmStress<3, float><<<g, kBlock, 0, s>>>(m, of, u, v, h, a, damage, s11, s12, s22, contrib, p, err); break;
-        case 6: kBbmStress<6, float><<<g, kBlock, 0, s>>>(m, of, u, v, h, a, damage, s11, s12, s22, contrib, p, err); break;
-        default: return cudaErrorInvalidValue;
-        }
-        return cudaGetLastError();
-    }
-    const BbmOps<double> od { o.gx, o.gy, o.w, o.wdam, o.d1, o.d2, o.hsize, o.gm, o.dm };
-    switch (dg) {
-    case 1: kBbmStress<1, double><<<g, kBlock, 0, s>>>(m, od, u, v, h, a, damage, s11, s12, s22, contrib, p, err); break;
-    case 3: kBbmStress<3, double><<<g, kBlock, 0, s>>>(m, od, u, v, h, a, damage, s11, s12, s22, contrib, p, err); break;
-    case 6: kBbmStress<6, double><<<g, kBlock, 0, s>>>(m, od, u, v, h, a, damage, s11, s12, s22, contrib, p, err); break;
-    default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launchBbmMomentum(cudaStream_t s, const DevMesh& m, const DevOps& o, const BbmNodeState& st,
-    const double* contrib, const BbmParams& p, int* err, const float2* invmHL, const BbmNodeConst32* c)
-{
-    if (invmHL && c && c->k0)
-        kBbmMomentum32<<<blocksFor(m.Ncg), kBlock, 0, s>>>(m, st, *c, contrib, p, err, invmHL);
-    else if (invmHL)
-        kBbmMomentum<float><<<blocksFor(m.Ncg), kBlock, 0, s>>>(m, o, st, contrib, p, err, invmHL);
-    else
-        kBbmMomentum<double><<<blocksFor(m.Ncg), kBlock, 0, s>>>(m, o, st, contrib, p, err, nullptr);
     return cudaGetLastError();
 }
 

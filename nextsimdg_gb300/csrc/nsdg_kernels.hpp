@@ -47,23 +47,16 @@ struct DevOps {
     const double* minv8 = nullptr;
     const double* gx = nullptr;
     const double* gy = nullptr;
-    const double* w = nullptr;
     const double* a1 = nullptr;
     const double* a2 = nullptr;
-    const double* d1 = nullptr;
-    const double* d2 = nullptr;
-    const double* wdam = nullptr;
     const double* dxssh = nullptr;
     const double* dyssh = nullptr;
     const double* hsize = nullptr;
     const double* invm2 = nullptr;   // 1 / lumped CG2 mass
     const double* lumped1 = nullptr; // lumped CG1 mass
     // spherical metric terms (null on Cartesian meshes)
-    const double* gm = nullptr;      // strain term iMM at the Gauss points [q][j]
     const double* minvP = nullptr;   // CG2DG inverse mass (the transport's minv carries 1 / R)
     const double* minv8P = nullptr;
-    const double* a3 = nullptr;      // divM iMJwPSI [j][q]
-    const double* dm = nullptr;      // divM [j][k] (BBM)
 };
 
 // Status bits written by kernels into the handle's device error word.
@@ -317,9 +310,6 @@ cudaError_t launchMevpPrepNodes32(cudaStream_t s, const DevMesh& m, const MevpNo
     const MevpNodeState32& st32, const double* invm2, const MevpParams& p,
     float* uLast = nullptr, float* vLast = nullptr);
 // (the Dirichlet flags of the nodes come from m.cg2Dir)
-// The unit square's strain operators (G_xi, G_eta [q][j]) for the
-// parallelogram BBM kernel, in constant memory (they depend only on the basis).
-cudaError_t uploadAffineReference(const double ref[4][81]);
 // The sum-factorised element kernels with FP32 state (nsdg_sumfact.cuh), Pw
 // the weighted pressure as pairs of floats: on parallelograms (4 coefficients
 // per element) and on general quadrilaterals or a sphere.  viscosityMode
@@ -446,43 +436,43 @@ struct BbmNodeState {
     const double* uGrad;
     const double* vGrad;
 };
-// Mixed-precision BBM: the node terms that stay fixed through the elastic
-// sub-steps, in FP32, formed once per step by the preparation kernel:
-// k0 = (dt_sub / (rho H), A F_ocean, u_ocean, v_ocean), k1 = (the wind
-// stress tau_atm,x, tau_atm,y, rho H g dX_ssh, rho H g dY_ssh).
-struct BbmNodeConst32 {
-    float4* k0;
-    float4* k1;
+// The BBM sub-cycle (nsdg_bbm.cu), T = double or, on the mixed path, float.
+// Step constants and point values at the 3 x 3 Gauss points.
+template <typename T> struct BbmPoints {
+    T* c = nullptr; // [6][9][N] constants of the step
+    T* s = nullptr; // [3][9][N] stress
+    T* d = nullptr; // [9][N] damage
 };
-// c (mixed precision, with p): also forms the FP32 node constants.
-cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const BbmNodeState& st,
-    const BbmParams* p = nullptr, const BbmNodeConst32* c = nullptr);
-// Per-step Gauss-point constants of the BBM update from h and A:
-// 0 hG, 1 expC, 2 Pmax, 3 elasticity, 4 Dunit_factor / dt ... (9 x 5 per element)
-// FP32 copies of the BBM element operators (mixed precision)
-struct BbmOps32 {
-    const float* gx;
-    const float* gy;
-    const float* w;
-    const float* wdam;
-    const float* d1;
-    const float* d2;
-    const float* gm; // spherical only
-    const float* dm; // spherical only
-    // parallelogram meshes: [5][ld] coefficients; the stress kernel then takes
-    // the unit square's operators (uploadAffineReference,
-    // uploadAffineBbmReference) instead of the per-element ones above
-    const float* coef = nullptr;
-    size_t ld = 0;
+template <typename T> struct BbmElements {
+    StressGeometry<T> geo {};
+    const T* wdam = nullptr; // [DG][9][N] damage projection (general quadrilaterals)
+    const T* w = nullptr;    // StressMetric::w there; 2 J (times k_x on rectangles) per element else
+    BbmPoints<T> pt {};
 };
-cudaError_t uploadAffineBbmReference(const double* w, const double* wdam, int dg, const double* dxi,
-    const double* deta);
-cudaError_t launchBbmStress(cudaStream_t s, const DevMesh& m, const DevOps& o, int dg, const double* u,
-    const double* v, const double* h, const double* a, double* damage, double* s11, double* s12,
-    double* s22, double* contrib, const BbmParams& p, int* err, const BbmOps32* o32 = nullptr);
-cudaError_t launchBbmMomentum(cudaStream_t s, const DevMesh& m, const DevOps& o,
-    const BbmNodeState& st, const double* contrib, const BbmParams& p, int* err,
-    const float2* invmHL = nullptr, const BbmNodeConst32* c = nullptr);
+// Step constants of the nodes and the velocity of the sub-cycle.
+template <typename T> struct BbmNodeConst {
+    T *a = nullptr, *kx = nullptr, *ky = nullptr, *im = nullptr, *imLo = nullptr;
+    T *uo = nullptr, *vo = nullptr, *uor = nullptr, *vor = nullptr;
+    T *u = nullptr, *v = nullptr;
+};
+constexpr int kBbmElems = 32; // elements per block
+template <typename T>
+cudaError_t launchBbmLoad(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, const double* h,
+    const double* a, const double* damage, const double* s11, const double* s12, const double* s22,
+    const double* hsize, const BbmParams& p);
+template <typename T>
+cudaError_t launchBbmStore(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, double* damage,
+    double* s11, double* s12, double* s22);
+template <typename T>
+cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const BbmNodeState& st, const BbmNodeConst<T>& c,
+    const double* invm2, const BbmParams& p);
+// contrib: [18][N], zero on land
+template <typename T>
+cudaError_t launchBbmStress(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, const T* u,
+    const T* v, T* contrib, const BbmParams& p, int* err);
+template <typename T>
+cudaError_t launchBbmMomentum(cudaStream_t s, const DevMesh& m, const BbmNodeState& st, const BbmNodeConst<T>& c,
+    const T* contrib, const BbmParams& p, int* err);
 
 // --- layout conversion, reductions ---------------------------------------
 // host ModelArray layout (AoS, nin comps) -> device SoA with `dg` comps,
