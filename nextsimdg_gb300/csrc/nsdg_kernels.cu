@@ -1769,10 +1769,9 @@ __device__ __forceinline__ void mevpMomentum32Node(int nx, int ny, size_t N, siz
     const float uOcnRel = uo - u, vOcnRel = v - vo;
     const float afocn = a * (p.F_oceanf * sqrtf(uOcnRel * uOcnRel + vOcnRel * vOcnRel));
     const float rden = 1.0f / (p.onePlusBetaf + afocn);
-    // (beta u + ku + a focn uo - fc dt u + mx) / (1 + beta + a focn), VPCGDynamicsKernel.hpp:132-172 over c1,
-    // as the increment of u (kMevpMomentum)
-    float un = fmaf(rden, fmaf(-(p.onePlusFcf + afocn), u, fmaf(afocn, uo, ku + mx)), u);
-    float vn = fmaf(rden, fmaf(-(p.oneMinusFcf + afocn), v, fmaf(afocn, vo, kv + my)), v);
+    // (beta u + ku + a focn uo - fc dt u + mx) / (1 + beta + a focn), VPCGDynamicsKernel.hpp:132-172 over c1
+    float un = rden * (p.betaf * u + ku + afocn * uo - p.fcdtf * u + mx);
+    float vn = rden * (p.betaf * v + kv + afocn * vo + p.fcdtf * v + my);
     if (!isfinite(un) || !isfinite(vn))
         atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
     if (dir) {

@@ -156,7 +156,7 @@ struct MevpParams {
     double onePlusBeta = 0, onePlusFc = 0, oneMinusFc = 0; // 1 + beta, 1 +- fc dt
     float keep = 0, dmin2f = 0, F_oceanf = 0;  // FP32 copies (dmin2f: DeltaMin^2)
     float dmin2lo = 0;                         // DeltaMin^2 - dmin2f (its float-pair low part)
-    float onePlusBetaf = 0, onePlusFcf = 0, oneMinusFcf = 0;
+    float betaf = 0, onePlusBetaf = 0, fcdtf = 0; // beta, 1 + beta, fc dt
 };
 inline MevpParams withDerived(MevpParams p)
 {
@@ -168,9 +168,9 @@ inline MevpParams withDerived(MevpParams p)
     p.dmin2f = static_cast<float>(p.DeltaMin * p.DeltaMin);
     p.dmin2lo = static_cast<float>(std::fma(p.DeltaMin, p.DeltaMin, -static_cast<double>(p.dmin2f)));
     p.F_oceanf = static_cast<float>(p.F_ocean);
+    p.betaf = static_cast<float>(p.beta);
     p.onePlusBetaf = static_cast<float>(1.0 + p.beta);
-    p.onePlusFcf = static_cast<float>(p.onePlusFc);
-    p.oneMinusFcf = static_cast<float>(p.oneMinusFc);
+    p.fcdtf = static_cast<float>(p.fc * p.dt);
     return p;
 }
 cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* invm2,
