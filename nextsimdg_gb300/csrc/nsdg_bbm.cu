@@ -431,7 +431,9 @@ __device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const
 // Per launch: 96 x 80 rectangles, FP64, 21.7 us (121.8 us with coefficients and
 // per-element operators, 60 blocks of one thread per element); 256 x 256
 // parallelograms, mixed, 11.5 us (45.2 us: conversions of the FP64 state and
-// 168 registers).
+// 168 registers).  One thread per element, as the mEVP kernel takes on large
+// grids, was slower here: 8.5 against 4.3 us on 128 x 128, 10.4 to 11.1 against
+// 11.5 on 256 x 256.
 template <typename T, Geometry GEO, int DG, int E>
 __global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T> geo, const T* __restrict__ wdam,
     const T* __restrict__ wj, const T* __restrict__ u, const T* __restrict__ v, BbmPoints<T> pt,

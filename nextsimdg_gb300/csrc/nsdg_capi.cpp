@@ -2451,12 +2451,17 @@ struct nsdg_ensemble {
     // operators, 2 parallelogram coefficients (every member a parallelogram mesh)
     int elementKind = 0;
     int viscMode = 3;
+    size_t elements = 0;
+    // parallelograms by one thread per element, 64 to a block
+    bool oneThread() const { return elementKind == 2 && viscMode == 3 && elements >= kOneThreadElems; }
     cudaError_t launchElements(cudaStream_t s, const EnsembleMember* table, const MevpParams& mp)
     {
+        if (oneThread())
+            return launchMevpStress32AffineThreadBatched(s, table, dStressMap, stressBlocks, mp);
         if (elementKind == 2)
             return launchMevpStress32AffineBatched(s, table, dTmaMap, tmaBlocks, mp, viscMode);
         return elementKind == 1 ? launchMevpStress32TmaBatched(s, table, dTmaMap, tmaBlocks, mp, derr)
-                                : launchMevpStress32Batched(s, table, dStressMap, stressBlocks, mp);
+                                : launchMevpStress32Batched(s, table, dStressMap, stressBlocks, elements, mp);
     }
     cudaGraphExec_t graph = nullptr;
     double graphDt = -1.0;
@@ -2522,6 +2527,7 @@ int nsdg_ensemble::build()
     const size_t perP = static_cast<size_t>(persistentNodesPerBlock());
     for (size_t mi = 0; mi < members.size(); ++mi) {
         EnsembleMember d = describe(members[mi]);
+        elements += d.N;
         d.stressBlock0 = static_cast<int>(smap.size());
         d.nodeBlock0 = static_cast<int>(nmap.size());
         d.tmaBlock0 = static_cast<int>(tmap.size());
@@ -2809,7 +2815,7 @@ int nsdg_ensemble_tile(nsdg_ensemble* ens, int member, int* tile_w, int* tile_h)
 {
     if (!ens || !tile_w || !tile_h || member < 0 || member >= static_cast<int>(ens->members.size()))
         return NSDG_ERR_BAD_ARG;
-    if (ens->elementKind != 0) {
+    if (ens->elementKind != 0 && !ens->oneThread()) {
         *tile_w = kTmaElems; // consecutive elements (operators staged by TMA, or parallelogram coefficients)
         *tile_h = 1;
     } else {

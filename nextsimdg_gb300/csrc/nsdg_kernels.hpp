@@ -321,6 +321,7 @@ cudaError_t launchMevpPrepNodes32(cudaStream_t s, const DevMesh& m, const MevpNo
 // fails (bitwise form 2).
 constexpr int kAffElems = 32;  // elements per block
 constexpr int kQuadElems = 64;
+constexpr size_t kOneThreadElems = 16384; // from here one thread per element (the reason stands at the kernels)
 cudaError_t launchMevpStress32Affine(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo,
     const float* u, const float* v, const float2* Pw, float* tdiv, const MevpParams& p, int viscosityMode);
 cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo, const float* u,
@@ -365,14 +366,19 @@ cudaError_t launchEnsembleSubcyclePersistent(cudaStream_t s, const EnsembleMembe
     int elemBlocks, const uint16_t* nodeMap, int nodeBlocks, const MevpParams& p, int viscosityMode,
     int iterations, unsigned* bar, int* err);
 // One launch each for the element and the node phase of every member.
+// Blocks of kQuadElems elements; `elements`: the members' total.
 cudaError_t launchMevpStress32Batched(cudaStream_t s, const EnsembleMember* members, const uint16_t* blockMember,
-    int blocks, const MevpParams& p);
+    int blocks, size_t elements, const MevpParams& p);
 cudaError_t launchMevpMomentum32Batched(cudaStream_t s, const EnsembleMember* members, const uint16_t* blockMember,
     int blocks, const MevpParams& p, int* err);
 // The element phase of every member with the TMA-staged kernel: blocks of
 // kTmaElems consecutive elements, tensor maps read from the member table.
 cudaError_t launchMevpStress32TmaBatched(cudaStream_t s, const EnsembleMember* members,
     const uint16_t* blockMember, int blocks, const MevpParams& p, int* err);
+// The element phase on parallelograms, one thread per element (blocks as for
+// launchMevpStress32Batched).
+cudaError_t launchMevpStress32AffineThreadBatched(cudaStream_t s, const EnsembleMember* members,
+    const uint16_t* blockMember, int blocks, const MevpParams& p);
 // The element phase of every member with the parallelogram kernel (every
 // member must have coefficients); blocks as for the TMA-staged launch.
 cudaError_t launchMevpStress32AffineBatched(cudaStream_t s, const EnsembleMember* members,

@@ -39,6 +39,14 @@ __global__ void __launch_bounds__(3 * kElems) kMevpStress(DevMesh m, StressGeome
 // unit-square operators and the viscosity in FP64, which was bound by FP64
 // issue), 9.6 us for 384 x 320 quadrilaterals (42.7 us with TMA-staged
 // operators), 7.3 us for 301 x 257 cells of a sphere (38.6 us).
+//
+// Three threads per element keep small grids' latency down; from
+// kOneThreadElems elements the SMs are full either way and one thread per
+// element issues about 950 instructions instead of 1,700 (shared-memory
+// exchange, indices).  Parallelograms: 64 x 64 2.2 against 2.6 us, 128 x 128 2.7
+// against 2.7, 256 x 256 4.6 against 4.1, 512 x 512 13.9 against 10.3;
+// quadrilaterals: 96 x 96 2.9 against 3.4, 192 x 192 4.5 against 4.2, 384 x 384
+// 12.0 against 9.6.
 template <Geometry GEO, int VM, int E>
 __global__ void __launch_bounds__(3 * E) kMevpStress32(DevMesh m, StressGeometry<float> geo,
     const float* __restrict__ u, const float* __restrict__ v, const float2* __restrict__ Pw, float* __restrict__ tdiv,
@@ -47,6 +55,16 @@ __global__ void __launch_bounds__(3 * E) kMevpStress32(DevMesh m, StressGeometry
     __shared__ Exchange<float, E> ex;
     __shared__ float sums[GEO == AFFINE ? 1 : 2][3][3][E];
     stressBlock<float, GEO, VM, E>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, rh, keep, blockIdx.x * size_t(E), ex, sums);
+}
+
+// One thread per element, for kOneThreadElems elements or more.
+template <Geometry GEO>
+__global__ void __launch_bounds__(kQuadElems) kMevpStress32Thread(DevMesh m, StressGeometry<float> geo,
+    const float* __restrict__ u, const float* __restrict__ v, const float2* __restrict__ Pw, float* __restrict__ tdiv,
+    Rheology<float> rh, float keep)
+{
+    stressThread<float, GEO, 3>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, rh, keep,
+        blockIdx.x * size_t(kQuadElems) + threadIdx.x);
 }
 
 // One launch over the elements of every member of an ensemble: block b belongs
@@ -62,6 +80,18 @@ __global__ void __launch_bounds__(3 * E) kMevpStress32Batched(const EnsembleMemb
     stressBlock<float, GEO, VM, E>(M.nx, M.N, M.ice, GEO == AFFINE ? M.aff : M.quad, M.st.u, M.st.v, M.Pw, M.tdiv, rh,
         keep, size_t(b) * E, ex, sums);
 }
+
+template <Geometry GEO>
+__global__ void __launch_bounds__(kQuadElems) kMevpStress32ThreadBatched(const EnsembleMember* __restrict__ members,
+    const uint16_t* __restrict__ blockMember, Rheology<float> rh, float keep)
+{
+    const EnsembleMember& M = members[blockMember[blockIdx.x]];
+    const int b = static_cast<int>(blockIdx.x) - M.stressBlock0;
+    stressThread<float, GEO, 3>(M.nx, M.N, M.ice, GEO == AFFINE ? M.aff : M.quad, M.st.u, M.st.v, M.Pw, M.tdiv, rh,
+        keep, size_t(b) * kQuadElems + threadIdx.x);
+}
+
+size_t blocksOf(size_t n) { return (n + kQuadElems - 1) / kQuadElems; }
 
 template <typename... KArgs, typename... Args>
 cudaError_t launch(cudaStream_t s, void (*kernel)(KArgs...), size_t blocks, int threads, Args... args)
@@ -95,6 +125,9 @@ cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const StressGeo
 {
     const MevpParams p = withDerived(pIn);
     const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
+    if (m.N >= kOneThreadElems)
+        return launch(s, geo.m ? kMevpStress32Thread<SPHERE> : kMevpStress32Thread<QUAD>, blocksOf(m.N), kQuadElems, m,
+            geo, u, v, Pw, tdiv, rh, p.keep);
     auto kernel = geo.m ? kMevpStress32<SPHERE, 3, kQuadElems> : kMevpStress32<QUAD, 3, kQuadElems>;
     return launch(s, kernel, (m.N + kQuadElems - 1) / kQuadElems, 3 * kQuadElems, m, geo, u, v, Pw, tdiv, rh, p.keep);
 }
@@ -110,16 +143,28 @@ cudaError_t launchMevpStress32Affine(cudaStream_t s, const DevMesh& m, const Str
               kMevpStress32<AFFINE, 2, kAffElems>, kMevpStress32<AFFINE, 3, kAffElems>,
               kMevpStress32<AFFINE, 4, kAffElems> };
     const int vm = viscosityMode >= 0 && viscosityMode <= 4 ? viscosityMode : 3;
+    if (vm == 3 && m.N >= kOneThreadElems)
+        return launch(s, kMevpStress32Thread<AFFINE>, blocksOf(m.N), kQuadElems, m, geo, u, v, Pw, tdiv, rh, p.keep);
     return launch(s, kernels[vm], (m.N + kAffElems - 1) / kAffElems, 3 * kAffElems, m, geo, u, v, Pw, tdiv, rh, p.keep);
 }
 
 cudaError_t launchMevpStress32Batched(cudaStream_t s, const EnsembleMember* members, const uint16_t* blockMember,
-    int blocks, const MevpParams& pIn)
+    int blocks, size_t elements, const MevpParams& pIn)
 {
     const MevpParams p = withDerived(pIn);
     const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
+    if (elements >= kOneThreadElems)
+        return launch(s, kMevpStress32ThreadBatched<QUAD>, blocks, kQuadElems, members, blockMember, rh, p.keep);
     return launch(s, kMevpStress32Batched<QUAD, 3, kQuadElems>, blocks, 3 * kQuadElems, members, blockMember, rh,
         p.keep);
+}
+
+cudaError_t launchMevpStress32AffineThreadBatched(cudaStream_t s, const EnsembleMember* members,
+    const uint16_t* blockMember, int blocks, const MevpParams& pIn)
+{
+    const MevpParams p = withDerived(pIn);
+    const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
+    return launch(s, kMevpStress32ThreadBatched<AFFINE>, blocks, kQuadElems, members, blockMember, rh, p.keep);
 }
 
 cudaError_t launchMevpStress32AffineBatched(cudaStream_t s, const EnsembleMember* members,

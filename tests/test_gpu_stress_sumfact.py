@@ -68,3 +68,22 @@ def test_ensemble_of_mixed_geometries(gpu, kinds):
             if "quads" not in kinds:
                 assert np.all(d == 0.0), name
             assert np.sqrt(np.mean(d * d)) <= 1e-5, name
+
+
+@pytest.mark.parametrize("kind", ["stretched", "quads"])
+def test_one_thread_per_element_is_bitwise_three(gpu, kind):
+    """From 16,384 elements the element kernels run one thread per element: an
+    ensemble above that of members below it is bitwise their single runs."""
+    sizes = [(127, 90), (61, 83)]
+    ref = [_step(MEVPDynamicsKernel(dg_comp=3, n_steps=20, precision=1), kind, *s) for s in sizes]
+    members = [MEVPDynamicsKernel(dg_comp=3, n_steps=20, precision=1) for _ in sizes]
+    for m, s in zip(members, sizes):
+        _step(m, kind, *s, steps=0)
+    ens = Ensemble(members)
+    for i in range(2):
+        ens.update(120.0 * i, 120.0)
+    ens.synchronize()
+    assert ens.tile(0) == (64, 1)
+    for m, r in zip(members, ref):
+        for name in ("u", "v"):
+            np.testing.assert_array_equal(m.getDG0Data(name), r[name])
