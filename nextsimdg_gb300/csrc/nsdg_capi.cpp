@@ -2512,7 +2512,7 @@ struct nsdg_ensemble {
     }
     static int nodeBlocksOf(const EnsembleMember& d)
     {
-        return static_cast<int>((d.Ncg + nodesPerBlock() - 1) / nodesPerBlock());
+        return static_cast<int>((cellsAndBorder(d.nx, d.ny) + cellsPerNodeBlock() - 1) / cellsPerNodeBlock());
     }
     static int tmaBlocksOf(const EnsembleMember& d) { return static_cast<int>((d.N + kTmaElems - 1) / kTmaElems); }
     void chooseElementKernel();
@@ -2524,7 +2524,7 @@ int nsdg_ensemble::build()
 {
     std::vector<EnsembleMember> table;
     std::vector<uint16_t> smap, nmap, tmap, pmap;
-    const size_t perP = static_cast<size_t>(persistentNodesPerBlock());
+    const size_t perP = static_cast<size_t>(persistentCellsPerBlock());
     for (size_t mi = 0; mi < members.size(); ++mi) {
         EnsembleMember d = describe(members[mi]);
         elements += d.N;
@@ -2535,7 +2535,7 @@ int nsdg_ensemble::build()
         smap.insert(smap.end(), stressBlocksOf(d), static_cast<uint16_t>(mi));
         nmap.insert(nmap.end(), nodeBlocksOf(d), static_cast<uint16_t>(mi));
         tmap.insert(tmap.end(), tmaBlocksOf(d), static_cast<uint16_t>(mi));
-        pmap.insert(pmap.end(), (d.Ncg + perP - 1) / perP, static_cast<uint16_t>(mi));
+        pmap.insert(pmap.end(), (cellsAndBorder(d.nx, d.ny) + perP - 1) / perP, static_cast<uint16_t>(mi));
         table.push_back(d);
     }
     stressBlocks = static_cast<int>(smap.size());

@@ -1719,76 +1719,58 @@ __global__ void kViscositySelfTestChecked(size_t n, const float* __restrict__ in
     out[i] = viscosity8<4>(inv[i], Pa[i], dmin, d2h, nsdg_ff::narrowAny(fma(dmin, dmin, -nsdg_ff::widenPos(d2h))));
 }
 
-// Body of the mixed-precision node kernel for CG2 node i.
-__device__ __forceinline__ void mevpMomentum32Node(int nx, int ny, size_t N, size_t i, const uint8_t* __restrict__ cg2Dir,
-    const MevpNodeState32& st, const float* __restrict__ tdiv, const MevpParams& p, int* __restrict__ err)
+// Body of the mixed-precision node kernel for the nodes of cell t.
+__device__ __forceinline__ void mevpMomentum32Cell(int nx, int ny, size_t N, unsigned t, const MevpNodeState32& st,
+    const float* __restrict__ tdiv, const MevpParams& p, int* __restrict__ err)
 {
-    // 32-bit index arithmetic (node counts stay far below 2^31)
-    const unsigned s2 = 2u * static_cast<unsigned>(nx) + 1u;
-    const int i2 = static_cast<int>(static_cast<unsigned>(i) % s2), j2 = static_cast<int>(static_cast<unsigned>(i) / s2);
-    // per-step constants first, two 16-byte loads (a programmatic dependent
-    // launch overlaps them with the stress kernel's tail), then the wait for
-    // its results
-    const float4 c0 = st.k0[i], c1 = st.k1[i];
-    const float a = c0.x, ku = c0.y, kv = c0.z, uo = c0.w, vo = c1.x;
-    const float2 im = make_float2(c1.y, c1.z);
-    const bool dir = c1.w != 0.f;
+    const CellNodes c(t, nx, ny);
+    // before the wait for the stress kernel: the step's constants, two 16-byte
+    // loads per node, and the velocity, which the node kernel before that one wrote
+    float4 k0[4], k1[4];
+    float u[4], v[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        k0[n] = c.exists[n] ? st.k0[c.id[n]] : make_float4(0.f, 0.f, 0.f, 0.f);
+        k1[n] = c.exists[n] ? st.k1[c.id[n]] : make_float4(0.f, 0.f, 0.f, 1.f);
+        u[n] = c.exists[n] ? st.u[c.id[n]] : 0.f;
+        v[n] = c.exists[n] ? st.v[c.id[n]] : 0.f;
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    float dSx = 0.f, dSy = 0.f;
-    if (!dir) {
-        const NodeCand X = nodeCand(i2, nx);
-        NodeCand Y = nodeCand(j2, ny);
-        if (Y.n == 2 && (Y.c0 & 1)) { // even cell rows first (the reference's accumulation order)
-            const int c = Y.c0, l = Y.l0;
-            Y.c0 = Y.c1;
-            Y.l0 = Y.l1;
-            Y.c1 = c;
-            Y.l1 = l;
-        }
+    float dx[4], dy[4];
+    gatherCell(c, nx, ny, N, tdiv, dx, dy);
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            if (r < Y.n) {
-                const int cy = r ? Y.c1 : Y.c0, ly = r ? Y.l1 : Y.l0;
-#pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    if (k < X.n) {
-                        const size_t c = size_t(cy) * nx + (k ? X.c1 : X.c0);
-                        const int j = (k ? X.l1 : X.l0) + 3 * ly;
-                        dSx -= tdiv[j * N + c];
-                        dSy -= tdiv[(9 + j) * N + c];
-                    }
-                }
-            }
+    for (int n = 0; n < 4; ++n) {
+        if (!c.exists[n])
+            continue;
+        const float a = k0[n].x, ku = k0[n].y, kv = k0[n].z, uo = k0[n].w, vo = k1[n].x;
+        const float2 im = make_float2(k1[n].y, k1[n].z);
+        const bool dir = k1[n].w != 0.f;
+        const float dSx = dir ? 0.f : dx[n], dSy = dir ? 0.f : dy[n];
+        // the divergence over the lumped mass and c1: that factor is FP64, held
+        // as the unevaluated sum hi + lo of two floats and applied with FP32 FMAs
+        const float mx = fmaf(dSx, im.y, dSx * im.x);
+        const float my = fmaf(dSy, im.y, dSy * im.x);
+        const float uOcnRel = uo - u[n], vOcnRel = v[n] - vo;
+        const float afocn = a * (p.F_oceanf * sqrtf(uOcnRel * uOcnRel + vOcnRel * vOcnRel));
+        const float rden = 1.0f / (p.onePlusBetaf + afocn);
+        // (beta u + ku + a focn uo - fc dt u + mx) / (1 + beta + a focn), VPCGDynamicsKernel.hpp:132-172 over c1
+        float un = rden * (p.betaf * u[n] + ku + afocn * uo - p.fcdtf * u[n] + mx);
+        float vn = rden * (p.betaf * v[n] + kv + afocn * vo + p.fcdtf * v[n] + my);
+        if (!isfinite(un) || !isfinite(vn))
+            atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
+        if (dir) {
+            un = 0.f;
+            vn = 0.f;
         }
+        st.u[c.id[n]] = un;
+        st.v[c.id[n]] = vn;
     }
-    // the divergence over the lumped mass and c1: that factor is FP64, held
-    // as the unevaluated sum hi + lo of two floats and applied with FP32 FMAs
-    const float mx = fmaf(dSx, im.y, dSx * im.x);
-    const float my = fmaf(dSy, im.y, dSy * im.x);
-    const float u = st.u[i], v = st.v[i];
-    const float uOcnRel = uo - u, vOcnRel = v - vo;
-    const float afocn = a * (p.F_oceanf * sqrtf(uOcnRel * uOcnRel + vOcnRel * vOcnRel));
-    const float rden = 1.0f / (p.onePlusBetaf + afocn);
-    // (beta u + ku + a focn uo - fc dt u + mx) / (1 + beta + a focn), VPCGDynamicsKernel.hpp:132-172 over c1
-    float un = rden * (p.betaf * u + ku + afocn * uo - p.fcdtf * u + mx);
-    float vn = rden * (p.betaf * v + kv + afocn * vo + p.fcdtf * v + my);
-    if (!isfinite(un) || !isfinite(vn))
-        atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
-    if (dir) {
-        un = 0.f;
-        vn = 0.f;
-    }
-    st.u[i] = un;
-    st.v[i] = vn;
 }
 
 __global__ void __launch_bounds__(kBlock) kMevpMomentum32(DevMesh m, MevpNodeState32 st,
     const float* __restrict__ tdiv, MevpParams p, int* __restrict__ err)
 {
-    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i >= m.Ncg)
-        return;
-    mevpMomentum32Node(m.nx, m.ny, m.N, i, m.cg2Dir, st, tdiv, p, err);
+    mevpMomentum32Cell(m.nx, m.ny, m.N, blockIdx.x * kBlock + threadIdx.x, st, tdiv, p, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -1888,9 +1870,8 @@ __global__ void __launch_bounds__(kAffElems * kStressParts) kEnsembleSubcyclePer
             break;
         for (int b = blockIdx.x; b < nodeBlocks; b += gridDim.x) {
             const EnsembleMember& M = members[nodeMap[b]];
-            const size_t i = size_t(b - M.nodeBlockP) * kThreads + threadIdx.x;
-            if (i < M.Ncg)
-                mevpMomentum32Node(M.nx, M.ny, M.N, i, M.cg2Dir, M.st, M.tdiv, p, err);
+            mevpMomentum32Cell(M.nx, M.ny, M.N, static_cast<unsigned>(b - M.nodeBlockP) * kThreads + threadIdx.x,
+                M.st, M.tdiv, p, err);
         }
         if (!gridBarrierBounded(bar, err, &okShared))
             break;
@@ -1901,10 +1882,8 @@ __global__ void __launch_bounds__(kBlock) kMevpMomentum32Batched(const EnsembleM
     const uint16_t* __restrict__ blockMember, MevpParams p, int* __restrict__ err)
 {
     const EnsembleMember& M = members[blockMember[blockIdx.x]];
-    const size_t i = (static_cast<size_t>(blockIdx.x) - M.nodeBlock0) * kBlock + threadIdx.x;
-    if (i >= M.Ncg)
-        return;
-    mevpMomentum32Node(M.nx, M.ny, M.N, i, M.cg2Dir, M.st, M.tdiv, p, err);
+    mevpMomentum32Cell(M.nx, M.ny, M.N, (blockIdx.x - static_cast<unsigned>(M.nodeBlock0)) * kBlock + threadIdx.x, M.st,
+        M.tdiv, p, err);
 }
 
 __global__ void kWidenVelocity(size_t n, const float* __restrict__ u32, const float* __restrict__ v32,
@@ -2375,7 +2354,7 @@ cudaError_t launchMevpMomentum32(cudaStream_t s, const DevMesh& m, const MevpNod
 {
     const MevpParams p = withDerived(pIn);
     cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(blocksFor(m.Ncg));
+    cfg.gridDim = dim3(blocksFor(cellsAndBorder(m.nx, m.ny)));
     cfg.blockDim = dim3(kBlock);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -2416,7 +2395,7 @@ cudaError_t launchMevpStress32TmaBatched(cudaStream_t s, const EnsembleMember* m
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kMevpStress32TmaBatched, members, blockMember, p, err);
 }
-int persistentNodesPerBlock() { return kAffElems * kStressParts; }
+int persistentCellsPerBlock() { return kAffElems * kStressParts; }
 
 cudaError_t launchEnsembleSubcyclePersistent(cudaStream_t s, const EnsembleMember* members, const uint16_t* elemMap,
     int elemBlocks, const uint16_t* nodeMap, int nodeBlocks, const MevpParams& pIn, int viscosityMode,
@@ -2453,7 +2432,7 @@ cudaError_t launchEnsembleSubcyclePersistent(cudaStream_t s, const EnsembleMembe
     return cudaLaunchKernelEx(&cfg, kern, members, elemMap, elemBlocks, nodeMap, nodeBlocks, p, iterations, bar, err);
 }
 
-int nodesPerBlock() { return kBlock; }
+int cellsPerNodeBlock() { return kBlock; }
 
 cudaError_t launchWidenVelocity(cudaStream_t s, size_t n, const float* u32, const float* v32, double* u, double* v)
 {

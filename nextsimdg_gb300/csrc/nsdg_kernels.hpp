@@ -358,10 +358,10 @@ struct EnsembleMember {
 // The whole mEVP sub-cycle of a parallelogram ensemble (every member has
 // coefficients) as one cooperative, persistent launch: `iterations` times the
 // element phase (the parallelogram kernel, blocks of elemMap as in the batched
-// launch) and the node phase (nodeMap: blocks of persistentNodesPerBlock()
+// launch) and the node phase (nodeMap: blocks of persistentCellsPerBlock()
 // nodes), separated by bounded grid barriers on bar[2] (set to zero here
 // first).  Bitwise the same results as the per-phase launches.
-int persistentNodesPerBlock();
+int persistentCellsPerBlock();
 cudaError_t launchEnsembleSubcyclePersistent(cudaStream_t s, const EnsembleMember* members, const uint16_t* elemMap,
     int elemBlocks, const uint16_t* nodeMap, int nodeBlocks, const MevpParams& p, int viscosityMode,
     int iterations, unsigned* bar, int* err);
@@ -383,7 +383,10 @@ cudaError_t launchMevpStress32AffineThreadBatched(cudaStream_t s, const Ensemble
 // member must have coefficients); blocks as for the TMA-staged launch.
 cudaError_t launchMevpStress32AffineBatched(cudaStream_t s, const EnsembleMember* members,
     const uint16_t* blockMember, int blocks, const MevpParams& p, int viscosityMode);
-int nodesPerBlock();
+// node blocks of the batched and the persistent launches: cells and border
+// cells, each with the nodes it owns
+inline size_t cellsAndBorder(int nx, int ny) { return (size_t(nx) + 1) * (size_t(ny) + 1); }
+int cellsPerNodeBlock();
 
 // u, v (FP64) from the FP32 iterate at the end of the sub-cycle
 cudaError_t launchWidenVelocity(cudaStream_t s, size_t n, const float* u32, const float* v32, double* u,

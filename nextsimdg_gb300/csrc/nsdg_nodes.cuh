@@ -72,5 +72,75 @@ __device__ __forceinline__ void gatherDivergence(const DevMesh& m, int i2, int j
     dy = ay;
 }
 
+// The four CG2 nodes that cell (ix, iy) of the (nx + 1) x (ny + 1) cells and
+// border cells owns: its lower left corner and, where the cell is one of the
+// mesh, the middles of its lower and left sides and its centre.
+struct CellNodes {
+    size_t id[4];   // (2 ix, 2 iy), (2 ix + 1, 2 iy), (2 ix, 2 iy + 1), (2 ix + 1, 2 iy + 1)
+    bool exists[4];
+    int ix, iy;
+    __device__ __forceinline__ CellNodes(unsigned t, int nx, int ny)
+    {
+        const unsigned w = static_cast<unsigned>(nx) + 1u;
+        iy = static_cast<int>(t / w);
+        ix = static_cast<int>(t % w);
+        const size_t s2 = 2 * size_t(nx) + 1;
+        id[0] = 2 * s2 * iy + 2 * ix;
+        id[1] = id[0] + 1;
+        id[2] = id[0] + s2;
+        id[3] = id[2] + 1;
+        exists[0] = iy <= ny;
+        exists[1] = exists[0] && ix < nx;
+        exists[2] = iy < ny;
+        exists[3] = exists[2] && ix < nx;
+    }
+};
+
+// minus the sums of the contributions of the cells around those four nodes,
+// in the order of gatherDivergence (even cell rows first, ascending x).  One
+// thread for four nodes: every lane of a warp does the same loads, where one
+// thread per node makes the lanes of a warp wait for each other's cells.  The
+// mixed mEVP node kernel takes this form (1025 x 1025 nodes 9.1 -> 6.9 us per
+// launch, the same results bit for bit); with the FP64 and the BBM kernels'
+// larger node state it is slower (513 x 513 nodes: FP64 18.6 -> 20.5 us, BBM
+// FP64 23.1 -> 27.0, BBM mixed 4.6 -> 5.5), and they keep one thread per node.
+template <typename T>
+__device__ __forceinline__ void gatherCell(const CellNodes& c, int nx, int ny, size_t N,
+    const T* __restrict__ contrib, T (&dx)[4], T (&dy)[4])
+{
+    const bool left = c.ix > 0, right = c.ix < nx, below = c.iy > 0, above = c.iy < ny;
+    const size_t e = size_t(c.iy) * nx + c.ix; // the cell itself
+    auto at = [&](bool ok, int j, size_t cell, T& x, T& y) {
+        x = ok ? contrib[j * N + cell] : T(0);
+        y = ok ? contrib[(9 + j) * N + cell] : T(0);
+    };
+    // corner: local nodes 8, 6 of the row below and 2, 0 of the cell's row
+    T bx[2], by[2], ax[2], ay[2], mbx, mby, max_, may, lx[2], ly[2], cx, cy;
+    at(below && left, 8, e - nx - 1, bx[0], by[0]);
+    at(below && right, 6, e - nx, bx[1], by[1]);
+    at(above && left, 2, e - 1, ax[0], ay[0]);
+    at(above && right, 0, e, ax[1], ay[1]);
+    at(below && right, 7, e - nx, mbx, mby);  // middle of the lower side
+    at(above && right, 1, e, max_, may);
+    at(above && left, 5, e - 1, lx[0], ly[0]); // middle of the left side
+    at(above && right, 3, e, lx[1], ly[1]);
+    at(above && right, 4, e, cx, cy);          // centre
+    const bool belowFirst = (c.iy & 1) != 0;   // row iy - 1 is even
+    auto four = [&](const T (&b)[2], const T (&a)[2]) {
+        const T p0 = belowFirst ? b[0] : a[0], p1 = belowFirst ? b[1] : a[1];
+        const T q0 = belowFirst ? a[0] : b[0], q1 = belowFirst ? a[1] : b[1];
+        return T(0) - p0 - p1 - q0 - q1;
+    };
+    auto two = [&](T b, T a) { return belowFirst ? T(0) - b - a : T(0) - a - b; };
+    dx[0] = four(bx, ax);
+    dy[0] = four(by, ay);
+    dx[1] = two(mbx, max_);
+    dy[1] = two(mby, may);
+    dx[2] = T(0) - lx[0] - lx[1];
+    dy[2] = T(0) - ly[0] - ly[1];
+    dx[3] = T(0) - cx;
+    dy[3] = T(0) - cy;
+}
+
 } // namespace
 } // namespace nsdg
