@@ -23,7 +23,7 @@ LIB = PKG / "libnsdg_gb300.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 
-CU_SOURCES = ["nsdg_kernels.cu", "nsdg_stress_sumfact.cu", "nsdg_bbm.cu", "nsdg_stress_pairs.cu", "nsdg_forcing.cu", "nsdg_noalloc.cu", "nsdg_surrogate.cu", "nsdg_ice_growth.cu"]
+CU_SOURCES = ["nsdg_kernels.cu", "nsdg_stress_sumfact.cu", "nsdg_bbm.cu", "nsdg_step.cu", "nsdg_stress_pairs.cu", "nsdg_forcing.cu", "nsdg_noalloc.cu", "nsdg_surrogate.cu", "nsdg_ice_growth.cu"]
 CXX_SOURCES = ["nsdg_host.cpp", "nsdg_capi.cpp", "nsdg_transport_capi.cpp", "nsdg_ice_growth_capi.cpp",
                "nsdg_restart.cpp", "nsdg_restart_write.cpp", "nsdg_restart_capi.cpp"]
 # per-file nvcc flags: the column thermodynamics and the benchmark forcing

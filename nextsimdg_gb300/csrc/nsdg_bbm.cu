@@ -15,8 +15,12 @@
 #include <cmath>
 #include <type_traits>
 
+#include "nsdg_exp64.cuh"
+#include "nsdg_modes.cuh"
 #include "nsdg_nodes.cuh"
+#include "nsdg_prep.cuh"
 #include "nsdg_sumfact.cuh"
+#include "nsdg_visc_ff.hpp"
 
 namespace nsdg {
 namespace {
@@ -36,6 +40,26 @@ template <typename T> __device__ __forceinline__ T powByMode(T x, T y, int mode,
     return mode == 2 ? r * sqrt(x) : r;
 }
 
+// FP64 <-> the point values' and node constants' type on the integer pipe
+template <typename T> __device__ __forceinline__ T store(double x)
+{
+    if constexpr (sizeof(T) == 8)
+        return x;
+    else
+        return nsdg_ff::narrowAny(x);
+}
+__device__ __forceinline__ double load(double x) { return x; }
+__device__ __forceinline__ double load(float x)
+{
+    const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
+    if (m >= 0x7f800000u)
+        return static_cast<double>(x);
+    const double y = nsdg_ff::widenNonneg(__uint_as_float(m));
+    return __hiloint2double(__double2hiint(y) | static_cast<int>(b & 0x80000000u), __double2loint(y));
+}
+// sqrt(x), x often 0 (open water, calm)
+__device__ __forceinline__ double rootOf(double x) { return __double_as_longlong(x) == 0 ? 0.0 : sqrt64(x); }
+
 // 1-D Gauss weights and points on [-1/2, 1/2], Legendre mode 2 there
 constexpr double kG = 0.38729833462074168852;
 constexpr double kL2Norm = 1. / 180.; // sum w L2^2
@@ -49,15 +73,16 @@ __device__ constexpr int modeX(int j) { return j == 1 || j == 5 || j == 7 ? 1 : 
 __device__ constexpr int modeY(int j) { return j == 2 || j == 5 || j == 6 ? 1 : j == 4 || j == 7 ? 2 : 0; }
 __device__ __forceinline__ constexpr double leg(int n, int i) { return n == 0 ? 1.0 : n == 1 ? kX(i) : kL2(i); }
 __device__ __forceinline__ constexpr double psiAt(int j, int q) { return leg(modeX(j), q % 3) * leg(modeY(j), q / 3); }
-__device__ __forceinline__ constexpr double invNorm(int n) { return n == 0 ? 1.0 : n == 1 ? 12.0 : 180.0; }
-__device__ __forceinline__ constexpr double invNormOf(int j) { return invNorm(modeX(j)) * invNorm(modeY(j)); }
 
-// Step constants and point values from the advected fields.
+// Step constants and point values from the advected fields, and the Lagrange
+// values of h and A for the nodes.  Bound by FP64 issue: 256 x 256 elements with
+// six modes, FP32 targets, 130 us (155 us with dense products and CUDA's exp,
+// roots and divisions, without the Lagrange values).
 template <typename T, int DG>
 __global__ void __launch_bounds__(128) kBbmLoad(size_t N, const double* __restrict__ h, const double* __restrict__ a,
     const double* __restrict__ damage, const double* __restrict__ s11, const double* __restrict__ s12,
     const double* __restrict__ s22, const double* __restrict__ hsize, const double* __restrict__ invKx2,
-    BbmPoints<T> pt, BbmParams p)
+    BbmPoints<T> pt, double* __restrict__ lagH, double* __restrict__ lagA, BbmParams p)
 {
     const size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
     if (e >= N)
@@ -69,53 +94,50 @@ __global__ void __launch_bounds__(128) kBbmLoad(size_t N, const double* __restri
         ac[j] = a[j * N + e];
         dc[j] = damage[j * N + e];
     }
+    storeLagrange<DG>(hc, ac, N, e, lagH, lagA);
+    double hg[9], ag[9], dg[9];
+    gaussValues<DG>(hc, hg);
+    gaussValues<DG>(ac, ag);
+    gaussValues<DG>(dc, dg);
     const double size = hsize[e];
-    const double sizeScale = sqrt(0.1 / size);
+    const double sizeScale = sqrt64(0.1 * recip64(size));
     // relax = (1 - dcrit) dt / td, td = size sqrt(2 (1 + nu0) rho) / sqrt(elasticity)
-    const double relaxScale = p.dt / (size * sqrt(2. * (1. + p.nu0) * p.rho_ice));
+    const double relaxScale = p.dt * recip64(size * p.soundRoot);
     // the kernels' half strains, over k_x on rectangles
-    const double strain = (invKx2 ? 2. / sqrt(invKx2[e]) : 2.) * p.dt * p.young / (1. - p.nu0 * p.nu0);
-#pragma unroll 1
-    for (int q = 0; q < 9; ++q) {
-        double hs = 0.0, as = 0.0, ds = 0.0;
+    const double strain = invKx2 ? timesRsqrt64(p.strainScale, invKx2[e]) : p.strainScale;
+    const double lab = p.C_lab * sizeScale, crush = p.compr_strength * sizeScale;
 #pragma unroll
-        for (int j = 0; j < DG; ++j) {
-            const double ps = psiAt(j, q);
-            hs = fma(hc[j], ps, hs);
-            as = fma(ac[j], ps, as);
-            ds = fma(dc[j], ps, ds);
-        }
-        const double hG = fmax(hs, 0.0), aG = fmin(fmax(as, 0.0), 1.0);
-        const double expC = exp(p.compaction_param * (1.0 - aG));
-        const double el = hG * p.young * expC; // elasticity / damage
+    for (int q = 0; q < 9; ++q) {
+        const double hG = atLeast(hg[q], 0.0), aG = atMost(atLeast(ag[q], 0.0), 1.0);
+        const double expC = exp64(p.compaction_param * (1.0 - aG));
+        const double hE = hG * expC;
         const size_t at = q * N + e;
-        pt.c[0 * 9 * N + at] = static_cast<T>(hG * expC * strain);
-        pt.c[1 * 9 * N + at] = static_cast<T>(
+        pt.c[0 * 9 * N + at] = store<T>(hE * strain);
+        pt.c[1 * 9 * N + at] = store<T>(
             p.P0 * powByMode(hG, p.exponent_compression_factor + 1., p.powCmode, p.powCk) * expC);
         const double tv = p.lambda * powByMode(expC, p.exponent_relaxation_sigma - 1., p.powRmode, p.powRk);
         // FP64: the viscous relaxation time over damage^(n-1); FP32: dt over it
         // (the time itself underflows in open water)
-        pt.c[2 * 9 * N + at] = static_cast<T>(sizeof(T) == 8 ? tv : p.dt / tv);
-        pt.c[3 * 9 * N + at] = static_cast<T>(p.C_lab * sizeScale * hG);
-        pt.c[4 * 9 * N + at] = static_cast<T>(p.compr_strength * sizeScale * hG);
-        pt.c[5 * 9 * N + at] = static_cast<T>(relaxScale * sqrt(el));
-        pt.d[at] = static_cast<T>(ds);
+        if constexpr (sizeof(T) == 8)
+            pt.c[2 * 9 * N + at] = tv;
+        else
+            pt.c[2 * 9 * N + at] = store<T>(p.dt * recip64(tv));
+        pt.c[3 * 9 * N + at] = store<T>(lab * hG);
+        pt.c[4 * 9 * N + at] = store<T>(crush * hG);
+        pt.c[5 * 9 * N + at] = store<T>(relaxScale * rootOf(hE * p.young)); // of elasticity / damage
+        pt.d[at] = store<T>(dg[q]);
     }
     const double* src[3] = { s11, s12, s22 };
-#pragma unroll 1
+#pragma unroll
     for (int c = 0; c < 3; ++c) {
-        double m[8];
+        double m[8], v[9];
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             m[j] = src[c][j * N + e];
+        gaussValues<8>(m, v);
 #pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            double s = 0.0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                s = fma(m[j], psiAt(j, q), s);
-            pt.s[(c * 9 + q) * N + e] = static_cast<T>(s);
-        }
+        for (int q = 0; q < 9; ++q)
+            pt.s[(c * 9 + q) * N + e] = store<T>(v[q]);
     }
 }
 
@@ -129,18 +151,15 @@ __global__ void __launch_bounds__(128) kBbmStore(size_t N, BbmPoints<T> pt, doub
     if (e >= N)
         return;
     auto project = [&](const T* src, auto modes, double* out) {
-        double v[9];
+        constexpr int M = decltype(modes)::value;
+        double v[9], c[M];
 #pragma unroll
         for (int q = 0; q < 9; ++q)
-            v[q] = static_cast<double>(src[q * N + e]);
+            v[q] = load(src[q * N + e]);
+        modesOf<M>(v, c);
 #pragma unroll
-        for (int j = 0; j < decltype(modes)::value; ++j) {
-            double s = 0.0;
-#pragma unroll
-            for (int q = 0; q < 9; ++q)
-                s = fma(v[q], psiAt(j, q) * kW(q % 3) * kW(q / 3) * invNormOf(j), s);
-            out[j * N + e] = s;
-        }
+        for (int j = 0; j < M; ++j)
+            out[j * N + e] = c[j];
     };
     project(pt.d, std::integral_constant<int, DG>(), damage);
     double* dst[3] = { s11, s12, s22 };
@@ -524,36 +543,41 @@ __global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T>
 // with c = dt / (rho H):
 //   a = c A F_ocean, kx = c (A F_atm |wind| uwind - rho H g dxSSH), ky likewise,
 //   im = c / lumped mass, and the ocean velocity turned by the ocean angle.
-template <typename T>
-__global__ void __launch_bounds__(128) kBbmPrepNodes(size_t n, BbmNodeState st, BbmNodeConst<T> c,
-    const double* __restrict__ invm2, BbmParams p)
+template <typename T, bool CONST>
+__global__ void __launch_bounds__(128) kBbmPrepNodes(int nx, int ny, size_t N, NodeInputs in, BbmNodeState st,
+    BbmNodeConst<T> c, BbmParams p)
 {
-    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i >= n)
+    const CellNodes cell(blockIdx.x * 128 + threadIdx.x, nx, ny);
+    if (!cell.exists[0])
         return;
-    const double A = fmax(fmin(st.cgA[i], 1.0), 1.e-4);
-    const double H = fmax(st.cgH[i], 1.e-4);
-    st.cgA[i] = A;
-    st.cgH[i] = H;
-    st.avgU[i] = 0.0;
-    st.avgV[i] = 0.0;
-    const double rhoH = p.rho_ice * H, cm = p.dt / rhoH;
-    const double ua = st.ua[i], va = st.va[i], uo = st.uo[i], vo = st.vo[i];
-    const double drag = A * p.F_atm * sqrt(ua * ua + va * va);
-    const double im = invm2[i] * cm;
-    c.a[i] = static_cast<T>(cm * A * p.F_ocean);
-    c.kx[i] = static_cast<T>(cm * (drag * ua - rhoH * p.gravity * st.uGrad[i]));
-    c.ky[i] = static_cast<T>(cm * (drag * va - rhoH * p.gravity * st.vGrad[i]));
-    c.im[i] = static_cast<T>(im);
-    if (c.imLo)
-        c.imLo[i] = static_cast<T>(im - static_cast<double>(c.im[i]));
-    c.uo[i] = static_cast<T>(uo);
-    c.vo[i] = static_cast<T>(vo);
-    c.uor[i] = static_cast<T>(uo * p.cosA - vo * p.sinA);
-    c.vor[i] = static_cast<T>(vo * p.cosA + uo * p.sinA);
-    if (c.u != reinterpret_cast<T*>(st.u)) {
-        c.u[i] = static_cast<T>(st.u[i]);
-        c.v[i] = static_cast<T>(st.v[i]);
+    double A[4], H[4], gx[4], gy[4];
+    nodeFields<CONST>(cell, nx, ny, N, in, A, H, gx, gy);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        if (!cell.exists[n])
+            continue;
+        const size_t i = cell.id[n];
+        st.avgU[i] = 0.0;
+        st.avgV[i] = 0.0;
+        const double cm = p.dt * recip64(p.rho_ice * H[n]);
+        const double ua = in.ua[i], va = in.va[i], uo = in.uo[i], vo = in.vo[i];
+        const double ca = cm * A[n], drag = ca * (p.F_atm * rootOf(fma(ua, ua, va * va)));
+        const double im = in.invm2[i] * cm;
+        c.a[i] = store<T>(ca * p.F_ocean);
+        c.kx[i] = store<T>(fma(drag, ua, -p.dt * p.gravity * gx[n]));
+        c.ky[i] = store<T>(fma(drag, va, -p.dt * p.gravity * gy[n]));
+        const T hi = store<T>(im);
+        c.im[i] = hi;
+        if constexpr (sizeof(T) == 4)
+            c.imLo[i] = store<T>(im - load(hi));
+        c.uo[i] = store<T>(uo);
+        c.vo[i] = store<T>(vo);
+        c.uor[i] = store<T>(fma(uo, p.cosA, -vo * p.sinA));
+        c.vor[i] = store<T>(fma(vo, p.cosA, uo * p.sinA));
+        if constexpr (sizeof(T) == 4) {
+            c.u[i] = store<T>(in.u[i]);
+            c.v[i] = store<T>(in.v[i]);
+        }
     }
 }
 
@@ -650,16 +674,16 @@ cudaError_t stressFor(cudaStream_t s, const DevMesh& m, const BbmElements<T>& el
 template <typename T>
 cudaError_t launchBbmLoad(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, const double* h,
     const double* a, const double* damage, const double* s11, const double* s12, const double* s22,
-    const double* hsize, const BbmParams& p)
+    const double* hsize, double* lagH, double* lagA, const BbmParams& p)
 {
     const unsigned g = static_cast<unsigned>((m.N + 127) / 128);
     const double* invKx2 = nullptr;
     if constexpr (sizeof(T) == 8)
         invKx2 = el.geo.rect ? el.geo.k + m.N : nullptr;
     switch (dg) {
-    case 1: kBbmLoad<T, 1><<<g, 128, 0, s>>>(m.N, h, a, damage, s11, s12, s22, hsize, invKx2, el.pt, p); break;
-    case 3: kBbmLoad<T, 3><<<g, 128, 0, s>>>(m.N, h, a, damage, s11, s12, s22, hsize, invKx2, el.pt, p); break;
-    case 6: kBbmLoad<T, 6><<<g, 128, 0, s>>>(m.N, h, a, damage, s11, s12, s22, hsize, invKx2, el.pt, p); break;
+    case 1: kBbmLoad<T, 1><<<g, 128, 0, s>>>(m.N, h, a, damage, s11, s12, s22, hsize, invKx2, el.pt, lagH, lagA, p); break;
+    case 3: kBbmLoad<T, 3><<<g, 128, 0, s>>>(m.N, h, a, damage, s11, s12, s22, hsize, invKx2, el.pt, lagH, lagA, p); break;
+    case 6: kBbmLoad<T, 6><<<g, 128, 0, s>>>(m.N, h, a, damage, s11, s12, s22, hsize, invKx2, el.pt, lagH, lagA, p); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -680,10 +704,14 @@ cudaError_t launchBbmStore(cudaStream_t s, const DevMesh& m, int dg, const BbmEl
 }
 
 template <typename T>
-cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const BbmNodeState& st, const BbmNodeConst<T>& c,
-    const double* invm2, const BbmParams& p)
+cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const NodeInputs& in, const BbmNodeState& st,
+    const BbmNodeConst<T>& c, const BbmParams& p)
 {
-    kBbmPrepNodes<T><<<static_cast<unsigned>((m.Ncg + 127) / 128), 128, 0, s>>>(m.Ncg, st, c, invm2, p);
+    const unsigned g = static_cast<unsigned>((cellsAndBorder(m.nx, m.ny) + 127) / 128);
+    if (in.constant)
+        kBbmPrepNodes<T, true><<<g, 128, 0, s>>>(m.nx, m.ny, m.N, in, st, c, p);
+    else
+        kBbmPrepNodes<T, false><<<g, 128, 0, s>>>(m.nx, m.ny, m.N, in, st, c, p);
     return cudaGetLastError();
 }
 
@@ -712,11 +740,12 @@ cudaError_t launchBbmMomentum(cudaStream_t s, const DevMesh& m, const BbmNodeSta
 
 #define NSDG_BBM_INSTANCES(T)                                                                                       \
     template cudaError_t launchBbmLoad<T>(cudaStream_t, const DevMesh&, int, const BbmElements<T>&, const double*,  \
-        const double*, const double*, const double*, const double*, const double*, const double*, const BbmParams&); \
+        const double*, const double*, const double*, const double*, const double*, const double*, double*, double*,  \
+        const BbmParams&);                                                                                          \
     template cudaError_t launchBbmStore<T>(cudaStream_t, const DevMesh&, int, const BbmElements<T>&, double*,       \
         double*, double*, double*);                                                                                 \
-    template cudaError_t launchBbmPrepNodes<T>(cudaStream_t, const DevMesh&, const BbmNodeState&,                   \
-        const BbmNodeConst<T>&, const double*, const BbmParams&);                                                   \
+    template cudaError_t launchBbmPrepNodes<T>(cudaStream_t, const DevMesh&, const NodeInputs&,                     \
+        const BbmNodeState&, const BbmNodeConst<T>&, const BbmParams&);                                             \
     template cudaError_t launchBbmStress<T>(cudaStream_t, const DevMesh&, int, const BbmElements<T>&, const T*,     \
         const T*, T*, const BbmParams&, int*);                                                                      \
     template cudaError_t launchBbmMomentum<T>(cudaStream_t, const DevMesh&, const BbmNodeState&,                    \

@@ -106,7 +106,6 @@ struct nsdg_kernel {
     double *u = nullptr, *v = nullptr, *uo = nullptr, *vo = nullptr, *ua = nullptr, *va = nullptr;
     double *avgU = nullptr, *avgV = nullptr;
     // per-step work
-    double *u0 = nullptr, *v0 = nullptr, *cgH = nullptr, *cgA = nullptr, *uGrad = nullptr, *vGrad = nullptr;
     double *nodeA = nullptr, *nodeKu = nullptr, *nodeKv = nullptr, *nodeIm = nullptr; // FP64 mEVP node constants
     double *Pg = nullptr, *contrib = nullptr;
     // the element maps of the sum-factorised stress kernels, the weights and
@@ -123,7 +122,8 @@ struct nsdg_kernel {
     double *phiA = nullptr, *k1 = nullptr; // 3 fields x dg x N
     double *velx8 = nullptr, *vely8 = nullptr, *nvX8 = nullptr, *nvY8 = nullptr;
     double *sA = nullptr, *sK1 = nullptr;  // 3 x 8 x N
-    double *sshScratch = nullptr, *staging = nullptr, *dgTmp = nullptr, *cgTmp = nullptr;
+    double *sshScratch = nullptr; // CG1 heights and gradient, Ncg1 each
+    double *staging = nullptr, *dgTmp = nullptr, *cgTmp = nullptr, *cgTmp2 = nullptr;
     // mixed precision (NSDG_PRECISION_MIXED)
     DevOps32 dops32;
     StressMaps maps32 {};
@@ -335,7 +335,8 @@ struct nsdg_kernel {
     SetTarget setTarget(const std::string& s);
     void storeField(const std::string& s, const double* data, size_t nComp);
     // the conversion of a field copied to `staging` into its target, on `stream`
-    int enqueueConversion(const SetTarget& t, const double* staging, size_t nComp);
+    int enqueueConversion(const SetTarget& t, const double* staging, size_t nComp, AverageFields& batch);
+    int flushAverages(AverageFields& batch);
     // the cell averages of a field into host memory `out`: projections and
     // the copy enqueued on `stream` (a stored field is copied at once)
     int enqueueReadout(const std::string& s, double* out, HostMoves* batch = nullptr);
@@ -470,7 +471,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     // state and work
     add(size_t(dg) * N); add(size_t(dg) * N); add(N); add(size_t(dg) * N);
     add(8 * N); add(8 * N); add(8 * N);
-    for (int i = 0; i < 22; ++i) add(Ncg);
+    for (int i = 0; i < 17; ++i) add(Ncg);
     add(9 * N); add(18 * N);
     add(size_t(dg) * N); add(size_t(dg) * N); add(ED * nXe); add(ED * nYe);
     add(3 * size_t(dg) * N); add(3 * size_t(dg) * N);
@@ -577,7 +578,10 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     for (size_t i = 0; i < Ncg; ++i)
         invm[i] = 1.0 / ops.lumped2[i];
     dops.invm2 = upd(invm);
-    dops.lumped1 = upd(ops.lumped1);
+    std::vector<double> invm1(ops.lumped1.size());
+    for (size_t i = 0; i < invm1.size(); ++i)
+        invm1[i] = 1.0 / ops.lumped1[i];
+    dops.invm1 = upd(invm1);
     if (bbm) {
         dops.cellX8 = upd(ops.cellX8);
         dops.cellY8 = upd(ops.cellY8);
@@ -609,8 +613,8 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     s12 = z(8 * N);
     s22 = z(8 * N);
     u = z(Ncg); v = z(Ncg); uo = z(Ncg); vo = z(Ncg); ua = z(Ncg); va = z(Ncg);
-    avgU = z(Ncg); avgV = z(Ncg); u0 = z(Ncg); v0 = z(Ncg); cgH = z(Ncg); cgA = z(Ncg);
-    uGrad = z(Ncg); vGrad = z(Ncg); nodeA = z(Ncg); nodeKu = z(Ncg); nodeKv = z(Ncg); nodeIm = z(Ncg);
+    avgU = z(Ncg); avgV = z(Ncg);
+    nodeA = z(Ncg); nodeKu = z(Ncg); nodeKv = z(Ncg); nodeIm = z(Ncg);
     Pg = z(9 * N);
     contrib = z(18 * N);
     if (!bbm) {
@@ -636,6 +640,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     stage2 = z(8 * N);
     dgTmp = z(8 * N);
     cgTmp = z(Ncg);
+    cgTmp2 = z(Ncg);
     partials = z((N + 255) / 256 + 1);
     dsum = z(1);
     if (pairs) {
@@ -955,21 +960,24 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
             nvY8, STAGE_RK2_B, dt, b, cx8, cy8));
     }
     // --- prepareIteration (CGDynamicsKernel.cpp:260-276) ---
-    {
-        const double* in[2] = { hice, cice };
-        double* out[2] = { cgH, cgA };
-        LCH(launchDG2CG(s, dm, dg, 2, in, out));
-        e = launchSSHGradient(s, dm, dops, ssh, sshScratch, uGrad, vGrad);
-        if (e != cudaSuccess)
-            return fail(NSDG_ERR_CUDA, std::string("ssh gradient: ") + cudaGetErrorString(e));
-        launches += 3;
-    }
+    LCH(launchSSHGradient(s, dm, dops, ssh, sshScratch, sshScratch + Ncg1, sshScratch + 2 * Ncg1));
+    ++launches; // two kernels
     } // prep
     const int nS = P.n_steps;
+    // the transport's work arrays hold the cells' Lagrange values of h and A
+    // between the elements' and the nodes' preparation
+    double *const lagH = phiA, *const lagA = k1;
+    NodeInputs ni;
+    ni.constant = dg == 1;
+    ni.h = dg == 1 ? hice : lagH;
+    ni.a = dg == 1 ? cice : lagA;
+    ni.ug = sshScratch + Ncg1;
+    ni.vg = sshScratch + 2 * Ncg1;
+    ni.u = u; ni.v = v; ni.uo = uo; ni.vo = vo; ni.ua = ua; ni.va = va;
+    ni.invm2 = dops.invm2;
     if (!bbm) {
         const MevpParams mp = mevpParams(dt);
-        MevpNodeState st { u, v, u0, v0, cgH, cgA, uo, vo, ua, va, uGrad, vGrad, nodeA, nodeKu, nodeKv,
-            nodeIm };
+        MevpNodeState st { u, v, uo, vo, nodeA, nodeKu, nodeKv, nodeIm };
         if (prep) {
             // a full mixed-precision update also records the sub-cycle's
             // start (the warm-start features of the next update) inside
@@ -984,14 +992,14 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
                 po.visc = pressureOps ? Pg : nullptr;
                 po.half = hP32;
             }
-            LCH(launchMevpPrepElements(s, dm, dg, hice, cice, po, mp, save ? tdiv32 : nullptr,
+            LCH(launchMevpPrepElements(s, dm, dg, hice, cice, lagH, lagA, po, mp, save ? tdiv32 : nullptr,
                 save ? tdivLast : nullptr));
             // after the elements' preparation: the first stress kernel reads
             // its pressure before it waits for the launch just before it
             if (!mixed())
-                LCH(launchMevpPrepNodes(s, dm, st, dops.invm2, mp));
+                LCH(launchMevpPrepNodes(s, dm, ni, st, mp));
             else
-                LCH(launchMevpPrepNodes32(s, dm, st, st32, dops.invm2, mp, save ? uLast : nullptr,
+                LCH(launchMevpPrepNodes32(s, dm, ni, st32, mp, save ? uLast : nullptr,
                     save ? vLast : nullptr));
         }
         if (loop && mixed() && !prep) {
@@ -1025,12 +1033,13 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
             P.compaction_param, P.nu0, P.young, P.P0, P.undamaged_time_relaxation_sigma,
             P.exponent_relaxation_sigma, P.exponent_compression_factor, P.tan_phi, P.compr_strength, P.C_lab };
         bbmPowModes(bp);
-        BbmNodeState st { u, v, avgU, avgV, cgH, cgA, uo, vo, ua, va, uGrad, vGrad };
+        BbmNodeState st { u, v, avgU, avgV };
         auto subcycle = [&](auto& el, auto& node, auto* div) -> int {
             // the nodes' preparation last: the first stress kernel reads the
             // point values before it waits for the launch just before it
-            LCH(launchBbmLoad(s, dm, dg, el, hice, cice, damage, s11, s12, s22, dops.hsize, bp));
-            LCH(launchBbmPrepNodes(s, dm, st, node, dops.invm2, bp));
+            LCH(launchBbmLoad(s, dm, dg, el, hice, cice, damage, s11, s12, s22, dops.hsize, lagH, lagA,
+                bp));
+            LCH(launchBbmPrepNodes(s, dm, ni, st, node, bp));
             for (int it = 0; it < nS; ++it) {
                 LCH(launchBbmStress(s, dm, dg, el, node.u, node.v, div, bp, derr));
                 LCH(launchBbmMomentum(s, dm, st, node, div, bp, derr));
@@ -1506,9 +1515,8 @@ namespace {
 // targets t0, t1, as set_data of an H field does (CGDynamicsKernel.cpp:54-90)
 int cellsToNodes(nsdg_kernel* k, const double* f0, const double* f1, double* t0, double* t1)
 {
-    const double* in[2] = { f0, f1 };
-    double* out[2] = { t0, t1 };
-    const cudaError_t e = launchDG2CG(k->stream, k->dm, 1, 2, in, out);
+    const AverageFields f { { f0, f1 }, { t0, t1 }, 2 };
+    const cudaError_t e = launchAverage(k->stream, k->dm, f);
     return e == cudaSuccess ? NSDG_OK : k->fail(NSDG_ERR_CUDA, std::string("benchmark forcing: ") + cudaGetErrorString(e));
 }
 int forcingArgs(nsdg_kernel* k, const nsdg_benchmark_forcing* f)
@@ -1588,24 +1596,34 @@ void nsdg_kernel::storeField(const std::string& s, const double* data, size_t nC
     bucketComps[s] = static_cast<int>(nComp);
 }
 
-int nsdg_kernel::enqueueConversion(const SetTarget& t, const double* staging, size_t nComp)
+int nsdg_kernel::flushAverages(AverageFields& batch)
+{
+    const cudaError_t e = batch.count ? launchAverage(stream, dm, batch) : cudaSuccess;
+    batch = AverageFields();
+    return e == cudaSuccess ? NSDG_OK : fail(NSDG_ERR_CUDA, std::string("set_data convert: ") + cudaGetErrorString(e));
+}
+
+// The conversion of one staged input; node averages of one component are
+// collected in batch, which the caller flushes.
+int nsdg_kernel::enqueueConversion(const SetTarget& t, const double* staging, size_t nComp, AverageFields& batch)
 {
     cudaError_t e;
-    if (t.cg && nComp != size_t(dg)) {
+    if (t.cg && (nComp != size_t(dg) || dg == 1)) {
         // CGDynamicsKernel.cpp:54-90: ma2dg keeps component 0 only, so DG2CG
         // of the one-component field gives the same node values (the higher
         // components' contributions are exact zeros)
-        const double* in[1] = { staging };
-        double* out[1] = { t.cg };
-        e = launchDG2CG(stream, dm, 1, 1, in, out);
-    } else if (t.cg) {
+        batch.src[batch.count] = staging;
+        batch.dst[batch.count] = t.cg;
+        return ++batch.count == kAverageFields ? flushAverages(batch) : NSDG_OK;
+    }
+    const int r = flushAverages(batch); // targets are written in the inputs' order
+    if (r)
+        return r;
+    if (t.cg) {
         // CGDynamicsKernel.cpp:54-90: ma2dg into a DG vector, then DG2CG
         e = launchAosToSoa(stream, N, static_cast<int>(nComp), dg, staging, dgTmp);
-        if (e == cudaSuccess) {
-            const double* in[1] = { dgTmp };
-            double* out[1] = { t.cg };
-            e = launchDG2CG(stream, dm, dg, 1, in, out);
-        }
+        if (e == cudaSuccess)
+            e = launchDG2CG(stream, dm, dg, dgTmp, t.cg);
     } else {
         e = launchAosToSoa(stream, N, static_cast<int>(nComp), t.comps, staging, t.dg);
     }
@@ -1660,8 +1678,11 @@ int nsdg_kernel_set_data(nsdg_kernel* k, const char* name, const double* data, s
         return r;
     }
     r = cu(cudaStreamWaitEvent(st, k->copied, 0), "set_data wait");
+    AverageFields average;
     if (r == NSDG_OK)
-        r = k->enqueueConversion(target, staging, n_comp);
+        r = k->enqueueConversion(target, staging, n_comp, average);
+    if (r == NSDG_OK)
+        r = k->flushAverages(average);
     // recorded after whatever reads this staging buffer, also on a failure
     const cudaError_t er = cudaEventRecord(k->converted[slot], st);
     if (r == NSDG_OK)
@@ -1721,7 +1742,7 @@ int nsdg_kernel::enqueueReadout(const std::string& s, double* out, HostMoves* ba
             const double rad = 0x1.1df46a2529d39p-6;
             const double ang = bbm ? P.ocean_turning_angle : 0.0;
             double* tx = cgTmp;
-            double* ty = u0; // reused as scratch outside update
+            double* ty = cgTmp2;
             e = launchIceOceanStress(stream, Ncg, bbm ? 1 : 0, bbm ? avgU : u, bbm ? avgV : v, uo, vo, P.F_ocean,
                 std::cos(rad * ang), std::sin(rad * ang), tx, ty, mixed());
             const double* in[2] = { tx, ty };
@@ -1871,12 +1892,15 @@ int nsdg_kernel_module_step(nsdg_kernel* k, const nsdg_field_in* in, size_t n_in
         return r;
     }
     off = 0;
+    AverageFields averages;
     for (size_t i = 0; i < n_in && r == NSDG_OK; ++i) {
         if (!targets[i].cg && !targets[i].dg)
             continue;
-        r = k->enqueueConversion(targets[i], k->moduleStage + off, in[i].n_comp);
+        r = k->enqueueConversion(targets[i], k->moduleStage + off, in[i].n_comp, averages);
         off += N * in[i].n_comp;
     }
+    if (r == NSDG_OK)
+        r = k->flushAverages(averages);
     if (r == NSDG_OK)
         r = k->launchStep(dt);
     HostMoves outMoves; // pageable outputs, written by one kernel
@@ -2100,8 +2124,7 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
     const double dt = k->graphDt > 0 ? k->graphDt : 120.0;
     MevpParams mp { k->P.rho_ice, k->P.F_atm, k->P.F_ocean, k->P.fc, k->P.gravity, k->P.Pstar, k->P.DeltaMin,
         k->P.alpha, k->P.beta, dt };
-    MevpNodeState st { k->u, k->v, k->u0, k->v0, k->cgH, k->cgA, k->uo, k->vo, k->ua, k->va, k->uGrad,
-        k->vGrad, k->nodeA, k->nodeKu, k->nodeKv, k->nodeIm };
+    MevpNodeState st { k->u, k->v, k->uo, k->vo, k->nodeA, k->nodeKu, k->nodeKv, k->nodeIm };
     const double rad = 0x1.1df46a2529d39p-6;
     BbmParams bp { k->P.rho_ice, k->P.F_atm, k->P.F_ocean, k->P.fc, k->P.gravity, dt / k->P.n_steps,
         double(k->P.n_steps), std::cos(rad * k->P.ocean_turning_angle), std::sin(rad * k->P.ocean_turning_angle),
@@ -2109,7 +2132,7 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
         k->P.exponent_relaxation_sigma, k->P.exponent_compression_factor, k->P.tan_phi, k->P.compr_strength,
         k->P.C_lab };
     bbmPowModes(bp);
-    BbmNodeState bs { k->u, k->v, k->avgU, k->avgV, k->cgH, k->cgA, k->uo, k->vo, k->ua, k->va, k->uGrad, k->vGrad };
+    BbmNodeState bs { k->u, k->v, k->avgU, k->avgV };
     const size_t dN = size_t(k->dg) * k->N;
     StageFields a;
     a.nf = bbm ? 3 : 2;

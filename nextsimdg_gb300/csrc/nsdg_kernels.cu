@@ -1155,9 +1155,9 @@ __global__ void __launch_bounds__(kTrX * kTrY, 4) kTransportStageAffine(Transpor
 // reference's reversed-parity stripes), cells in ascending x; then the
 // boundary rows and columns are doubled.
 // ===========================================================================
-template <int DG, int NF>
-__global__ void __launch_bounds__(kBlock) kDG2CG(DevMesh m, const double* __restrict__ in0,
-    const double* __restrict__ in1, double* __restrict__ out0, double* __restrict__ out1)
+template <int DG>
+__global__ void __launch_bounds__(kBlock) kDG2CG(DevMesh m, const double* __restrict__ in,
+    double* __restrict__ out)
 {
     const size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
     if (t >= m.Ncg)
@@ -1173,11 +1173,7 @@ __global__ void __launch_bounds__(kBlock) kDG2CG(DevMesh m, const double* __rest
         Y.c1 = c;
         Y.l1 = l;
     }
-    const double* in[2] = { in0, in1 };
-    double acc[NF];
-#pragma unroll
-    for (int f = 0; f < NF; ++f)
-        acc[f] = 0.0;
+    double acc = 0.0;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         if (r >= Y.n)
@@ -1190,19 +1186,16 @@ __global__ void __launch_bounds__(kBlock) kDG2CG(DevMesh m, const double* __rest
             const int cx = k ? X.c1 : X.c0, lx = k ? X.l1 : X.l0;
             const size_t c = size_t(cy) * m.nx + cx;
             const int q = lx + 3 * ly;
+            double at = 0.0;
 #pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                double at = 0.0;
-#pragma unroll
-                for (int j = 0; j < DG; ++j)
-                    at += in[f][j * m.N + c] * cT.psiLag3[j][q];
-                if (q == 4)
-                    acc[f] += at;
-                else if (q == 1 || q == 3 || q == 5 || q == 7)
-                    acc[f] += 0.5 * at;
-                else
-                    acc[f] += 0.25 * at;
-            }
+            for (int j = 0; j < DG; ++j)
+                at += in[j * m.N + c] * cT.psiLag3[j][q];
+            if (q == 4)
+                acc += at;
+            else if (q == 1 || q == 3 || q == 5 || q == 7)
+                acc += 0.5 * at;
+            else
+                acc += 0.25 * at;
         }
     }
     double scale = 1.0;
@@ -1210,208 +1203,12 @@ __global__ void __launch_bounds__(kBlock) kDG2CG(DevMesh m, const double* __rest
         scale *= 2.0;
     if (i2 == 0 || i2 == 2 * m.nx)
         scale *= 2.0;
-    out0[t] = acc[0] * scale;
-    if constexpr (NF > 1)
-        out1[t] = acc[1] * scale;
-}
-
-// ===========================================================================
-// Sea-surface-height gradient (CGDynamicsKernel.cpp:126-258)
-// ===========================================================================
-// CG1 Lagrange average of the DG0 ssh (reversed parity: odd rows first)
-__global__ void __launch_bounds__(kBlock) kSSHToCG1(DevMesh m, const double* __restrict__ ssh, double* __restrict__ cg1)
-{
-    const size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (t >= m.Ncg1)
-        return;
-    const unsigned s1 = static_cast<unsigned>(m.nx) + 1u;
-    const int i1 = static_cast<int>(static_cast<unsigned>(t) % s1), j1 = static_cast<int>(static_cast<unsigned>(t) / s1);
-    // the cell rows touching the node, odd rows first (registers, no local arrays)
-    const bool below = j1 >= 1, above = j1 < m.ny;
-    const int nr = int(below) + int(above);
-    int row0 = below ? j1 - 1 : j1, row1 = j1;
-    if (nr == 2 && (row0 % 2) == 0) {
-        row0 = j1;
-        row1 = j1 - 1;
-    }
-    double acc = 0.0;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        if (r >= nr)
-            continue;
-        const int row = r ? row1 : row0;
-        for (int cx = i1 - 1; cx <= i1; ++cx) {
-            if (cx < 0 || cx >= m.nx)
-                continue;
-            acc += 0.25 * ssh[size_t(row) * m.nx + cx];
-        }
-    }
-    double scale = 1.0;
-    if (j1 == 0 || j1 == m.ny)
-        scale *= 2.0;
-    if (i1 == 0 || i1 == m.nx)
-        scale *= 2.0;
-    cg1[t] = acc * scale;
-}
-// CG1 gradient by element gather (even rows first), divided by the lumped mass
-__global__ void __launch_bounds__(kBlock) kSSHGrad1(DevMesh m, DevOps o, const double* __restrict__ cg1,
-    double* __restrict__ ug, double* __restrict__ vg)
-{
-    const size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (t >= m.Ncg1)
-        return;
-    const unsigned s1 = static_cast<unsigned>(m.nx) + 1u;
-    const int i1 = static_cast<int>(static_cast<unsigned>(t) % s1), j1 = static_cast<int>(static_cast<unsigned>(t) / s1);
-    // the cell rows touching the node with the node's local row in each, even
-    // rows first (registers, no local arrays)
-    const bool below = j1 >= 1, above = j1 < m.ny;
-    const int nr = int(below) + int(above);
-    int row0 = below ? j1 - 1 : j1, ly0 = below ? 1 : 0, row1 = j1, ly1 = 0;
-    if (nr == 2 && (row0 % 2) == 1) {
-        row0 = j1;
-        ly0 = 0;
-        row1 = j1 - 1;
-        ly1 = 1;
-    }
-    double au = 0.0, av = 0.0;
-    const size_t N = m.N;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        if (r >= nr)
-            continue;
-        for (int lx = 1; lx >= 0; --lx) {
-            const int cx = i1 - lx;
-            if (cx < 0 || cx >= m.nx)
-                continue;
-            const int cy = r ? row1 : row0, ly = r ? ly1 : ly0;
-            const size_t e = size_t(cy) * m.nx + cx;
-            const size_t n0 = size_t(cy) * s1 + cx;
-            const double loc[4] = { cg1[n0], cg1[n0 + 1], cg1[n0 + s1], cg1[n0 + s1 + 1] };
-            const int k = lx + 2 * ly;
-            double tx = 0.0, ty = 0.0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                tx += o.dxssh[(k * 4 + j) * N + e] * loc[j];
-                ty += o.dyssh[(k * 4 + j) * N + e] * loc[j];
-            }
-            au -= tx;
-            av -= ty;
-        }
-    }
-    ug[t] = au / o.lumped1[t];
-    vg[t] = av / o.lumped1[t];
-}
-// boundary extension of the CG1 gradient (the value a boundary node copies
-// from the neighbouring interior node) followed by CG1 -> CG2 interpolation
-__device__ __forceinline__ size_t sshSource(int i1, int j1, int nx, int ny)
-{
-    int si = i1, sj = j1;
-    if (i1 == 0) si = 1;
-    if (i1 == nx) si = nx - 1;
-    if (j1 == 0) sj = 1;
-    if (j1 == ny) sj = ny - 1;
-    return size_t(sj) * (nx + 1) + si;
-}
-__global__ void __launch_bounds__(kBlock) kSSHToCG2(DevMesh m, const double* __restrict__ ug,
-    const double* __restrict__ vg, double* __restrict__ uGrad, double* __restrict__ vGrad)
-{
-    const size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (t >= m.Ncg)
-        return;
-    const int s2 = 2 * m.nx + 1;
-    const int i2 = static_cast<int>(static_cast<unsigned>(t) % static_cast<unsigned>(s2)), j2 = static_cast<int>(static_cast<unsigned>(t) / static_cast<unsigned>(s2));
-    const int nx = m.nx, ny = m.ny;
-    const int ix = i2 / 2, iy = j2 / 2;
-    double u, v;
-    if (!(i2 & 1) && !(j2 & 1)) {
-        const size_t a = sshSource(ix, iy, nx, ny);
-        u = ug[a];
-        v = vg[a];
-    } else if ((i2 & 1) && !(j2 & 1)) {
-        const size_t a = sshSource(ix, iy, nx, ny), b = sshSource(ix + 1, iy, nx, ny);
-        u = 0.5 * (ug[a] + ug[b]);
-        v = 0.5 * (vg[a] + vg[b]);
-    } else if (!(i2 & 1) && (j2 & 1)) {
-        const size_t a = sshSource(ix, iy, nx, ny), b = sshSource(ix, iy + 1, nx, ny);
-        u = 0.5 * (ug[a] + ug[b]);
-        v = 0.5 * (vg[a] + vg[b]);
-    } else {
-        const size_t a = sshSource(ix, iy, nx, ny), b = sshSource(ix + 1, iy, nx, ny);
-        const size_t c = sshSource(ix, iy + 1, nx, ny), d = sshSource(ix + 1, iy + 1, nx, ny);
-        u = 0.25 * (ug[a] + ug[b] + ug[c] + ug[d]);
-        v = 0.25 * (vg[a] + vg[b] + vg[c] + vg[d]);
-    }
-    uGrad[t] = u;
-    vGrad[t] = v;
+    out[t] = acc * scale;
 }
 
 // ===========================================================================
 // mEVP
 // ===========================================================================
-__global__ void __launch_bounds__(kBlock) kMevpPrepNodes(size_t n, MevpNodeState st,
-    const double* __restrict__ invm2, MevpParams p)
-{
-    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i >= n)
-        return;
-    // clamps of prepareIteration (CGDynamicsKernel.cpp:273-275)
-    const double A = fmax(fmin(st.cgA[i], 1.0), 1.e-4);
-    const double H = fmax(st.cgH[i], 1.e-4);
-    st.cgA[i] = A;
-    st.cgH[i] = H;
-    const double rhoH = p.rho_ice * H;
-    const double rc1 = p.dt / rhoH;
-    const double ua = st.ua[i], va = st.va[i];
-    const double fatm = p.F_atm * sqrt(ua * ua + va * va);
-    st.a[i] = A * p.F_ocean * rc1;
-    st.ku[i] = st.u[i] + (A * (fatm * ua) - rhoH * p.gravity * st.uGrad[i]) * rc1;
-    st.kv[i] = st.v[i] + (A * (fatm * va) - rhoH * p.gravity * st.vGrad[i]) * rc1;
-    st.im[i] = invm2[i] * rc1;
-}
-
-template <int DG>
-__global__ void __launch_bounds__(kBlock) kMevpPrepElements(size_t N, const double* __restrict__ h,
-    const double* __restrict__ a, PressureOut out, double Pstar, double invAlpha, const float* __restrict__ tdiv32,
-    float* __restrict__ tdivLast)
-{
-    const size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (e >= N)
-        return;
-    if (tdivLast) // the divergence at the start of this sub-cycle (warm-start features)
-#pragma unroll
-        for (int k = 0; k < 18; ++k)
-            tdivLast[k * N + e] = tdiv32[k * N + e];
-    double hc[DG], ac[DG];
-    loadCell<DG>(h, N, e, hc);
-    loadCell<DG>(a, N, e, ac);
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        double hs = 0.0, as = 0.0;
-#pragma unroll
-        for (int j = 0; j < DG; ++j) {
-            hs += hc[j] * cT.psi[3][j][q];
-            as += ac[j] * cT.psi[3][j][q];
-        }
-        const double hq = fmax(hs, 0.0);
-        const double aq = fmin(fmax(as, 0.0), 1.0);
-        const double pa = Pstar * hq * exp(-20.0 * (1.0 - aq)) * invAlpha;
-        const size_t at = q * N + e;
-        if (out.weighted)
-            out.weighted[at] = 0.25 * pa * out.w[at];
-        if (out.weightedPair) {
-            const double x = 0.25 * pa * out.w[at];
-            const float hi = static_cast<float>(x);
-            out.weightedPair[at] = make_float2(hi, static_cast<float>(x - static_cast<double>(hi)));
-        }
-        if (out.alpha)
-            out.alpha[at] = pa;
-        if (out.visc) {
-            out.visc[at] = 0.125 * pa;
-            out.half[at] = static_cast<float>(0.5 * pa);
-        }
-    }
-}
-
 // One mEVP iteration, element part, carried in divergence space.
 //
 // The reference updates the stress coefficients s (8 per component,
@@ -1476,46 +1273,6 @@ __global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, MevpNodeState
 // ===========================================================================
 // mEVP, mixed precision
 // ===========================================================================
-__global__ void __launch_bounds__(kBlock) kMevpPrepNodes32(size_t n, MevpNodeState st, MevpNodeState32 f,
-    const double* __restrict__ invm2, const uint8_t* __restrict__ dir, MevpParams p, float* __restrict__ uLast,
-    float* __restrict__ vLast)
-{
-    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-    if (i >= n)
-        return;
-    // clamps of prepareIteration (CGDynamicsKernel.cpp:273-275)
-    const double A = fmax(fmin(st.cgA[i], 1.0), 1.e-4);
-    const double H = fmax(st.cgH[i], 1.e-4);
-    st.cgA[i] = A;
-    st.cgH[i] = H;
-    const double u = st.u[i], v = st.v[i];
-    st.u0[i] = u;
-    st.v0[i] = v;
-    // c1 = rho H / dt and its reciprocal: one FP64 division per node
-    const double rhoH = p.rho_ice * H;
-    const double rc1 = p.dt / rhoH;
-    const double ua = st.ua[i], va = st.va[i];
-    const double fatm = p.F_atm * sqrt(ua * ua + va * va);
-    const float uf = static_cast<float>(u), vf = static_cast<float>(v);
-    f.u[i] = uf;
-    f.v[i] = vf;
-    f.u0[i] = uf;
-    f.v0[i] = vf;
-    if (uLast) { // the velocity at the start of this sub-cycle (warm-start features)
-        uLast[i] = uf;
-        vLast[i] = vf;
-    }
-    // u0 + (A F_atm |wind| uwind - rho H g dxSSH) / c1, in FP64
-    const double ku = u + (A * (fatm * ua) - rhoH * p.gravity * st.uGrad[i]) * rc1;
-    const double kv = v + (A * (fatm * va) - rhoH * p.gravity * st.vGrad[i]) * rc1;
-    const double im = invm2[i] * rc1;
-    const float hi = static_cast<float>(im);
-    f.k0[i] = make_float4(static_cast<float>(A * rc1), static_cast<float>(ku), static_cast<float>(kv),
-        static_cast<float>(st.uo[i]));
-    f.k1[i] = make_float4(static_cast<float>(st.vo[i]), hi, static_cast<float>(im - static_cast<double>(hi)),
-        dir[i] ? 1.f : 0.f);
-}
-
 // ---------------------------------------------------------------------------
 // TMA-staged FP32 stress kernel
 // ---------------------------------------------------------------------------
@@ -2135,48 +1892,10 @@ cudaError_t launchTransportStageAffine(cudaStream_t s, const DevMesh& m, int dg,
     return cudaGetLastError();
 }
 
-cudaError_t launchDG2CG(cudaStream_t s, const DevMesh& m, int dg, int nf, const double* const* dgIn,
-    double* const* cgOut)
+cudaError_t launchDG2CG(cudaStream_t s, const DevMesh& m, int dg, const double* dgIn, double* cgOut)
 {
     const unsigned g = blocksFor(m.Ncg);
-    if (nf == 1) {
-        NSDG_DG_SWITCH(dg, (kDG2CG<D, 1><<<g, kBlock, 0, s>>>(m, dgIn[0], nullptr, cgOut[0], nullptr)));
-    } else {
-        NSDG_DG_SWITCH(dg, (kDG2CG<D, 2><<<g, kBlock, 0, s>>>(m, dgIn[0], dgIn[1], cgOut[0], cgOut[1])));
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launchSSHGradient(cudaStream_t s, const DevMesh& m, const DevOps& o, const double* ssh,
-    double* scratch, double* uGrad, double* vGrad)
-{
-    double* cg1 = scratch;
-    double* ug = scratch + m.Ncg1;
-    double* vg = scratch + 2 * m.Ncg1;
-    kSSHToCG1<<<blocksFor(m.Ncg1), kBlock, 0, s>>>(m, ssh, cg1);
-    kSSHGrad1<<<blocksFor(m.Ncg1), kBlock, 0, s>>>(m, o, cg1, ug, vg);
-    kSSHToCG2<<<blocksFor(m.Ncg), kBlock, 0, s>>>(m, ug, vg, uGrad, vGrad);
-    return cudaGetLastError();
-}
-
-cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* invm2,
-    const MevpParams& p)
-{
-    kMevpPrepNodes<<<blocksFor(m.Ncg), kBlock, 0, s>>>(m.Ncg, st, invm2, p);
-    return cudaGetLastError();
-}
-
-cudaError_t launchMevpPrepElements(cudaStream_t s, const DevMesh& m, int dg, const double* h,
-    const double* a, const PressureOut& out, const MevpParams& p, const float* tdiv32, float* tdivLast)
-{
-    const unsigned g = blocksFor(m.N);
-    const double ia = 1.0 / p.alpha;
-    switch (dg) {
-    case 1: kMevpPrepElements<1><<<g, kBlock, 0, s>>>(m.N, h, a, out, p.Pstar, ia, tdiv32, tdivLast); break;
-    case 3: kMevpPrepElements<3><<<g, kBlock, 0, s>>>(m.N, h, a, out, p.Pstar, ia, tdiv32, tdivLast); break;
-    case 6: kMevpPrepElements<6><<<g, kBlock, 0, s>>>(m.N, h, a, out, p.Pstar, ia, tdiv32, tdivLast); break;
-    default: return cudaErrorInvalidValue;
-    }
+    NSDG_DG_SWITCH(dg, (kDG2CG<D><<<g, kBlock, 0, s>>>(m, dgIn, cgOut)));
     return cudaGetLastError();
 }
 
@@ -2196,12 +1915,6 @@ cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const MevpNodeS
     return cudaLaunchKernelEx(&cfg, kMevpMomentum, m, st, contrib, p, err);
 }
 
-cudaError_t launchMevpPrepNodes32(cudaStream_t s, const DevMesh& m, const MevpNodeState& st64,
-    const MevpNodeState32& st32, const double* invm2, const MevpParams& p, float* uLast, float* vLast)
-{
-    kMevpPrepNodes32<<<blocksFor(m.Ncg), kBlock, 0, s>>>(m.Ncg, st64, st32, invm2, m.cg2Dir, p, uLast, vLast);
-    return cudaGetLastError();
-}
 namespace {
 template <bool SPH> constexpr size_t tmaSmem() { return size_t(tmaTileBytes<SPH>()) + 3 * 9 * kTmaElems * 4 + 2 * 8; }
 constexpr size_t kTmaSmem = tmaSmem<false>();

@@ -53,7 +53,7 @@ struct DevOps {
     const double* dyssh = nullptr;
     const double* hsize = nullptr;
     const double* invm2 = nullptr;   // 1 / lumped CG2 mass
-    const double* lumped1 = nullptr; // lumped CG1 mass
+    const double* invm1 = nullptr;   // 1 / lumped CG1 mass
     // spherical metric terms (null on Cartesian meshes)
     const double* minvP = nullptr;   // CG2DG inverse mass (the transport's minv carries 1 / R)
     const double* minv8P = nullptr;
@@ -118,30 +118,40 @@ cudaError_t launchTransportStageAffine(cudaStream_t s, const DevMesh& m, int dg,
     int mode, double dt, const StageFields& f);
 
 // --- interpolation / preparation ----------------------------------------
-// DG -> CG2 Lagrange averaging of nf (<=2) DG fields (Interpolations.cpp:144-204).
-cudaError_t launchDG2CG(cudaStream_t s, const DevMesh& m, int dg, int nf,
-    const double* const* dgIn, double* const* cgOut);
-// Gradient of the sea-surface height on CG2 (CGDynamicsKernel.cpp:126-258);
-// scratch needs 3*Ncg1 doubles.
-cudaError_t launchSSHGradient(cudaStream_t s, const DevMesh& m, const DevOps& o, const double* ssh,
-    double* scratch, double* uGrad, double* vGrad);
+// DG -> CG2 Lagrange averaging of a DG field (Interpolations.cpp:144-204).
+cudaError_t launchDG2CG(cudaStream_t s, const DevMesh& m, int dg, const double* dgIn, double* cgOut);
+// CG2 node values of up to four one-component fields (DG2CG of DG 1).
+constexpr int kAverageFields = 4;
+struct AverageFields {
+    const double* src[kAverageFields] = {};
+    double* dst[kAverageFields] = {};
+    int count = 0;
+};
+cudaError_t launchAverage(cudaStream_t s, const DevMesh& m, const AverageFields& f);
+// CG1 gradient of the sea-surface height (CGDynamicsKernel.cpp:126-204);
+// cg1, ug, vg: Ncg1 doubles each.
+cudaError_t launchSSHGradient(cudaStream_t s, const DevMesh& m, const DevOps& o, const double* ssh, double* cg1,
+    double* ug, double* vg);
 
-// mEVP per-step node constants (CGDynamicsKernel.cpp:260-276 clamps plus the
-// loop-invariant parts of VPCGDynamicsKernel.hpp:132-172).
+// What the nodes' preparation reads: thickness and concentration as Lagrange
+// values [9][N] of the cells (constant: one value per cell), the CG1 gradient
+// of the sea-surface height, and node fields.
+struct NodeInputs {
+    const double* h = nullptr;
+    const double* a = nullptr;
+    bool constant = false;
+    const double *ug = nullptr, *vg = nullptr;
+    const double *u = nullptr, *v = nullptr, *uo = nullptr, *vo = nullptr, *ua = nullptr, *va = nullptr;
+    const double* invm2 = nullptr; // 1 / lumped CG2 mass
+};
+// The FP64 mEVP node state and its step constants, over c1 = rho H / dt
+// (CGDynamicsKernel.cpp:260-276 clamps plus the loop-invariant parts of
+// VPCGDynamicsKernel.hpp:132-172).
 struct MevpNodeState {
     double* u;
     double* v;
-    double* u0;
-    double* v0;
-    double* cgH;     // in: DG2CG(h) ; out: clamped
-    double* cgA;     // in: DG2CG(A) ; out: clamped
     const double* uo;
     const double* vo;
-    const double* ua;
-    const double* va;
-    const double* uGrad;
-    const double* vGrad;
-    // the FP64 path's step constants, over c1 = rho H / dt:
     double* a;  // A F_ocean / c1
     double* ku; // u0 + (A F_atm |wind| uwind - rho H g dxSSH) / c1
     double* kv;
@@ -173,7 +183,7 @@ inline MevpParams withDerived(MevpParams p)
     p.fcdtf = static_cast<float>(p.fc * p.dt);
     return p;
 }
-cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* invm2,
+cudaError_t launchMevpPrepNodes(cudaStream_t s, const DevMesh& m, const NodeInputs& in, const MevpNodeState& st,
     const MevpParams& p);
 // P at the 3x3 Gauss points from h and A (MEVPStressUpdateStep.hpp:54-57,75-77),
 // in every form whose target is given ([9][N] each).
@@ -185,10 +195,11 @@ struct PressureOut {
     float2* weightedPair = nullptr; // the same as a pair of floats (mixed)
     const double* w = nullptr;      // StressMetric::w
 };
+// Also the Lagrange values of h and A (lagH, lagA: [9][N] each, dg > 1).
 // tdivLast (mixed precision, optional): also copies tdiv32 there (the
 // sub-cycle's starting divergence, a warm-start feature).
-cudaError_t launchMevpPrepElements(cudaStream_t s, const DevMesh& m, int dg, const double* h,
-    const double* a, const PressureOut& out, const MevpParams& p, const float* tdiv32 = nullptr,
+cudaError_t launchMevpPrepElements(cudaStream_t s, const DevMesh& m, int dg, const double* h, const double* a,
+    double* lagH, double* lagA, const PressureOut& out, const MevpParams& p, const float* tdiv32 = nullptr,
     float* tdivLast = nullptr);
 // One mEVP iteration, element part, carried in divergence space: the strain at
 // the Gauss points, Delta, and the relaxed update of the element's stress
@@ -303,12 +314,9 @@ struct MevpNodeState32 {
 };
 // The per-step node preparation of the mixed path (prepareIteration's clamps,
 // CGDynamicsKernel.cpp:260-276, and the constants of updateMomentum,
-// VPCGDynamicsKernel.hpp:132-172): FP64 inputs, the FP32 state above; the
-// clamped cgA, cgH and u0, v0 are written back in FP64.  invm2: the FP64
-// inverse lumped CG2 mass.
-cudaError_t launchMevpPrepNodes32(cudaStream_t s, const DevMesh& m, const MevpNodeState& st64,
-    const MevpNodeState32& st32, const double* invm2, const MevpParams& p,
-    float* uLast = nullptr, float* vLast = nullptr);
+// VPCGDynamicsKernel.hpp:132-172): FP64 inputs, the FP32 state above.
+cudaError_t launchMevpPrepNodes32(cudaStream_t s, const DevMesh& m, const NodeInputs& in, const MevpNodeState32& st32,
+    const MevpParams& p, float* uLast = nullptr, float* vLast = nullptr);
 // (the Dirichlet flags of the nodes come from m.cg2Dir)
 // The sum-factorised element kernels with FP32 state (nsdg_sumfact.cuh), Pw
 // the weighted pressure as pairs of floats: on parallelograms (4 coefficients
@@ -406,12 +414,17 @@ struct BbmParams {
     // how the kernels evaluate d^(n-1) (relaxation) and h^(m+1) (compression):
     // mode 1 = integer power k by multiplication, 2 = x^k sqrt(x), 0 = pow()
     int powRmode = 0, powRk = 0, powCmode = 0, powCk = 0;
-    double invNSteps = 0; // 1 / nSteps (set by bbmPowModes)
+    // set by bbmPowModes
+    double invNSteps = 0;   // 1 / nSteps
+    double soundRoot = 0;   // sqrt(2 (1 + nu0) rho)
+    double strainScale = 0; // 2 dt young / (1 - nu0^2)
 };
 // Sets the power modes of p from its exponents (integers and half-integers up to 8).
 inline void bbmPowModes(BbmParams& p)
 {
     p.invNSteps = 1.0 / p.nSteps;
+    p.soundRoot = std::sqrt(2. * (1. + p.nu0) * p.rho_ice);
+    p.strainScale = 2. * p.dt * p.young / (1. - p.nu0 * p.nu0);
     auto classify = [](double y, int& mode, int& k) {
         mode = 0;
         k = 0;
@@ -436,14 +449,6 @@ struct BbmNodeState {
     double* v;
     double* avgU;
     double* avgV;
-    double* cgH;
-    double* cgA;
-    const double* uo;
-    const double* vo;
-    const double* ua;
-    const double* va;
-    const double* uGrad;
-    const double* vGrad;
 };
 // The BBM sub-cycle (nsdg_bbm.cu), T = double or, on the mixed path, float.
 // Step constants and point values at the 3 x 3 Gauss points.
@@ -468,13 +473,13 @@ constexpr int kBbmElems = 32; // elements per block
 template <typename T>
 cudaError_t launchBbmLoad(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, const double* h,
     const double* a, const double* damage, const double* s11, const double* s12, const double* s22,
-    const double* hsize, const BbmParams& p);
+    const double* hsize, double* lagH, double* lagA, const BbmParams& p);
 template <typename T>
 cudaError_t launchBbmStore(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, double* damage,
     double* s11, double* s12, double* s22);
 template <typename T>
-cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const BbmNodeState& st, const BbmNodeConst<T>& c,
-    const double* invm2, const BbmParams& p);
+cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const NodeInputs& in, const BbmNodeState& st,
+    const BbmNodeConst<T>& c, const BbmParams& p);
 // contrib: [18][N], zero on land
 template <typename T>
 cudaError_t launchBbmStress(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, const T* u,
