@@ -110,7 +110,8 @@ struct nsdg_kernel {
     double *Pg = nullptr, *contrib = nullptr;
     // the element maps of the sum-factorised stress kernels, the weights and
     // the weighted pressure (FP64, or pairs of floats on the mixed path)
-    StressGeometry<double> geo {};
+    StressGeometry<double> geo {}; // BBM
+    FixedGeometry fixedGeo {};     // mEVP
     StressGeometry<float> quad32 {}, aff32 {};
     const double* metricW = nullptr;
     double* Pw = nullptr;
@@ -400,6 +401,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     stepNumber = 0;
     readCache = 0;
     geo = {};
+    fixedGeo = {};
     quad32 = {};
     aff32 = {};
     Pw = nullptr;
@@ -483,7 +485,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     buildStressMetric(mesh, P.precision == NSDG_PRECISION_FP64, metric);
     {
         const size_t sz = P.precision == NSDG_PRECISION_FP64 ? 8 : 4;
-        add(metric.k.size(), sz); add(metric.n.size(), sz); add(metric.m.size(), sz);
+        add(metric.k.size(), sz); add(metric.n.size(), sz); add(metric.m.size(), sz); add(N, 4);
         add(4 * N, 4);                            // the same on parallelograms
         add(9 * N); add(9 * N);                   // weights, weighted pressure
         if (bbm) {
@@ -589,11 +591,22 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         dops.hsize = upd(ops.hsize);
     }
     metricW = upd(metric.w);
-    if (!mixed()) {
+    if (!mixed() && (bbm || metric.rect)) {
         geo.rect = metric.rect;
         geo.k = upd(metric.k);
         geo.n = metric.n.empty() ? nullptr : upd(metric.n);
         geo.m = metric.m.empty() ? nullptr : upd(metric.m);
+        fixedGeo.rect = geo.k;
+    } else if (!mixed()) {
+        FixedMetric fixed;
+        buildFixedMetric(metric, N, fixed);
+        auto upi = [&](const std::vector<long long>& src) {
+            return src.empty() ? nullptr : static_cast<const long long*>(up(src.data(), src.size(), 8, e));
+        };
+        fixedGeo.k = upi(fixed.k);
+        fixedGeo.n = upi(fixed.n);
+        fixedGeo.m = upi(fixed.m);
+        fixedGeo.exponent = static_cast<const int*>(up(fixed.exponent.data(), N, 4, e));
     }
     if (e != cudaSuccess)
         return fail(NSDG_ERR_CUDA, std::string("initialise: upload failed: ") + cudaGetErrorString(e));
@@ -1016,7 +1029,7 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
                     else if (opsPairs && fp64Stress == 1)
                         LCH(launchMevpStressPairs(s, dm, opsPairs, pairsLdN, u, v, Pg, contrib, mp));
                     else
-                        LCH(launchMevpStress(s, dm, geo, u, v, Pw, contrib, mp));
+                        LCH(launchMevpStress(s, dm, fixedGeo, u, v, Pw, contrib, mp));
                     LCH(launchMevpMomentum(s, dm, st, contrib, mp, derr));
                 } else {
                     LCH(launchStress32(s, mp, derr));
@@ -2159,9 +2172,9 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
             if (k->opsPairs && k->fp64Stress == 1)
                 return launchMevpStressPairs(k->stream, k->dm, k->opsPairs, k->pairsLdN, k->u, k->v, k->Pg,
                     k->contrib, mp);
-            return launchMevpStress(k->stream, k->dm, k->geo, k->u, k->v, k->Pw, k->contrib, mp);
+            return launchMevpStress(k->stream, k->dm, k->fixedGeo, k->u, k->v, k->Pw, k->contrib, mp);
         case 9:
-            return launchMevpStress(k->stream, k->dm, k->geo, k->u, k->v, k->Pw, k->contrib, mp);
+            return launchMevpStress(k->stream, k->dm, k->fixedGeo, k->u, k->v, k->Pw, k->contrib, mp);
         case 10:
             return launchMevpStressPairs(k->stream, k->dm, k->opsPairs, k->pairsLdN, k->u, k->v, k->Pg, k->contrib,
                 mp);

@@ -435,6 +435,32 @@ void transportOps(const HostMesh& m, int dg, ElementOps& ops, unsigned threads)
 
 } // namespace
 
+void buildFixedMetric(const StressMetric& s, size_t N, FixedMetric& out, unsigned threads)
+{
+    out.k.resize(s.k.size());
+    out.n.resize(s.n.size());
+    out.m.resize(s.m.size());
+    out.exponent.assign(N, 0);
+    parallelFor(N, threads, [&](size_t lo, size_t hi) {
+        for (size_t e = lo; e < hi; ++e) {
+            double most = 0.0;
+            for (size_t i = e; i < s.k.size(); i += N)
+                most = std::max(most, std::fabs(s.k[i]));
+            for (size_t i = e; i < s.m.size(); i += N)
+                most = std::max(most, std::fabs(s.m[i]));
+            int x;
+            std::frexp(most, &x);
+            out.exponent[e] = x;
+            for (size_t i = e; i < s.k.size(); i += N)
+                out.k[i] = std::llrint(std::ldexp(s.k[i], 62 - x));
+            for (size_t i = e; i < s.m.size(); i += N)
+                out.m[i] = std::llrint(std::ldexp(s.m[i], 62 - x));
+            for (size_t i = e; i < s.n.size(); i += N)
+                out.n[i] = std::llrint(std::ldexp(s.n[i], 62));
+        }
+    });
+}
+
 void buildStressMetric(const HostMesh& m, bool allowRect, StressMetric& out, unsigned threads)
 {
     const Basis& b = basis();
@@ -444,6 +470,18 @@ void buildStressMetric(const HostMesh& m, bool allowRect, StressMetric& out, uns
     for (size_t j = 0; j <= ny && out.rect; ++j)
         for (size_t i = 0; i <= nx && out.rect; ++i)
             out.rect = m.vx[j * sv + i] == m.vx[i] && m.vy[j * sv + i] == m.vy[j * sv];
+    if (out.rect) { // the rectangles' fixed-point maps take side ratios up to kRectRatio
+        double hx[2] = { m.vx[1] - m.vx[0], m.vx[1] - m.vx[0] }, hy[2] = { m.vy[sv] - m.vy[0], m.vy[sv] - m.vy[0] };
+        for (size_t i = 0; i < nx; ++i) {
+            hx[0] = std::min(hx[0], m.vx[i + 1] - m.vx[i]);
+            hx[1] = std::max(hx[1], m.vx[i + 1] - m.vx[i]);
+        }
+        for (size_t j = 0; j < ny; ++j) {
+            hy[0] = std::min(hy[0], m.vy[(j + 1) * sv] - m.vy[j * sv]);
+            hy[1] = std::max(hy[1], m.vy[(j + 1) * sv] - m.vy[j * sv]);
+        }
+        out.rect = hx[0] > 0.0 && hy[0] > 0.0 && hx[1] < kRectRatio * hy[0] && hy[1] < kRectRatio * hx[0];
+    }
     out.k.assign((out.rect ? 2 : 36) * N, 0.0);
     out.w.assign(9 * N, 0.0);
     if (!out.rect)

@@ -126,9 +126,11 @@ void buildElementOps(const HostMesh& m, int dg, bool stressTransport, ElementOps
 //   n = W^{-1} nu / (nu W^{-1} nu),  W = w J [cos lat],  nu = (1,-2,1) x (1,-2,1)
 //   m = tan(lat) / (2 R)                              (spherical meshes)
 //   w = 2 w_q J
-// A mesh whose vertices form a tensor grid (rect) has k_x = 1 / (2 dx) and
+// A mesh whose vertices form a tensor grid with k_y / k_x and k_x / k_y below
+// kRectRatio (rect) has k_x = 1 / (2 dx) and
 // k_y = 1 / (2 dy) at every point and needs no n: it keeps k = (k_y / k_x,
 // 1 / k_x^2) per element, and w = 2 w_q J k_x.
+constexpr double kRectRatio = 32.0;
 struct StressMetric {
     bool rect = false;
     std::vector<double> k; // [2][N] (rect) or [4][9][N]
@@ -138,6 +140,14 @@ struct StressMetric {
 };
 // With allowRect false the general form is built on every mesh.
 void buildStressMetric(const HostMesh& m, bool allowRect, StressMetric& out, unsigned threads = 0);
+// The general form as integers for the FP64 element kernel
+// (nsdg_stress_fixed.cuh): per element |k| and |m| below 2^exponent, k and m as
+// multiples of 2^(exponent - 62), n (below 1) of 2^-62.
+struct FixedMetric {
+    std::vector<long long> k, n, m;
+    std::vector<int> exponent;
+};
+void buildFixedMetric(const StressMetric& s, size_t N, FixedMetric& out, unsigned threads = 0);
 // The largest relative difference between an element's operators (gx, gy,
 // a1, a2 and on a sphere gm, a3 of `ops`) and those rebuilt from `s`.
 double stressMetricMismatch(const HostMesh& m, const ElementOps& ops, const StressMetric& s, unsigned threads = 0);

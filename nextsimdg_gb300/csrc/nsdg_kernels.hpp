@@ -208,13 +208,20 @@ cudaError_t launchMevpPrepElements(cudaStream_t s, const DevMesh& m, int dg, con
 // MEVPStressUpdateStep.hpp:30-118), by sum factorisation (nsdg_sumfact.cuh).
 // Device copy of StressMetric (nsdg_host.hpp).
 template <typename T> struct StressGeometry {
-    const T* k = nullptr; // [2][N] on rectangles (FP64), [4][N] on parallelograms (FP32), else [4][9][N]
+    const T* k = nullptr; // [2][N] on rectangles (FP64 BBM), [4][N] on parallelograms (FP32), else [4][9][N]
     const T* n = nullptr; // [9][N] (null on rectangles and parallelograms)
     const T* m = nullptr; // [9][N] (spherical meshes)
     bool rect = false;
 };
+// The map for the FP64 mEVP kernel (nsdg_stress_fixed.cuh): StressMetric::k on
+// rectangles, else device copies of FixedMetric (m on a sphere).
+struct FixedGeometry {
+    const double* rect = nullptr;
+    const long long *k = nullptr, *n = nullptr, *m = nullptr;
+    const int* exponent = nullptr;
+};
 // Pw holds w P/(4 alpha) at the Gauss points.
-cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const StressGeometry<double>& geo, const double* u,
+cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const FixedGeometry& geo, const double* u,
     const double* v, const double* Pw, double* tdiv, const MevpParams& p);
 // The benchmark forcing on the cell centres (nsdg_forcing.cu):
 // BenchmarkAtmosphere.cpp:29-77 and BenchmarkOcean.cpp:15-39.

@@ -1,6 +1,7 @@
 // nsdg_stress_sumfact.cu — the sum-factorised mEVP element kernels
 // (nsdg_sumfact.cuh): FP64, mixed precision, and mixed precision batched over
 // an ensemble's members.
+#include "nsdg_stress_fixed.cuh"
 #include "nsdg_sumfact.cuh"
 
 namespace nsdg {
@@ -8,26 +9,21 @@ namespace {
 
 using namespace sf;
 
-// FP64.
-// Bound by FP64 issue: about 480 FP64 instructions per element on rectangles,
-// 720 on quadrilaterals and 800 on a sphere; at the rate cuBLAS DGEMM reaches
-// (0.55 T FMA/s) 57 us for 256 x 256 rectangles.  Timed alone (CUDA events):
-// 60.8 us for 256 x 256 rectangles (112 us with 9 x 9 operators streamed from
-// memory), 42 us for 201 x 143 quadrilaterals (49 us), 32 us for 154 x 121
-// cells of a sphere (44 us), 7.4 us for 64 x 64 rectangles (20.5 us).  Three
-// threads per element rather than one: the same time on large grids, but on
-// 64 x 64 one warp per SM waits out every instruction's latency (17.1 us).
+// FP64 (nsdg_stress_fixed.cuh).  Bound by FP64 issue (126 instructions per
+// element) and the integer work beside it.  Timed alone (CUDA events): 22.2 us
+// for 256 x 256 rectangles (60.8 us with the linear maps in FP64, 112 us with
+// 9 x 9 operators streamed from memory), 18.4 us for 201 x 143 quadrilaterals (42
+// and 49 us), 12.5 us for 154 x 121 cells of a sphere (32 and 44 us), 4.6 us for
+// 64 x 64 rectangles (7.4 and 20.5 us).  Three threads per element: with one, a
+// 64 x 64 grid is one warp per SM that waits out every instruction's latency.
 constexpr int kElems = 32;
 
 template <Geometry GEO>
-__global__ void __launch_bounds__(3 * kElems) kMevpStress(DevMesh m, StressGeometry<double> geo,
-    const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ Pw,
-    double* __restrict__ tdiv, Rheology<double> rh, double keep)
+__global__ void __launch_bounds__(3 * kElems) kMevpStress(DevMesh m, FixedGeometry geo, const double* __restrict__ u,
+    const double* __restrict__ v, const double* __restrict__ Pw, double* __restrict__ tdiv, double dmin2, double keep)
 {
-    __shared__ Exchange<double, kElems> ex;
-    __shared__ double sums[GEO == RECT ? 1 : 2][3][3][kElems];
-    stressBlock<double, GEO, 0, kElems>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, rh, keep, blockIdx.x * size_t(kElems),
-        ex, sums);
+    __shared__ FixedShared<GEO, kElems> sh;
+    stressFixed<GEO, kElems>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, dmin2, keep, blockIdx.x * size_t(kElems), sh);
 }
 
 // Mixed precision: FP32 velocities, divergence and arithmetic, Delta^2 and the
@@ -110,14 +106,13 @@ cudaError_t launch(cudaStream_t s, void (*kernel)(KArgs...), size_t blocks, int 
 
 } // namespace
 
-cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const StressGeometry<double>& geo, const double* u,
+cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const FixedGeometry& geo, const double* u,
     const double* v, const double* Pw, double* tdiv, const MevpParams& pIn)
 {
     const MevpParams p = withDerived(pIn);
-    const Rheology<double> rh { 0.25 * (p.DeltaMin * p.DeltaMin) };
     const size_t blocks = (m.N + kElems - 1) / kElems;
     auto kernel = geo.rect ? kMevpStress<RECT> : geo.m ? kMevpStress<SPHERE> : kMevpStress<QUAD>;
-    return launch(s, kernel, blocks, 3 * kElems, m, geo, u, v, Pw, tdiv, rh, p.keepd);
+    return launch(s, kernel, blocks, 3 * kElems, m, geo, u, v, Pw, tdiv, p.DeltaMin * p.DeltaMin, p.keepd);
 }
 
 cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo, const float* u,

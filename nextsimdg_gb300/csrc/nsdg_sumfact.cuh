@@ -20,11 +20,9 @@
 // 1 / (R cos lat) and 1 / R, and the metric terms of the strain and of the
 // divergence are point multiplications by m = tan(lat) / R.
 //
-// The 1-D maps are written for a type T.  FP64 issue bounds the FP64 kernels
-// (GB300 issues FP64 at about 1/60 of its FP32 rate), so what counts there is
-// the number of FP64 instructions: about 480 per element and iteration on
-// rectangles and 720 on general quadrilaterals, against 850 with the 9 x 9
-// operators.
+// The 1-D maps are written for a type T: FP32 here and in the BBM kernels, FP64
+// in the latter; the FP64 mEVP kernel runs them in fixed point
+// (nsdg_stress_fixed.cuh).
 //
 // Half strains are used throughout: a = e11 / 2, b = e22 / 2, s = e12.
 #pragma once
@@ -142,26 +140,17 @@ template <typename T> __device__ __forceinline__ void columnT(const T (&x)[3], c
     o[2] = p + q;
 }
 
-// -x / 2 for x >= 0 (subnormal results flushed to zero), on the integer pipe
-__device__ __forceinline__ double minusHalf(double x)
-{
-    const int hi = __double2hiint(x);
-    return hi >= (2 << 20) ? __hiloint2double((hi - (1 << 20)) | static_cast<int>(0x80000000u), __double2loint(x)) : 0.0;
-}
-
 // How an element's map is given: one pair (k_y / k_x, 1 / k_x^2) on
-// rectangles, four derivatives on parallelograms, four per Gauss point else.
+// rectangles (FP64), four derivatives on parallelograms (FP32), four per Gauss
+// point else.  On rectangles the strain is carried over k_x (strain' = strain /
+// k_x, the eta derivatives times rho = k_y / k_x, DeltaMin^2 over k_x^2) and k_x
+// is part of the pressure's weight, so only rho is multiplied in.
 enum Geometry { RECT = 0, AFFINE = 1, QUAD = 2, SPHERE = 3 };
 
 // What the stress increments take besides the strain: the weighted pressure
 // pq = w P / (4 alpha) (FP32 kernels: as a pair of floats, 48 bits) and
 // DeltaMin^2.
 template <typename T> struct Rheology;
-template <> struct Rheology<double> {
-    using Weight = double;
-    double dminQ; // DeltaMin^2 / 4
-    static __device__ __forceinline__ double none() { return 0.0; }
-};
 template <> struct Rheology<float> {
     using Weight = float2;
     float d2h, d2l; // DeltaMin^2 as a pair of floats
@@ -173,19 +162,6 @@ template <> struct Rheology<float> {
 // f11, f12, f22 of P/(8 alpha Delta) (5 e11 + 3 e22) - P/(2 alpha) etc. from
 // a = e11/2, b = e22/2, s = e12 and Delta^2 = DeltaMin^2 + 4 (a + b)^2 + (a - b)^2 + s^2
 // (MEVPStressUpdateStep.hpp:63-77, 80-116).
-template <int VM>
-__device__ __forceinline__ void pointStress(double a, double b, double s, double pq, const Rheology<double>& rh,
-    double& f11, double& f12, double& f22)
-{
-    const double pl = a + b, mi = a - b;
-    const double t = fma(4.0, fma(pl, pl, rh.dminQ), fma(mi, mi, mulT(s, s)));
-    const double z = timesRsqrt64(pq, t); // 2 P / (8 alpha Delta), weighted
-    const double w = fma(z, pl, minusHalf(pq));
-    const double d = mulT(z, mi);
-    f12 = mulT(z, s);
-    f11 = fma(4.0, w, d);
-    f22 = fma(4.0, w, -d);
-}
 // FP32: the invariant is a sum of squares (no cancellation); Delta^2 and the
 // viscosity in float pairs (VM 3, the default) or in FP64 (VM 0, 1, 2; 4 is
 // 3 checked against 2)
@@ -215,9 +191,6 @@ __device__ __forceinline__ void pointStress(float a, float b, float s, float2 pq
 // 24 and 36 values in between go through shared memory, as do the sums of the
 // two projections on general quadrilaterals.
 //
-// On rectangles the strain is carried over k_x (strain' = strain / k_x, the
-// eta derivatives times rho = k_y / k_x, DeltaMin^2 over k_x^2) and k_x is
-// part of the pressure's weight, so only rho is multiplied in.
 template <typename T, int E> struct Exchange {
     union {
         struct {
@@ -251,7 +224,6 @@ __device__ __forceinline__ void gaussRow(int R, bool active, size_t e, size_t N,
 {
     T I[3], D[3], uxi[3], uet[3], vxi[3], vet[3], f11[3], f12[3], f22[3], x[3], y[3];
     [[maybe_unused]] T up[3], vp[3];
-    const Scaled<T> sc(GEO == RECT ? ke[0] : T(1));
     auto take = [&](int c) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
@@ -261,37 +233,15 @@ __device__ __forceinline__ void gaussRow(int R, bool active, size_t e, size_t N,
     };
     take(0);
     deriv(I, uxi);
-    if constexpr (GEO == RECT)
-        sc.interp(D, uet);
-    else
-        interp(D, uet);
+    interp(D, uet);
     if constexpr (GEO == SPHERE)
         interp(I, up);
     take(1);
     deriv(I, vxi);
-    if constexpr (GEO == RECT)
-        sc.interp(D, vet);
-    else
-        interp(D, vet);
+    interp(D, vet);
     if constexpr (GEO == SPHERE)
         interp(I, vp);
-    if constexpr (GEO == RECT) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            pointStress<VM>(uxi[i], vet[i], uet[i] + vxi[i], pq[i], rh, f11[i], f12[i], f22[i]);
-        __syncthreads(); // every warp has taken its row: the buffer changes hands
-        auto put = [&](int c, const T (&fx)[3], const T (&fy)[3]) {
-            derivT(fx, x);
-            sc.interpT(fy, y);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                ex.out.x[c][R][i][le] = x[i];
-                ex.out.y[c][R][i][le] = y[i];
-            }
-        };
-        put(0, f11, f12);
-        put(1, f12, f22);
-    } else if constexpr (GEO == AFFINE) {
+    if constexpr (GEO == AFFINE) {
 #pragma unroll
         for (int i = 0; i < 3; ++i)
             pointStress<VM>(fmaT(ke[0], uxi[i], mulT(ke[1], uet[i])), fmaT(ke[2], vxi[i], mulT(ke[3], vet[i])),
@@ -402,7 +352,7 @@ __device__ __forceinline__ void gaussRow(int R, bool active, size_t e, size_t N,
 template <typename T, Geometry GEO, int VM, int E>
 __device__ __forceinline__ void stressBlock(int nx, size_t N, const uint8_t* __restrict__ ice,
     const StressGeometry<T>& geo, const T* __restrict__ u, const T* __restrict__ v,
-    const typename Rheology<T>::Weight* __restrict__ Pw, T* __restrict__ tdiv, Rheology<T> rh, T keep, size_t x0,
+    const typename Rheology<T>::Weight* __restrict__ Pw, T* __restrict__ tdiv, const Rheology<T>& rh, T keep, size_t x0,
     Exchange<T, E>& ex, T (*sums)[3][3][E])
 {
     const int le = threadIdx.x % E, R = threadIdx.x / E; // R is the same in a warp
@@ -417,10 +367,6 @@ __device__ __forceinline__ void stressBlock(int nx, size_t N, const uint8_t* __r
 #pragma unroll
         for (int i = 0; i < 3; ++i)
             pq[i] = Pw[(3 * R + i) * N + e];
-        if constexpr (GEO == RECT) {
-            ke[0] = geo.k[e];
-            rh.dminQ *= geo.k[N + e];
-        }
         if constexpr (GEO == AFFINE)
 #pragma unroll
             for (int c = 0; c < 4; ++c)
