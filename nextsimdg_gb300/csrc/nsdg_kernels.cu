@@ -1230,13 +1230,13 @@ constexpr int kStressParts = 3;
 // The FP64 node update, divided through by c1 = rho H / dt (kMevpPrepNodes):
 //   u_new = (beta u + ku + f u_o - fc dt u + im dSx) / (1 + beta + f),  f = a |u_o - u|,
 // and likewise v with + fc dt v (VPCGDynamicsKernel.hpp:132-172), as the
-// increment (ku + f u_o + im dSx - (1 + f + fc dt) u) / (1 + beta + f): a
+// increment (ku + f (u_o - u) + im dSx - (1 + fc dt) u) / (1 + beta + f): a
 // rounding of the factors then acts on the increment, where in the quotient
-// it would act on u in each of the iterations with the same sign.  Bound by
-// FP64 issue: about 30 FP64 instructions per node, with the square root and
-// the reciprocal from FP32 seeds (CUDA's were more than half of the 60
-// before); 513 x 513 nodes 18.6 us instead of 26.8 us, 129 x 129
-// 3.0 us instead of 6.2 us (latency of the dependent chain).
+// it would act on u in each of the iterations with the same sign.  All but the
+// divergence's part is formed before the wait for the stress kernel.  Bound by
+// FP64 issue: about 25 FP64 instructions per node; 513 x 513 nodes 15.7 us
+// (18.1 us with 30 of them after the wait, 26.8 us with CUDA's square root and
+// division), 129 x 129 2.8 us (latency of the dependent chain).
 __global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, MevpNodeState st,
     const double* __restrict__ contrib, MevpParams p, int* __restrict__ err)
 {
@@ -1251,16 +1251,17 @@ __global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, MevpNodeState
     const double a = st.a[i], ku = st.ku[i], kv = st.kv[i], im = st.im[i];
     const double u = st.u[i], v = st.v[i];
     const double uo = st.uo[i], vo = st.vo[i];
+    const double ur = uo - u, vr = vo - v;
+    const double f = a * sf::sqrt64(fma(ur, ur, vr * vr));
+    const double rden = sf::recip64(p.onePlusBeta + f);
+    const double gu = fma(-p.onePlusFc, u, fma(f, ur, ku)), gv = fma(-p.oneMinusFc, v, fma(f, vr, kv));
     asm volatile("griddepcontrol.wait;" ::: "memory");
     double dSx = 0.0, dSy = 0.0;
     if (!dir)
         gatherDivergence(m, i2, j2, contrib, dSx, dSy);
-    const double ur = uo - u, vr = vo - v;
-    const double f = a * sf::sqrt64(fma(ur, ur, vr * vr));
-    const double rden = sf::recip64(p.onePlusBeta + f);
-    double un = fma(rden, fma(-(p.onePlusFc + f), u, fma(f, uo, fma(dSx, im, ku))), u);
-    double vn = fma(rden, fma(-(p.oneMinusFc + f), v, fma(f, vo, fma(dSy, im, kv))), v);
-    if (!isfinite(un) || !isfinite(vn))
+    double un = fma(rden, fma(dSx, im, gu), u);
+    double vn = fma(rden, fma(dSy, im, gv), v);
+    if (max(__double2hiint(un) & 0x7fffffff, __double2hiint(vn) & 0x7fffffff) >= 0x7ff00000)
         atomicOr(err, DEV_ERR_NONFINITE_VELOCITY);
     if (dir) {
         un = 0.0;

@@ -52,21 +52,19 @@ __device__ __forceinline__ void gatherDivergence(const DevMesh& m, int i2, int j
         Y.l1 = l;
     }
     const size_t N = m.N;
-    T ax = T(0), ay = T(0);
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        if (r < Y.n) {
-            const int cy = r ? Y.c1 : Y.c0, ly = r ? Y.l1 : Y.l0;
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (k < X.n) {
-                    const size_t c = size_t(cy) * m.nx + (k ? X.c1 : X.c0);
-                    const int j = (k ? X.l1 : X.l0) + 3 * ly;
-                    ax -= contrib[j * N + c];
-                    ay -= contrib[(9 + j) * N + c];
-                }
-            }
-        }
+    auto at = [&](int cy, int cx, int j) { return contrib + size_t(j) * N + size_t(cy) * m.nx + cx; };
+    const T* p = at(Y.c0, X.c0, X.l0 + 3 * Y.l0); // the first one is only negated
+    T ax = -p[0], ay = -p[9 * N];
+    auto subtract = [&](const T* q) {
+        ax -= q[0];
+        ay -= q[9 * N];
+    };
+    if (X.n == 2)
+        subtract(at(Y.c0, X.c1, X.l1 + 3 * Y.l0));
+    if (Y.n == 2) {
+        subtract(at(Y.c1, X.c0, X.l0 + 3 * Y.l1));
+        if (X.n == 2)
+            subtract(at(Y.c1, X.c1, X.l1 + 3 * Y.l1));
     }
     dx = ax;
     dy = ay;
