@@ -471,8 +471,8 @@ __global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T>
             c[i][j] = in ? pt.c[(9 * j + q) * N + e] : T(1);
 #pragma unroll
         for (int f = 0; f < 3; ++f)
-            g[f][i] = in ? pt.s[(9 * f + q) * N + e] : T(0);
-        d[i] = in ? pt.d[q * N + e] : T(1);
+            g[f][i] = in ? beforeWait(pt.s + (9 * f + q) * N + e) : T(0);
+        d[i] = in ? beforeWait(pt.d + q * N + e) : T(1);
     }
     if (in) {
         if constexpr (GEO == RECT) {
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T>
             weight = wj[e];
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    waitForPrevious(sizeof(T) == 4);
     {
         T n[2][3] = { { T(0), T(0), T(0) }, { T(0), T(0), T(0) } };
         if (ice) {
@@ -496,8 +496,8 @@ __global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T>
             const size_t base = 2 * size_t(s2) * iy + 2 * ix + R;
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
-                n[0][r] = u[base + size_t(r) * s2];
-                n[1][r] = v[base + size_t(r) * s2];
+                n[0][r] = afterWait(u + base + size_t(r) * s2);
+                n[1][r] = afterWait(v + base + size_t(r) * s2);
             }
         }
 #pragma unroll
@@ -607,10 +607,10 @@ __global__ void __launch_bounds__(128) kBbmMomentum(DevMesh m, BbmNodeConst<T> c
     // the node kernel before that one wrote
     const T a = c.a[i], kx = c.kx[i], ky = c.ky[i], im = c.im[i];
     const T uo = c.uo[i], vo = c.vo[i], uor = c.uor[i], vor = c.vor[i];
-    const T u = c.u[i], v = c.v[i];
+    const T u = beforeWait(c.u + i), v = beforeWait(c.v + i);
     const T imLo = sizeof(T) == 4 ? c.imLo[i] : T(0);
-    const double au = avgU[i], av = avgV[i];
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const double au = beforeWait(avgU + i), av = beforeWait(avgV + i);
+    waitForPrevious(sizeof(T) == 4);
     T dSx = T(0), dSy = T(0);
     if (!dir)
         gatherDivergence(m, i2, j2, contrib, dSx, dSy);

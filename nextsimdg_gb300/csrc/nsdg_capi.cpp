@@ -1030,7 +1030,7 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
                         LCH(launchMevpStressPairs(s, dm, opsPairs, pairsLdN, u, v, Pg, contrib, mp));
                     else
                         LCH(launchMevpStress(s, dm, fixedGeo, u, v, Pw, contrib, mp));
-                    LCH(launchMevpMomentum(s, dm, st, contrib, mp, derr));
+                    LCH(launchMevpMomentum(s, dm, st, contrib, mp, fp64Stress == 0 && releaseEarly64(N, fixedGeo), derr));
                 } else {
                     LCH(launchStress32(s, mp, derr));
                     LCH(launchMevpMomentum32(s, dm, st32, tdiv32, mp, derr));
@@ -2187,7 +2187,7 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
             if (bbm && k->mixed())
                 return launchBbmMomentum(k->stream, k->dm, bs, k->bbmNode32, k->contrib32, bp, k->derr);
             return bbm ? launchBbmMomentum(k->stream, k->dm, bs, k->bbmNode64, k->contrib, bp, k->derr)
-                       : launchMevpMomentum(k->stream, k->dm, st, k->contrib, mp, k->derr);
+                       : launchMevpMomentum(k->stream, k->dm, st, k->contrib, mp, false, k->derr);
         case 3:
         case 4:
             return k->launchStress32(k->stream, mp, k->derr, kernel_id == 4 ? 1 : 0);

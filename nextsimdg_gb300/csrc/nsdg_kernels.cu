@@ -1238,7 +1238,7 @@ constexpr int kStressParts = 3;
 // (18.1 us with 30 of them after the wait, 26.8 us with CUDA's square root and
 // division), 129 x 129 2.8 us (latency of the dependent chain).
 __global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, MevpNodeState st,
-    const double* __restrict__ contrib, MevpParams p, int* __restrict__ err)
+    const double* __restrict__ contrib, MevpParams p, bool release, int* __restrict__ err)
 {
     const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
     if (i >= m.Ncg)
@@ -1249,13 +1249,13 @@ __global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, MevpNodeState
     // velocity, which the node kernel before that one wrote
     const bool dir = m.cg2Dir[i] != 0;
     const double a = st.a[i], ku = st.ku[i], kv = st.kv[i], im = st.im[i];
-    const double u = st.u[i], v = st.v[i];
+    const double u = beforeWait(st.u + i), v = beforeWait(st.v + i);
     const double uo = st.uo[i], vo = st.vo[i];
     const double ur = uo - u, vr = vo - v;
     const double f = a * sf::sqrt64(fma(ur, ur, vr * vr));
     const double rden = sf::recip64(p.onePlusBeta + f);
     const double gu = fma(-p.onePlusFc, u, fma(f, ur, ku)), gv = fma(-p.oneMinusFc, v, fma(f, vr, kv));
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    waitForPrevious(release);
     double dSx = 0.0, dSy = 0.0;
     if (!dir)
         gatherDivergence(m, i2, j2, contrib, dSx, dSy);
@@ -1333,7 +1333,7 @@ __device__ __forceinline__ void stress32TmaBlock(const CUtensorMap* mapG, const 
             hP[qq] = hPg[(3 * part + qq) * N + e];
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    waitForPrevious();
     if (active) {
         const size_t s2 = 2 * size_t(nx) + 1;
         const size_t ix = static_cast<unsigned>(e) % static_cast<unsigned>(nx);
@@ -1342,8 +1342,8 @@ __device__ __forceinline__ void stress32TmaBlock(const CUtensorMap* mapG, const 
 #pragma unroll
         for (int j = 0; j < 9; ++j) {
             const size_t nd = base + (j % 3) + (j / 3) * s2;
-            ul[j] = u[nd];
-            vl[j] = v[nd];
+            ul[j] = afterWait(u + nd);
+            vl[j] = afterWait(v + nd);
         }
     }
     __syncthreads(); // the barriers are initialised before anyone polls them
@@ -1490,10 +1490,10 @@ __device__ __forceinline__ void mevpMomentum32Cell(int nx, int ny, size_t N, uns
     for (int n = 0; n < 4; ++n) {
         k0[n] = c.exists[n] ? st.k0[c.id[n]] : make_float4(0.f, 0.f, 0.f, 0.f);
         k1[n] = c.exists[n] ? st.k1[c.id[n]] : make_float4(0.f, 0.f, 0.f, 1.f);
-        u[n] = c.exists[n] ? st.u[c.id[n]] : 0.f;
-        v[n] = c.exists[n] ? st.v[c.id[n]] : 0.f;
+        u[n] = c.exists[n] ? beforeWait(st.u + c.id[n]) : 0.f;
+        v[n] = c.exists[n] ? beforeWait(st.v + c.id[n]) : 0.f;
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    waitForPrevious();
     float dx[4], dy[4];
     gatherCell(c, nx, ny, N, tdiv, dx, dy);
 #pragma unroll
@@ -1901,7 +1901,7 @@ cudaError_t launchDG2CG(cudaStream_t s, const DevMesh& m, int dg, const double* 
 }
 
 cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* contrib,
-    const MevpParams& pIn, int* err)
+    const MevpParams& pIn, bool release, int* err)
 {
     const MevpParams p = withDerived(pIn);
     cudaLaunchConfig_t cfg {};
@@ -1913,7 +1913,7 @@ cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const MevpNodeS
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kMevpMomentum, m, st, contrib, p, err);
+    return cudaLaunchKernelEx(&cfg, kMevpMomentum, m, st, contrib, p, release, err);
 }
 
 namespace {

@@ -220,6 +220,20 @@ struct FixedGeometry {
     const long long *k = nullptr, *n = nullptr, *m = nullptr;
     const int* exponent = nullptr;
 };
+// Whether the FP64 stress and node kernels let the next launch go at their wait
+// (nsdg_pdl.cuh).  Where the stress kernel has five or more blocks per SM they
+// do: 160 x 160 rectangles 1.77 against 1.93 ms per update, quadrilaterals 2.53
+// against 2.63, sphere 2.57 against 2.84 (128 x 128: 1.33 / 1.38, 1.82 / 1.74, 1.76 /
+// 1.83; 154 x 121 sphere 2.06 / 1.90).  And where it has at most one, but on
+// quadrilaterals: 48 x 48 rectangles 0.73 against 0.84, 64 x 64 0.80 against 0.87,
+// sphere 1.06 against 1.17, quadrilaterals 1.18 against 1.12.
+constexpr size_t kSMs = 152;
+constexpr size_t kFixedElems = 32; // elements per block of the FP64 stress kernel
+inline bool releaseEarly64(size_t N, const FixedGeometry& geo)
+{
+    const size_t blocks = (N + kFixedElems - 1) / kFixedElems;
+    return blocks >= 5 * kSMs || (blocks <= kSMs && (geo.rect || geo.m));
+}
 // Pw holds w P/(4 alpha) at the Gauss points.
 cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const FixedGeometry& geo, const double* u,
     const double* v, const double* Pw, double* tdiv, const MevpParams& p);
@@ -258,7 +272,7 @@ cudaError_t launchPairsSelfTest(cudaStream_t s, size_t n, const double* a, const
 // Node gather of the divergence, Dirichlet zero, implicit velocity update and
 // boundary zero (CGDynamicsKernel.cpp:365-444, VPCGDynamicsKernel.hpp:132-172).
 cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* contrib,
-    const MevpParams& p, int* err);
+    const MevpParams& p, bool release, int* err);
 
 // --- mEVP, mixed precision (NSDG_PRECISION_MIXED) ----------------------
 // FP32 operators, velocities, divergence coefficients and momentum

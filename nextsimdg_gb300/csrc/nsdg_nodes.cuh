@@ -3,6 +3,7 @@
 #pragma once
 
 #include "nsdg_kernels.hpp"
+#include "nsdg_pdl.cuh"
 
 namespace nsdg {
 namespace {
@@ -53,18 +54,31 @@ __device__ __forceinline__ void gatherDivergence(const DevMesh& m, int i2, int j
     }
     const size_t N = m.N;
     auto at = [&](int cy, int cx, int j) { return contrib + size_t(j) * N + size_t(cy) * m.nx + cx; };
-    const T* p = at(Y.c0, X.c0, X.l0 + 3 * Y.l0); // the first one is only negated
-    T ax = -p[0], ay = -p[9 * N];
-    auto subtract = [&](const T* q) {
-        ax -= q[0];
-        ay -= q[9 * N];
-    };
-    if (X.n == 2)
-        subtract(at(Y.c0, X.c1, X.l1 + 3 * Y.l0));
-    if (Y.n == 2) {
-        subtract(at(Y.c1, X.c0, X.l0 + 3 * Y.l1));
-        if (X.n == 2)
-            subtract(at(Y.c1, X.c1, X.l1 + 3 * Y.l1));
+    // all loads first, a missing cell's from the first one's place
+    const bool x2 = X.n == 2, y2 = Y.n == 2;
+    const T* p[4] = { at(Y.c0, X.c0, X.l0 + 3 * Y.l0), at(Y.c0, X.c1, X.l1 + 3 * Y.l0),
+        at(Y.c1, X.c0, X.l0 + 3 * Y.l1), at(Y.c1, X.c1, X.l1 + 3 * Y.l1) };
+    p[1] = x2 ? p[1] : p[0];
+    p[2] = y2 ? p[2] : p[0];
+    p[3] = x2 && y2 ? p[3] : p[0];
+    T x[4], y[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        x[k] = afterWait(p[k]);
+        y[k] = afterWait(p[k] + 9 * N);
+    }
+    T ax = -x[0], ay = -y[0];
+    if (x2) {
+        ax -= x[1];
+        ay -= y[1];
+    }
+    if (y2) {
+        ax -= x[2];
+        ay -= y[2];
+        if (x2) {
+            ax -= x[3];
+            ay -= y[3];
+        }
     }
     dx = ax;
     dy = ay;
@@ -109,8 +123,8 @@ __device__ __forceinline__ void gatherCell(const CellNodes& c, int nx, int ny, s
     const bool left = c.ix > 0, right = c.ix < nx, below = c.iy > 0, above = c.iy < ny;
     const size_t e = size_t(c.iy) * nx + c.ix; // the cell itself
     auto at = [&](bool ok, int j, size_t cell, T& x, T& y) {
-        x = ok ? contrib[j * N + cell] : T(0);
-        y = ok ? contrib[(9 + j) * N + cell] : T(0);
+        x = ok ? afterWait(contrib + j * N + cell) : T(0);
+        y = ok ? afterWait(contrib + (9 + j) * N + cell) : T(0);
     };
     // corner: local nodes 8, 6 of the row below and 2, 0 of the cell's row
     T bx[2], by[2], ax[2], ay[2], mbx, mby, max_, may, lx[2], ly[2], cx, cy;

@@ -56,7 +56,7 @@ __device__ __forceinline__ void pointStress64(double pl, double mi, double s, do
 template <Geometry GEO, int E>
 __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __restrict__ ice,
     const FixedGeometry& geo, const double* __restrict__ u, const double* __restrict__ v,
-    const double* __restrict__ Pw, double* __restrict__ tdiv, double dmin2, double keep, size_t x0,
+    const double* __restrict__ Pw, double* __restrict__ tdiv, double dmin2, double keep, bool release, size_t x0,
     FixedShared<GEO, E>& sh)
 {
     using fx::i64;
@@ -74,14 +74,9 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
             dmin2 *= geo.rect[N + e];
         } else
             ke = geo.exponent[e];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            told[r] = tdiv[(3 * r + R) * N + e];
-            told[3 + r] = tdiv[(9 + 3 * r + R) * N + e];
-        }
     }
     sh.top[1][R][le] = topOf(max(fx::magnitudeWord(pq[0]), max(fx::magnitudeWord(pq[1]), fx::magnitudeWord(pq[2]))));
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    waitForPrevious(release);
     double n[2][3] = { { 0.0, 0.0, 0.0 }, { 0.0, 0.0, 0.0 } };
     if (active) {
         const unsigned s2 = 2u * static_cast<unsigned>(nx) + 1u;
@@ -90,8 +85,13 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
         const size_t base = 2 * size_t(s2) * iy + 2 * ix + R;
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            n[0][r] = u[base + size_t(r) * s2];
-            n[1][r] = v[base + size_t(r) * s2];
+            n[0][r] = afterWait(u + base + size_t(r) * s2);
+            n[1][r] = afterWait(v + base + size_t(r) * s2);
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) { // needed at the end
+            told[r] = afterWait(tdiv + (3 * r + R) * N + e);
+            told[3 + r] = afterWait(tdiv + (9 + 3 * r + R) * N + e);
         }
     }
     int word = 0;

@@ -16,14 +16,15 @@ using namespace sf;
 // and 49 us), 12.5 us for 154 x 121 cells of a sphere (32 and 44 us), 4.6 us for
 // 64 x 64 rectangles (7.4 and 20.5 us).  Three threads per element: with one, a
 // 64 x 64 grid is one warp per SM that waits out every instruction's latency.
-constexpr int kElems = 32;
+constexpr int kElems = kFixedElems;
 
 template <Geometry GEO>
 __global__ void __launch_bounds__(3 * kElems) kMevpStress(DevMesh m, FixedGeometry geo, const double* __restrict__ u,
-    const double* __restrict__ v, const double* __restrict__ Pw, double* __restrict__ tdiv, double dmin2, double keep)
+    const double* __restrict__ v, const double* __restrict__ Pw, double* __restrict__ tdiv, double dmin2, double keep, bool release)
 {
     __shared__ FixedShared<GEO, kElems> sh;
-    stressFixed<GEO, kElems>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, dmin2, keep, blockIdx.x * size_t(kElems), sh);
+    stressFixed<GEO, kElems>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, dmin2, keep, release, blockIdx.x * size_t(kElems),
+        sh);
 }
 
 // Mixed precision: FP32 velocities, divergence and arithmetic, Delta^2 and the
@@ -112,7 +113,8 @@ cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const FixedGeomet
     const MevpParams p = withDerived(pIn);
     const size_t blocks = (m.N + kElems - 1) / kElems;
     auto kernel = geo.rect ? kMevpStress<RECT> : geo.m ? kMevpStress<SPHERE> : kMevpStress<QUAD>;
-    return launch(s, kernel, blocks, 3 * kElems, m, geo, u, v, Pw, tdiv, p.DeltaMin * p.DeltaMin, p.keepd);
+    return launch(s, kernel, blocks, 3 * kElems, m, geo, u, v, Pw, tdiv, p.DeltaMin * p.DeltaMin, p.keepd,
+        releaseEarly64(m.N, geo));
 }
 
 cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo, const float* u,

@@ -31,6 +31,7 @@
 #include <cstdint>
 
 #include "nsdg_kernels.hpp"
+#include "nsdg_pdl.cuh"
 #include "nsdg_seed64.cuh"
 #include "nsdg_viscosity.cuh"
 
@@ -373,11 +374,11 @@ __device__ __forceinline__ void stressBlock(int nx, size_t N, const uint8_t* __r
                 ke[c] = geo.k[c * N + e];
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            told[r] = tdiv[(3 * r + R) * N + e];
-            told[3 + r] = tdiv[(9 + 3 * r + R) * N + e];
+            told[r] = beforeWait(tdiv + (3 * r + R) * N + e);
+            told[3 + r] = beforeWait(tdiv + (9 + 3 * r + R) * N + e);
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    waitForPrevious();
     {
         T n[2][3] = { { T(0), T(0), T(0) }, { T(0), T(0), T(0) } };
         if (active) {
@@ -387,8 +388,8 @@ __device__ __forceinline__ void stressBlock(int nx, size_t N, const uint8_t* __r
             const size_t base = 2 * size_t(s2) * iy + 2 * ix + R;
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
-                n[0][r] = u[base + size_t(r) * s2];
-                n[1][r] = v[base + size_t(r) * s2];
+                n[0][r] = afterWait(u + base + size_t(r) * s2);
+                n[1][r] = afterWait(v + base + size_t(r) * s2);
             }
         }
 #pragma unroll
@@ -444,9 +445,9 @@ __device__ __forceinline__ void stressThread(int nx, size_t N, const uint8_t* __
                 ke[c] = geo.k[c * N + e];
 #pragma unroll
         for (int j = 0; j < 18; ++j)
-            told[j] = tdiv[j * N + e];
+            told[j] = beforeWait(tdiv + j * N + e);
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    waitForPrevious();
     if (!active)
         return;
     T val[2][3][3], der[2][3][3]; // [u, v][Gauss row][column]
@@ -460,7 +461,7 @@ __device__ __forceinline__ void stressThread(int nx, size_t N, const uint8_t* __
             const T* src = (c ? v : u) + base;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                const T n[3] = { src[i], src[s2 + i], src[2 * s2 + i] };
+                const T n[3] = { afterWait(src + i), afterWait(src + s2 + i), afterWait(src + 2 * s2 + i) };
                 T vr[3], dr[3];
                 interpDeriv(n, vr, dr);
 #pragma unroll
