@@ -341,20 +341,7 @@ struct nsdg_kernel {
     // the cell averages of a field into host memory `out`: projections and
     // the copy enqueued on `stream` (a stored field is copied at once)
     int enqueueReadout(const std::string& s, double* out, HostMoves* batch = nullptr);
-    // the GPU reads and writes pageable host memory directly (Grace: address
-    // translation over the CPU-GPU link; NSDG_HOST_DIRECT=0 turns it off):
-    // host arrays that are not page-locked then move by a kernel, which runs
-    // at the link's rate, instead of a copy staged through a driver buffer
-    bool hostDirect = false;
-    static bool isPageable(const void* p)
-    {
-        cudaPointerAttributes a {};
-        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        return a.type == cudaMemoryTypeUnregistered;
-    }
+    bool hostDirect = false; // hostDirectAvailable()
     bool moveByKernel(const void* p) const { return hostDirect && isPageable(p); }
 };
 
@@ -857,14 +844,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         if (r)
             return r;
     }
-    {
-        int dev = 0, pageableAccess = 0;
-        const char* hd = std::getenv("NSDG_HOST_DIRECT");
-        hostDirect = cudaGetDevice(&dev) == cudaSuccess
-            && cudaDeviceGetAttribute(&pageableAccess, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess
-            && pageableAccess == 1 && !(hd && std::strcmp(hd, "0") == 0);
-        cudaGetLastError();
-    }
+    hostDirect = hostDirectAvailable();
     ready = true;
     return ok();
 }

@@ -17,6 +17,7 @@ struct nsdg_ice_growth {
     double* fields = nullptr;   // [NSDG_IG_NFIELDS][n] on the device
     uint8_t* ocean = nullptr;   // n, 1 = ocean element
     double* staging = nullptr;  // pinned host buffer of n doubles
+    bool hostDirect = false;    // hostDirectAvailable()
     std::string err;
     int fail(int code, const std::string& m)
     {

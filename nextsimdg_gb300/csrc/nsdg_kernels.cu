@@ -6,6 +6,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
+#include <cstdlib>
+#include <cstring>
 
 #include "nsdg_host.hpp"
 
@@ -2185,6 +2187,26 @@ __global__ void __launch_bounds__(256) kHostMove(HostMoves m)
         }
         m.dst[f][off] = m.src[f][off];
     }
+}
+
+bool hostDirectAvailable()
+{
+    int dev = 0, pageableAccess = 0;
+    const char* hd = std::getenv("NSDG_HOST_DIRECT");
+    const bool direct = cudaGetDevice(&dev) == cudaSuccess
+        && cudaDeviceGetAttribute(&pageableAccess, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess
+        && pageableAccess == 1 && !(hd && std::strcmp(hd, "0") == 0);
+    cudaGetLastError();
+    return direct;
+}
+bool isPageable(const void* p)
+{
+    cudaPointerAttributes a {};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
 }
 
 cudaError_t launchHostMove(cudaStream_t s, const HostMoves& m)

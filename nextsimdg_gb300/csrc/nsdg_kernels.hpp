@@ -523,6 +523,12 @@ struct HostMoves {
     int count = 0;
 };
 cudaError_t launchHostMove(cudaStream_t s, const HostMoves& m);
+// Whether the GPU reads and writes pageable host memory directly (Grace:
+// address translation over the CPU-GPU link; NSDG_HOST_DIRECT=0 turns it off).
+// Host arrays that are not page-locked then move by that kernel, which runs at
+// the link's rate, instead of a copy staged through a buffer.
+bool hostDirectAvailable();
+bool isPageable(const void* p);
 // device SoA -> AoS with `nout` comps (all, or component 0 only)
 cudaError_t launchSoaToAos(cudaStream_t s, size_t N, int dg, int nout, const double* soa, double* aos);
 // Tools::MeanValue: writes partial sums per block into `partials` and the
