@@ -128,6 +128,9 @@ struct AverageFields {
     int count = 0;
 };
 cudaError_t launchAverage(cudaStream_t s, const DevMesh& m, const AverageFields& f);
+// An empty kernel: one launch after which a programmatic dependent may follow
+// several streams joined before it.
+cudaError_t launchJoin(cudaStream_t s);
 // CG1 gradient of the sea-surface height (CGDynamicsKernel.cpp:126-204);
 // cg1, ug, vg: Ncg1 doubles each.
 cudaError_t launchSSHGradient(cudaStream_t s, const DevMesh& m, const DevOps& o, const double* ssh, double* cg1,
