@@ -5,8 +5,8 @@
 // 1e-6 of their size within an element, rectangles) is 0.35 to 0.5 of that of
 // the maps in FP64.
 //
-// What stays in FP64 is the rheology, twelve instructions per Gauss point, and
-// the relaxation of the 18 divergence coefficients: 126 FP64 instructions per
+// What stays in FP64 is the rheology, ten instructions per Gauss point, and
+// the relaxation of the 18 divergence coefficients: 108 FP64 instructions per
 // element where the maps in FP64 make it 480 on rectangles and 720 on
 // quadrilaterals.
 //

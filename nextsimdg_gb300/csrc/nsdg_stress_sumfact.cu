@@ -9,11 +9,11 @@ namespace {
 
 using namespace sf;
 
-// FP64 (nsdg_stress_fixed.cuh).  Bound by FP64 issue (126 instructions per
-// element) and the integer work beside it.  Timed alone (CUDA events): 22.2 us
+// FP64 (nsdg_stress_fixed.cuh).  Bound by FP64 issue (108 instructions per
+// element) and the integer work beside it.  Timed alone (CUDA events): 21.1 us
 // for 256 x 256 rectangles (60.8 us with the linear maps in FP64, 112 us with
-// 9 x 9 operators streamed from memory), 18.4 us for 201 x 143 quadrilaterals (42
-// and 49 us), 12.5 us for 154 x 121 cells of a sphere (32 and 44 us), 4.6 us for
+// 9 x 9 operators streamed from memory), 16.6 us for 201 x 143 quadrilaterals (42
+// and 49 us), 12.2 us for 154 x 121 cells of a sphere (32 and 44 us), 4.6 us for
 // 64 x 64 rectangles (7.4 and 20.5 us).  Three threads per element: with one, a
 // 64 x 64 grid is one warp per SM that waits out every instruction's latency.
 constexpr int kElems = kFixedElems;
