@@ -103,23 +103,38 @@ NSDG_FX_HD constexpr Coef coefOf(u64 c) // c 2^-64
 {
     return Coef { static_cast<int>((c >> 32) + ((c >> 31) & 1)), static_cast<int>(static_cast<unsigned>(c)) };
 }
-// c x, floored (within two units)
-NSDG_FX_HD i64 mul(i64 x, Coef c)
+// x = hi 2^32 + lo with lo signed (|x| < 2^63 - 2^32)
+struct Split {
+    int hi, lo;
+    NSDG_FX_HD explicit Split(i64 x) : lo(static_cast<int>(static_cast<unsigned>(x)))
+    {
+        hi = static_cast<int>(x >> 32) + static_cast<int>(static_cast<unsigned>(x) >> 31);
+    }
+};
+NSDG_FX_HD i64 wide(int a, int b, i64 c) { return static_cast<i64>(a) * b + c; }
+// c x, floored (within two units): three multiplications with 64-bit addends
+NSDG_FX_HD i64 mul(Split x, Coef c) { return wide(x.hi, c.hi, wide(x.lo, c.hi, wide(x.hi, c.lo, 0)) >> 32); }
+NSDG_FX_HD i64 mul(i64 x, Coef c) { return mul(Split(x), c); }
+// a factor |k| < 2^62 for the products below, hi and lo as in Split
+NSDG_FX_HD i64 packed(i64 k)
 {
-    const int xh = static_cast<int>(x >> 32);
-    const unsigned xl = static_cast<unsigned>(x);
-    const i64 t = static_cast<i64>(xh) * c.lo;
-    const u64 s = static_cast<u64>(xl) * static_cast<unsigned>(c.hi);
-    return static_cast<i64>(xh) * c.hi + (t >> 32) + static_cast<i64>(s >> 32);
+    const Split s(k);
+    return static_cast<i64>((static_cast<u64>(static_cast<unsigned>(s.hi)) << 32) | static_cast<unsigned>(s.lo));
 }
-// k x 2^-64, floored
-NSDG_FX_HD i64 mulHigh(i64 x, i64 k)
+NSDG_FX_HD Split unpacked(i64 p)
 {
-#if defined(__CUDA_ARCH__)
-    return __mul64hi(x, k);
-#else
-    return static_cast<i64>((static_cast<__int128>(x) * k) >> 64);
-#endif
+    Split s(0);
+    s.hi = static_cast<int>(p >> 32);
+    s.lo = static_cast<int>(static_cast<unsigned>(p));
+    return s;
+}
+// (k x) 2^-64 and (k x + l y) 2^-64, floored (within two and three units), for
+// |x|, |y| < 2^61.5: the middle sums stay below 2^63
+NSDG_FX_HD i64 mulHigh(Split x, Split k) { return wide(x.hi, k.hi, wide(x.lo, k.hi, wide(x.hi, k.lo, 0)) >> 32); }
+NSDG_FX_HD i64 mulHigh(Split x, Split k, Split y, Split l)
+{
+    const i64 t = wide(y.lo, l.hi, wide(y.hi, l.lo, wide(x.lo, k.hi, wide(x.hi, k.lo, 0))));
+    return wide(x.hi, k.hi, wide(y.hi, l.hi, t >> 32));
 }
 
 // The 1-D maps of the element update on a line of three nodes or Gauss points

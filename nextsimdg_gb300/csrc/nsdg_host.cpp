@@ -3,6 +3,7 @@
 // Compiled with -ffp-contract=off so the operators are identical on x86-64
 // and aarch64 hosts.
 #include "nsdg_host.hpp"
+#include "nsdg_fixed.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -452,11 +453,11 @@ void buildFixedMetric(const StressMetric& s, size_t N, FixedMetric& out, unsigne
             std::frexp(most, &x);
             out.exponent[e] = x;
             for (size_t i = e; i < s.k.size(); i += N)
-                out.k[i] = std::llrint(std::ldexp(s.k[i], 62 - x));
+                out.k[i] = fx::packed(std::llrint(std::ldexp(s.k[i], 62 - x)));
             for (size_t i = e; i < s.m.size(); i += N)
-                out.m[i] = std::llrint(std::ldexp(s.m[i], 62 - x));
+                out.m[i] = fx::packed(std::llrint(std::ldexp(s.m[i], 62 - x)));
             for (size_t i = e; i < s.n.size(); i += N)
-                out.n[i] = std::llrint(std::ldexp(s.n[i], 62));
+                out.n[i] = fx::packed(std::llrint(std::ldexp(s.n[i], 62)));
         }
     });
 }

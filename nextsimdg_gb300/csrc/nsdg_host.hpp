@@ -141,8 +141,8 @@ struct StressMetric {
 // With allowRect false the general form is built on every mesh.
 void buildStressMetric(const HostMesh& m, bool allowRect, StressMetric& out, unsigned threads = 0);
 // The general form as integers for the FP64 element kernel
-// (nsdg_stress_fixed.cuh): per element |k| and |m| below 2^exponent, k and m as
-// multiples of 2^(exponent - 62), n (below 1) of 2^-62.
+// (nsdg_stress_fixed.cuh), in the form of fx::packed: per element |k| and |m| below
+// 2^exponent, k and m as multiples of 2^(exponent - 62), n (below 1) of 2^-62.
 struct FixedMetric {
     std::vector<long long> k, n, m;
     std::vector<int> exponent;

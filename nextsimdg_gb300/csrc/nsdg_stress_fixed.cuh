@@ -18,8 +18,9 @@
 //              <= 122 V and the projected strain <= 130 V -> bits 55
 // and the weighted pressure, F = its largest, bounds the stress increments
 // (|2 zp -+ d| <= sqrt(5) pq, so |f11|, |f22| <= 4.3 F, |f12| <= F); through the
-// transposed maps they stay within 56 (1 + rho) F, and on quadrilaterals, after
-// the products with k / 4, within 304 F.
+// transposed maps they stay within 56 (1 + rho) F.  On quadrilaterals they are
+// within 22 F after the projection (F = 2^57: below 2^61.5), and after the
+// products with k / 4 and a shift by 3 the maps stay within 38 F.
 #pragma once
 
 #include "nsdg_fixed.hpp"
@@ -127,7 +128,7 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
     __syncthreads();
     // Gauss row R
     const int scale = bits - top + 1022; // of the strain (on quadrilaterals before the products with k / 4)
-    const int bitsP = GEO == RECT ? 58 - sc.shift : 59;
+    const int bitsP = GEO == RECT ? 58 - sc.shift : 58;
     const int atP = fx::fixedShift(bitsP, topP);
     i64 I[3], D[3], uxi[3], uet[3], vxi[3], vet[3], F11[3], F12[3], F22[3], x[3], y[3];
     [[maybe_unused]] i64 up[3], vp[3];
@@ -184,24 +185,24 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
         put(1, F12, F22);
     } else {
         const int atStrain = fx::doubleExponent(scale - ke - 2);
-        i64 k0[3], k1[3], k2[3], k3[3], nq[3], a[3], b[3], s[3];
-        [[maybe_unused]] i64 mq[3];
+        i64 a[3], b[3], s[3];
+        auto factor = [&](const i64* p, size_t row) { return fx::unpacked(active ? p[row * N + e] : 0); };
+        fx::Split k0[3] = { factor(geo.k, 3 * R), factor(geo.k, 3 * R + 1), factor(geo.k, 3 * R + 2) };
+        fx::Split k1[3] = { factor(geo.k, 9 + 3 * R), factor(geo.k, 10 + 3 * R), factor(geo.k, 11 + 3 * R) };
+        fx::Split k2[3] = { factor(geo.k, 18 + 3 * R), factor(geo.k, 19 + 3 * R), factor(geo.k, 20 + 3 * R) };
+        fx::Split k3[3] = { factor(geo.k, 27 + 3 * R), factor(geo.k, 28 + 3 * R), factor(geo.k, 29 + 3 * R) };
+        fx::Split nq[3] = { factor(geo.n, 3 * R), factor(geo.n, 3 * R + 1), factor(geo.n, 3 * R + 2) };
+        auto metric = [&](int i) { return GEO == SPHERE ? factor(geo.m, 3 * R + i) : fx::Split(0); };
+        [[maybe_unused]] fx::Split mq[3] = { metric(0), metric(1), metric(2) };
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            const size_t q = 3 * R + i;
-            k0[i] = active ? geo.k[q * N + e] : 0;
-            k1[i] = active ? geo.k[(9 + q) * N + e] : 0;
-            k2[i] = active ? geo.k[(18 + q) * N + e] : 0;
-            k3[i] = active ? geo.k[(27 + q) * N + e] : 0;
-            nq[i] = active ? geo.n[q * N + e] : 0;
-            a[i] = fx::mulHigh(uxi[i], k0[i]) + fx::mulHigh(uet[i], k1[i]);
-            b[i] = fx::mulHigh(vxi[i], k2[i]) + fx::mulHigh(vet[i], k3[i]);
-            s[i] = fx::mulHigh(uxi[i], k2[i]) + fx::mulHigh(uet[i], k3[i]) + fx::mulHigh(vxi[i], k0[i])
-                + fx::mulHigh(vet[i], k1[i]);
+            const fx::Split ux(uxi[i]), ue(uet[i]), vx(vxi[i]), ve(vet[i]);
+            a[i] = fx::mulHigh(ux, k0[i], ue, k1[i]);
+            b[i] = fx::mulHigh(vx, k2[i], ve, k3[i]);
+            s[i] = fx::mulHigh(ux, k2[i], ue, k3[i]) + fx::mulHigh(vx, k0[i], ve, k1[i]);
             if constexpr (GEO == SPHERE) {
-                mq[i] = active ? geo.m[q * N + e] : 0;
-                a[i] -= fx::mulHigh(vp[i], mq[i]);
-                s[i] += fx::mulHigh(up[i], mq[i]);
+                a[i] -= fx::mulHigh(fx::Split(vp[i]), mq[i]);
+                s[i] += fx::mulHigh(fx::Split(up[i]), mq[i]);
             }
         }
         const int nr = R == 1 ? -2 : 1; // nu on this row: nr, -2 nr, nr
@@ -211,33 +212,33 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
             times(s[0] + s[2] - 2 * s[1], nr) };
         sumRows<i64, E>(sh.sums[0], R, le, c);
         i64 d[3] = { 0, 0, 0 };
+        const fx::Split c0(c[0]), c1(c[1]), c2(c[2]);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            increments(i, a[i] - fx::four(fx::mulHigh(c[0], nq[i])), b[i] - fx::four(fx::mulHigh(c[1], nq[i])),
-                s[i] - fx::four(fx::mulHigh(c[2], nq[i])), atStrain);
-            d[0] += fx::mulHigh(F11[i], nq[i]);
-            d[1] += fx::mulHigh(F22[i], nq[i]);
-            d[2] += fx::mulHigh(F12[i], nq[i]);
+            increments(i, a[i] - fx::four(fx::mulHigh(c0, nq[i])), b[i] - fx::four(fx::mulHigh(c1, nq[i])),
+                s[i] - fx::four(fx::mulHigh(c2, nq[i])), atStrain);
+            d[0] += fx::mulHigh(fx::Split(F11[i]), nq[i]);
+            d[1] += fx::mulHigh(fx::Split(F22[i]), nq[i]);
+            d[2] += fx::mulHigh(fx::Split(F12[i]), nq[i]);
         }
         // P^T: subtract nu (n . f)
         sumRows<i64, E>(sh.sums[1], R, le, d);
         i64 t0[3], t1[3], t2[3], t3[3];
         [[maybe_unused]] i64 mu[3], mv[3];
-        // sums of products with k / 4, over 16
-        auto sixteenth = [](i64 t) { return (t + 8) >> 4; };
+        // sums of products with k / 4, over 8
+        auto eighth = [](i64 t) { return (t + 4) >> 3; };
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             const int w = i == 1 ? -2 * nr : nr;
-            F11[i] -= times(fx::four(d[0]), w);
-            F22[i] -= times(fx::four(d[1]), w);
-            F12[i] -= times(fx::four(d[2]), w);
-            t0[i] = sixteenth(fx::mulHigh(F11[i], k0[i]) + fx::mulHigh(F12[i], k2[i]));
-            t1[i] = sixteenth(fx::mulHigh(F11[i], k1[i]) + fx::mulHigh(F12[i], k3[i]));
-            t2[i] = sixteenth(fx::mulHigh(F12[i], k0[i]) + fx::mulHigh(F22[i], k2[i]));
-            t3[i] = sixteenth(fx::mulHigh(F12[i], k1[i]) + fx::mulHigh(F22[i], k3[i]));
+            const fx::Split f11(F11[i] - times(fx::four(d[0]), w)), f22(F22[i] - times(fx::four(d[1]), w)),
+                f12(F12[i] - times(fx::four(d[2]), w));
+            t0[i] = eighth(fx::mulHigh(f11, k0[i], f12, k2[i]));
+            t1[i] = eighth(fx::mulHigh(f11, k1[i], f12, k3[i]));
+            t2[i] = eighth(fx::mulHigh(f12, k0[i], f22, k2[i]));
+            t3[i] = eighth(fx::mulHigh(f12, k1[i], f22, k3[i]));
             if constexpr (GEO == SPHERE) {
-                mu[i] = sixteenth(fx::mulHigh(F12[i], mq[i]));
-                mv[i] = sixteenth(-fx::mulHigh(F11[i], mq[i]));
+                mu[i] = eighth(fx::mulHigh(f12, mq[i]));
+                mv[i] = eighth(-fx::mulHigh(f11, mq[i]));
             }
         }
         auto put = [&](int c, const i64 (&tx)[3], const i64 (&ty)[3], [[maybe_unused]] const i64 (&tm)[3]) {
@@ -270,7 +271,7 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
         return;
     bad = (sh.top[0][0][le] | sh.top[0][1][le] | sh.top[0][2][le]) != 0;
     const int scaleP = bitsP - topP + 1022;
-    const int atOut = fx::doubleExponent(GEO == RECT ? scaleP : scaleP - 4 - ke - 2);
+    const int atOut = fx::doubleExponent(GEO == RECT ? scaleP : scaleP - 3 - ke - 2);
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         i64 o[3];

@@ -10,12 +10,15 @@ namespace {
 using namespace sf;
 
 // FP64 (nsdg_stress_fixed.cuh).  Bound by FP64 issue (108 instructions per
-// element) and the integer work beside it.  Timed alone (CUDA events): 21.1 us
+// element) and the integer work beside it.  Timed alone (CUDA events): 19.3 us
 // for 256 x 256 rectangles (60.8 us with the linear maps in FP64, 112 us with
-// 9 x 9 operators streamed from memory), 16.6 us for 201 x 143 quadrilaterals (42
-// and 49 us), 12.2 us for 154 x 121 cells of a sphere (32 and 44 us), 4.6 us for
+// 9 x 9 operators streamed from memory), 16.7 us for 201 x 143 quadrilaterals (42
+// and 49 us), 11.7 us for 154 x 121 cells of a sphere (32 and 44 us), 4.6 us for
 // 64 x 64 rectangles (7.4 and 20.5 us).  Three threads per element: with one, a
 // 64 x 64 grid is one warp per SM that waits out every instruction's latency.
+// Without a bound on the registers (80, 128 and 166): with six or more blocks per
+// SM forced, quadrilaterals and spheres spill (16.9 and 14.6 us) and rectangles
+// gain nothing.
 constexpr int kElems = kFixedElems;
 
 template <Geometry GEO>

@@ -67,6 +67,16 @@ int main(int argc, char** argv)
         if (c < (0x7fffffffull << 32))
             prod = std::max(prod, R(std::llabs(mul(Y, coefOf(c)) - static_cast<i64>((static_cast<__int128>(Y) * c) >> 64))));
     }
+    const R unit = ldexpl(1, 64);
+    R high = 0;
+    for (int i = 0; i < 200000; ++i) {
+        const i64 most = static_cast<i64>(0x1p61 * 1.41), one = 1ll << 62;
+        auto any = [&](i64 m) { return i < 64 ? (gen() & 1 ? m - 1 : 1 - m) : static_cast<i64>(U(gen) * m) >> (gen() % 40); };
+        const i64 x = any(most), y = any(most), k = any(one), l = any(one);
+        const R a = R(x) * k / unit, b = R(y) * l / unit;
+        high = std::max(high, fabsl(mulHigh(Split(x), unpacked(packed(k))) - a) / 2);
+        high = std::max(high, fabsl(mulHigh(Split(x), unpacked(packed(k)), Split(y), unpacked(packed(l))) - (a + b)) / 3);
+    }
     const Scaled sc(rho);
     const int bits = std::min(58, 61 - sc.shift), bitsP = 58 - sc.shift;
     for (int i = 0; i < 20000; ++i) {
@@ -124,7 +134,7 @@ int main(int argc, char** argv)
                 share = std::max(share, fabsl(R(o[r]) - (a[r] + b[r])));
         }
     }
-    std::printf("%.6Lf %.6Lf %.6Lf %.6Lf %.6Lf %d\n", conv, near, prod, strain, share, sc.shift);
+    std::printf("%.6Lf %.6Lf %.6Lf %.6Lf %.6Lf %.6Lf %d\n", conv, near, prod, high, strain, share, sc.shift);
 }
 """
 
@@ -142,15 +152,16 @@ def program(tmp_path_factory):
 def test_within_units_of_the_exact_maps(program, rho):
     """A conversion to fixed point is truncated (below one unit), one to FP64
     rounded to nearest (half an ulp, at most 2^-53 of the value), a product
-    within two units.  A strain then has at most 4 units from a column's value
+    within two units (a sum of two with packed factors within three).  A strain then has at most 4 units from a column's value
     and 8 from its derivative, 8 + 4 (2 + 16 g) = 41 in a row's derivative and
     rho (1.2 8 + 2^shift / rho 3 2) from a row's scaled interpolation; a share 2 4
     = 8 from a row's transposed derivative and 2^shift 4 from its transposed
     interpolation, which a column's maps multiply by at most 2 (1.2 + 4 g) with 12
     of their own."""
-    conv, near, prod, strain, share, shift = map(float, subprocess.check_output([str(program), repr(rho)]).split())
+    conv, near, prod, high, strain, share, shift = map(float, subprocess.check_output([str(program), repr(rho)]).split())
     assert conv < 1.0
     assert near <= 1.0
     assert prod <= 2.0
+    assert high <= 1.0
     assert strain <= 41 + 10 * rho + 6 * 2 ** shift
     assert share <= 12 + 6.2 * (8 + 4 * 2 ** shift)
