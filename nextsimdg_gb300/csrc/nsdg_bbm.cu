@@ -19,6 +19,7 @@
 #include "nsdg_modes.cuh"
 #include "nsdg_nodes.cuh"
 #include "nsdg_prep.cuh"
+#include "nsdg_stress_fixed.cuh"
 #include "nsdg_sumfact.cuh"
 #include "nsdg_visc_ff.hpp"
 
@@ -239,88 +240,17 @@ __device__ __forceinline__ void bbmPoint(T a, T b, T s, const T (&c)[6], const B
     g22 *= keep;
 }
 
-template <typename T, int E> struct BbmShared {
-    Exchange<T, E> ex;
-    T strain[3][3][E];   // nu . strain per row
-    T sum[3][9][E];      // per row: nu . f (3) and the damage's moments (2, or DG)
-};
-
-// Row R of an element: see kBbmStress.
+// P f and the damage's projection of row R, and the new state: sums over the
+// three rows in sum[row][9][E] (nu . f, 3, and the damage's moments, 3 or DG).
 template <typename T, Geometry GEO, int DG, int E>
-__device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const StressGeometry<T>& geo,
-    const T* __restrict__ wdam, const T* __restrict__ wj, const BbmPoints<T>& pt, const T (&ke)[4], T weight,
-    const T (&c)[3][6], T (&g)[3][3], T (&d)[3], const BbmScalars<T>& k, BbmShared<T, E>& sh, int le)
+__device__ __forceinline__ void bbmProject(int R, size_t e, size_t N, bool in, const T* __restrict__ wdam,
+    const T (&nq)[3], const BbmPoints<T>& pt, T (&g)[3][3], T (&d)[3], T (*sum)[9][E], int le)
 {
-    T I[3], D[3], uxi[3], uet[3], vxi[3], vet[3], a[3], b[3], s[3];
-    const Scaled<T> sc(GEO == RECT ? ke[0] : T(1));
-    auto take = [&](int f) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            I[i] = sh.ex.in.v[f][R][i][le];
-            D[i] = sh.ex.in.dv[f][R][i][le];
-        }
-    };
-    take(0);
-    deriv(I, uxi);
-    if constexpr (GEO == RECT)
-        sc.interp(D, uet);
-    else
-        interp(D, uet);
-    take(1);
-    deriv(I, vxi);
-    if constexpr (GEO == RECT)
-        sc.interp(D, vet);
-    else
-        interp(D, vet);
     const bool mid = R == 1;
     const T nr = mid ? T(-2) : T(1);
-    [[maybe_unused]] T k0[3], k1[3], k2[3], k3[3], nq[3];
-    if constexpr (GEO == RECT) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            a[i] = uxi[i];
-            b[i] = vet[i];
-            s[i] = uet[i] + vxi[i];
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const size_t q = 3 * R + i;
-            if constexpr (GEO == AFFINE) {
-                k0[i] = ke[0];
-                k1[i] = ke[1];
-                k2[i] = ke[2];
-                k3[i] = ke[3];
-            } else {
-                k0[i] = in ? geo.k[q * N + e] : T(0);
-                k1[i] = in ? geo.k[(9 + q) * N + e] : T(0);
-                k2[i] = in ? geo.k[(18 + q) * N + e] : T(0);
-                k3[i] = in ? geo.k[(27 + q) * N + e] : T(0);
-                nq[i] = in ? geo.n[q * N + e] : T(0);
-            }
-            a[i] = fmaT(k0[i], uxi[i], k1[i] * uet[i]);
-            b[i] = fmaT(k2[i], vxi[i], k3[i] * vet[i]);
-            s[i] = fmaT(k2[i], uxi[i], fmaT(k3[i], uet[i], fmaT(k0[i], vxi[i], k1[i] * vet[i])));
-        }
-        if constexpr (GEO == QUAD) {
-            T l[3] = { nr * fmaT(T(-2), a[1], a[0] + a[2]), nr * fmaT(T(-2), b[1], b[0] + b[2]),
-                nr * fmaT(T(-2), s[1], s[0] + s[2]) };
-            sumRows<T, E>(sh.strain, R, le, l);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                a[i] = fmaT(-l[0], nq[i], a[i]);
-                b[i] = fmaT(-l[1], nq[i], b[i]);
-                s[i] = fmaT(-l[2], nq[i], s[i]);
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-        bbmPoint(a[i], b[i], s[i], c[i], k, g[0][i], g[1][i], g[2][i], d[i]);
-    // P f and the damage's projection: sums over the three rows
 #pragma unroll
     for (int f = 0; f < 3; ++f)
-        sh.sum[R][f][le] = nr * fmaT(T(-2), g[f][1], g[f][0] + g[f][2]);
+        sum[R][f][le] = nr * fmaT(T(-2), g[f][1], g[f][0] + g[f][2]);
     [[maybe_unused]] T m0 = T(0), m1 = T(0), m2 = T(0);
     if constexpr (GEO == QUAD) {
 #pragma unroll
@@ -329,7 +259,7 @@ __device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const
 #pragma unroll
             for (int i = 0; i < 3; ++i)
                 t = fmaT(in ? wdam[(j * 9 + 3 * R + i) * N + e] : T(0), d[i], t);
-            sh.sum[R][3 + j][le] = t;
+            sum[R][3 + j][le] = t;
         }
     } else {
         // the row's Legendre coefficients along xi
@@ -338,15 +268,15 @@ __device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const
         m0 = fmaT(T(kW(0)), t2, d[1]);
         m1 = T(0.5 / kG) * (d[2] - d[0]);
         m2 = T(0.5 / (kG * kG)) * t2;
-        sh.sum[R][3][le] = m0;
-        sh.sum[R][4][le] = m1;
-        sh.sum[R][5][le] = m2;
+        sum[R][3][le] = m0;
+        sum[R][4][le] = m1;
+        sum[R][5][le] = m2;
     }
     __syncthreads();
     [[maybe_unused]] const T nRow = mid ? T(kN(1)) : T(kN(0));
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
-        const T l = sh.sum[0][f][le] + sh.sum[1][f][le] + sh.sum[2][f][le];
+        const T l = sum[0][f][le] + sum[1][f][le] + sum[2][f][le];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
             g[f][i] = fmaT(-l, GEO == QUAD ? nq[i] : nRow * T(kN(i)), g[f][i]);
@@ -355,7 +285,7 @@ __device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const
         T cf[DG];
 #pragma unroll
         for (int j = 0; j < DG; ++j)
-            cf[j] = sh.sum[0][3 + j][le] + sh.sum[1][3 + j][le] + sh.sum[2][3 + j][le];
+            cf[j] = sum[0][3 + j][le] + sum[1][3 + j][le] + sum[2][3 + j][le];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             T t = T(0);
@@ -366,7 +296,7 @@ __device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const
         }
     } else {
         // modes of total degree <= 2 (DG 6), 1 (DG 3) or 0 (DG 1) stay
-        auto at = [&](int m, int r) { return sh.sum[r][3 + m][le]; };
+        auto at = [&](int m, int r) { return sum[r][3 + m][le]; };
         auto second = [&](int m) { return fmaT(T(-2), at(m, 1), at(m, 0) + at(m, 2)); };
         auto mean = [&](int m) { return fmaT(T(kW(0)), second(m), at(m, 1)); };
         // the row value of the part of a coefficient that is quadratic in eta
@@ -399,14 +329,79 @@ __device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const
                 pt.s[(9 * f + q) * N + e] = g[f][i];
         }
     }
+}
+
+template <typename T, int E> struct BbmShared {
+    Exchange<T, E> ex;
+    T strain[3][3][E]; // nu . strain per row
+    T sum[3][9][E];
+};
+
+// Row R of an element in FP32: see kBbmStress.
+template <Geometry GEO, int DG, int E>
+__device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const StressGeometry<float>& geo,
+    const float* __restrict__ wdam, const float* __restrict__ wj, const BbmPoints<float>& pt, const float (&ke)[4],
+    float weight, const float (&c)[3][6], float (&g)[3][3], float (&d)[3], const BbmScalars<float>& k,
+    BbmShared<float, E>& sh, int le)
+{
+    using T = float;
+    T I[3], D[3], uxi[3], uet[3], vxi[3], vet[3], a[3], b[3], s[3];
+    auto take = [&](int f) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            I[i] = sh.ex.in.v[f][R][i][le];
+            D[i] = sh.ex.in.dv[f][R][i][le];
+        }
+    };
+    take(0);
+    deriv(I, uxi);
+    interp(D, uet);
+    take(1);
+    deriv(I, vxi);
+    interp(D, vet);
+    const bool mid = R == 1;
+    const T nr = mid ? T(-2) : T(1);
+    T k0[3], k1[3], k2[3], k3[3];
+    [[maybe_unused]] T nq[3] = { T(0), T(0), T(0) };
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const size_t q = 3 * R + i;
+        if constexpr (GEO == AFFINE) {
+            k0[i] = ke[0];
+            k1[i] = ke[1];
+            k2[i] = ke[2];
+            k3[i] = ke[3];
+        } else {
+            k0[i] = in ? geo.k[q * N + e] : T(0);
+            k1[i] = in ? geo.k[(9 + q) * N + e] : T(0);
+            k2[i] = in ? geo.k[(18 + q) * N + e] : T(0);
+            k3[i] = in ? geo.k[(27 + q) * N + e] : T(0);
+            nq[i] = in ? geo.n[q * N + e] : T(0);
+        }
+        a[i] = fmaT(k0[i], uxi[i], k1[i] * uet[i]);
+        b[i] = fmaT(k2[i], vxi[i], k3[i] * vet[i]);
+        s[i] = fmaT(k2[i], uxi[i], fmaT(k3[i], uet[i], fmaT(k0[i], vxi[i], k1[i] * vet[i])));
+    }
+    if constexpr (GEO == QUAD) {
+        T l[3] = { nr * fmaT(T(-2), a[1], a[0] + a[2]), nr * fmaT(T(-2), b[1], b[0] + b[2]),
+            nr * fmaT(T(-2), s[1], s[0] + s[2]) };
+        sumRows<T, E>(sh.strain, R, le, l);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            a[i] = fmaT(-l[0], nq[i], a[i]);
+            b[i] = fmaT(-l[1], nq[i], b[i]);
+            s[i] = fmaT(-l[2], nq[i], s[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        bbmPoint(a[i], b[i], s[i], c[i], k, g[0][i], g[1][i], g[2][i], d[i]);
+    bbmProject<T, GEO, DG, E>(R, e, N, in, wdam, nq, pt, g, d, sh.sum, le);
     // the divergence K^T (w J g) of this row: xi maps transposed
     T x[3], y[3];
     auto put = [&](int f, const T (&tx)[3], const T (&ty)[3]) {
         derivT(tx, x);
-        if constexpr (GEO == RECT)
-            sc.interpT(ty, y);
-        else
-            interpT(ty, y);
+        interpT(ty, y);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             sh.ex.out.x[f][R][i][le] = x[i];
@@ -423,20 +418,15 @@ __device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const
 #pragma unroll
         for (int i = 0; i < 3; ++i)
             g[f][i] *= w[i];
-    if constexpr (GEO == RECT) {
-        put(0, g[0], g[1]);
-        put(1, g[1], g[2]);
-    } else {
 #pragma unroll
-        for (int f = 0; f < 2; ++f) {
-            T p[3], q[3];
+    for (int f = 0; f < 2; ++f) {
+        T p[3], q[3];
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                p[i] = fmaT(k0[i], g[f][i], k2[i] * g[f + 1][i]);
-                q[i] = fmaT(k1[i], g[f][i], k3[i] * g[f + 1][i]);
-            }
-            put(f, p, q);
+        for (int i = 0; i < 3; ++i) {
+            p[i] = fmaT(k0[i], g[f][i], k2[i] * g[f + 1][i]);
+            q[i] = fmaT(k1[i], g[f][i], k3[i] * g[f + 1][i]);
         }
+        put(f, p, q);
     }
 }
 
@@ -444,20 +434,18 @@ __device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const
 // per element in three warps, as the mEVP kernel (nsdg_sumfact.cuh): node
 // column R, Gauss row R, node column R.
 //
-// Bound by FP64 issue in FP64 (about 1000 FP64 instructions per element where
-// the coefficient form took 3000, most of them in divisions, roots and
-// exponentials) and by memory on the mixed path (900 bytes per element, FP32).
-// Per launch: 96 x 80 rectangles, FP64, 21.7 us (121.8 us with coefficients and
-// per-element operators, 60 blocks of one thread per element); 256 x 256
-// parallelograms, mixed, 11.5 us (45.2 us: conversions of the FP64 state and
+// In FP32 bound by memory (900 bytes per element): 256 x 256 parallelograms 10.2
+// us per launch (45.2 us with the FP64 state as coefficients, its conversions and
 // 168 registers).  One thread per element, as the mEVP kernel takes on large
 // grids, was slower here: 8.5 against 4.3 us on 128 x 128, 10.4 to 11.1 against
 // 11.5 on 256 x 256.
-template <typename T, Geometry GEO, int DG, int E>
-__global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T> geo, const T* __restrict__ wdam,
-    const T* __restrict__ wj, const T* __restrict__ u, const T* __restrict__ v, BbmPoints<T> pt,
-    T* __restrict__ contrib, BbmScalars<T> k, int* __restrict__ err)
+template <Geometry GEO, int DG, int E>
+__global__ void __launch_bounds__(3 * E) kBbmStress32(DevMesh m, StressGeometry<float> geo,
+    const float* __restrict__ wdam, const float* __restrict__ wj, const float* __restrict__ u,
+    const float* __restrict__ v, BbmPoints<float> pt, float* __restrict__ contrib, BbmScalars<float> k,
+    int* __restrict__ err)
 {
+    using T = float;
     __shared__ BbmShared<T, E> sh;
     const int le = threadIdx.x % E, R = threadIdx.x / E;
     const size_t N = m.N, e = blockIdx.x * size_t(E) + le;
@@ -475,10 +463,6 @@ __global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T>
         d[i] = in ? beforeWait(pt.d + q * N + e) : T(1);
     }
     if (in) {
-        if constexpr (GEO == RECT) {
-            ke[0] = geo.k[e];
-            weight = wj[e];
-        }
         if constexpr (GEO == AFFINE) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -486,7 +470,7 @@ __global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T>
             weight = wj[e];
         }
     }
-    waitForPrevious(sizeof(T) == 4);
+    waitForPrevious();
     {
         T n[2][3] = { { T(0), T(0), T(0) }, { T(0), T(0), T(0) } };
         if (ice) {
@@ -512,7 +496,7 @@ __global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T>
         }
     }
     __syncthreads();
-    bbmRow<T, GEO, DG, E>(R, e, N, in, geo, wdam, wj, pt, ke, weight, c, g, d, k, sh, le);
+    bbmRow<GEO, DG, E>(R, e, N, in, geo, wdam, wj, pt, ke, weight, c, g, d, k, sh, le);
     bool finite = true; // g holds the weighted stress
 #pragma unroll
     for (int f = 0; f < 3; ++f)
@@ -536,6 +520,140 @@ __global__ void __launch_bounds__(3 * E) kBbmStress(DevMesh m, StressGeometry<T>
 #pragma unroll
         for (int r = 0; r < 3; ++r)
             contrib[(9 * f + 3 * r + R) * N + e] = o[r];
+    }
+}
+
+// The same in FP64, its linear maps in fixed point as the mEVP kernel's
+// (nsdg_stress_fixed.cuh): the strain's scale comes from the velocities, the
+// divergence's from the new weighted stress, F its largest (exchanged by a
+// barrier of its own); the maps stay within 16 (1 + rho) F on rectangles and 9 F
+// elsewhere.  The brittle update and the projections of the state stay in FP64.
+// Bound by FP64 issue (about 600 instructions per element, most in the update's
+// divisions and roots; 900 with the maps in FP64, 3000 on coefficients): 96 x 80
+// rectangles 17.4 us per launch (21.8 and 121.8 us); update of 100 sub-steps,
+// 192 x 192 rectangles 10.2 -> 7.2 ms, quadrilaterals 10.8 -> 7.7.
+template <Geometry GEO, int E> struct BbmFixedShared {
+    Exchange<fx::i64, E> ex;
+    fx::i64 strain[3][3][E];
+    double sum[3][9][E];
+    int top[2][3][E];
+};
+template <Geometry GEO, int DG, int E>
+__global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry geo, const double* __restrict__ proj,
+    const double* __restrict__ wdam, const double* __restrict__ wj, const double* __restrict__ u,
+    const double* __restrict__ v, BbmPoints<double> pt, double* __restrict__ contrib, BbmScalars<double> k,
+    int* __restrict__ err)
+{
+    using fx::i64;
+    __shared__ BbmFixedShared<GEO, E> sh;
+    const int le = threadIdx.x % E, R = threadIdx.x / E;
+    const size_t N = m.N, e = blockIdx.x * size_t(E) + le;
+    const bool in = e < N, ice = in && m.ice[e];
+    double c[3][6], g[3][3], d[3], w[3], nq[3], rho = 1.0;
+    [[maybe_unused]] int ke = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const size_t q = 3 * R + i;
+#pragma unroll
+        for (int j = 0; j < 6; ++j)
+            c[i][j] = in ? pt.c[(9 * j + q) * N + e] : 1.0;
+#pragma unroll
+        for (int f = 0; f < 3; ++f)
+            g[f][i] = in ? beforeWait(pt.s + (9 * f + q) * N + e) : 0.0;
+        d[i] = in ? beforeWait(pt.d + q * N + e) : 1.0;
+        if constexpr (GEO == RECT) {
+            w[i] = in ? kW(i) * wj[e] : 0.0; // the row's weight below
+            nq[i] = 0.0;
+        } else {
+            w[i] = in ? wj[q * N + e] : 0.0;
+            nq[i] = in ? proj[q * N + e] : 0.0;
+        }
+    }
+    if (in) {
+        if constexpr (GEO == RECT)
+            rho = geo.rect[e];
+        else
+            ke = geo.exponent[e];
+    }
+    waitForPrevious(false);
+    double n[2][3] = { { 0.0, 0.0, 0.0 }, { 0.0, 0.0, 0.0 } };
+    if (ice) {
+        const unsigned s2 = 2u * static_cast<unsigned>(m.nx) + 1u;
+        const unsigned ix = static_cast<unsigned>(e) % static_cast<unsigned>(m.nx);
+        const unsigned iy = static_cast<unsigned>(e) / static_cast<unsigned>(m.nx);
+        const size_t base = 2 * size_t(s2) * iy + 2 * ix + R;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            n[0][r] = afterWait(u + base + size_t(r) * s2);
+            n[1][r] = afterWait(v + base + size_t(r) * s2);
+        }
+    }
+    int word = 0;
+#pragma unroll
+    for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            word = max(word, fx::magnitudeWord(n[f][r]));
+    sh.top[0][R][le] = topOf(word);
+    __syncthreads();
+    const int top = topOfRows<E>(sh.top[0], le);
+    const bool bad = top > kTopMost; // not finite
+    const fx::Scaled sc(rho);
+    const int bits = strainBits<GEO>(sc);
+    fixedColumn<E>(n, fx::fixedShift(bits, top), R, le, sh.ex);
+    __syncthreads();
+    const FixedMap<GEO> map(geo, R, e, N, in);
+    i64 F11[3], F12[3], F22[3];
+    {
+        i64 a[3], b[3], s[3];
+        fixedStrain<GEO, E>(R, le, sc, map, sh.ex, sh.strain, a, b, s);
+        const int scale = bits - top + 1022;
+        const int at = fx::doubleExponent(GEO == RECT ? scale : scale - ke - 2);
+        const double none = __longlong_as_double(0x7ff8000000000000ll);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            bbmPoint(bad ? none : fx::toDouble(a[i], at), bad ? none : fx::toDouble(b[i], at),
+                bad ? none : fx::toDouble(s[i], at), c[i], k, g[0][i], g[1][i], g[2][i], d[i]);
+    }
+    bbmProject<double, GEO, DG, E>(R, e, N, in, wdam, nq, pt, g, d, sh.sum, le);
+    word = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        if constexpr (GEO == RECT)
+            w[i] *= R == 1 ? kW(1) : kW(0);
+#pragma unroll
+        for (int f = 0; f < 3; ++f) {
+            g[f][i] *= w[i];
+            word = max(word, fx::magnitudeWord(g[f][i]));
+        }
+    }
+    if (in && word >= 0x7ff00000)
+        atomicOr(err, DEV_ERR_NONFINITE_STRESS);
+    sh.top[1][R][le] = topOf(word);
+    __syncthreads();
+    const int topG = topOfRows<E>(sh.top[1], le);
+    const int bitsG = GEO == RECT ? 59 - sc.shift : 59;
+    const int atG = fx::fixedShift(bitsG, topG);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        F11[i] = fx::toFixed(g[0][i], atG);
+        F12[i] = fx::toFixed(g[1][i], atG);
+        F22[i] = fx::toFixed(g[2][i], atG);
+    }
+    fixedShares<GEO, 0, E>(R, le, sc, map, F11, F12, F22, sh.ex);
+    __syncthreads();
+    if (!ice)
+        return;
+    const int scale = bitsG - topG + 1022;
+    const int at = fx::doubleExponent(GEO == RECT ? scale : scale - ke - 2);
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+        i64 o[3];
+        fixedColumnShares<E>(f, R, le, sh.ex, o);
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            contrib[(9 * f + 3 * r + R) * N + e]
+                = topG > kTopMost ? __longlong_as_double(0x7ff8000000000000ll) : fx::toDouble(o[r], at);
     }
 }
 
@@ -657,16 +775,22 @@ cudaError_t launch(cudaStream_t s, void (*kernel)(KArgs...), size_t blocks, int 
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-template <typename T, int DG>
-cudaError_t stressFor(cudaStream_t s, const DevMesh& m, const BbmElements<T>& el, const T* u, const T* v,
-    T* contrib, const BbmScalars<T>& k, int* err)
+template <int DG>
+cudaError_t stressFor(cudaStream_t s, const DevMesh& m, const BbmElements<float>& el, const float* u, const float* v,
+    float* contrib, const BbmScalars<float>& k, int* err)
 {
     constexpr int E = kBbmElems;
-    const size_t blocks = (m.N + E - 1) / E;
-    if (el.geo.n)
-        return launch(s, kBbmStress<T, QUAD, DG, E>, blocks, 3 * E, m, el.geo, el.wdam, el.w, u, v, el.pt, contrib, k, err);
-    constexpr Geometry simple = sizeof(T) == 8 ? RECT : AFFINE;
-    return launch(s, kBbmStress<T, simple, DG, E>, blocks, 3 * E, m, el.geo, el.wdam, el.w, u, v, el.pt, contrib, k, err);
+    auto kernel = el.geo.n ? kBbmStress32<QUAD, DG, E> : kBbmStress32<AFFINE, DG, E>;
+    return launch(s, kernel, (m.N + E - 1) / E, 3 * E, m, el.geo, el.wdam, el.w, u, v, el.pt, contrib, k, err);
+}
+template <int DG>
+cudaError_t stressFor(cudaStream_t s, const DevMesh& m, const BbmElements<double>& el, const double* u,
+    const double* v, double* contrib, const BbmScalars<double>& k, int* err)
+{
+    constexpr int E = kBbmElems;
+    auto kernel = el.fixed.rect ? kBbmStress64<RECT, DG, E> : kBbmStress64<QUAD, DG, E>;
+    return launch(s, kernel, (m.N + E - 1) / E, 3 * E, m, el.fixed, el.geo.n, el.wdam, el.w, u, v, el.pt, contrib, k,
+        err);
 }
 
 } // namespace
@@ -722,9 +846,9 @@ cudaError_t launchBbmStress(cudaStream_t s, const DevMesh& m, int dg, const BbmE
     const BbmScalars<T> k { static_cast<T>(p.dt), static_cast<T>(p.nu0), static_cast<T>(0.5 * (1. - p.nu0)),
         static_cast<T>(p.tan_phi), static_cast<T>(p.exponent_relaxation_sigma - 1.), p.powRmode, p.powRk };
     switch (dg) {
-    case 1: return stressFor<T, 1>(s, m, el, u, v, contrib, k, err);
-    case 3: return stressFor<T, 3>(s, m, el, u, v, contrib, k, err);
-    case 6: return stressFor<T, 6>(s, m, el, u, v, contrib, k, err);
+    case 1: return stressFor<1>(s, m, el, u, v, contrib, k, err);
+    case 3: return stressFor<3>(s, m, el, u, v, contrib, k, err);
+    case 6: return stressFor<6>(s, m, el, u, v, contrib, k, err);
     default: return cudaErrorInvalidValue;
     }
 }

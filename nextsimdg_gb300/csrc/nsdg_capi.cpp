@@ -110,8 +110,8 @@ struct nsdg_kernel {
     double *Pg = nullptr, *contrib = nullptr;
     // the element maps of the sum-factorised stress kernels, the weights and
     // the weighted pressure (FP64, or pairs of floats on the mixed path)
-    StressGeometry<double> geo {}; // BBM
-    FixedGeometry fixedGeo {};     // mEVP
+    StressGeometry<double> geo {}; // FP64: rectangles, and the BBM projection
+    FixedGeometry fixedGeo {};
     StressGeometry<float> quad32 {}, aff32 {};
     const double* metricW = nullptr;
     double* Pw = nullptr;
@@ -473,6 +473,8 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     {
         const size_t sz = P.precision == NSDG_PRECISION_FP64 ? 8 : 4;
         add(metric.k.size(), sz); add(metric.n.size(), sz); add(metric.m.size(), sz); add(N, 4);
+        if (bbm)
+            add(metric.n.size(), sz); // the projection in both forms
         add(4 * N, 4);                            // the same on parallelograms
         add(9 * N); add(9 * N);                   // weights, weighted pressure
         if (bbm) {
@@ -578,11 +580,9 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         dops.hsize = upd(ops.hsize);
     }
     metricW = upd(metric.w);
-    if (!mixed() && (bbm || metric.rect)) {
-        geo.rect = metric.rect;
+    if (!mixed() && metric.rect) {
+        geo.rect = true;
         geo.k = upd(metric.k);
-        geo.n = metric.n.empty() ? nullptr : upd(metric.n);
-        geo.m = metric.m.empty() ? nullptr : upd(metric.m);
         fixedGeo.rect = geo.k;
     } else if (!mixed()) {
         FixedMetric fixed;
@@ -594,6 +594,8 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         fixedGeo.n = upi(fixed.n);
         fixedGeo.m = upi(fixed.m);
         fixedGeo.exponent = static_cast<const int*>(up(fixed.exponent.data(), N, 4, e));
+        if (bbm)
+            geo.n = upd(metric.n);
     }
     if (e != cudaSuccess)
         return fail(NSDG_ERR_CUDA, std::string("initialise: upload failed: ") + cudaGetErrorString(e));
@@ -700,6 +702,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
             bbmNode64.u = u;
             bbmNode64.v = v;
             bbm64.geo = geo;
+            bbm64.fixed = fixedGeo;
             bbm64.w = geo.rect ? upd(perElement()) : metricW;
             bbm64.wdam = geo.rect ? nullptr : upd(ops.wdam);
         } else {

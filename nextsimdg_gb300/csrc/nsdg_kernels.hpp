@@ -482,7 +482,8 @@ template <typename T> struct BbmPoints {
     T* d = nullptr; // [9][N] damage
 };
 template <typename T> struct BbmElements {
-    StressGeometry<T> geo {};
+    StressGeometry<T> geo {}; // FP64: rectangles' k (kBbmLoad), else n alone
+    FixedGeometry fixed {};   // FP64
     const T* wdam = nullptr; // [DG][9][N] damage projection (general quadrilaterals)
     const T* w = nullptr;    // StressMetric::w there; 2 J (times k_x on rectangles) per element else
     BbmPoints<T> pt {};

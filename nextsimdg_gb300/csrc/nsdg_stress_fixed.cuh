@@ -52,6 +52,209 @@ __device__ __forceinline__ void pointStress64(double pl, double mi, double s, do
     f = z * s;
 }
 
+// The maps of Gauss row R (nothing on rectangles).
+template <Geometry GEO> struct FixedMap {
+    fx::Split k0[3], k1[3], k2[3], k3[3], n[3], m[3];
+    __device__ __forceinline__ FixedMap(const FixedGeometry& geo, int R, size_t e, size_t N, bool active)
+        : FixedMap([&](const fx::i64* p, int row) { return fx::unpacked(active ? p[size_t(row) * N + e] : 0); }, geo,
+            3 * R)
+    {
+    }
+    template <typename F>
+    __device__ __forceinline__ FixedMap(F at, const FixedGeometry& geo, int q)
+        : k0 { at(geo.k, q), at(geo.k, q + 1), at(geo.k, q + 2) }
+        , k1 { at(geo.k, q + 9), at(geo.k, q + 10), at(geo.k, q + 11) }
+        , k2 { at(geo.k, q + 18), at(geo.k, q + 19), at(geo.k, q + 20) }
+        , k3 { at(geo.k, q + 27), at(geo.k, q + 28), at(geo.k, q + 29) }
+        , n { at(geo.n, q), at(geo.n, q + 1), at(geo.n, q + 2) }
+        , m { metric(at, geo, q), metric(at, geo, q + 1), metric(at, geo, q + 2) }
+    {
+    }
+    template <typename F> static __device__ __forceinline__ fx::Split metric(F at, const FixedGeometry& geo, int q)
+    {
+        return GEO == SPHERE ? at(geo.m, q) : fx::Split(0);
+    }
+};
+template <> struct FixedMap<RECT> {
+    __device__ __forceinline__ FixedMap(const FixedGeometry&, int, size_t, size_t, bool) { }
+};
+
+// nu (1, -2 or 4) times t
+__device__ __forceinline__ fx::i64 nuTimes(fx::i64 t, int f) { return f == 1 ? t : f == -2 ? -2 * t : fx::four(t); }
+
+// The velocities n[u, v][row] of node column R through the eta maps.
+template <int E>
+__device__ __forceinline__ void fixedColumn(const double (&n)[2][3], int at, int R, int le, Exchange<fx::i64, E>& ex)
+{
+    using fx::i64;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const i64 a[3] = { fx::toFixed(n[c][0], at), fx::toFixed(n[c][1], at), fx::toFixed(n[c][2], at) };
+        i64 val[3], der[3];
+        fx::interp(a, val);
+        fx::deriv(a, der);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            ex.in.v[c][r][R][le] = val[r];
+            ex.in.dv[c][r][R][le] = der[r];
+        }
+    }
+}
+
+// The half strains of Gauss row R (on quadrilaterals over 4 and projected; sums
+// takes the three rows' parts of nu . g).
+template <Geometry GEO, int E>
+__device__ __forceinline__ void fixedStrain(int R, int le, const fx::Scaled& sc, const FixedMap<GEO>& map,
+    const Exchange<fx::i64, E>& ex, fx::i64 (*sums)[3][E], fx::i64 (&a)[3], fx::i64 (&b)[3], fx::i64 (&s)[3])
+{
+    using fx::i64;
+    i64 I[3], D[3], uxi[3], uet[3], vxi[3], vet[3];
+    [[maybe_unused]] i64 up[3], vp[3];
+    auto take = [&](int c) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            I[i] = ex.in.v[c][R][i][le];
+            D[i] = ex.in.dv[c][R][i][le];
+        }
+    };
+    take(0);
+    fx::deriv(I, uxi);
+    if constexpr (GEO == RECT)
+        sc.interp(D, uet);
+    else
+        fx::interp(D, uet);
+    if constexpr (GEO == SPHERE)
+        fx::interp(I, up);
+    take(1);
+    fx::deriv(I, vxi);
+    if constexpr (GEO == RECT)
+        sc.interp(D, vet);
+    else
+        fx::interp(D, vet);
+    if constexpr (GEO == SPHERE)
+        fx::interp(I, vp);
+    if constexpr (GEO == RECT) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            a[i] = uxi[i];
+            b[i] = vet[i];
+            s[i] = uet[i] + vxi[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const fx::Split ux(uxi[i]), ue(uet[i]), vx(vxi[i]), ve(vet[i]);
+            a[i] = fx::mulHigh(ux, map.k0[i], ue, map.k1[i]);
+            b[i] = fx::mulHigh(vx, map.k2[i], ve, map.k3[i]);
+            s[i] = fx::mulHigh(ux, map.k2[i], ue, map.k3[i]) + fx::mulHigh(vx, map.k0[i], ve, map.k1[i]);
+            if constexpr (GEO == SPHERE) {
+                a[i] -= fx::mulHigh(fx::Split(vp[i]), map.m[i]);
+                s[i] += fx::mulHigh(fx::Split(up[i]), map.m[i]);
+            }
+        }
+        const int nr = R == 1 ? -2 : 1; // nu on this row: nr, -2 nr, nr
+        // P: subtract n (nu . g)
+        i64 c[3] = { nuTimes(a[0] + a[2] - 2 * a[1], nr), nuTimes(b[0] + b[2] - 2 * b[1], nr),
+            nuTimes(s[0] + s[2] - 2 * s[1], nr) };
+        sumRows<i64, E>(sums, R, le, c);
+        const fx::Split c0(c[0]), c1(c[1]), c2(c[2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            a[i] -= fx::four(fx::mulHigh(c0, map.n[i]));
+            b[i] -= fx::four(fx::mulHigh(c1, map.n[i]));
+            s[i] -= fx::four(fx::mulHigh(c2, map.n[i]));
+        }
+    }
+}
+
+// Row R's stresses F through the transposed xi maps (on quadrilaterals times
+// k / 4 and over 2^SHIFT).
+template <Geometry GEO, int SHIFT, int E>
+__device__ __forceinline__ void fixedShares(int R, int le, const fx::Scaled& sc, const FixedMap<GEO>& map,
+    const fx::i64 (&F11)[3], const fx::i64 (&F12)[3], const fx::i64 (&F22)[3], Exchange<fx::i64, E>& ex)
+{
+    using fx::i64;
+    auto put = [&](int c, const i64 (&tx)[3], const i64 (&ty)[3], [[maybe_unused]] const i64 (&tm)[3]) {
+        i64 x[3], y[3];
+        fx::derivT(tx, x);
+        if constexpr (GEO == RECT)
+            sc.interpT(ty, y);
+        else
+            fx::interpT(ty, y);
+        if constexpr (GEO == SPHERE) {
+            i64 z[3];
+            fx::interpT(tm, z);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                x[i] += z[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            ex.out.x[c][R][i][le] = x[i];
+            ex.out.y[c][R][i][le] = y[i];
+        }
+    };
+    if constexpr (GEO == RECT) {
+        put(0, F11, F12, F11);
+        put(1, F12, F22, F12);
+    } else {
+        auto over = [](i64 t) {
+            if constexpr (SHIFT > 0)
+                return (t + (1ll << (SHIFT - 1))) >> SHIFT;
+            else
+                return t;
+        };
+        i64 t0[3], t1[3], t2[3], t3[3];
+        [[maybe_unused]] i64 mu[3], mv[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const fx::Split f11(F11[i]), f12(F12[i]), f22(F22[i]);
+            t0[i] = over(fx::mulHigh(f11, map.k0[i], f12, map.k2[i]));
+            t1[i] = over(fx::mulHigh(f11, map.k1[i], f12, map.k3[i]));
+            t2[i] = over(fx::mulHigh(f12, map.k0[i], f22, map.k2[i]));
+            t3[i] = over(fx::mulHigh(f12, map.k1[i], f22, map.k3[i]));
+            if constexpr (GEO == SPHERE) {
+                mu[i] = over(fx::mulHigh(f12, map.m[i]));
+                mv[i] = over(-fx::mulHigh(f11, map.m[i]));
+            }
+        }
+        if constexpr (GEO == SPHERE) {
+            put(0, t0, t1, mu);
+            put(1, t2, t3, mv);
+        } else {
+            put(0, t0, t1, t0);
+            put(1, t2, t3, t2);
+        }
+    }
+}
+
+// Node column R's shares of component c.
+template <int E>
+__device__ __forceinline__ void fixedColumnShares(int c, int R, int le, const Exchange<fx::i64, E>& ex,
+    fx::i64 (&o)[3])
+{
+    fx::i64 x[3], y[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        x[r] = ex.out.x[c][r][R][le];
+        y[r] = ex.out.y[c][r][R][le];
+    }
+    fx::columnT(x, y, o);
+}
+
+// the velocities' scale: bits below the largest one
+template <Geometry GEO> __device__ __forceinline__ int strainBits(const fx::Scaled& sc)
+{
+    return GEO == RECT ? min(58, 61 - sc.shift) : 55;
+}
+// the largest of the three rows' or columns' exponents, at least 2^-900 (below
+// which values count as 0)
+template <int E> __device__ __forceinline__ int topOfRows(const int (*top)[E], int le)
+{
+    return max(max(top[0][le], 123), max(top[1][le], top[2][le]));
+}
+constexpr int kTopMost = 1923; // above: beyond 2^900, or not finite
+
 // Three threads per element as stressBlock: node column R, Gauss row R, node
 // column R.
 template <Geometry GEO, int E>
@@ -103,168 +306,55 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
             word = max(word, fx::magnitudeWord(n[c][r]));
     sh.top[0][R][le] = topOf(word);
     __syncthreads();
-    int top = max(sh.top[0][0][le], max(sh.top[0][1][le], sh.top[0][2][le]));
-    int topP = max(sh.top[1][0][le], max(sh.top[1][1][le], sh.top[1][2][le]));
-    // not finite, or beyond 2^900
-    bool bad = max(top, topP) > 1923;
-    // 2^-900 counts as 0; the increments' products may round up to 2^topP
-    top = max(top, 123);
-    topP = max(topP, 123) + 1;
+    const int top = topOfRows<E>(sh.top[0], le);
+    // the increments' products may round up to 2^topP
+    const int topP = topOfRows<E>(sh.top[1], le) + 1;
+    bool bad = max(top, topP - 1) > kTopMost;
     const fx::Scaled sc(rho);
-    const int bits = GEO == RECT ? min(58, 61 - sc.shift) : 55;
-    const int at = fx::fixedShift(bits, top);
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        const i64 a[3] = { fx::toFixed(n[c][0], at), fx::toFixed(n[c][1], at), fx::toFixed(n[c][2], at) };
-        i64 val[3], der[3];
-        fx::interp(a, val);
-        fx::deriv(a, der);
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            sh.ex.in.v[c][r][R][le] = val[r];
-            sh.ex.in.dv[c][r][R][le] = der[r];
-        }
-    }
+    const int bits = strainBits<GEO>(sc);
+    fixedColumn<E>(n, fx::fixedShift(bits, top), R, le, sh.ex);
     __syncthreads();
     // Gauss row R
-    const int scale = bits - top + 1022; // of the strain (on quadrilaterals before the products with k / 4)
+    const int scale = bits - top + 1022; // of the strain
+    const int atStrain = fx::doubleExponent(GEO == RECT ? scale : scale - ke - 2);
     const int bitsP = GEO == RECT ? 58 - sc.shift : 58;
     const int atP = fx::fixedShift(bitsP, topP);
-    i64 I[3], D[3], uxi[3], uet[3], vxi[3], vet[3], F11[3], F12[3], F22[3], x[3], y[3];
-    [[maybe_unused]] i64 up[3], vp[3];
-    auto take = [&](int c) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            I[i] = sh.ex.in.v[c][R][i][le];
-            D[i] = sh.ex.in.dv[c][R][i][le];
-        }
-    };
-    take(0);
-    fx::deriv(I, uxi);
-    if constexpr (GEO == RECT)
-        sc.interp(D, uet);
-    else
-        fx::interp(D, uet);
-    if constexpr (GEO == SPHERE)
-        fx::interp(I, up);
-    take(1);
-    fx::deriv(I, vxi);
-    if constexpr (GEO == RECT)
-        sc.interp(D, vet);
-    else
-        fx::interp(D, vet);
-    if constexpr (GEO == SPHERE)
-        fx::interp(I, vp);
+    const FixedMap<GEO> map(geo, R, e, N, active);
+    i64 a[3], b[3], s[3], F11[3], F12[3], F22[3];
+    fixedStrain<GEO, E>(R, le, sc, map, sh.ex, sh.sums[0], a, b, s);
     int most = 0;
-    auto increments = [&](int i, i64 a, i64 b, i64 s, int atStrain) {
+    [[maybe_unused]] i64 nf[3] = { 0, 0, 0 }; // n . f
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
         double zp, d, f;
-        pointStress64(fx::toDouble(a + b, atStrain + 1), fx::toDouble(a - b, atStrain), fx::toDouble(s, atStrain), pq[i],
-            dmin2, zp, d, f);
+        pointStress64(fx::toDouble(a[i] + b[i], atStrain + 1), fx::toDouble(a[i] - b[i], atStrain),
+            fx::toDouble(s[i], atStrain), pq[i], dmin2, zp, d, f);
         most = max(most, max(fx::magnitudeWord(zp), max(fx::magnitudeWord(d), fx::magnitudeWord(f))));
-        const i64 w = 2 * (fx::toFixed(zp, atP) - fx::toFixed(pq[i], atP)), D1 = fx::toFixed(d, atP);
-        F11[i] = w + D1;
-        F22[i] = w - D1;
+        const i64 w = 2 * (fx::toFixed(zp, atP) - fx::toFixed(pq[i], atP)), D = fx::toFixed(d, atP);
+        F11[i] = w + D;
+        F22[i] = w - D;
         F12[i] = fx::toFixed(f, atP);
-    };
+        if constexpr (GEO != RECT) {
+            nf[0] += fx::mulHigh(fx::Split(F11[i]), map.n[i]);
+            nf[1] += fx::mulHigh(fx::Split(F22[i]), map.n[i]);
+            nf[2] += fx::mulHigh(fx::Split(F12[i]), map.n[i]);
+        }
+    }
     if constexpr (GEO == RECT) {
-        const int atStrain = fx::doubleExponent(scale);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            increments(i, uxi[i], vet[i], uet[i] + vxi[i], atStrain);
         __syncthreads(); // every warp has taken its row: the buffer changes hands
-        auto put = [&](int c, const i64 (&fx_)[3], const i64 (&fy)[3]) {
-            fx::derivT(fx_, x);
-            sc.interpT(fy, y);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                sh.ex.out.x[c][R][i][le] = x[i];
-                sh.ex.out.y[c][R][i][le] = y[i];
-            }
-        };
-        put(0, F11, F12);
-        put(1, F12, F22);
     } else {
-        const int atStrain = fx::doubleExponent(scale - ke - 2);
-        i64 a[3], b[3], s[3];
-        auto factor = [&](const i64* p, size_t row) { return fx::unpacked(active ? p[row * N + e] : 0); };
-        fx::Split k0[3] = { factor(geo.k, 3 * R), factor(geo.k, 3 * R + 1), factor(geo.k, 3 * R + 2) };
-        fx::Split k1[3] = { factor(geo.k, 9 + 3 * R), factor(geo.k, 10 + 3 * R), factor(geo.k, 11 + 3 * R) };
-        fx::Split k2[3] = { factor(geo.k, 18 + 3 * R), factor(geo.k, 19 + 3 * R), factor(geo.k, 20 + 3 * R) };
-        fx::Split k3[3] = { factor(geo.k, 27 + 3 * R), factor(geo.k, 28 + 3 * R), factor(geo.k, 29 + 3 * R) };
-        fx::Split nq[3] = { factor(geo.n, 3 * R), factor(geo.n, 3 * R + 1), factor(geo.n, 3 * R + 2) };
-        auto metric = [&](int i) { return GEO == SPHERE ? factor(geo.m, 3 * R + i) : fx::Split(0); };
-        [[maybe_unused]] fx::Split mq[3] = { metric(0), metric(1), metric(2) };
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const fx::Split ux(uxi[i]), ue(uet[i]), vx(vxi[i]), ve(vet[i]);
-            a[i] = fx::mulHigh(ux, k0[i], ue, k1[i]);
-            b[i] = fx::mulHigh(vx, k2[i], ve, k3[i]);
-            s[i] = fx::mulHigh(ux, k2[i], ue, k3[i]) + fx::mulHigh(vx, k0[i], ve, k1[i]);
-            if constexpr (GEO == SPHERE) {
-                a[i] -= fx::mulHigh(fx::Split(vp[i]), mq[i]);
-                s[i] += fx::mulHigh(fx::Split(up[i]), mq[i]);
-            }
-        }
-        const int nr = R == 1 ? -2 : 1; // nu on this row: nr, -2 nr, nr
-        auto times = [&](i64 t, int f) { return f == 1 ? t : f == -2 ? -2 * t : 4 * t; };
-        // P: subtract n (nu . g)
-        i64 c[3] = { times(a[0] + a[2] - 2 * a[1], nr), times(b[0] + b[2] - 2 * b[1], nr),
-            times(s[0] + s[2] - 2 * s[1], nr) };
-        sumRows<i64, E>(sh.sums[0], R, le, c);
-        i64 d[3] = { 0, 0, 0 };
-        const fx::Split c0(c[0]), c1(c[1]), c2(c[2]);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            increments(i, a[i] - fx::four(fx::mulHigh(c0, nq[i])), b[i] - fx::four(fx::mulHigh(c1, nq[i])),
-                s[i] - fx::four(fx::mulHigh(c2, nq[i])), atStrain);
-            d[0] += fx::mulHigh(fx::Split(F11[i]), nq[i]);
-            d[1] += fx::mulHigh(fx::Split(F22[i]), nq[i]);
-            d[2] += fx::mulHigh(fx::Split(F12[i]), nq[i]);
-        }
         // P^T: subtract nu (n . f)
-        sumRows<i64, E>(sh.sums[1], R, le, d);
-        i64 t0[3], t1[3], t2[3], t3[3];
-        [[maybe_unused]] i64 mu[3], mv[3];
-        // sums of products with k / 4, over 8
-        auto eighth = [](i64 t) { return (t + 4) >> 3; };
+        sumRows<i64, E>(sh.sums[1], R, le, nf);
+        const int nr = R == 1 ? -2 : 1;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             const int w = i == 1 ? -2 * nr : nr;
-            const fx::Split f11(F11[i] - times(fx::four(d[0]), w)), f22(F22[i] - times(fx::four(d[1]), w)),
-                f12(F12[i] - times(fx::four(d[2]), w));
-            t0[i] = eighth(fx::mulHigh(f11, k0[i], f12, k2[i]));
-            t1[i] = eighth(fx::mulHigh(f11, k1[i], f12, k3[i]));
-            t2[i] = eighth(fx::mulHigh(f12, k0[i], f22, k2[i]));
-            t3[i] = eighth(fx::mulHigh(f12, k1[i], f22, k3[i]));
-            if constexpr (GEO == SPHERE) {
-                mu[i] = eighth(fx::mulHigh(f12, mq[i]));
-                mv[i] = eighth(-fx::mulHigh(f11, mq[i]));
-            }
-        }
-        auto put = [&](int c, const i64 (&tx)[3], const i64 (&ty)[3], [[maybe_unused]] const i64 (&tm)[3]) {
-            fx::derivT(tx, x);
-            fx::interpT(ty, y);
-            if constexpr (GEO == SPHERE) {
-                i64 z[3];
-                fx::interpT(tm, z);
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-                    x[i] += z[i];
-            }
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                sh.ex.out.x[c][R][i][le] = x[i];
-                sh.ex.out.y[c][R][i][le] = y[i];
-            }
-        };
-        if constexpr (GEO == SPHERE) {
-            put(0, t0, t1, mu);
-            put(1, t2, t3, mv);
-        } else {
-            put(0, t0, t1, t0);
-            put(1, t2, t3, t2);
+            F11[i] -= nuTimes(fx::four(nf[0]), w);
+            F22[i] -= nuTimes(fx::four(nf[1]), w);
+            F12[i] -= nuTimes(fx::four(nf[2]), w);
         }
     }
+    fixedShares<GEO, 3, E>(R, le, sc, map, F11, F12, F22, sh.ex);
     sh.top[0][R][le] = bad || most >= 0x7ff00000;
     __syncthreads();
     if (!active)
@@ -275,12 +365,7 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         i64 o[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            x[r] = sh.ex.out.x[c][r][R][le];
-            y[r] = sh.ex.out.y[c][r][R][le];
-        }
-        fx::columnT(x, y, o);
+        fixedColumnShares<E>(c, R, le, sh.ex, o);
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
             const double div = bad ? __longlong_as_double(0x7ff8000000000000ll) : fx::toDouble(o[r], atOut);

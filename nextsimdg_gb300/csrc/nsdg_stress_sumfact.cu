@@ -10,20 +10,21 @@ namespace {
 using namespace sf;
 
 // FP64 (nsdg_stress_fixed.cuh).  Bound by FP64 issue (108 instructions per
-// element) and the integer work beside it.  Timed alone (CUDA events): 19.3 us
+// element) and the integer work beside it.  Timed alone (CUDA events): 19.1 us
 // for 256 x 256 rectangles (60.8 us with the linear maps in FP64, 112 us with
-// 9 x 9 operators streamed from memory), 16.7 us for 201 x 143 quadrilaterals (42
-// and 49 us), 11.7 us for 154 x 121 cells of a sphere (32 and 44 us), 4.6 us for
+// 9 x 9 operators streamed from memory), 16.5 us for 201 x 143 quadrilaterals (42
+// and 49 us), 11.5 us for 154 x 121 cells of a sphere (32 and 44 us), 4.6 us for
 // 64 x 64 rectangles (7.4 and 20.5 us).  Three threads per element: with one, a
 // 64 x 64 grid is one warp per SM that waits out every instruction's latency.
-// Without a bound on the registers (80, 128 and 166): with six or more blocks per
-// SM forced, quadrilaterals and spheres spill (16.9 and 14.6 us) and rectangles
-// gain nothing.
+// The blocks per SM bound the registers at 80, 128 and 168: left alone the
+// compiler takes 72, 128 and 130 (sphere 12.4 us); six or more blocks make
+// quadrilaterals and spheres spill (16.9 and 14.6 us), four leave the former a
+// longer tail (update 2.73 against 2.54 ms).
 constexpr int kElems = kFixedElems;
 
 template <Geometry GEO>
-__global__ void __launch_bounds__(3 * kElems) kMevpStress(DevMesh m, FixedGeometry geo, const double* __restrict__ u,
-    const double* __restrict__ v, const double* __restrict__ Pw, double* __restrict__ tdiv, double dmin2, double keep, bool release)
+__global__ void __launch_bounds__(3 * kElems, GEO == RECT ? 8 : GEO == QUAD ? 5 : 4) kMevpStress(DevMesh m,
+    FixedGeometry geo, const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ Pw, double* __restrict__ tdiv, double dmin2, double keep, bool release)
 {
     __shared__ FixedShared<GEO, kElems> sh;
     stressFixed<GEO, kElems>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, dmin2, keep, release, blockIdx.x * size_t(kElems),

@@ -1,4 +1,4 @@
-"""The fixed-point FP64 element update on the GPU against the CPU oracle, on
+"""The fixed-point FP64 element updates on the GPU against the CPU oracle, on
 what its scales depend on: side ratios on both sides of the rectangles' limit
 of 32, open water (a pressure of zero), and neighbouring velocities of very
 different size."""
@@ -6,13 +6,13 @@ import numpy as np
 import pytest
 
 from nextsimdg_gb300._lib import NsdgError
-from nextsimdg_gb300.dynamics import MEVPDynamicsKernel
+from nextsimdg_gb300.dynamics import BBMDynamicsKernel, MEVPDynamicsKernel
 from test_stress_metric import _coords
 
 pytestmark = pytest.mark.gpu
 
 
-def _step(k, ratio, spread, steps=2):
+def _step(k, ratio, spread, steps=2, damage=None):
     nx, ny = 11, 9
     c = np.array(_coords("stretched", nx, ny), dtype=float)
     c[..., 1] *= ratio
@@ -23,6 +23,8 @@ def _step(k, ratio, spread, steps=2):
          "vwind": rng.uniform(-3, 3, n), "uocean": np.zeros(n), "vocean": np.full(n, 0.02), "ssh": np.zeros(n)}
     f["u"], f["v"] = (rng.uniform(-0.1, 0.1, n) * 10.0 ** rng.uniform(-spread, 0, n) for _ in range(2))
     f["hice"][: n // 3] = f["cice"][: n // 3] = 0.0
+    if damage is not None:
+        f["damage"] = rng.uniform(damage, 1.0, n)
     for name, a in f.items():
         k.setData(name, a)
     for s in range(steps):
@@ -35,6 +37,16 @@ def test_matches_oracle(gpu, oracle, ratio, spread):
     """1e-10 of the largest value, the bar of the FP64 path."""
     got = _step(MEVPDynamicsKernel(dg_comp=3, n_steps=60), ratio, spread)
     ref = _step(oracle.OracleKernel(0, 3, n_steps=60), ratio, spread)
+    for name, r in ref.items():
+        assert np.abs(got[name] - r).max() <= 1e-10 * max(np.abs(r).max(), 1e-300), name
+
+
+@pytest.mark.parametrize("ratio,spread", [(1 / 60, 0), (1 / 20, 3), (20.0, 0), (60.0, 0)])
+def test_bbm_matches_oracle(gpu, oracle, ratio, spread):
+    """Ten sub-steps: 1e-10 of the largest value (the oracle's own response to
+    h x (1 + 1e-14) is below 3e-14)."""
+    got = _step(BBMDynamicsKernel(dg_comp=3, n_steps=10), ratio, spread, steps=1, damage=0.5)
+    ref = _step(oracle.OracleKernel(1, 3, n_steps=10), ratio, spread, steps=1, damage=0.5)
     for name, r in ref.items():
         assert np.abs(got[name] - r).max() <= 1e-10 * max(np.abs(r).max(), 1e-300), name
 
