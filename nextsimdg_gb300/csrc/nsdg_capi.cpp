@@ -163,7 +163,8 @@ struct nsdg_kernel {
     // mixed path on a parallelogram mesh without periodic edges: the tiled
     // transport stage (edge fluxes staged in shared memory, cell term from
     // affCoef, diagonal M^{-1}); NSDG_TRANSPORT_KERNEL=element keeps the
-    // per-element kernel
+    // per-element kernel (256 x 256 BBM, three fields of six modes: 19 us per
+    // stage against 50)
     double* minvDiag = nullptr;      // [dg][N]
     bool trAffine = false;
     double trAffWorst[2] = { -1, -1 }; // cell-operator mismatch, relative off-diagonal of M^{-1}
@@ -394,6 +395,8 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     Pw = nullptr;
     Pw32 = nullptr;
     affCoef = nullptr;
+    minvDiag = nullptr;
+    trAffine = false;
 
     // --- host mesh (DynamicsKernel.hpp:44-75) ---
     mesh = HostMesh();
@@ -488,17 +491,17 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         add(324 * pairsLd(N), 8);                 // float-pair stress operators
     if (P.precision == NSDG_PRECISION_MIXED && !bbm) {
         add((mesh.spherical ? 486 : 324) * ops32Ld(N), 4);
-        add(5 * ops32Ld(N), 4);                   // parallelogram coefficients
         add(18 * N, 4);
         for (int i = 0; i < 4; ++i) add(Ncg, 4);  // FP32 u, v, u0, v0
         add(8 * Ncg, 4);                          // the packed per-step node constants
         add(18 * N, 4); add(Ncg, 4); add(Ncg, 4); // start of the previous sub-cycle
         add(9 * N, 4);                            // P/(2 alpha)
-        add(size_t(dg) * N);                      // diagonal of M^{-1} (parallelogram transport)
     }
     if (P.precision == NSDG_PRECISION_MIXED) {
         add(ops.cellX.size(), 4); add(ops.cellY.size(), 4); // FP32 transport operators
         add(ops.jwA.size(), 4);                             // FP32 J w of the CG2DG quadrature
+        add(5 * ops32Ld(N), 4);                             // parallelogram coefficients
+        add(size_t(dg) * N);                                // diagonal of M^{-1} (parallelogram transport)
     }
     if (P.precision == NSDG_PRECISION_MIXED && bbm) {
         add(ops.cellX8.size(), 4); add(ops.cellY8.size(), 4);
@@ -673,6 +676,36 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         cellY32 = upf(ops.cellY);
         jwA32 = upf(ops.jwA);
     }
+    auto takeAffine = [&](const AffineStressOps& aff) {
+        affCoef = arena.take<float>(aff.coef.size());
+        if (!affCoef)
+            e = cudaErrorMemoryAllocation;
+        else if (e == cudaSuccess)
+            e = cudaMemcpy(affCoef, aff.coef.data(), aff.coef.size() * sizeof(float), cudaMemcpyHostToDevice);
+        affLd = ops32Ld(N);
+    };
+    // the transport on the same coefficients: the rebuilt cell operators within
+    // 1e-9 of the exact ones (far below FP32 rounding), M^{-1} diagonal to 1e-12
+    // of its diagonal
+    auto tiledTransport = [&] {
+        const char* tk = std::getenv("NSDG_TRANSPORT_KERNEL");
+        if (!affCoef || !transport32 || !flags.perEntry.empty())
+            return;
+        AffineTransportOps atr;
+        const bool fits = buildAffineTransportOps(mesh, ops, 1e-9, 1e-12, atr);
+        trAffWorst[0] = atr.worstCell;
+        trAffWorst[1] = atr.worstOffDiag;
+        if (!fits || (tk && std::strcmp(tk, "element") == 0))
+            return;
+        minvDiag = arena.take<double>(atr.minvDiag.size());
+        if (!minvDiag)
+            e = cudaErrorMemoryAllocation;
+        else if (e == cudaSuccess)
+            e = cudaMemcpy(minvDiag, atr.minvDiag.data(), atr.minvDiag.size() * sizeof(double), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+            e = uploadAffineTransportReference(dg, atr.ref);
+        trAffine = e == cudaSuccess;
+    };
     if (bbm) {
         // 2 J (times k_x on rectangles) from the weight of the centre point
         auto perElement = [&]() {
@@ -724,6 +757,10 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
                 bbmAffine = buildAffineStressOps(mesh, ops, ops32Ld(N), 1e-9, aff)
                     && buildAffineBbmOps(mesh, ops, 1e-9, abb);
                 affWorst = std::max(aff.worst, abb.worst);
+                if (bbmAffine) {
+                    takeAffine(aff);
+                    tiledTransport();
+                }
             }
             if (bbmAffine) {
                 std::vector<double> centre(4 * N);
@@ -782,39 +819,14 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
             AffineStressOps aff;
             const size_t ld = ops32Ld(N);
             if (buildAffineStressOps(mesh, ops, ld, 1e-9, aff)) {
-                affCoef = arena.take<float>(aff.coef.size());
-                if (!affCoef)
-                    e = cudaErrorMemoryAllocation;
-                else if (e == cudaSuccess)
-                    e = cudaMemcpy(affCoef, aff.coef.data(), aff.coef.size() * sizeof(float), cudaMemcpyHostToDevice);
-                affLd = ld;
+                takeAffine(aff);
                 std::vector<double> centre(4 * N); // the map is the same at every point
                 for (size_t c = 0; c < 4; ++c)
                     std::copy_n(metric.k.begin() + (9 * c + 4) * N, N, centre.begin() + c * N);
                 aff32.k = upf(centre);
             }
             affWorst = aff.worst;
-            // the transport on the same coefficients: the rebuilt cell
-            // operators within 1e-9 of the exact ones (far below FP32
-            // rounding), M^{-1} diagonal to 1e-12 of its diagonal
-            const char* tk = std::getenv("NSDG_TRANSPORT_KERNEL");
-            if (affCoef && transport32 && flags.perEntry.empty()) {
-                AffineTransportOps atr;
-                const bool fits = buildAffineTransportOps(mesh, ops, 1e-9, 1e-12, atr);
-                trAffWorst[0] = atr.worstCell;
-                trAffWorst[1] = atr.worstOffDiag;
-                if (fits && !(tk && std::strcmp(tk, "element") == 0)) {
-                    minvDiag = arena.take<double>(atr.minvDiag.size());
-                    if (!minvDiag)
-                        e = cudaErrorMemoryAllocation;
-                    else if (e == cudaSuccess)
-                        e = cudaMemcpy(minvDiag, atr.minvDiag.data(), atr.minvDiag.size() * sizeof(double),
-                            cudaMemcpyHostToDevice);
-                    if (e == cudaSuccess)
-                        e = uploadAffineTransportReference(dg, atr.ref);
-                    trAffine = e == cudaSuccess;
-                }
-            }
+            tiledTransport();
         }
         auto zf = [&](size_t n) {
             float* p = arena.take<float>(n);

@@ -24,7 +24,8 @@ constexpr int kElems = kFixedElems;
 
 template <Geometry GEO>
 __global__ void __launch_bounds__(3 * kElems, GEO == RECT ? 8 : GEO == QUAD ? 5 : 4) kMevpStress(DevMesh m,
-    FixedGeometry geo, const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ Pw, double* __restrict__ tdiv, double dmin2, double keep, bool release)
+    FixedGeometry geo, const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ Pw,
+    double* __restrict__ tdiv, double dmin2, double keep, bool release)
 {
     __shared__ FixedShared<GEO, kElems> sh;
     stressFixed<GEO, kElems>(m.nx, m.N, m.ice, geo, u, v, Pw, tdiv, dmin2, keep, release, blockIdx.x * size_t(kElems),
