@@ -5,7 +5,8 @@ Workload (the configuration the headline metric is quoted on, one GPU): the
 512 x 512 box test with DG2 transport (6 components), CG2 velocity, DG-stress
 8, 100 mEVP iterations (alpha = beta = 300) per 120 s step, in the mixed
 precision mode (FP32 stress/momentum arithmetic and state; FP64 for the
-conservation sums, the inverse mass matrices, Delta and the viscosity).
+conservation sums, the inverse mass matrices and the node constants; Delta
+and the viscosity in pairs of floats).
 One "step" is one model step: the DG transport of concentration and
 thickness with limiters, the preparation of the momentum solve and the 100
 mEVP iterations (strain, stress, divergence, momentum, boundaries).
@@ -100,11 +101,21 @@ def bytes_per_element_iteration_stress(word: int = 8, spherical: bool = False, p
     return operators + pressure + tdiv + velocity
 
 
-def flops_per_element_iteration_stress() -> int:
-    """Flops of kMevpStress per element (FMA = 2): strain 4 x 81 FMA, Delta,
-    viscosity and stress increments ~12 per Gauss point, divergence update
-    4 x 81 FMA + 18."""
-    return 2 * (4 * 81) + 9 * 12 + 2 * (4 * 81) + 2 * 18
+def launched_stress_bytes(kind: str, word: int, spherical: bool = False) -> int:
+    """Algorithmic bytes per element of the element kernel a step launches:
+    the operator kernels' above ("pairs", "tma"), and of the sum-factorised
+    ones the map (FP64 tensor grid 2 words, parallelograms 4, else 36 + 9 and
+    on a sphere 9 more), the weighted pressure at 9 Gauss points (8 bytes: FP64
+    or a pair of floats), the divergence and the velocity."""
+    if kind in ("pairs", "tma"):
+        return bytes_per_element_iteration_stress(word, spherical=spherical)
+    words = {"fp64": 2, "affine": 4}.get(kind, 54 if spherical else 45)
+    return words * word + 9 * 8 + 2 * 18 * word + 4 * 2 * word
+
+
+# FP64 instructions per element of the FP64 stress kernel: ten per Gauss point
+# and one per divergence coefficient (its linear maps run in fixed point)
+FP64_STRESS_INSTRUCTIONS = 9 * 10 + 18
 
 
 def bytes_per_cell_update(n_iter: int = NSTEPS, word: int = 8) -> float:
@@ -134,13 +145,13 @@ def launched_bytes_per_cell_update(box, prec: int, stress_kind: str, tiled_trans
     actually launches (each array counted once per launch), by part:
     100 x (element stress kernel + node momentum kernel) + transport,
     preparation and read-outs.  stress_kind names the element kernel:
-    "fp64" (FP64 operators), "pairs" (the same bytes as float pairs),
-    "affine" (5 FP32 coefficients per element), "tma"/"global" (FP32
+    "fp64" (tensor grid), "pairs" (9 x 9 operators as float pairs), "affine"
+    (parallelograms), "global" (the map at every Gauss point), "tma" (FP32
     operators)."""
     N = box.nelements
     ncg = (2 * box.nx + 1) * (2 * box.ny + 1)
     word = 8 if prec == 0 else 4
-    stress = bytes_per_element_iteration_stress(word, parallelogram=stress_kind == "affine")
+    stress = launched_stress_bytes(stress_kind, word)
     if prec == 0:
         # 15 FP64 node streams read, u and v written, the Dirichlet flag
         node = ncg * (15 * 8 + 2 * 8 + 1) / N
@@ -402,7 +413,7 @@ def stress_roofline(k, N: int, prec: int, ms_step: float, local: int, nx: int):
     nms, nname = k.time_kernel(1, 50)
     kind, mismatch = k.stress_variant()
     affine = kind == "affine"
-    bpe = bytes_per_element_iteration_stress(4 if prec else 8, parallelogram=affine)
+    bpe = launched_stress_bytes(kind if prec else "pairs" if "Pairs" in kname else "fp64", 4 if prec else 8)
     achieved = N * bpe / (kms * 1e-3) / 1e9
     hbm, hbm_kind = measured_peaks()
     traffic = None
@@ -417,9 +428,9 @@ def stress_roofline(k, N: int, prec: int, ms_step: float, local: int, nx: int):
             "kernel_timing": "CUDA events on the library's stream around 50 back-to-back launches of the kernel "
                              "on the workload's state, right after the timed steps"}
     if prec:
-        # every FP32 stress kernel on this mesh: the operator-streaming ones
-        # (global loads, TMA tiles) and, on a parallelogram mesh, the
-        # coefficient kernel with each FP64 viscosity form
+        # every FP32 stress kernel on this mesh: the map at every Gauss point,
+        # the TMA-staged operators and, on a parallelogram mesh, the
+        # coefficient kernel with each viscosity form
         names = {3: "global", 4: "tma", 5: "affine_rsqrt_f64", 6: "affine_newton_f64", 7: "affine_newton_f64_intcvt",
                  8: "affine_float_pairs", 12: "affine_float_pairs_checked"}
         ids = (3, 4, 5, 6, 7, 8, 12) if affine else (3, 4)
@@ -427,11 +438,10 @@ def stress_roofline(k, N: int, prec: int, ms_step: float, local: int, nx: int):
         roof["stress_kernel"] = kind
         roof["parallelogram_mismatch"] = mismatch
         if affine:
-            # form 2 (the default: the FP64 Newton step, 3 DFMA + 2 DMUL per
-            # Gauss point) is bound by FP64 issue, against the FMA-lane rate
-            # of the measured FP64 DGEMM; form 4 computes the same step in
-            # float pairs, bitwise equal, and runs the FP64 step only where
-            # its rounding check fails (about 1e-4 of the Gauss points)
+            # form 3 (the default: the Newton step in float pairs) leaves the
+            # kernel to its memory traffic; form 2 (the same step in FP64, 3
+            # DFMA + 2 DMUL per Gauss point) is bound by FP64 issue, against
+            # the FMA-lane rate of the measured FP64 DGEMM
             form = k.viscosity_form()
             roof["viscosity_form"] = form
             fp64_tf, fp64_kind = fp64_peak_tflops(local)
@@ -444,14 +454,17 @@ def stress_roofline(k, N: int, prec: int, ms_step: float, local: int, nx: int):
                 roof["limiter"] = "fp64 issue (Delta and viscosity in FP64), see fp64_issue"
                 roof["fp64_issue"] = issue
             else:
-                roof["limiter"] = ("memory and FP32 issue: Delta and the viscosity by float pairs checked against "
-                                   "the FP64 form's rounding (bitwise equal); fp64_issue_form2 is the FP64 form")
+                roof["limiter"] = ("memory: Delta and the viscosity in float pairs on the FP32 pipe; "
+                                   "fp64_issue_form2 is the kernel with their FP64 form")
                 roof["fp64_issue_form2"] = issue
     if prec == 0:
         fp64_tf, fp64_kind = fp64_peak_tflops(local)
-        ach = N * flops_per_element_iteration_stress() / (kms * 1e-3) / 1e12
-        roof["fp64"] = {"achieved_tflops": ach, "peak_tflops": fp64_tf, "frac": ach / fp64_tf,
-                        "peak_kind": fp64_kind}
+        if "Pairs" not in kname:
+            rate = N * FP64_STRESS_INSTRUCTIONS / (kms * 1e-3) / 1e12
+            roof["limiter"] = "fp64 issue and the integer work of the fixed-point maps"
+            roof["fp64"] = {"instructions_per_element": FP64_STRESS_INSTRUCTIONS, "achieved_T_lane_inst_per_s": rate,
+                            "peak_T_fma_lanes_per_s": fp64_tf / 2, "frac": rate / (fp64_tf / 2),
+                            "peak_kind": fp64_kind}
     return roof, {"name": nname, "ms": nms}
 
 
@@ -482,9 +495,8 @@ def fp64_pairs_variant(args, box, N: int, local: int) -> dict:
 def distorted_variant(args, local: int) -> dict:
     """Mixed precision on a 512 x 512 box whose vertices are displaced
     (sinusoidally, 3 % of the box: the elements are general quadrilaterals,
-    not parallelograms), so the element kernel streams the per-element FP32
-    operators (TMA tiles or global loads, whichever the library times as
-    faster on this mesh) instead of the parallelogram coefficients."""
+    not parallelograms), so the element kernel reads the map's derivatives at
+    every Gauss point instead of four coefficients per element."""
     from nextsimdg_gb300.boxtest import BoxTest
     box = BoxTest(args.nx, distort=0.03)
     N = box.nelements
@@ -701,7 +713,7 @@ def spherical_variant(args, N: int, local: int):
         steps = max(3, args.steps // 2)
         ms = k.time_updates(DT, steps) / steps
         kms, kname = k.time_kernel(0, 30)
-        bpe = bytes_per_element_iteration_stress(4 if prec else 8, spherical=True)
+        bpe = launched_stress_bytes("global", 4 if prec else 8, spherical=True)
         out[name] = {"value": N / (ms * 1e-3), "unit": UNIT, "ms_per_step": ms, "stress_kernel": kname,
                      "stress_kernel_ms": kms, "stress_GBps": N * bpe / (kms * 1e-3) / 1e9,
                      "algorithmic_bytes_per_element": bpe}
@@ -974,7 +986,8 @@ def run_ours(args, world, rank, local):
             "config": {"workload": f"box test {args.nx}x{args.nx}, DG2 transport, CG2 velocity, mEVP {NSTEPS} "
                                    f"iterations, alpha=beta={ALPHA:g}, dt={DT:g} s",
                        "precision": args.precision,
-                       "method": ("FP32 bulk (FP64: conservation sums, inverse mass matrices, Delta, viscosity); "
+                       "method": ("FP32 bulk (FP64: conservation sums, inverse mass matrices, node constants; Delta and the "
+                                  "viscosity in float pairs); "
                                   "the learned warm start is measured in variants.learned_fp32 (1024 x 1024), not enabled here"
                                   if prec else "FP64 throughout (the reference's arithmetic)"),
                        "parallelism": "replicas" if world > 1 else "single",

@@ -228,19 +228,19 @@ int nsdg_kernel_time_updates(nsdg_kernel* k, double dt, int steps, float* ms);
  * TMA.  *name gets its name. */
 int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean_ms,
     const char** name);
-/* Which mixed-precision mEVP stress kernel the updates use: *kind 0 =
- * operators by global loads, 1 = operator tiles by TMA, 2 = parallelogram
- * coefficients (chosen by timing at initialise; NSDG_STRESS_KERNEL =
- * global|tma|affine fixes it); for a mixed-precision BBM handle 2 = the
- * parallelogram BBM stress kernel, 0 = per-element operators
+/* Which mixed-precision mEVP stress kernel the updates use: *kind 0 = the
+ * map's derivatives at every Gauss point, 1 = operator tiles by TMA, 2 =
+ * parallelogram coefficients (2 on parallelogram meshes, else 0;
+ * NSDG_STRESS_KERNEL = global|tma|affine fixes it); for a mixed-precision BBM
+ * handle 2 = parallelogram coefficients, 0 = the map at every Gauss point
  * (NSDG_BBM_STRESS_KERNEL=general); *mismatch = the largest relative
  * difference, in FP64, between the exact operators and those rebuilt from
  * parallelogram coefficients (-1 when not evaluated, e.g. spherical or FP64
  * handles). */
 int nsdg_kernel_stress_variant(nsdg_kernel* k, int* kind, double* mismatch);
 /* Which transport stage the updates use: *tiled 1 = the parallelogram-mesh
- * kernel (mixed-precision mEVP on a Cartesian parallelogram mesh without
- * periodic edges: tiles of 32 x 8 elements, each interior edge flux evaluated
+ * kernel (mixed precision on a Cartesian parallelogram mesh without periodic
+ * edges; with BBM for thickness, concentration and damage: tiles of 32 x 8 elements, each interior edge flux evaluated
  * once into shared memory, the cell term from the Jacobian coefficients,
  * diagonal M^{-1}), 0 = the per-element kernel (NSDG_TRANSPORT_KERNEL=element
  * before initialise fixes it); *cell_mismatch = the largest relative
@@ -258,7 +258,7 @@ int nsdg_kernel_transport_variant(nsdg_kernel* k, int* tiled, double* cell_misma
 int nsdg_kernel_host_direct(nsdg_kernel* k, int* direct);
 /* The evaluation of P/(8 alpha Delta) in the parallelogram stress kernel:
  * 0 CUDA's rsqrt(double), 1 and 2 one FP64 Newton step from an FP32 seed
- * (2, the default: conversions on the integer pipe), 3 the same step in
+ * (2: conversions on the integer pipe), 3, the default, the same step in
  * float pairs, 4 form 3 checked against form 2's rounding, with form 2 where
  * the check fails: bitwise form 2.  NSDG_VISC_FORM=0..4 in the environment
  * before initialise selects one.  No reference counterpart. */
@@ -276,11 +276,11 @@ int nsdg_kernel_launches_per_update(nsdg_kernel* k, int* launches);
  * runs one model (one kernel) per process.  Members must be initialised
  * Cartesian mEVP kernels in NSDG_PRECISION_MIXED with the same parameters; they keep
  * their own setData / getDG0Data, which are ordered after the ensemble's
- * update.  The element tile shape of every grid size is chosen at creation by
- * timing the candidates on the GPU; then the whole element phase is timed with
- * those tiles and with the TMA-staged kernel (32 consecutive elements per
- * block, 32 x 1) and the faster is kept (nsdg_ensemble_tile reports the
- * choice; NSDG_STRESS_KERNEL=tma|global in the environment fixes it). */
+ * update.  The element kernel is chosen as for a single handle, over the
+ * members' elements together: parallelogram coefficients when every member is
+ * a parallelogram mesh, else the map at every Gauss point
+ * (nsdg_ensemble_tile reports a block's consecutive elements;
+ * NSDG_STRESS_KERNEL=tma|global|affine in the environment fixes it). */
 typedef struct nsdg_ensemble nsdg_ensemble;
 int nsdg_ensemble_create(nsdg_kernel* const* members, int n_members, nsdg_ensemble** out);
 int nsdg_ensemble_destroy(nsdg_ensemble* ens);

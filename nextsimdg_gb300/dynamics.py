@@ -381,8 +381,8 @@ class _KernelBase:
 
     def viscosity_form(self) -> int:
         """The parallelogram stress kernel's evaluation of P/(8 alpha Delta)
-        (nsdg_kernel_viscosity_form: 2, the default, the FP64 Newton step;
-        4 float pairs checked against it, bitwise equal)."""
+        (nsdg_kernel_viscosity_form: 3, the default, the Newton step in float
+        pairs; 2 in FP64; 4 float pairs checked against it, bitwise equal)."""
         f = c_int()
         self._check(self._l.nsdg_kernel_viscosity_form(self._h, byref(f)))
         return f.value
