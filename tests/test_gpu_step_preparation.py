@@ -58,3 +58,17 @@ def test_module_step_converts_as_set_data(gpu, dg, precision):
     out = k.module_step(0.0, 120.0, f, list(ref))
     for name, r in ref.items():
         np.testing.assert_array_equal(np.asarray(out[name]).ravel(), np.asarray(r).ravel())
+
+
+@pytest.mark.parametrize("bbm", [False, True])
+def test_second_initialise_takes_the_new_mesh(gpu, bbm):
+    """Parallelograms (tiled transport), then general quadrilaterals on the same
+    handle: bitwise a fresh handle's step."""
+    new = lambda: (BBMDynamicsKernel if bbm else MEVPDynamicsKernel)(dg_comp=3, n_steps=40, precision=1)  # noqa: E731
+    k = new()
+    _step(k, "sheared", 9, 6, bbm)
+    assert k.transport_variant()[0] == "tiled"
+    again, ref = _step(k, "quads", 9, 6, bbm), _step(new(), "quads", 9, 6, bbm)
+    assert k.transport_variant()[0] == "element"
+    for name, r in ref.items():
+        np.testing.assert_array_equal(again[name], r)
