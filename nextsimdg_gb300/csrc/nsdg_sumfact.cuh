@@ -20,8 +20,7 @@
 // 1 / (R cos lat) and 1 / R, and the metric terms of the strain and of the
 // divergence are point multiplications by m = tan(lat) / R.
 //
-// The 1-D maps are written for a type T: FP32 here and in the BBM kernels, FP64
-// in the latter; the FP64 mEVP kernel runs them in fixed point
+// The FP32 kernels use the 1-D maps below; the FP64 ones run them in fixed point
 // (nsdg_stress_fixed.cuh).
 //
 // Half strains are used throughout: a = e11 / 2, b = e22 / 2, s = e12.
@@ -104,29 +103,6 @@ template <typename T> __device__ __forceinline__ void derivT(const T (&t)[3], T 
     o[1] = mulT(T(-2), k);
     o[2] = k + s;
 }
-// interp and interpT times a factor r, with r g, 0.3 r and 0.4 r given
-template <typename T> struct Scaled {
-    T r, g, c3, c4;
-    __device__ __forceinline__ explicit Scaled(T f) : r(f), g(Line<T>::g * f), c3(Line<T>::c3 * f), c4(Line<T>::c4 * f) { }
-    __device__ __forceinline__ void interp(const T (&n)[3], T (&o)[3]) const
-    {
-        const T d = n[2] - n[0];
-        const T e = fmaT(T(-2), n[1], n[2] + n[0]);
-        o[1] = mulT(r, n[1]);
-        const T m = fmaT(c3, e, o[1]);
-        o[0] = fmaT(-g, d, m);
-        o[2] = fmaT(g, d, m);
-    }
-    __device__ __forceinline__ void interpT(const T (&t)[3], T (&o)[3]) const
-    {
-        const T s = t[0] + t[2], d = t[2] - t[0];
-        const T m = mulT(c3, s);
-        o[0] = fmaT(-g, d, m);
-        o[1] = fmaT(c4, s, mulT(r, t[1]));
-        o[2] = fmaT(g, d, m);
-    }
-};
-
 // The transposed eta maps of one column of nodes: x[r] (to the transposed
 // interpolation) and y[r] (to the transposed derivative) from the Gauss rows
 // r = 0, 1, 2; o[r] is the node in row r.
