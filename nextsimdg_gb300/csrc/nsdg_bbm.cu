@@ -780,7 +780,7 @@ cudaError_t stressFor(cudaStream_t s, const DevMesh& m, const BbmElements<float>
     float* contrib, const BbmScalars<float>& k, int* err)
 {
     constexpr int E = kBbmElems;
-    auto kernel = el.geo.n ? kBbmStress32<QUAD, DG, E> : kBbmStress32<AFFINE, DG, E>;
+    auto kernel = el.parallelogram ? kBbmStress32<AFFINE, DG, E> : kBbmStress32<QUAD, DG, E>;
     return launch(s, kernel, (m.N + E - 1) / E, 3 * E, m, el.geo, el.wdam, el.w, u, v, el.pt, contrib, k, err);
 }
 template <int DG>

@@ -87,16 +87,11 @@ int deviceCheck(std::string& msg)
 // ===========================================================================
 // Dynamics kernel handle
 // ===========================================================================
-struct nsdg_kernel {
-    int rheology = NSDG_RHEOLOGY_MEVP;
-    int dg = 6;
-    nsdg_params P {};
-    std::string err;
-    bool ready = false;
-    cudaStream_t stream = nullptr;
-    Arena arena;
-    HostMesh mesh;
-    BoundaryFlags flags;
+// What initialise sets for a mesh: device arrays (in the arena, or uploaded to
+// it), the kernels chosen for the mesh and what follows from its sizes.  A
+// second initialise starts from a fresh one, so nothing of the old mesh, whose
+// arena is released, decides a kernel or is read.
+struct MeshState {
     DevMesh dm;
     DevOps dops;
     size_t N = 0, Ncg = 0, Ncg1 = 0;
@@ -138,7 +133,6 @@ struct nsdg_kernel {
     BbmNodeConst<double> bbmNode64 {};
     BbmNodeConst<float> bbmNode32 {};
     float* contrib32 = nullptr;
-    bool bbmAffine = false; // the mixed path's parallelogram form
     float *cellX8_32 = nullptr, *cellY8_32 = nullptr; // FP32 DG8 stress-transport operators
     // which FP32 stress kernel the updates use: 0 the element map's
     // derivatives at the Gauss points from global memory, 1 operator tiles by
@@ -168,6 +162,26 @@ struct nsdg_kernel {
     double* minvDiag = nullptr;      // [dg][N]
     bool trAffine = false;
     double trAffWorst[2] = { -1, -1 }; // cell-operator mismatch, relative off-diagonal of M^{-1}
+    float* tdiv32 = nullptr;
+    MevpNodeState32 st32 {};
+    // FP32 u, v and divergence at the start of the previous sub-cycle (the
+    // warm-start features), refreshed by every mixed-precision mEVP update
+    float *uLast = nullptr, *vLast = nullptr, *tdivLast = nullptr;
+    double *partials = nullptr, *dsum = nullptr;
+    int* derr = nullptr;
+    double* stage2 = nullptr;
+};
+
+struct nsdg_kernel : MeshState {
+    int rheology = NSDG_RHEOLOGY_MEVP;
+    int dg = 6;
+    nsdg_params P {};
+    std::string err;
+    bool ready = false;
+    cudaStream_t stream = nullptr;
+    Arena arena;
+    HostMesh mesh;
+    BoundaryFlags flags;
     cudaError_t launchTransport(cudaStream_t s, int mode, double dt, const StageFields& f, bool forceElement = false)
     {
         if (trAffine && !forceElement)
@@ -186,14 +200,7 @@ struct nsdg_kernel {
                          : launchMevpStress32(s, dm, quad32, st32.u, st32.v, Pw32, tdiv32, mp);
     }
     int chooseStress32();
-    float* tdiv32 = nullptr;
-    MevpNodeState32 st32 {};
-    // FP32 u, v and divergence at the start of the previous sub-cycle (the
-    // warm-start features), refreshed by every mixed-precision mEVP update
-    float *uLast = nullptr, *vLast = nullptr, *tdivLast = nullptr;
     bool mixed() const { return P.precision == NSDG_PRECISION_MIXED; }
-    double *partials = nullptr, *dsum = nullptr;
-    int* derr = nullptr;
     // pinned host copy of derr (a pageable target would make the read a
     // staged, synchronous copy) and the event set_data waits on
     int* hErr = nullptr;
@@ -203,7 +210,6 @@ struct nsdg_kernel {
     // converted[i]: the last conversion that read staging buffer i
     cudaStream_t copyStream = nullptr;
     cudaEvent_t converted[2] = { nullptr, nullptr };
-    double* stage2 = nullptr;
     int stageSlot = 0;
     // nsdg_kernel_module_step's staging for all of a step's inputs at once
     double* moduleStage = nullptr;
@@ -388,15 +394,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     bucketComps.clear();
     stepNumber = 0;
     readCache = 0;
-    geo = {};
-    fixedGeo = {};
-    quad32 = {};
-    aff32 = {};
-    Pw = nullptr;
-    Pw32 = nullptr;
-    affCoef = nullptr;
-    minvDiag = nullptr;
-    trAffine = false;
+    static_cast<MeshState&>(*this) = MeshState();
 
     // --- host mesh (DynamicsKernel.hpp:44-75) ---
     mesh = HostMesh();
@@ -750,19 +748,18 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
             // parallelogram meshes: 4 coefficients per element
             // (NSDG_BBM_STRESS_KERNEL=general keeps the map at every point)
             const char* bk = std::getenv("NSDG_BBM_STRESS_KERNEL");
-            bbmAffine = false;
             if (!(bk && std::strcmp(bk, "general") == 0)) {
                 AffineStressOps aff;
                 AffineBbmOps abb;
-                bbmAffine = buildAffineStressOps(mesh, ops, ops32Ld(N), 1e-9, aff)
+                bbm32.parallelogram = buildAffineStressOps(mesh, ops, ops32Ld(N), 1e-9, aff)
                     && buildAffineBbmOps(mesh, ops, 1e-9, abb);
                 affWorst = std::max(aff.worst, abb.worst);
-                if (bbmAffine) {
+                if (bbm32.parallelogram) {
                     takeAffine(aff);
                     tiledTransport();
                 }
             }
-            if (bbmAffine) {
+            if (bbm32.parallelogram) {
                 std::vector<double> centre(4 * N);
                 for (size_t c = 0; c < 4; ++c)
                     std::copy_n(metric.k.begin() + (9 * c + 4) * N, N, centre.begin() + c * N);
@@ -2249,7 +2246,7 @@ int nsdg_kernel_stress_variant(nsdg_kernel* k, int* kind, double* mismatch)
     if (k->mixed() && k->rheology == NSDG_RHEOLOGY_MEVP)
         *kind = k->stressKind;
     else if (k->mixed())
-        *kind = k->bbmAffine ? 2 : 0; // BBM: parallelogram coefficients or the map at every point
+        *kind = k->bbm32.parallelogram ? 2 : 0; // BBM: parallelogram coefficients or the map at every point
     else
         *kind = -1;
     *mismatch = k->affWorst;

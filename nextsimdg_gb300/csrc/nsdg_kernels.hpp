@@ -487,6 +487,7 @@ template <typename T> struct BbmElements {
     const T* wdam = nullptr; // [DG][9][N] damage projection (general quadrilaterals)
     const T* w = nullptr;    // StressMetric::w there; 2 J (times k_x on rectangles) per element else
     BbmPoints<T> pt {};
+    bool parallelogram = false; // FP32: geo.k and w are per element
 };
 // Step constants of the nodes and the velocity of the sub-cycle.
 template <typename T> struct BbmNodeConst {
