@@ -1062,9 +1062,17 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
     return NSDG_OK;
 }
 
+// Opens with an empty launch: the first stress kernel reads the divergence
+// before it waits for the launch just before it (nsdg_pdl.cuh), and what comes
+// before these iterations may write it (the network's increments, a restore).
 int nsdg_kernel::mixedIterations(cudaStream_t s, double dt, int count, int* errWord, int& launches)
 {
+    if (count < 1)
+        return NSDG_OK;
     const MevpParams mp = mevpParams(dt);
+    if (const cudaError_t e = launchJoin(s); e != cudaSuccess)
+        return fail(NSDG_ERR_CUDA, std::string("mEVP iterations: ") + cudaGetErrorString(e));
+    ++launches;
     for (int it = 0; it < count; ++it) {
         cudaError_t e = launchStress32(s, mp, errWord);
         if (e == cudaSuccess)
