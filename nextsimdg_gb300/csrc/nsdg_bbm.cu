@@ -760,37 +760,24 @@ __global__ void __launch_bounds__(128) kBbmMomentum(DevMesh m, BbmNodeConst<T> c
     c.v[i] = vn;
 }
 
-template <typename... KArgs, typename... Args>
-cudaError_t launch(cudaStream_t s, void (*kernel)(KArgs...), size_t blocks, int threads, Args... args)
-{
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
-    cfg.blockDim = dim3(threads);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <int DG>
 cudaError_t stressFor(cudaStream_t s, const DevMesh& m, const BbmElements<float>& el, const float* u, const float* v,
-    float* contrib, const BbmScalars<float>& k, int* err)
+    float* contrib, const BbmScalars<float>& k, int* err, bool programmatic)
 {
     constexpr int E = kBbmElems;
     auto kernel = el.parallelogram ? kBbmStress32<AFFINE, DG, E> : kBbmStress32<QUAD, DG, E>;
-    return launch(s, kernel, (m.N + E - 1) / E, 3 * E, m, el.geo, el.wdam, el.w, u, v, el.pt, contrib, k, err);
+    return launchAfter(programmatic, s, kernel, (m.N + E - 1) / E, 3 * E, 0, m, el.geo, el.wdam, el.w, u, v, el.pt,
+        contrib, k, err);
 }
 template <int DG>
 cudaError_t stressFor(cudaStream_t s, const DevMesh& m, const BbmElements<double>& el, const double* u,
-    const double* v, double* contrib, const BbmScalars<double>& k, int* err)
+    const double* v, double* contrib, const BbmScalars<double>& k, int* err,
+    bool programmatic)
 {
     constexpr int E = kBbmElems;
     auto kernel = el.fixed.rect ? kBbmStress64<RECT, DG, E> : kBbmStress64<QUAD, DG, E>;
-    return launch(s, kernel, (m.N + E - 1) / E, 3 * E, m, el.fixed, el.geo.n, el.wdam, el.w, u, v, el.pt, contrib, k,
-        err);
+    return launchAfter(programmatic, s, kernel, (m.N + E - 1) / E, 3 * E, 0, m, el.fixed, el.geo.n, el.wdam, el.w, u,
+        v, el.pt, contrib, k, err);
 }
 
 } // namespace
@@ -841,25 +828,26 @@ cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const NodeInput
 
 template <typename T>
 cudaError_t launchBbmStress(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, const T* u,
-    const T* v, T* contrib, const BbmParams& p, int* err)
+    const T* v, T* contrib, const BbmParams& p, int* err, bool programmatic)
 {
     const BbmScalars<T> k { static_cast<T>(p.dt), static_cast<T>(p.nu0), static_cast<T>(0.5 * (1. - p.nu0)),
         static_cast<T>(p.tan_phi), static_cast<T>(p.exponent_relaxation_sigma - 1.), p.powRmode, p.powRk };
     switch (dg) {
-    case 1: return stressFor<1>(s, m, el, u, v, contrib, k, err);
-    case 3: return stressFor<3>(s, m, el, u, v, contrib, k, err);
-    case 6: return stressFor<6>(s, m, el, u, v, contrib, k, err);
+    case 1: return stressFor<1>(s, m, el, u, v, contrib, k, err, programmatic);
+    case 3: return stressFor<3>(s, m, el, u, v, contrib, k, err, programmatic);
+    case 6: return stressFor<6>(s, m, el, u, v, contrib, k, err, programmatic);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename T>
 cudaError_t launchBbmMomentum(cudaStream_t s, const DevMesh& m, const BbmNodeState& st, const BbmNodeConst<T>& c,
-    const T* contrib, const BbmParams& p, int* err)
+    const T* contrib, const BbmParams& p, int* err, bool programmatic)
 {
     const BbmNodeScalars<T> k { static_cast<T>(p.cosA), static_cast<T>(p.sinA), static_cast<T>(p.dt * p.fc),
         p.invNSteps };
-    return launch(s, kBbmMomentum<T>, (m.Ncg + 127) / 128, 128, m, c, st.avgU, st.avgV, contrib, k, err);
+    return launchAfter(programmatic, s, kBbmMomentum<T>, (m.Ncg + 127) / 128, 128, 0, m, c, st.avgU, st.avgV, contrib,
+        k, err);
 }
 
 #define NSDG_BBM_INSTANCES(T)                                                                                       \
@@ -871,9 +859,9 @@ cudaError_t launchBbmMomentum(cudaStream_t s, const DevMesh& m, const BbmNodeSta
     template cudaError_t launchBbmPrepNodes<T>(cudaStream_t, const DevMesh&, const NodeInputs&,                     \
         const BbmNodeState&, const BbmNodeConst<T>&, const BbmParams&);                                             \
     template cudaError_t launchBbmStress<T>(cudaStream_t, const DevMesh&, int, const BbmElements<T>&, const T*,     \
-        const T*, T*, const BbmParams&, int*);                                                                      \
+        const T*, T*, const BbmParams&, int*, bool);                                                                \
     template cudaError_t launchBbmMomentum<T>(cudaStream_t, const DevMesh&, const BbmNodeState&,                    \
-        const BbmNodeConst<T>&, const T*, const BbmParams&, int*);
+        const BbmNodeConst<T>&, const T*, const BbmParams&, int*, bool);
 NSDG_BBM_INSTANCES(double)
 NSDG_BBM_INSTANCES(float)
 

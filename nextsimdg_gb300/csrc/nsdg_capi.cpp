@@ -191,13 +191,15 @@ struct nsdg_kernel : MeshState {
             t32 ? cellX32 : nullptr, t32 ? cellY32 : nullptr);
     }
     cudaError_t launchStress32(cudaStream_t s, const MevpParams& mp, int* errWord, int variant = -1,
-        int vm = -1)
+        int vm = -1, bool programmatic = true)
     {
         const int kind = variant < 0 ? stressKind : variant;
         if (kind == 2 && affCoef)
-            return launchMevpStress32Affine(s, dm, aff32, st32.u, st32.v, Pw32, tdiv32, mp, vm < 0 ? viscMode : vm);
-        return kind == 1 ? launchMevpStress32Tma(s, dm, maps32, st32.u, st32.v, Pg, hP32, tdiv32, mp, errWord)
-                         : launchMevpStress32(s, dm, quad32, st32.u, st32.v, Pw32, tdiv32, mp);
+            return launchMevpStress32Affine(s, dm, aff32, st32.u, st32.v, Pw32, tdiv32, mp, vm < 0 ? viscMode : vm,
+                programmatic);
+        return kind == 1 ? launchMevpStress32Tma(s, dm, maps32, st32.u, st32.v, Pg, hP32, tdiv32, mp, errWord,
+                   programmatic)
+                         : launchMevpStress32(s, dm, quad32, st32.u, st32.v, Pw32, tdiv32, mp, programmatic);
     }
     int chooseStress32();
     bool mixed() const { return P.precision == NSDG_PRECISION_MIXED; }
@@ -2156,25 +2158,28 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
         a.k1[i] = k->k1 + i * dN;
         a.dst[i] = k->phiA + i * dN;
     }
+    // ordinary launches: each one here follows another of the same kernel, whose
+    // output it reads (nsdg_pdl.cuh)
+    constexpr bool programmatic = false;
     auto launch = [&]() -> cudaError_t {
         switch (kernel_id) {
         case 0:
             if (!bbm && k->mixed())
-                return k->launchStress32(k->stream, mp, k->derr);
+                return k->launchStress32(k->stream, mp, k->derr, -1, -1, programmatic);
             if (bbm)
                 return k->mixed() ? launchBbmStress(k->stream, k->dm, k->dg, k->bbm32, k->bbmNode32.u, k->bbmNode32.v,
-                                       k->contrib32, bp, k->derr)
+                                       k->contrib32, bp, k->derr, programmatic)
                                    : launchBbmStress(k->stream, k->dm, k->dg, k->bbm64, k->u, k->v, k->contrib, bp,
-                                       k->derr);
+                                       k->derr, programmatic);
             if (k->opsPairs && k->fp64Stress == 2)
                 return launchMevpStressPairsTma(k->stream, k->dm, k->pairsMaps, k->u, k->v, k->Pg, k->contrib, mp,
                     k->derr);
             if (k->opsPairs && k->fp64Stress == 1)
                 return launchMevpStressPairs(k->stream, k->dm, k->opsPairs, k->pairsLdN, k->u, k->v, k->Pg,
                     k->contrib, mp);
-            return launchMevpStress(k->stream, k->dm, k->fixedGeo, k->u, k->v, k->Pw, k->contrib, mp);
+            return launchMevpStress(k->stream, k->dm, k->fixedGeo, k->u, k->v, k->Pw, k->contrib, mp, programmatic);
         case 9:
-            return launchMevpStress(k->stream, k->dm, k->fixedGeo, k->u, k->v, k->Pw, k->contrib, mp);
+            return launchMevpStress(k->stream, k->dm, k->fixedGeo, k->u, k->v, k->Pw, k->contrib, mp, programmatic);
         case 10:
             return launchMevpStressPairs(k->stream, k->dm, k->opsPairs, k->pairsLdN, k->u, k->v, k->Pg, k->contrib,
                 mp);
@@ -2183,21 +2188,21 @@ int nsdg_kernel_time_kernel(nsdg_kernel* k, int kernel_id, int reps, float* mean
                 k->derr);
         case 1:
             if (!bbm && k->mixed())
-                return launchMevpMomentum32(k->stream, k->dm, k->st32, k->tdiv32, mp, k->derr);
+                return launchMevpMomentum32(k->stream, k->dm, k->st32, k->tdiv32, mp, k->derr, programmatic);
             if (bbm && k->mixed())
-                return launchBbmMomentum(k->stream, k->dm, bs, k->bbmNode32, k->contrib32, bp, k->derr);
-            return bbm ? launchBbmMomentum(k->stream, k->dm, bs, k->bbmNode64, k->contrib, bp, k->derr)
-                       : launchMevpMomentum(k->stream, k->dm, st, k->contrib, mp, false, k->derr);
+                return launchBbmMomentum(k->stream, k->dm, bs, k->bbmNode32, k->contrib32, bp, k->derr, programmatic);
+            return bbm ? launchBbmMomentum(k->stream, k->dm, bs, k->bbmNode64, k->contrib, bp, k->derr, programmatic)
+                       : launchMevpMomentum(k->stream, k->dm, st, k->contrib, mp, false, k->derr, programmatic);
         case 3:
         case 4:
-            return k->launchStress32(k->stream, mp, k->derr, kernel_id == 4 ? 1 : 0);
+            return k->launchStress32(k->stream, mp, k->derr, kernel_id == 4 ? 1 : 0, -1, programmatic);
         case 5:
         case 6:
         case 7:
         case 8:
-            return k->launchStress32(k->stream, mp, k->derr, 2, kernel_id - 5);
+            return k->launchStress32(k->stream, mp, k->derr, 2, kernel_id - 5, programmatic);
         case 12:
-            return k->launchStress32(k->stream, mp, k->derr, 2, 4);
+            return k->launchStress32(k->stream, mp, k->derr, 2, 4, programmatic);
         default: // 2: the step's transport stage; 13: the per-element transport kernel
             return k->launchTransport(k->stream, STAGE_RK2_A, dt, a, kernel_id == 13);
         }

@@ -1903,19 +1903,10 @@ cudaError_t launchDG2CG(cudaStream_t s, const DevMesh& m, int dg, const double* 
 }
 
 cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* contrib,
-    const MevpParams& pIn, bool release, int* err)
+    const MevpParams& pIn, bool release, int* err, bool programmatic)
 {
     const MevpParams p = withDerived(pIn);
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(blocksFor(m.Ncg));
-    cfg.blockDim = dim3(kBlock);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kMevpMomentum, m, st, contrib, p, release, err);
+    return launchAfter(programmatic, s, kMevpMomentum, blocksFor(m.Ncg), kBlock, 0, m, st, contrib, p, release, err);
 }
 
 namespace {
@@ -2026,22 +2017,16 @@ cudaError_t makeStressMaps(const DevOps32& o, StressMaps* out)
 }
 
 cudaError_t launchMevpStress32Tma(cudaStream_t s, const DevMesh& m, const StressMaps& maps, const float* u,
-    const float* v, const double* Pg, const float* hP, float* tdiv, const MevpParams& pIn, int* err)
+    const float* v, const double* Pg, const float* hP, float* tdiv, const MevpParams& pIn, int* err,
+    bool programmatic)
 {
     const MevpParams p = withDerived(pIn);
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(blocksFor(m.N, kTmaElems));
-    cfg.blockDim = dim3(kTmaElems * kStressParts);
-    cfg.dynamicSmemBytes = m.spherical ? tmaSmem<true>() : tmaSmem<false>();
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    const size_t blocks = blocksFor(m.N, kTmaElems), shared = m.spherical ? tmaSmem<true>() : tmaSmem<false>();
     if (m.spherical)
-        return cudaLaunchKernelEx(&cfg, kMevpStress32Tma<true>, maps.g, maps.a, m, u, v, Pg, hP, tdiv, p, err);
-    return cudaLaunchKernelEx(&cfg, kMevpStress32Tma<false>, maps.g, maps.a, m, u, v, Pg, hP, tdiv, p, err);
+        return launchAfter(programmatic, s, kMevpStress32Tma<true>, blocks, kTmaElems * kStressParts, shared, maps.g,
+            maps.a, m, u, v, Pg, hP, tdiv, p, err);
+    return launchAfter(programmatic, s, kMevpStress32Tma<false>, blocks, kTmaElems * kStressParts, shared, maps.g,
+        maps.a, m, u, v, Pg, hP, tdiv, p, err);
 }
 
 cudaError_t launchViscositySelfTest(cudaStream_t s, size_t n, const float* inv, const double* Pa, double dmin,
@@ -2066,50 +2051,24 @@ cudaError_t launchViscositySelfTestChecked(cudaStream_t s, size_t n, const float
 }
 
 cudaError_t launchMevpMomentum32(cudaStream_t s, const DevMesh& m, const MevpNodeState32& st,
-    const float* tdiv, const MevpParams& pIn, int* err)
+    const float* tdiv, const MevpParams& pIn, int* err, bool programmatic)
 {
     const MevpParams p = withDerived(pIn);
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(blocksFor(cellsAndBorder(m.nx, m.ny)));
-    cfg.blockDim = dim3(kBlock);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kMevpMomentum32, m, st, tdiv, p, err);
+    return launchAfter(programmatic, s, kMevpMomentum32, blocksFor(cellsAndBorder(m.nx, m.ny)), kBlock, 0, m, st,
+        tdiv, p, err);
 }
 cudaError_t launchMevpMomentum32Batched(cudaStream_t s, const EnsembleMember* members, const uint16_t* blockMember,
     int blocks, const MevpParams& pIn, int* err)
 {
     const MevpParams p = withDerived(pIn);
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(kBlock);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kMevpMomentum32Batched, members, blockMember, p, err);
+    return launchAfter(true, s, kMevpMomentum32Batched, blocks, kBlock, 0, members, blockMember, p, err);
 }
 cudaError_t launchMevpStress32TmaBatched(cudaStream_t s, const EnsembleMember* members, const uint16_t* blockMember,
     int blocks, const MevpParams& pIn, int* err)
 {
     const MevpParams p = withDerived(pIn);
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(kTmaElems * kStressParts);
-    cfg.dynamicSmemBytes = kTmaSmem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kMevpStress32TmaBatched, members, blockMember, p, err);
+    return launchAfter(true, s, kMevpStress32TmaBatched, blocks, kTmaElems * kStressParts, kTmaSmem, members,
+        blockMember, p, err);
 }
 int persistentCellsPerBlock() { return kAffElems * kStressParts; }
 

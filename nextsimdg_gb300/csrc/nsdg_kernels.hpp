@@ -239,7 +239,7 @@ inline bool releaseEarly64(size_t N, const FixedGeometry& geo)
 }
 // Pw holds w P/(4 alpha) at the Gauss points.
 cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const FixedGeometry& geo, const double* u,
-    const double* v, const double* Pw, double* tdiv, const MevpParams& p);
+    const double* v, const double* Pw, double* tdiv, const MevpParams& p, bool programmatic = true);
 // The benchmark forcing on the cell centres (nsdg_forcing.cu):
 // BenchmarkAtmosphere.cpp:29-77 and BenchmarkOcean.cpp:15-39.
 struct BenchmarkWindArgs {
@@ -275,7 +275,7 @@ cudaError_t launchPairsSelfTest(cudaStream_t s, size_t n, const double* a, const
 // Node gather of the divergence, Dirichlet zero, implicit velocity update and
 // boundary zero (CGDynamicsKernel.cpp:365-444, VPCGDynamicsKernel.hpp:132-172).
 cudaError_t launchMevpMomentum(cudaStream_t s, const DevMesh& m, const MevpNodeState& st, const double* contrib,
-    const MevpParams& p, bool release, int* err);
+    const MevpParams& p, bool release, int* err, bool programmatic = true);
 
 // --- mEVP, mixed precision (NSDG_PRECISION_MIXED) ----------------------
 // FP32 operators, velocities, divergence coefficients and momentum
@@ -319,7 +319,8 @@ cudaError_t encodeTiledNd(CUtensorMap* map, CUtensorMapDataType type, const void
 cudaError_t launchBoundedWaitSelfTest(cudaStream_t s, double limitSeconds, int* timedOut);
 // kMevpStress32 with the operator tiles staged in shared memory by TMA.
 cudaError_t launchMevpStress32Tma(cudaStream_t s, const DevMesh& m, const StressMaps& maps, const float* u,
-    const float* v, const double* Pg, const float* hP, float* tdiv, const MevpParams& p, int* err);
+    const float* v, const double* Pg, const float* hP, float* tdiv, const MevpParams& p, int* err,
+    bool programmatic = true);
 // The mixed-precision node state.  The momentum update is divided through by
 // c1 = rho H / dt, so that per node it needs only
 //   u_new = (beta u + ku + a F_ocean |u_o - u| u_o - fc dt u + im dSx)
@@ -355,9 +356,10 @@ constexpr int kAffElems = 32;  // elements per block
 constexpr int kQuadElems = 64;
 constexpr size_t kOneThreadElems = 16384; // from here one thread per element (the reason stands at the kernels)
 cudaError_t launchMevpStress32Affine(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo,
-    const float* u, const float* v, const float2* Pw, float* tdiv, const MevpParams& p, int viscosityMode);
+    const float* u, const float* v, const float2* Pw, float* tdiv, const MevpParams& p, int viscosityMode,
+    bool programmatic = true);
 cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo, const float* u,
-    const float* v, const float2* Pw, float* tdiv, const MevpParams& p);
+    const float* v, const float2* Pw, float* tdiv, const MevpParams& p, bool programmatic = true);
 // out[k n + i] = P/(8 alpha Delta) of (inv[i], Pa[i]) by viscosity mode k = 0, 1, 2.
 cudaError_t launchViscositySelfTest(cudaStream_t s, size_t n, const float* inv, const double* Pa, double dmin,
     float* out);
@@ -368,7 +370,7 @@ cudaError_t launchViscositySelfTestFF(cudaStream_t s, size_t n, const float* inv
 cudaError_t launchViscositySelfTestChecked(cudaStream_t s, size_t n, const float* inv, const double* Pa,
     double dmin, float* out);
 cudaError_t launchMevpMomentum32(cudaStream_t s, const DevMesh& m,
-    const MevpNodeState32& st, const float* tdiv, const MevpParams& p, int* err);
+    const MevpNodeState32& st, const float* tdiv, const MevpParams& p, int* err, bool programmatic = true);
 // One member of a batched ensemble (device-resident table entry).
 struct EnsembleMember {
     int nx, ny;
@@ -509,10 +511,10 @@ cudaError_t launchBbmPrepNodes(cudaStream_t s, const DevMesh& m, const NodeInput
 // contrib: [18][N], zero on land
 template <typename T>
 cudaError_t launchBbmStress(cudaStream_t s, const DevMesh& m, int dg, const BbmElements<T>& el, const T* u,
-    const T* v, T* contrib, const BbmParams& p, int* err);
+    const T* v, T* contrib, const BbmParams& p, int* err, bool programmatic = true);
 template <typename T>
 cudaError_t launchBbmMomentum(cudaStream_t s, const DevMesh& m, const BbmNodeState& st, const BbmNodeConst<T>& c,
-    const T* contrib, const BbmParams& p, int* err);
+    const T* contrib, const BbmParams& p, int* err, bool programmatic = true);
 
 // --- layout conversion, reductions ---------------------------------------
 // host ModelArray layout (AoS, nin comps) -> device SoA with `dg` comps,

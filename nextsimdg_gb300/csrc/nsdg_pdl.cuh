@@ -20,10 +20,32 @@
 //     of an L1 may be older);
 //   after it: as ordinary global loads (not through the read-only path, which
 //     takes memory that does not change while a kernel lives).
+//
+// A launch that follows another one of the same kernel (nsdg_kernel_time_kernel)
+// has no such order: it is an ordinary one (programmatic = false).
 #pragma once
+
+#include <cuda_runtime.h>
 
 namespace nsdg {
 namespace {
+
+template <typename... KArgs, typename... Args>
+cudaError_t launchAfter(bool programmatic, cudaStream_t s, void (*kernel)(KArgs...), size_t blocks, int threads,
+    size_t shared, Args... args)
+{
+    cudaLaunchConfig_t cfg {};
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = shared;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = programmatic ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 
 __device__ __forceinline__ void waitForPrevious(bool release = true)
 {

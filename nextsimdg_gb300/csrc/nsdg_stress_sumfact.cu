@@ -95,47 +95,34 @@ __global__ void __launch_bounds__(kQuadElems) kMevpStress32ThreadBatched(const E
 
 size_t blocksOf(size_t n) { return (n + kQuadElems - 1) / kQuadElems; }
 
-template <typename... KArgs, typename... Args>
-cudaError_t launch(cudaStream_t s, void (*kernel)(KArgs...), size_t blocks, int threads, Args... args)
-{
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
-    cfg.blockDim = dim3(threads);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 } // namespace
 
 cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const FixedGeometry& geo, const double* u,
-    const double* v, const double* Pw, double* tdiv, const MevpParams& pIn)
+    const double* v, const double* Pw, double* tdiv, const MevpParams& pIn, bool programmatic)
 {
     const MevpParams p = withDerived(pIn);
     const size_t blocks = (m.N + kElems - 1) / kElems;
     auto kernel = geo.rect ? kMevpStress<RECT> : geo.m ? kMevpStress<SPHERE> : kMevpStress<QUAD>;
-    return launch(s, kernel, blocks, 3 * kElems, m, geo, u, v, Pw, tdiv, p.DeltaMin * p.DeltaMin, p.keepd,
-        releaseEarly64(m.N, geo));
+    return launchAfter(programmatic, s, kernel, blocks, 3 * kElems, 0, m, geo, u, v, Pw, tdiv, p.DeltaMin *
+        p.DeltaMin, p.keepd, releaseEarly64(m.N, geo));
 }
 
 cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo, const float* u,
-    const float* v, const float2* Pw, float* tdiv, const MevpParams& pIn)
+    const float* v, const float2* Pw, float* tdiv, const MevpParams& pIn, bool programmatic)
 {
     const MevpParams p = withDerived(pIn);
     const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
     if (m.N >= kOneThreadElems)
-        return launch(s, geo.m ? kMevpStress32Thread<SPHERE> : kMevpStress32Thread<QUAD>, blocksOf(m.N), kQuadElems, m,
-            geo, u, v, Pw, tdiv, rh, p.keep);
+        return launchAfter(programmatic, s, geo.m ? kMevpStress32Thread<SPHERE> : kMevpStress32Thread<QUAD>,
+            blocksOf(m.N), kQuadElems, 0, m, geo, u, v, Pw, tdiv, rh, p.keep);
     auto kernel = geo.m ? kMevpStress32<SPHERE, 3, kQuadElems> : kMevpStress32<QUAD, 3, kQuadElems>;
-    return launch(s, kernel, (m.N + kQuadElems - 1) / kQuadElems, 3 * kQuadElems, m, geo, u, v, Pw, tdiv, rh, p.keep);
+    return launchAfter(programmatic, s, kernel, (m.N + kQuadElems - 1) / kQuadElems, 3 * kQuadElems, 0, m, geo, u, v,
+        Pw, tdiv, rh, p.keep);
 }
 
 cudaError_t launchMevpStress32Affine(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo,
-    const float* u, const float* v, const float2* Pw, float* tdiv, const MevpParams& pIn, int viscosityMode)
+    const float* u, const float* v, const float2* Pw, float* tdiv, const MevpParams& pIn, int viscosityMode,
+    bool programmatic)
 {
     const MevpParams p = withDerived(pIn);
     const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
@@ -146,8 +133,10 @@ cudaError_t launchMevpStress32Affine(cudaStream_t s, const DevMesh& m, const Str
               kMevpStress32<AFFINE, 4, kAffElems> };
     const int vm = viscosityMode >= 0 && viscosityMode <= 4 ? viscosityMode : 3;
     if (vm == 3 && m.N >= kOneThreadElems)
-        return launch(s, kMevpStress32Thread<AFFINE>, blocksOf(m.N), kQuadElems, m, geo, u, v, Pw, tdiv, rh, p.keep);
-    return launch(s, kernels[vm], (m.N + kAffElems - 1) / kAffElems, 3 * kAffElems, m, geo, u, v, Pw, tdiv, rh, p.keep);
+        return launchAfter(programmatic, s, kMevpStress32Thread<AFFINE>, blocksOf(m.N), kQuadElems, 0, m, geo, u, v,
+            Pw, tdiv, rh, p.keep);
+    return launchAfter(programmatic, s, kernels[vm], (m.N + kAffElems - 1) / kAffElems, 3 * kAffElems, 0, m, geo, u,
+        v, Pw, tdiv, rh, p.keep);
 }
 
 cudaError_t launchMevpStress32Batched(cudaStream_t s, const EnsembleMember* members, const uint16_t* blockMember,
@@ -156,9 +145,10 @@ cudaError_t launchMevpStress32Batched(cudaStream_t s, const EnsembleMember* memb
     const MevpParams p = withDerived(pIn);
     const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
     if (elements >= kOneThreadElems)
-        return launch(s, kMevpStress32ThreadBatched<QUAD>, blocks, kQuadElems, members, blockMember, rh, p.keep);
-    return launch(s, kMevpStress32Batched<QUAD, 3, kQuadElems>, blocks, 3 * kQuadElems, members, blockMember, rh,
-        p.keep);
+        return launchAfter(true, s, kMevpStress32ThreadBatched<QUAD>, blocks, kQuadElems, 0, members, blockMember, rh,
+            p.keep);
+    return launchAfter(true, s, kMevpStress32Batched<QUAD, 3, kQuadElems>, blocks, 3 * kQuadElems, 0, members,
+        blockMember, rh, p.keep);
 }
 
 cudaError_t launchMevpStress32AffineThreadBatched(cudaStream_t s, const EnsembleMember* members,
@@ -166,7 +156,8 @@ cudaError_t launchMevpStress32AffineThreadBatched(cudaStream_t s, const Ensemble
 {
     const MevpParams p = withDerived(pIn);
     const Rheology<float> rh { p.dmin2f, p.dmin2lo, p.DeltaMin };
-    return launch(s, kMevpStress32ThreadBatched<AFFINE>, blocks, kQuadElems, members, blockMember, rh, p.keep);
+    return launchAfter(true, s, kMevpStress32ThreadBatched<AFFINE>, blocks, kQuadElems, 0, members, blockMember, rh,
+        p.keep);
 }
 
 cudaError_t launchMevpStress32AffineBatched(cudaStream_t s, const EnsembleMember* members,
@@ -179,7 +170,7 @@ cudaError_t launchMevpStress32AffineBatched(cudaStream_t s, const EnsembleMember
               kMevpStress32Batched<AFFINE, 2, kAffElems>, kMevpStress32Batched<AFFINE, 3, kAffElems>,
               kMevpStress32Batched<AFFINE, 4, kAffElems> };
     const int vm = viscosityMode >= 0 && viscosityMode <= 4 ? viscosityMode : 3;
-    return launch(s, kernels[vm], blocks, 3 * kAffElems, members, blockMember, rh, p.keep);
+    return launchAfter(true, s, kernels[vm], blocks, 3 * kAffElems, 0, members, blockMember, rh, p.keep);
 }
 
 } // namespace nsdg
