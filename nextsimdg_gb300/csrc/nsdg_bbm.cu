@@ -537,6 +537,7 @@ template <Geometry GEO, int E> struct BbmFixedShared {
     fx::i64 strain[3][3][E];
     double sum[3][9][E];
     int top[2][3][E];
+    int scale[GEO == RECT ? 1 : 3][3][E];
 };
 template <Geometry GEO, int DG, int E>
 __global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry geo, const double* __restrict__ proj,
@@ -549,8 +550,7 @@ __global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry g
     const int le = threadIdx.x % E, R = threadIdx.x / E;
     const size_t N = m.N, e = blockIdx.x * size_t(E) + le;
     const bool in = e < N, ice = in && m.ice[e];
-    double c[3][6], g[3][3], d[3], w[3], nq[3], rho = 1.0;
-    [[maybe_unused]] int ke = 0;
+    double c[3][6], g[3][3], d[3], w[3], nq[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const size_t q = 3 * R + i;
@@ -568,12 +568,6 @@ __global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry g
             w[i] = in ? wj[q * N + e] : 0.0;
             nq[i] = in ? proj[q * N + e] : 0.0;
         }
-    }
-    if (in) {
-        if constexpr (GEO == RECT)
-            rho = geo.rect[e];
-        else
-            ke = geo.exponent[e];
     }
     waitForPrevious(false);
     double n[2][3] = { { 0.0, 0.0, 0.0 }, { 0.0, 0.0, 0.0 } };
@@ -598,17 +592,14 @@ __global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry g
     __syncthreads();
     const int top = topOfRows<E>(sh.top[0], le);
     const bool bad = top > kTopMost; // not finite
-    const fx::Scaled sc(rho);
-    const int bits = strainBits<GEO>(sc);
-    fixedColumn<E>(n, fx::fixedShift(bits, top), R, le, sh.ex);
+    const FixedMap<GEO> map = rowMap<GEO>(geo, R, e, N, in);
+    fixedColumn<E>(n, fx::fixedShift(kVelocityBits, top), R, le, sh.ex);
     __syncthreads();
-    const FixedMap<GEO> map(geo, R, e, N, in);
     i64 F11[3], F12[3], F22[3];
     {
         i64 a[3], b[3], s[3];
-        fixedStrain<GEO, E>(R, le, sc, map, sh.ex, sh.strain, a, b, s);
-        const int scale = bits - top + 1022;
-        const int at = fx::doubleExponent(GEO == RECT ? scale : scale - ke - 2);
+        const int scale = fixedStrain<GEO, E>(R, le, map, sh.ex, sh.strain, sh.scale[0], a, b, s);
+        const int at = fx::doubleExponent(kVelocityBits - top + 1022 - scale);
         const double none = __longlong_as_double(0x7ff8000000000000ll);
 #pragma unroll
         for (int i = 0; i < 3; ++i)
@@ -632,24 +623,22 @@ __global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry g
     sh.top[1][R][le] = topOf(word);
     __syncthreads();
     const int topG = topOfRows<E>(sh.top[1], le);
-    const int bitsG = GEO == RECT ? 59 - sc.shift : 59;
-    const int atG = fx::fixedShift(bitsG, topG);
+    const int atG = fx::fixedShift(kStressBits<GEO>, topG);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         F11[i] = fx::toFixed(g[0][i], atG);
         F12[i] = fx::toFixed(g[1][i], atG);
         F22[i] = fx::toFixed(g[2][i], atG);
     }
-    fixedShares<GEO, 0, E>(R, le, sc, map, F11, F12, F22, sh.ex);
+    fixedShares<GEO, E>(R, le, map, F11, F12, F22, sh.ex, sh.scale + (GEO == RECT ? 0 : 1));
     __syncthreads();
     if (!ice)
         return;
-    const int scale = bitsG - topG + 1022;
-    const int at = fx::doubleExponent(GEO == RECT ? scale : scale - ke - 2);
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
         i64 o[3];
-        fixedColumnShares<E>(f, R, le, sh.ex, o);
+        const int scale = fixedColumnShares<GEO, E>(f, R, le, sh.ex, sh.scale + (GEO == RECT ? 0 : 1), o);
+        const int at = fx::doubleExponent(kStressBits<GEO> - topG + 1022 - scale);
 #pragma unroll
         for (int r = 0; r < 3; ++r)
             contrib[(9 * f + 3 * r + R) * N + e]

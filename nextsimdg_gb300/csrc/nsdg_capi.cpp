@@ -475,7 +475,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
     buildStressMetric(mesh, P.precision == NSDG_PRECISION_FP64, metric);
     {
         const size_t sz = P.precision == NSDG_PRECISION_FP64 ? 8 : 4;
-        add(metric.k.size(), sz); add(metric.n.size(), sz); add(metric.m.size(), sz); add(N, 4);
+        add(metric.k.size(), sz); add(metric.n.size(), sz); add(metric.m.size(), sz); add(3 * N, 4);
         if (bbm)
             add(metric.n.size(), sz); // the projection in both forms
         add(4 * N, 4);                            // the same on parallelograms
@@ -596,7 +596,7 @@ int nsdg_kernel::initialise(size_t nx, size_t ny, const double* coords, int sphe
         fixedGeo.k = upi(fixed.k);
         fixedGeo.n = upi(fixed.n);
         fixedGeo.m = upi(fixed.m);
-        fixedGeo.exponent = static_cast<const int*>(up(fixed.exponent.data(), N, 4, e));
+        fixedGeo.exponent = static_cast<const int*>(up(fixed.exponent.data(), fixed.exponent.size(), 4, e));
         if (bbm)
             geo.n = upd(metric.n);
     }

@@ -438,24 +438,30 @@ void transportOps(const HostMesh& m, int dg, ElementOps& ops, unsigned threads)
 
 void buildFixedMetric(const StressMetric& s, size_t N, FixedMetric& out, unsigned threads)
 {
+    const bool sphere = !s.m.empty();
     out.k.resize(s.k.size());
     out.n.resize(s.n.size());
     out.m.resize(s.m.size());
-    out.exponent.assign(N, 0);
+    out.exponent.assign((sphere ? 3 : 2) * N, 0);
     parallelFor(N, threads, [&](size_t lo, size_t hi) {
         for (size_t e = lo; e < hi; ++e) {
-            double most = 0.0;
-            for (size_t i = e; i < s.k.size(); i += N)
-                most = std::max(most, std::fabs(s.k[i]));
+            double most[3] = { 0.0, 0.0, 0.0 };
+            for (size_t i = 0; i < 36; ++i)
+                most[i / 9 % 2] = std::max(most[i / 9 % 2], std::fabs(s.k[i * N + e]));
             for (size_t i = e; i < s.m.size(); i += N)
-                most = std::max(most, std::fabs(s.m[i]));
-            int x;
-            std::frexp(most, &x);
-            out.exponent[e] = x;
-            for (size_t i = e; i < s.k.size(); i += N)
-                out.k[i] = fx::packed(std::llrint(std::ldexp(s.k[i], 62 - x)));
+                most[2] = std::max(most[2], std::fabs(s.m[i]));
+            int x[3];
+            for (int g = 0; g < 3; ++g)
+                std::frexp(most[g], x + g);
+            // a metric term of 0 (the equator) or far below the others takes part
+            // with as many bits as matter
+            x[2] = most[2] > 0.0 ? std::max(x[2], std::min(x[0], x[1]) - 60) : std::min(x[0], x[1]) - 60;
+            for (int g = 0; g < (sphere ? 3 : 2); ++g)
+                out.exponent[g * N + e] = x[g];
+            for (size_t i = 0; i < 36; ++i)
+                out.k[i * N + e] = fx::packed(std::llrint(std::ldexp(s.k[i * N + e], 62 - x[i / 9 % 2])));
             for (size_t i = e; i < s.m.size(); i += N)
-                out.m[i] = fx::packed(std::llrint(std::ldexp(s.m[i], 62 - x)));
+                out.m[i] = fx::packed(std::llrint(std::ldexp(s.m[i], 62 - x[2])));
             for (size_t i = e; i < s.n.size(); i += N)
                 out.n[i] = fx::packed(std::llrint(std::ldexp(s.n[i], 62)));
         }
@@ -471,7 +477,7 @@ void buildStressMetric(const HostMesh& m, bool allowRect, StressMetric& out, uns
     for (size_t j = 0; j <= ny && out.rect; ++j)
         for (size_t i = 0; i <= nx && out.rect; ++i)
             out.rect = m.vx[j * sv + i] == m.vx[i] && m.vy[j * sv + i] == m.vy[j * sv];
-    if (out.rect) { // the rectangles' fixed-point maps take side ratios up to kRectRatio
+    if (out.rect) { // side ratios that the rectangles' fixed-point maps take
         double hx[2] = { m.vx[1] - m.vx[0], m.vx[1] - m.vx[0] }, hy[2] = { m.vy[sv] - m.vy[0], m.vy[sv] - m.vy[0] };
         for (size_t i = 0; i < nx; ++i) {
             hx[0] = std::min(hx[0], m.vx[i + 1] - m.vx[i]);
@@ -481,7 +487,7 @@ void buildStressMetric(const HostMesh& m, bool allowRect, StressMetric& out, uns
             hy[0] = std::min(hy[0], m.vy[(j + 1) * sv] - m.vy[j * sv]);
             hy[1] = std::max(hy[1], m.vy[(j + 1) * sv] - m.vy[j * sv]);
         }
-        out.rect = hx[0] > 0.0 && hy[0] > 0.0 && hx[1] < kRectRatio * hy[0] && hy[1] < kRectRatio * hx[0];
+        out.rect = hx[0] > 0.0 && hy[0] > 0.0 && hx[1] < kRectWide * hy[0] && hy[1] < kRectTall * hx[0];
     }
     out.k.assign((out.rect ? 2 : 36) * N, 0.0);
     out.w.assign(9 * N, 0.0);

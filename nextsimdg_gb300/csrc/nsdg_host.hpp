@@ -126,11 +126,14 @@ void buildElementOps(const HostMesh& m, int dg, bool stressTransport, ElementOps
 //   n = W^{-1} nu / (nu W^{-1} nu),  W = w J [cos lat],  nu = (1,-2,1) x (1,-2,1)
 //   m = tan(lat) / (2 R)                              (spherical meshes)
 //   w = 2 w_q J
-// A mesh whose vertices form a tensor grid with k_y / k_x and k_x / k_y below
-// kRectRatio (rect) has k_x = 1 / (2 dx) and
-// k_y = 1 / (2 dy) at every point and needs no n: it keeps k = (k_y / k_x,
-// 1 / k_x^2) per element, and w = 2 w_q J k_x.
-constexpr double kRectRatio = 32.0;
+// A mesh whose vertices form a tensor grid with every k_y / k_x below kRectWide
+// and k_x / k_y below kRectTall (rect) has k_x = 1 / (2 dx) and k_y = 1 / (2 dy)
+// at every point and needs no n: it keeps k = (k_y / k_x, 1 / k_x^2) per element,
+// and w = 2 w_q J k_x.  The rectangles' maps carry everything over k_x: beyond a
+// k_y / k_x of 2 their unit is too coarse for the xi direction (divergence against
+// the same maps in FP64: error 0.6 at 1, 1.06 at 2, 1.25 at 3.9, 7.5 at 8), down to
+// 1/32 it is not (0.5 to 0.8); wider elements take the general form.
+constexpr double kRectWide = 2.0, kRectTall = 32.0;
 struct StressMetric {
     bool rect = false;
     std::vector<double> k; // [2][N] (rect) or [4][9][N]
@@ -141,11 +144,13 @@ struct StressMetric {
 // With allowRect false the general form is built on every mesh.
 void buildStressMetric(const HostMesh& m, bool allowRect, StressMetric& out, unsigned threads = 0);
 // The general form as integers for the FP64 element kernel
-// (nsdg_stress_fixed.cuh), in the form of fx::packed: per element |k| and |m| below
-// 2^exponent, k and m as multiples of 2^(exponent - 62), n (below 1) of 2^-62.
+// (nsdg_fixed_rows.hpp), in the form of fx::packed: per element and group (k[0] and
+// k[2], the xi derivatives' factors; k[1] and k[3], the eta derivatives'; m) the
+// factors are below 2^exponent and multiples of 2^(exponent - 62), n (below 1) of
+// 2^-62.
 struct FixedMetric {
     std::vector<long long> k, n, m;
-    std::vector<int> exponent;
+    std::vector<int> exponent; // [2][N], [3][N] on a sphere
 };
 void buildFixedMetric(const StressMetric& s, size_t N, FixedMetric& out, unsigned threads = 0);
 // The largest relative difference between an element's operators (gx, gy,

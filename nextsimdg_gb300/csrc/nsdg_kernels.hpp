@@ -221,7 +221,7 @@ template <typename T> struct StressGeometry {
 struct FixedGeometry {
     const double* rect = nullptr;
     const long long *k = nullptr, *n = nullptr, *m = nullptr;
-    const int* exponent = nullptr;
+    const int* exponent = nullptr; // [2][N] ([3][N] on a sphere)
 };
 // Whether the FP64 stress and node kernels let the next launch go at their wait
 // (nsdg_pdl.cuh).  Where the stress kernel has five or more blocks per SM they

@@ -29,6 +29,7 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "nsdg_fixed_rows.hpp"
 #include "nsdg_kernels.hpp"
 #include "nsdg_pdl.cuh"
 #include "nsdg_seed64.cuh"
@@ -116,13 +117,6 @@ template <typename T> __device__ __forceinline__ void columnT(const T (&x)[3], c
     o[1] = fmaT(T(-2), k, fmaT(Line<T>::c4, sx, x[1]));
     o[2] = p + q;
 }
-
-// How an element's map is given: one pair (k_y / k_x, 1 / k_x^2) on
-// rectangles (FP64), four derivatives on parallelograms (FP32), four per Gauss
-// point else.  On rectangles the strain is carried over k_x (strain' = strain /
-// k_x, the eta derivatives times rho = k_y / k_x, DeltaMin^2 over k_x^2) and k_x
-// is part of the pressure's weight, so only rho is multiplied in.
-enum Geometry { RECT = 0, AFFINE = 1, QUAD = 2, SPHERE = 3 };
 
 // What the stress increments take besides the strain: the weighted pressure
 // pq = w P / (4 alpha) (FP32 kernels: as a pair of floats, 48 bits) and
