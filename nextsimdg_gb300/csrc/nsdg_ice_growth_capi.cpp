@@ -30,9 +30,16 @@ int slotOf(const char* name)
     return -1;
 }
 
-// Fields move between pageable host arrays and the device by one kernel over
-// the CPU-GPU link where the GPU can: a field of 512 x 512 cells 28 us in and 71 us
-// out into a fresh array, through the pinned buffer 118 and 147.
+// Large fields move between pageable host arrays and the device by one kernel
+// over the CPU-GPU link where the GPU can.  A move costs about 15 us whatever its
+// size (the array's kind is looked up, a launch, a wait); through the page-locked
+// buffer a field goes in at 8 us and out at 12 plus the copies.  us per field,
+// moved by the kernel / through the buffer:
+//   cells        1,000      4,000      8,000      16,000     24,000     64,000     262,144
+//   setData   15.5 /  8.6 15.4 / 10.0 15.8 / 11.8 16.2 / 14.6 16.6 / 16.5 18.1 / 31.2 27.5 / 117
+//   getData   15.4 / 15.1 15.5 / 15.6 16.2 / 16.8 16.5 / 19.6 17.1 / 22.3 22.3 / 38.0 61.4 / 157
+constexpr size_t kDirectIn = 24000, kDirectOut = 6000;
+
 HostMoves oneMove(const double* src, double* dst, size_t n)
 {
     HostMoves m;
@@ -156,7 +163,7 @@ int nsdg_ice_growth_set_field(nsdg_ice_growth* g, const char* name, const double
     if (n != g->n)
         return g->fail(NSDG_ERR_SIZE_MISMATCH, "set_field: expected one value per element");
     cudaError_t e;
-    if (g->hostDirect && isPageable(data)) {
+    if (n >= kDirectIn && g->hostDirect && isPageable(data)) {
         e = launchHostMove(g->stream, oneMove(data, g->fields + size_t(k) * g->n, n));
         const cudaError_t es = cudaStreamSynchronize(g->stream); // `data` has been read
         if (e == cudaSuccess)
@@ -182,7 +189,7 @@ int nsdg_ice_growth_get_field(nsdg_ice_growth* g, const char* name, double* out,
     if (n != g->n)
         return g->fail(NSDG_ERR_SIZE_MISMATCH, "get_field: expected one value per element");
     const double* src = g->fields + size_t(k) * g->n;
-    const bool direct = g->hostDirect && isPageable(out);
+    const bool direct = n >= kDirectOut && g->hostDirect && isPageable(out);
     cudaError_t e;
     if (direct) {
         populate(out, n);
