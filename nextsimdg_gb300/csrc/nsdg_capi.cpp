@@ -351,7 +351,7 @@ struct nsdg_kernel : MeshState {
     // the copy enqueued on `stream` (a stored field is copied at once)
     int enqueueReadout(const std::string& s, double* out, HostMoves* batch = nullptr);
     bool hostDirect = false; // hostDirectAvailable()
-    bool moveByKernel(const void* p) const { return hostDirect && isPageable(p); }
+    bool moveByKernel(const void* p) const { return hostDirect && movesDirectly(p); }
 };
 
 int nsdg_kernel::checkDeviceError()

@@ -163,7 +163,7 @@ int nsdg_ice_growth_set_field(nsdg_ice_growth* g, const char* name, const double
     if (n != g->n)
         return g->fail(NSDG_ERR_SIZE_MISMATCH, "set_field: expected one value per element");
     cudaError_t e;
-    if (n >= kDirectIn && g->hostDirect && isPageable(data)) {
+    if (n >= kDirectIn && g->hostDirect && movesDirectly(data)) {
         e = launchHostMove(g->stream, oneMove(data, g->fields + size_t(k) * g->n, n));
         const cudaError_t es = cudaStreamSynchronize(g->stream); // `data` has been read
         if (e == cudaSuccess)
@@ -189,7 +189,7 @@ int nsdg_ice_growth_get_field(nsdg_ice_growth* g, const char* name, double* out,
     if (n != g->n)
         return g->fail(NSDG_ERR_SIZE_MISMATCH, "get_field: expected one value per element");
     const double* src = g->fields + size_t(k) * g->n;
-    const bool direct = n >= kDirectOut && g->hostDirect && isPageable(out);
+    const bool direct = n >= kDirectOut && g->hostDirect && movesDirectly(out);
     cudaError_t e;
     if (direct) {
         populate(out, n);

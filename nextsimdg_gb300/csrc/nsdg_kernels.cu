@@ -2158,8 +2158,10 @@ bool hostDirectAvailable()
     cudaGetLastError();
     return direct;
 }
-bool isPageable(const void* p)
+bool movesDirectly(const void* p)
 {
+    if (reinterpret_cast<uintptr_t>(p) % alignof(double) != 0)
+        return false;
     cudaPointerAttributes a {};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();

@@ -535,7 +535,10 @@ cudaError_t launchHostMove(cudaStream_t s, const HostMoves& m);
 // Host arrays that are not page-locked then move by that kernel, which runs at
 // the link's rate, instead of a copy staged through a buffer.
 bool hostDirectAvailable();
-bool isPageable(const void* p);
+// Whether that kernel may move the host array: pageable, and aligned as its
+// accesses are (an array of packed records or a buffer read at an odd offset is
+// copied instead).
+bool movesDirectly(const void* p);
 // device SoA -> AoS with `nout` comps (all, or component 0 only)
 cudaError_t launchSoaToAos(cudaStream_t s, size_t N, int dg, int nout, const double* soa, double* aos);
 // Tools::MeanValue: writes partial sums per block into `partials` and the
