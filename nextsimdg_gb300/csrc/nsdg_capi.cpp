@@ -1623,8 +1623,8 @@ int nsdg_kernel::flushAverages(AverageFields& batch)
 int nsdg_kernel::enqueueConversion(const SetTarget& t, const double* staging, size_t nComp, AverageFields& batch)
 {
     cudaError_t e;
-    if (t.cg && (nComp != size_t(dg) || dg == 1)) {
-        // CGDynamicsKernel.cpp:54-90: ma2dg keeps component 0 only, so DG2CG
+    if (t.cg && nComp == 1) {
+        // CGDynamicsKernel.cpp:54-90: ma2dg sets component 0 only, so DG2CG
         // of the one-component field gives the same node values (the higher
         // components' contributions are exact zeros)
         batch.src[batch.count] = staging;
@@ -1635,7 +1635,8 @@ int nsdg_kernel::enqueueConversion(const SetTarget& t, const double* staging, si
     if (r)
         return r;
     if (t.cg) {
-        // CGDynamicsKernel.cpp:54-90: ma2dg into a DG vector, then DG2CG
+        // CGDynamicsKernel.cpp:54-90: ma2dg into a DG vector (of another number
+        // of components: component 0, the rest zero), then DG2CG
         e = launchAosToSoa(stream, N, static_cast<int>(nComp), dg, staging, dgTmp);
         if (e == cudaSuccess)
             e = launchDG2CG(stream, dm, dg, dgTmp, t.cg);
