@@ -4,6 +4,7 @@
 
 #include "nsdg_kernels.hpp"
 #include "nsdg_pdl.cuh"
+#include "nsdg_visc_ff.hpp"
 
 namespace nsdg {
 namespace {
@@ -73,11 +74,16 @@ __device__ __forceinline__ void gatherDivergence(const DevMesh& m, int i2, int j
         ay -= y[1];
     }
     if (y2) {
-        ax -= x[2];
-        ay -= y[2];
-        if (x2) {
-            ax -= x[3];
-            ay -= y[3];
+        if (sizeof(T) == 4 && x2) { // rounded once, as a sum in FP64 (which made the update 35 % longer)
+            ax = -nsdg_ff::sumOfFour(x[0], x[1], x[2], x[3]);
+            ay = -nsdg_ff::sumOfFour(y[0], y[1], y[2], y[3]);
+        } else {
+            ax -= x[2];
+            ay -= y[2];
+            if (x2) {
+                ax -= x[3];
+                ay -= y[3];
+            }
         }
     }
     dx = ax;

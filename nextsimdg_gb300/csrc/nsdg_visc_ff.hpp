@@ -115,6 +115,24 @@ NSDG_FF_HD float fma(float a, float b, float c)
 #endif
 }
 
+// a + b exactly, as the returned float and the rest (Knuth's TwoSum)
+NSDG_FF_HD float twoSum(float a, float b, float& rest)
+{
+    const float t = add(a, b), v = sub(t, a);
+    rest = add(sub(a, sub(t, v)), sub(b, v));
+    return t;
+}
+// a + b + c + d rounded once, as a sum in FP64 would be: the sums exact as a
+// float and three errors, those as a float and a rest that only decides a tie
+NSDG_FF_HD float sumOfFour(float a, float b, float c, float d)
+{
+    float e1, e2, e3, f1, f2, q;
+    const float s = twoSum(twoSum(twoSum(a, b, e1), c, e2), d, e3);
+    const float g = twoSum(twoSum(e1, e2, f1), e3, f2);
+    const float r = twoSum(s, g, q), f = add(f1, f2);
+    return add(r, f != 0.f && (bitsOf(f) ^ bitsOf(q)) >> 31 == 0 ? mul(q, 1.f + 0x1p-22f) : q);
+}
+
 // positive normal float -> double (exact)
 NSDG_FF_HD double widenPos(float f)
 {
