@@ -933,6 +933,18 @@ void buildElementOps(const HostMesh& m, int dg, bool stressTransport, ElementOps
                             s += imd[k * dg + mm] * (b.psi(mm, 3, q) * (b.weight(3, q) * g.J[q]));
                         ops.wdam[(k * 9 + q) * N + e] = s;
                     }
+                // a constant is its own projection: the rows' sums are made 1 and 0 at
+                // the centre point, past the inverse's rounding, which a sub-cycle
+                // would add up sub-step by sub-step
+                for (int k = 0; k < dg; ++k) {
+                    double sum = k == 0 ? -1.0 : 0.0, rest = 0;
+                    for (int q = 0; q < 9; ++q) {
+                        const double x = ops.wdam[(k * 9 + q) * N + e], t = sum + x, v = t - sum;
+                        rest += (sum - (t - v)) + (x - v);
+                        sum = t;
+                    }
+                    ops.wdam[(k * 9 + 4) * N + e] -= sum + rest;
+                }
                 ops.hsize[e] = std::sqrt(m.area(e));
             }
         }
