@@ -55,6 +55,10 @@ the host cores with all threads, on the same workload.  The reference's own
 build (oracle/_ref) needs the reference sources, which the timing host does
 not have.
 
+The benchmark line on stdout has the contract's keys and one number for each of
+the other measurements (about 2 kB); the whole record, named as above, goes to
+stderr as one JSON line and to --details FILE.
+
 python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 """
 from __future__ import annotations
@@ -110,6 +114,8 @@ def launched_stress_bytes(kind: str, word: int, spherical: bool = False) -> int:
     if kind in ("pairs", "tma"):
         return bytes_per_element_iteration_stress(word, spherical=spherical)
     words = {"fp64": 2, "affine": 4}.get(kind, 54 if spherical else 45)
+    if kind == "global" and word == 8: # the factors' exponents
+        return words * word + (3 if spherical else 2) * 4 + 9 * 8 + 2 * 18 * word + 4 * 2 * word
     return words * word + 9 * 8 + 2 * 18 * word + 4 * 2 * word
 
 
@@ -153,8 +159,9 @@ def launched_bytes_per_cell_update(box, prec: int, stress_kind: str, tiled_trans
     word = 8 if prec == 0 else 4
     stress = launched_stress_bytes(stress_kind, word)
     if prec == 0:
-        # 15 FP64 node streams read, u and v written, the Dirichlet flag
-        node = ncg * (15 * 8 + 2 * 8 + 1) / N
+        # eight FP64 node streams read (four constants of the step, the ice's and
+        # the ocean's velocity), u and v written, the Dirichlet flag
+        node = ncg * (8 * 8 + 2 * 8 + 1) / N
     else:
         # two float4 of per-step constants, u and v read and written (FP32)
         node = ncg * (32 + 4 * 4) / N
@@ -1022,7 +1029,42 @@ def run_ours(args, world, rank, local):
             line["cpu_baseline"] = base
         if variants:
             line["variants"] = variants
-        print(json.dumps(line), flush=True)
+        # the whole record on stderr (and in --details FILE), the benchmark line
+        # alone on stdout
+        print(json.dumps({"details": True, **line}), file=sys.stderr, flush=True)
+        if args.details:
+            Path(args.details).write_text(json.dumps(line) + "\n")
+        print(json.dumps(headline(line)), flush=True)
+
+
+def headline(full: dict) -> dict:
+    """The benchmark line: every key of its contract, the other figures as one
+    number each.  Short enough (about 2 kB) for a log that keeps a run's last
+    lines."""
+    keep = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "gpu_launches", "clocks")
+    line = {k: full[k] for k in keep if k in full}
+    line["config"] = {k: full["config"][k] for k in ("workload", "precision", "parallelism", "bytes_per_cell_update")}
+    line["config"]["l2"] = "inputs larger than L2, no flush"
+    line["e2e"] = {k: full["e2e"][k] for k in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step")}
+    line["e2e_other"] = {k[4:]: full[k]["value"] for k in full if k.startswith("e2e_")}
+    line["roofline"] = {k: full["roofline"].get(k) for k in ("bound", "achieved", "peak", "unit", "frac", "traffic",
+                                                             "kernel", "kernel_ms", "share_of_step")}
+    if "cpu_baseline" in full:
+        line["cpu_baseline"] = {k: full["cpu_baseline"][k] for k in ("value", "unit", "cores", "kind")}
+    if "variants" in full:
+        values = {}
+        for name, v in full["variants"].items():
+            if "value" in v:
+                values[name] = v["value"]
+                continue
+            values.update({f"{name}.{k}": w["value"] for k, w in v.items()
+                           if isinstance(w, dict) and "value" in w and k in ("fp64", "fp32", "plain_fp32")})
+        line["variants"] = values
+    err = full.get("velocity_error_vs_fp64")
+    if err:
+        line["velocity_rms_after_a_day"] = {k: err[k]["u_v_rms_m_per_s"] for k in ("fp32", "fp64_h_times_1p1e-14")}
+    return line
 
 
 def e2e_call_breakdown(k, cycle, start: int, steps: int) -> dict:
@@ -1443,6 +1485,7 @@ def main():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-variants", action="store_true")
+    ap.add_argument("--details", default="", help="file for the whole record (it also goes to stderr)")
     ap.add_argument("--e2e-calls", action="store_true",
                     help="add e2e.calls_us: median microseconds of each call of the module cycle")
     ap.add_argument("--ensemble", type=int, default=0,
