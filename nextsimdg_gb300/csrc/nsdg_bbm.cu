@@ -540,7 +540,7 @@ template <Geometry GEO, int E> struct BbmFixedShared {
     int scale[GEO == RECT ? 1 : 3][3][E];
 };
 template <Geometry GEO, int DG, int E>
-__global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry geo, const double* __restrict__ proj,
+__global__ void __launch_bounds__(3 * E, GEO == QUAD ? 4 : 1) kBbmStress64(DevMesh m, FixedGeometry geo, const double* __restrict__ proj,
     const double* __restrict__ wdam, const double* __restrict__ wj, const double* __restrict__ u,
     const double* __restrict__ v, BbmPoints<double> pt, double* __restrict__ contrib, BbmScalars<double> k,
     int* __restrict__ err)
@@ -565,7 +565,6 @@ __global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry g
             w[i] = in ? kW(i) * wj[e] : 0.0; // the row's weight below
             nq[i] = 0.0;
         } else {
-            w[i] = in ? wj[q * N + e] : 0.0;
             nq[i] = in ? proj[q * N + e] : 0.0;
         }
     }
@@ -592,7 +591,7 @@ __global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry g
     __syncthreads();
     const int top = topOfRows<E>(sh.top[0], le);
     const bool bad = top > kTopMost; // not finite
-    const FixedMap<GEO> map = rowMap<GEO>(geo, R, e, N, in);
+    FixedMap<GEO> map = rowMap<GEO>(geo, R, e, N, in);
     fixedColumn<E>(n, fx::fixedShift(kVelocityBits, top), R, le, sh.ex);
     __syncthreads();
     i64 F11[3], F12[3], F22[3];
@@ -612,6 +611,8 @@ __global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry g
     for (int i = 0; i < 3; ++i) {
         if constexpr (GEO == RECT)
             w[i] *= R == 1 ? kW(1) : kW(0);
+        else
+            w[i] = in ? wj[size_t(3 * R + i) * N + e] : 0.0;
 #pragma unroll
         for (int f = 0; f < 3; ++f) {
             g[f][i] *= w[i];
@@ -630,6 +631,8 @@ __global__ void __launch_bounds__(3 * E) kBbmStress64(DevMesh m, FixedGeometry g
         F12[i] = fx::toFixed(g[1][i], atG);
         F22[i] = fx::toFixed(g[2][i], atG);
     }
+    if constexpr (GEO == QUAD) // read again: kept through the brittle update it would cost registers and a block per SM
+        map = rowMap<GEO>(geo, R, e, N, in);
     fixedShares<GEO, E>(R, le, map, F11, F12, F22, sh.ex, sh.scale + (GEO == RECT ? 0 : 1));
     __syncthreads();
     if (!ice)

@@ -213,6 +213,7 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
             dmin2 *= geo.rect[N + e];
     }
     sh.top[1][R][le] = topOf(max(fx::magnitudeWord(pq[0]), max(fx::magnitudeWord(pq[1]), fx::magnitudeWord(pq[2]))));
+    const FixedMap<GEO> map = rowMap<GEO>(geo, R, e, N, active);
     waitForPrevious(release);
     double n[2][3] = { { 0.0, 0.0, 0.0 }, { 0.0, 0.0, 0.0 } };
     if (active) {
@@ -243,7 +244,6 @@ __device__ __forceinline__ void stressFixed(int nx, size_t N, const uint8_t* __r
     // the increments' products may round up to 2^topP
     const int topP = topOfRows<E>(sh.top[1], le) + 1;
     bool bad = max(top, topP - 1) > kTopMost;
-    const FixedMap<GEO> map = rowMap<GEO>(geo, R, e, N, active);
     fixedColumn<E>(n, fx::fixedShift(kVelocityBits, top), R, le, sh.ex);
     __syncthreads();
     // Gauss row R
