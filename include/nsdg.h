@@ -216,7 +216,8 @@ int nsdg_kernel_mean_value(nsdg_kernel* k, const char* name, double* out);
  * handle's stream with CUDA events; *ms is the total device time. */
 int nsdg_kernel_time_updates(nsdg_kernel* k, double dt, int steps, float* ms);
 /* Times `reps` launches of one kernel of the step in isolation on the handle's
- * stream and returns the mean duration.  kernel_id: 0 = element stress kernel,
+ * stream, each after the one before it, and returns the mean duration (the
+ * launch, 2 to 3.5 us, included).  kernel_id: 0 = element stress kernel,
  * 1 = node momentum kernel, 2 = the transport stage the updates use, 13 = the
  * per-element transport kernel (kTransportStage); for mixed-precision mEVP
  * also 3 = stress kernel with operators by global loads, 4 = with operator

@@ -434,11 +434,11 @@ __device__ __forceinline__ void bbmRow(int R, size_t e, size_t N, bool in, const
 // per element in three warps, as the mEVP kernel (nsdg_sumfact.cuh): node
 // column R, Gauss row R, node column R.
 //
-// In FP32 bound by memory (900 bytes per element): 256 x 256 parallelograms 10.2
-// us per launch (45.2 us with the FP64 state as coefficients, its conversions and
-// 168 registers).  One thread per element, as the mEVP kernel takes on large
-// grids, was slower here: 8.5 against 4.3 us on 128 x 128, 10.4 to 11.1 against
-// 11.5 on 256 x 256.
+// In FP32 bound by memory (900 bytes per element): 256 x 256 parallelograms 12.3
+// us per launch in a row of them, the launch included (45.2 us with the state as
+// FP64 coefficients, its conversions and 168 registers), quadrilaterals 16.4.  One
+// thread per element, as the mEVP kernel takes on large grids, was slower here on
+// 128 x 128 (twice the time) and no faster on 256 x 256.
 template <Geometry GEO, int DG, int E>
 __global__ void __launch_bounds__(3 * E) kBbmStress32(DevMesh m, StressGeometry<float> geo,
     const float* __restrict__ wdam, const float* __restrict__ wj, const float* __restrict__ u,
@@ -530,8 +530,11 @@ __global__ void __launch_bounds__(3 * E) kBbmStress32(DevMesh m, StressGeometry<
 // elsewhere.  The brittle update and the projections of the state stay in FP64.
 // Bound by FP64 issue (about 600 instructions per element, most in the update's
 // divisions and roots; 900 with the maps in FP64, 3000 on coefficients): 96 x 80
-// rectangles 17.4 us per launch (21.8 and 121.8 us); update of 100 sub-steps,
-// 192 x 192 rectangles 10.2 -> 7.2 ms, quadrilaterals 10.8 -> 7.7.
+// rectangles 20.2 us per launch, the launch included (without it 21.8 with the
+// maps in FP64 and 121.8 on coefficients); update of 100 sub-steps, 192 x 192
+// rectangles 7.5 ms, quadrilaterals 8.6 (10.2 and 10.8 with the maps in FP64).  On
+// quadrilaterals four blocks per SM, 168 registers: left alone the compiler takes
+// 254 and two blocks (9.8 ms).
 template <Geometry GEO, int E> struct BbmFixedShared {
     Exchange<fx::i64, E> ex;
     fx::i64 strain[3][3][E];
@@ -540,8 +543,8 @@ template <Geometry GEO, int E> struct BbmFixedShared {
     int scale[GEO == RECT ? 1 : 3][3][E];
 };
 template <Geometry GEO, int DG, int E>
-__global__ void __launch_bounds__(3 * E, GEO == QUAD ? 4 : 1) kBbmStress64(DevMesh m, FixedGeometry geo, const double* __restrict__ proj,
-    const double* __restrict__ wdam, const double* __restrict__ wj, const double* __restrict__ u,
+__global__ void __launch_bounds__(3 * E, GEO == QUAD ? 4 : 1) kBbmStress64(DevMesh m, FixedGeometry geo,
+    const double* __restrict__ proj, const double* __restrict__ wdam, const double* __restrict__ wj, const double* __restrict__ u,
     const double* __restrict__ v, BbmPoints<double> pt, double* __restrict__ contrib, BbmScalars<double> k,
     int* __restrict__ err)
 {
@@ -700,9 +703,10 @@ template <typename T> struct BbmNodeScalars {
 //   u_new = (al (u + Gx) + be (v + Gy)) / (al^2 + be^2),
 //   v_new = (al (v + Gy) + be (Gx - u)) / (al^2 + be^2)
 // as increments, so that roundings of the factors act on the increment.  Per
-// launch: 193 x 161 nodes, FP64, 5.0 us (12.4 us with hypot, a division and the
-// step's terms formed again in every sub-step); 513 x 513 nodes, mixed, 4.7 us
-// (11.4 us on FP64 arrays).
+// launch in a row of them, the launch included: 193 x 161 nodes, FP64, 6.2 us
+// (without it 5.0, and 12.4 with hypot, a division and the step's terms formed again
+// in every sub-step); 513 x 513 nodes, mixed, 7.0 us (without it 4.7, and 11.4 on
+// FP64 arrays).
 template <typename T>
 __global__ void __launch_bounds__(128) kBbmMomentum(DevMesh m, BbmNodeConst<T> c, double* __restrict__ avgU,
     double* __restrict__ avgV, const T* __restrict__ contrib, BbmNodeScalars<T> k, int* __restrict__ err)

@@ -1024,7 +1024,7 @@ int nsdg_kernel::enqueuePhases(cudaStream_t s, double dt, int phases, int& launc
                         LCH(launchMevpStressPairs(s, dm, opsPairs, pairsLdN, u, v, Pg, contrib, mp));
                     else
                         LCH(launchMevpStress(s, dm, fixedGeo, u, v, Pw, contrib, mp));
-                    LCH(launchMevpMomentum(s, dm, st, contrib, mp, fp64Stress == 0 && releaseEarly64(N, fixedGeo), derr));
+                    LCH(launchMevpMomentum(s, dm, st, contrib, mp, fp64Stress == 0 && releaseEarly64(N), derr));
                 } else {
                     LCH(launchStress32(s, mp, derr));
                     LCH(launchMevpMomentum32(s, dm, st32, tdiv32, mp, derr));

@@ -112,11 +112,8 @@ NSDG_FX_HD int strainRow(L load, const FixedMap<GEO>& map, fx::i64 (&a)[3], fx::
         int top = map.xi + fx::lengthOf(x);
         const int topE = map.eta + fx::lengthOf(e);
         top = top > topE ? top : topE;
-        if constexpr (GEO == SPHERE) {
-            int m = 0;
-            for (int i = 0; i < 3; ++i)
-                m |= fx::upperMagnitude(up[i]) | fx::upperMagnitude(vp[i]);
-            const int topM = map.metric + fx::lengthOf(m);
+        if constexpr (GEO == SPHERE) { // values, not differences: up to 1.4 V
+            const int topM = map.metric + kVelocityBits + 1;
             top = top > topM ? top : topM;
         }
         const fx::Shift sx(kRowBits - top + map.xi), se(kRowBits - top + map.eta);
@@ -127,10 +124,11 @@ NSDG_FX_HD int strainRow(L load, const FixedMap<GEO>& map, fx::i64 (&a)[3], fx::
             s[i] = fx::mulHigh(ux, map.k2[i], ue, map.k3[i]) + fx::mulHigh(vx, map.k0[i], ve, map.k1[i]);
         }
         if constexpr (GEO == SPHERE) {
-            const fx::Shift sm(kRowBits - top + map.metric);
+            const int d = top - kRowBits - map.metric; // at least 1
+            const int sm = d > 63 ? 63 : d;
             for (int i = 0; i < 3; ++i) {
-                a[i] -= fx::mulHigh(Split(sm(vp[i])), map.m[i]);
-                s[i] += fx::mulHigh(Split(sm(up[i])), map.m[i]);
+                a[i] -= fx::mulHigh(Split(vp[i] >> sm), map.m[i]);
+                s[i] += fx::mulHigh(Split(up[i] >> sm), map.m[i]);
             }
         }
         return top - kRowBits + 2;
@@ -165,13 +163,10 @@ NSDG_FX_HD int sharesRow(const FixedMap<GEO>& map, const fx::i64 (&F0)[3], const
         int top = map.xi + fx::lengthOf(o0);
         const int topE = map.eta + fx::lengthOf(o1);
         top = top > topE ? top : topE;
-        if constexpr (GEO == SPHERE) {
-            int om = 0;
-            for (int i = 0; i < 3; ++i) {
+        if constexpr (GEO == SPHERE) { // below 2^59.5
+            for (int i = 0; i < 3; ++i)
                 tm[i] = fx::mulHigh(Split(FM[i]), map.m[i]);
-                om |= fx::upperMagnitude(tm[i]);
-            }
-            const int topM = map.metric + fx::lengthOf(om);
+            const int topM = map.metric + 60;
             top = top > topM ? top : topM;
         }
         const fx::Shift sx(kRowBits - top + map.xi), se(kRowBits - top + map.eta);
@@ -182,10 +177,11 @@ NSDG_FX_HD int sharesRow(const FixedMap<GEO>& map, const fx::i64 (&F0)[3], const
         fx::derivT(t0, x);
         fx::interpT(t1, y);
         if constexpr (GEO == SPHERE) {
-            const fx::Shift sm(kRowBits - top + map.metric);
+            const int d = top - kRowBits - map.metric; // at least 2
+            const int sm = d > 63 ? 63 : d;
             i64 z[3];
             for (int i = 0; i < 3; ++i)
-                tm[i] = sm(tm[i]);
+                tm[i] >>= sm;
             fx::interpT(tm, z);
             for (int i = 0; i < 3; ++i)
                 x[i] += z[i];

@@ -126,14 +126,15 @@ void buildElementOps(const HostMesh& m, int dg, bool stressTransport, ElementOps
 //   n = W^{-1} nu / (nu W^{-1} nu),  W = w J [cos lat],  nu = (1,-2,1) x (1,-2,1)
 //   m = tan(lat) / (2 R)                              (spherical meshes)
 //   w = 2 w_q J
-// A mesh whose vertices form a tensor grid with every k_y / k_x below kRectWide
-// and k_x / k_y below kRectTall (rect) has k_x = 1 / (2 dx) and k_y = 1 / (2 dy)
-// at every point and needs no n: it keeps k = (k_y / k_x, 1 / k_x^2) per element,
-// and w = 2 w_q J k_x.  The rectangles' maps carry everything over k_x: beyond a
-// k_y / k_x of 2 their unit is too coarse for the xi direction (divergence against
-// the same maps in FP64: error 0.6 at 1, 1.06 at 2, 1.25 at 3.9, 7.5 at 8), down to
-// 1/32 it is not (0.5 to 0.8); wider elements take the general form.
-constexpr double kRectWide = 2.0, kRectTall = 32.0;
+// A mesh whose vertices form a tensor grid with k_y / k_x below kRectWide and k_x /
+// k_y below kRectTall (rect) has k_x = 1 / (2 dx) and k_y = 1 / (2 dy) at every point
+// and needs no n: it keeps k = (k_y / k_x, 1 / k_x^2) per element, and w = 2 w_q J k_x.
+// The rectangles' maps carry everything over k_x in one unit.  Above a k_y / k_x of 2
+// the strain's bound passes 2^63; below, the unit grows coarse for the eta
+// direction: the divergence of v has 0.6 of the error of the maps in FP64 at 1 and
+// 1/2, 1.2 at 1/4 (9 x 9 operators in FP64: 1.15 to 1.23) and 1.6 at 1/32.  More slender
+// rectangles take the general form.
+constexpr double kRectWide = 2.0, kRectTall = 4.0;
 struct StressMetric {
     bool rect = false;
     std::vector<double> k; // [2][N] (rect) or [4][9][N]

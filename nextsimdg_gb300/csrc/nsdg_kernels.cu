@@ -1236,9 +1236,10 @@ constexpr int kStressParts = 3;
 // rounding of the factors then acts on the increment, where in the quotient
 // it would act on u in each of the iterations with the same sign.  All but the
 // divergence's part is formed before the wait for the stress kernel.  Bound by
-// FP64 issue: about 22 FP64 instructions per node; 513 x 513 nodes 15.3 us
-// (18.1 us with 30 of them after the wait, 26.8 us with CUDA's square root and
-// division), 129 x 129 2.7 us (latency of the dependent chain).
+// FP64 issue: about 22 FP64 instructions per node; 513 x 513 nodes 17.5 us per
+// launch in a row of them, the launch included, 15.3 without it (18.1 us with 30 of
+// them after the wait, 26.8 us with CUDA's square root and division), 129 x 129 5.1
+// us (2.7: latency of the dependent chain).
 __global__ void __launch_bounds__(kBlock) kMevpMomentum(DevMesh m, MevpNodeState st,
     const double* __restrict__ contrib, MevpParams p, bool release, int* __restrict__ err)
 {

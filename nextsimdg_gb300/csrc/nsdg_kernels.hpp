@@ -224,18 +224,18 @@ struct FixedGeometry {
     const int* exponent = nullptr; // [2][N] ([3][N] on a sphere)
 };
 // Whether the FP64 stress and node kernels let the next launch go at their wait
-// (nsdg_pdl.cuh).  Where the stress kernel has five or more blocks per SM they
-// do: 160 x 160 rectangles 1.77 against 1.93 ms per update, quadrilaterals 2.53
-// against 2.63, sphere 2.57 against 2.84 (128 x 128: 1.33 / 1.38, 1.82 / 1.74, 1.76 /
-// 1.83; 154 x 121 sphere 2.06 / 1.90).  And where it has at most one, but on
-// quadrilaterals: 48 x 48 rectangles 0.73 against 0.84, 64 x 64 0.80 against 0.87,
-// sphere 1.06 against 1.17, quadrilaterals 1.18 against 1.12.
+// (nsdg_pdl.cuh): where the stress kernel has five or more blocks per SM, or at most
+// one.  ms per update of DG1 fields, with / without:
+//                   48^2         64^2         96^2         128^2        160^2        256^2
+//   rectangles      0.67 / 0.84  0.79 / 0.87  0.93 / 0.99  1.26 / 1.33  1.91 / 1.83  3.39 / 3.77
+//   quadrilaterals  0.88 / 1.05  1.04 / 1.11  1.41 / 1.27  1.87 / 1.73  2.33 / 2.50  4.68 / 5.09
+//   sphere          0.94 / 1.12  1.10 / 1.17  1.54 / 1.33  1.94 / 1.82  2.43 / 2.75  5.41 / 5.79
 constexpr size_t kSMs = 152;
 constexpr size_t kFixedElems = 32; // elements per block of the FP64 stress kernel
-inline bool releaseEarly64(size_t N, const FixedGeometry& geo)
+inline bool releaseEarly64(size_t N)
 {
     const size_t blocks = (N + kFixedElems - 1) / kFixedElems;
-    return blocks >= 5 * kSMs || (blocks <= kSMs && (geo.rect || geo.m));
+    return blocks >= 5 * kSMs || blocks <= kSMs;
 }
 // Pw holds w P/(4 alpha) at the Gauss points.
 cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const FixedGeometry& geo, const double* u,

@@ -118,8 +118,8 @@ struct CellNodes {
 // in the order of gatherDivergence (even cell rows first, ascending x).  One
 // thread for four nodes: every lane of a warp does the same loads, where one
 // thread per node makes the lanes of a warp wait for each other's cells.  The
-// mixed mEVP node kernel takes this form (1025 x 1025 nodes 9.1 -> 6.9 us per
-// launch, the same results bit for bit); with the FP64 and the BBM kernels'
+// mixed mEVP node kernel takes this form (1025 x 1025 nodes 9.1 -> 6.9 us,
+// 11.2 with the launch, the same results bit for bit); with the FP64 and the BBM kernels'
 // larger node state it is slower (513 x 513 nodes: FP64 18.6 -> 20.5 us, BBM
 // FP64 23.1 -> 27.0, BBM mixed 4.6 -> 5.5), and they keep one thread per node.
 template <typename T>

@@ -12,7 +12,7 @@
 // against 0.79, 192 x 192 1.18 against 1.42.  The FP64 kernels are bound by the
 // SM's FP64 unit: blocks that start while others run land unevenly, and with two
 // to four blocks per SM that costs more than it gives (mEVP 96 x 96
-// quadrilaterals 1.47 against 1.29, BBM 96 x 96 4.3 against 2.9), so they let the
+// quadrilaterals 1.41 against 1.27, BBM 96 x 96 4.3 against 2.9), so they let the
 // next launch go early only where releaseEarly64 says so, the BBM ones never.
 //
 //   before the wait: arrays that the sub-cycle changes are read from L2

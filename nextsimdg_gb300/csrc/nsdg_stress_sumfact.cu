@@ -10,16 +10,15 @@ namespace {
 using namespace sf;
 
 // FP64 (nsdg_stress_fixed.cuh).  Bound by FP64 issue (108 instructions per
-// element) and the integer work beside it.  Timed alone (CUDA events): 19.1 us
-// for 256 x 256 rectangles (60.8 us with the linear maps in FP64, 112 us with
-// 9 x 9 operators streamed from memory), 16.5 us for 201 x 143 quadrilaterals (42
-// and 49 us), 11.5 us for 154 x 121 cells of a sphere (32 and 44 us), 4.6 us for
-// 64 x 64 rectangles (7.4 and 20.5 us).  Three threads per element: with one, a
-// 64 x 64 grid is one warp per SM that waits out every instruction's latency.
-// The blocks per SM bound the registers at 80, 128 and 168: left alone the
-// compiler takes 72, 128 and 130 (sphere 12.4 us); six or more blocks make
-// quadrilaterals and spheres spill (16.9 and 14.6 us), four leave the former a
-// longer tail (update 2.73 against 2.54 ms).
+// element) and the integer work beside it.  Per launch in a row of them, the
+// launch included (about 3 us): 21.4 us for 256 x 256 rectangles, 20.4 us for 201 x
+// 143 quadrilaterals, 14.4 us for 154 x 121 cells of a sphere, 6.7 us for 64 x 64
+// rectangles.  (Without the launch, with the linear maps in FP64 60.8, 42, 32 and
+// 7.4 us, with 9 x 9 operators streamed from memory 112, 49, 44 and 20.5.)  Three
+// threads per element: with one, a 64 x 64 grid is one warp per SM that waits out
+// every instruction's latency.  The blocks per SM bound the registers at 80, 128
+// and 168: with five a sphere's kernel spills (update of 154 x 121 cells 2.08
+// against 1.92 ms), with six quadrilaterals' did (16.9 against 16.5 us per launch).
 constexpr int kElems = kFixedElems;
 
 template <Geometry GEO>
@@ -37,18 +36,20 @@ __global__ void __launch_bounds__(3 * kElems, GEO == RECT ? 8 : GEO == QUAD ? 5 
 // parallelograms (divergence 144, weighted pressure 72, coefficients 16, its
 // share of the velocities) and 430 on quadrilaterals (+ 180 of map, 216 on a
 // sphere), where the 9 x 9 operators were 1,580 (2,228).  Bound by L2 / HBM
-// traffic: 14.0 us for 512 x 512 parallelograms = 4.9 TB/s (24.9 us with dense
-// unit-square operators and the viscosity in FP64, which was bound by FP64
-// issue), 9.6 us for 384 x 320 quadrilaterals (42.7 us with TMA-staged
-// operators), 7.3 us for 301 x 257 cells of a sphere (38.6 us).
+// traffic: per launch in a row of them, the launch included, 12.3 us for 512 x 512
+// parallelograms = 5.6 TB/s (24.9 us with dense unit-square operators and the
+// viscosity in FP64, which was bound by FP64 issue), 10.3 us for 384 x 320
+// quadrilaterals (42.7 us with TMA-staged operators), 9.2 us for 301 x 257 cells of
+// a sphere (38.6 us).
 //
 // Three threads per element keep small grids' latency down; from
 // kOneThreadElems elements the SMs are full either way and one thread per
 // element issues about 950 instructions instead of 1,700 (shared-memory
-// exchange, indices).  Parallelograms: 64 x 64 2.2 against 2.6 us, 128 x 128 2.7
-// against 2.7, 256 x 256 4.6 against 4.1, 512 x 512 13.9 against 10.3;
-// quadrilaterals: 96 x 96 2.9 against 3.4, 192 x 192 4.5 against 4.2, 384 x 384
-// 12.0 against 9.6.
+// exchange, indices).  Updates of 100 iterations, three threads against one, ms:
+//   parallelograms  64^2 .459 / .489   96^2 .484 / .496  128^2 .540 / .519
+//                  192^2 .687 / .658  256^2 .875 / .838  512^2 2.66 / 2.29
+//   quadrilaterals  64^2 .530 / .565   96^2 .571 / .580  128^2 .684 / .621
+//                  192^2 .781 / .795  256^2 1.13 / .973  384^2 2.16 / 1.83
 template <Geometry GEO, int VM, int E>
 __global__ void __launch_bounds__(3 * E) kMevpStress32(DevMesh m, StressGeometry<float> geo,
     const float* __restrict__ u, const float* __restrict__ v, const float2* __restrict__ Pw, float* __restrict__ tdiv,
@@ -104,7 +105,7 @@ cudaError_t launchMevpStress(cudaStream_t s, const DevMesh& m, const FixedGeomet
     const size_t blocks = (m.N + kElems - 1) / kElems;
     auto kernel = geo.rect ? kMevpStress<RECT> : geo.m ? kMevpStress<SPHERE> : kMevpStress<QUAD>;
     return launchAfter(programmatic, s, kernel, blocks, 3 * kElems, 0, m, geo, u, v, Pw, tdiv, p.DeltaMin *
-        p.DeltaMin, p.keepd, releaseEarly64(m.N, geo));
+        p.DeltaMin, p.keepd, releaseEarly64(m.N));
 }
 
 cudaError_t launchMevpStress32(cudaStream_t s, const DevMesh& m, const StressGeometry<float>& geo, const float* u,

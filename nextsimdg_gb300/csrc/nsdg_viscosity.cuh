@@ -53,8 +53,9 @@ __device__ __forceinline__ float narrowPos(double d)
 // pair of floats (nsdg_ff::viscPair: no FP64 instruction).  Against extended
 // precision its RMS error is VM 2's to nine digits (0.2887 ulp, both round an
 // approximation far below the float's last place; they differ in 1e-7 of the
-// cases).  512 x 512 parallelograms: 14.0 us, VM 4 24.8 us, VM 2 36.9 us
-// (FP64 issue, the pair's sum included), VM 0 and 1 54 us.
+// cases).  512 x 512 parallelograms, launch included: 12.3 us (one thread
+// per element), VM 4 26.7 us, VM 2 39.0 us (FP64 issue, the pair's sum included), VM
+// 0 and 1 57.4 us (three threads).
 __device__ __forceinline__ float viscNewton64(float inv, double Pa, double dmin, float y0)
 {
     const double t = fma(dmin, dmin, widenNonneg(inv));
